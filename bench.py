@@ -248,7 +248,7 @@ def run_ours(args):
             dn, ds, done, res = window()
             nodes += dn
             dev_s += ds
-            launches += 1          # the explorer kernel (idle queue persists across launches)
+            launches += 1          # the explorer kernel (explorers persist across launches)
             steps_done += 1
             exchange_ub(res, done)
         torch.cuda.synchronize()

@@ -133,9 +133,9 @@ struct pbb_engine {
     DeviceInstance di;
     signed char *mat = nullptr, *vec = nullptr, *bestperm = nullptr;
     int* path = nullptr;   // per explorer and level: heads, tails, free loads
-    int *line = nullptr, *state = nullptr, *bestcost = nullptr, *qval = nullptr, *ub_d = nullptr, *root_d = nullptr;
+    int *line = nullptr, *state = nullptr, *bestcost = nullptr, *askid = nullptr, *ub_d = nullptr, *root_d = nullptr;
     int* ival_d = nullptr;   // [2][64] interval start / end vectors
-    unsigned* qseq = nullptr;
+    unsigned* ask = nullptr;
     GroupCtl* ctl = nullptr;
     DevGroup* group_d = nullptr;
     int* ngroups_d = nullptr;     // device copy of the group count (1)
@@ -283,7 +283,7 @@ int pbb_engine_destroy(pbb_engine* e)
     if (e->st) cudaStreamSynchronize(e->st);
     e->di.release();
     cudaFree(e->mat); cudaFree(e->vec); cudaFree(e->bestperm); cudaFree(e->path);
-    cudaFree(e->line); cudaFree(e->state); cudaFree(e->bestcost); cudaFree(e->qval); cudaFree(e->qseq);
+    cudaFree(e->line); cudaFree(e->state); cudaFree(e->bestcost); cudaFree(e->askid); cudaFree(e->ask);
     cudaFree(e->ub_d); cudaFree(e->root_d); cudaFree(e->ival_d); cudaFree(e->ctl); cudaFree(e->group_d);
     cudaFree(e->ngroups_d);
     cudaFree(e->sample_d);
@@ -329,8 +329,8 @@ static int engine_create(const pbb_instance* inst, const pbb_config* cfg, pbb_en
     CK(cudaMalloc(&e->line, sizeof(int) * B));
     CK(cudaMalloc(&e->state, sizeof(int) * B));
     CK(cudaMalloc(&e->bestcost, sizeof(int) * B));
-    CK(cudaMalloc(&e->qval, sizeof(int) * B));
-    CK(cudaMalloc(&e->qseq, sizeof(unsigned) * B));
+    CK(cudaMalloc(&e->askid, sizeof(int) * B));
+    CK(cudaMalloc(&e->ask, sizeof(unsigned) * B));
     CK(cudaMalloc(&e->ub_d, sizeof(int)));
     CK(cudaMalloc(&e->root_d, sizeof(int) * PBB_MAX_N));
     CK(cudaMalloc(&e->neh_d, sizeof(int) * (PBB_MAX_N + 1)));
@@ -363,6 +363,7 @@ static int engine_create(const pbb_instance* inst, const pbb_config* cfg, pbb_en
     g.search.sort_crit = cfg->sorting_criterion;
     g.search.core_warps = cfg->core_warps > 0 ? cfg->core_warps : PBB_CORE_WARPS;
     g.search.split_depth = cfg->split_depth > 0 ? cfg->split_depth : PBB_SPLIT_DEPTH;
+    g.search.split_narrow = cfg->split_depth > 0 ? cfg->split_depth : PBB_SPLIT_NARROW;
     g.search.share_after = cfg->share_after > 0 ? cfg->share_after : (cfg->share_after < 0 ? 0 : PBB_SHARE_AFTER);
     g.search.early_stop = cfg->early_stop_johnson ? 1 : 0;
     g.ivm.count = B;
@@ -376,8 +377,8 @@ static int engine_create(const pbb_instance* inst, const pbb_config* cfg, pbb_en
     g.ivm.state = e->state;
     g.ivm.bestcost = e->bestcost;
     g.ivm.bestperm = e->bestperm;
-    g.ivm.qseq = e->qseq;
-    g.ivm.qval = e->qval;
+    g.ivm.ask = e->ask;
+    g.ivm.askid = e->askid;
     g.ivm.path = e->path;
     g.ctl = e->ctl;
     g.first_cta = 0;
@@ -669,7 +670,7 @@ int pbb_diag_get_samples(pbb_engine* e, int32_t max_records, int32_t* out, int32
     return PBB_OK;
 }
 
-int pbb_explore(pbb_engine* e, double seconds, int32_t* done)
+static int explore_window(pbb_engine* e, double seconds, int32_t* done, int eager)
 {
     if (!e || !e->started) return fail(PBB_E_INVAL, "engine not started");
     pbbh::DeviceGuard keep_callers_device;
@@ -687,7 +688,7 @@ int pbb_explore(pbb_engine* e, double seconds, int32_t* done)
         if (variant == 0 && e->cfg.bounding_mode == 2 && e->cfg.branching_mode == 3 && !e->cfg.find_all && masks)
             variant = 3;
         CK(pbbl::launch_explore(e->nw, e->group_d, e->ngroups_d, e->ctas, e->warps, e->smem, budget, e->max_rounds,
-                                e->select_budget, e->st, variant));
+                                e->select_budget, e->st, variant, eager));
         CK(cudaEventRecord(e->ev1, e->st));
         rc = wait_event(e->ev1, e->wait_limit_s < 0 ? win + 60.0 : e->wait_limit_s);
         if (rc == PBB_E_TIMEOUT) {
@@ -705,6 +706,16 @@ int pbb_explore(pbb_engine* e, double seconds, int32_t* done)
     }
     if (done) *done = e->done ? 1 : 0;
     return PBB_OK;
+}
+
+// A window this short serves a caller that looks at the search between
+// windows (exports, exchanges or saves its intervals): it is not cut into more
+// intervals than share_after allows.
+#define PBB_SHORT_WINDOW_S 0.01
+
+int pbb_explore(pbb_engine* e, double seconds, int32_t* done)
+{
+    return explore_window(e, seconds, done, !(seconds > 0 && seconds < PBB_SHORT_WINDOW_S));
 }
 
 int pbb_get_result(pbb_engine* e, pbb_result* out)
@@ -766,7 +777,7 @@ int pbb_solve(pbb_engine* e, int32_t ub, const int32_t* root_perm, double time_l
             if (left <= 0) break;
             slice = std::min(slice, left);
         }
-        rc = pbb_explore(e, slice, &done);
+        rc = explore_window(e, slice, &done, 1);
         if (rc) return rc;
     }
     return pbb_get_result(e, out);

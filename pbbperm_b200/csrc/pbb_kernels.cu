@@ -1,9 +1,9 @@
 // Kernels of the IVM flow-shop engine (sm_100a).
 //
-//   pbb_reset_kernel     explorers empty, idle queue and counters cleared
+//   pbb_reset_kernel     explorers empty, requests for work and counters cleared
 //   pbb_root_kernel      root row bounded (weak, uncounted) + initial unfold
 //   pbb_explore_kernel   persistent explorer loop: select/decode/bound/prune
-//                        and work sharing through a device idle queue
+//                        and work sharing, inside the CTA and between CTAs
 //   pbb_bound_kernel     batched children bounds of given nodes (LB parity API)
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -35,21 +35,21 @@ __device__ __forceinline__ void st_release(int* p, int v)
     asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
-__device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* p)
+// a value other warps of the CTA update in shared memory
+template <class V>
+__device__ __forceinline__ V ld_shared(const V* p)
 {
-    unsigned v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-
-__device__ __forceinline__ void st_release_u32(unsigned* p, unsigned v)
-{
-    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+    return *reinterpret_cast<const volatile V*>(p);
 }
 
 __device__ __forceinline__ unsigned long long ld_volatile_u64(const unsigned long long* p)
 {
     return *reinterpret_cast<const volatile unsigned long long*>(p);
+}
+
+__device__ __forceinline__ unsigned ld_volatile_u32(const unsigned* p)
+{
+    return *reinterpret_cast<const volatile unsigned*>(p);
 }
 
 __device__ __forceinline__ int ld_volatile_s32(const int* p) { return *reinterpret_cast<const volatile int*>(p); }
@@ -413,67 +413,116 @@ __device__ __forceinline__ void bound_current(const DevGroup& G, const CtaTables
 }
 
 // ---------------------------------------------------------------------------
-// idle-explorer queue: bounded MPMC queue with per-cell sequence numbers
-// (D. Vyukov's design), one lane operates it
+// work sharing
 // ---------------------------------------------------------------------------
-__device__ bool queue_push(const DevGroup& G, int v)
+// Waiting warps are found in two places.  Inside a CTA the mask of waiting
+// warps, the explorers they offer and the handed-over ids live in shared
+// memory, so a working warp learns of a waiting one, and a waiting one of its
+// work, without a trip to L2.  Between CTAs one warp per CTA at most asks, by
+// a bit in the group's mask of asking CTAs, so a donor claims a CTA with one
+// atomic and thousands of idle warps never meet on one address.  What bounds a
+// search of up to some 10^6 nodes is how fast work reaches idle warps: a
+// single queue of idle explorers with compare-and-swap cursors took a third of
+// all warp time of an 18x20 search with the one-machine bound and left half of
+// the rest idle.  Measured with it and with this, explorer milliseconds:
+// 12x10 (1.7 k nodes) 2.4 / 0.22, 20x10 (0.12 M) 10 / 1.0, 18x20 one-machine
+// bound (8.8 M) 102 / 13, 30x10 (10 M) 97 / 27, 20x20 (13 M) 94 / 56, 50x20
+// (56 M) 515 / 500.
+
+// What a working warp is asked to do at this step: 0 nothing, 1 give work to
+// a warp of its CTA, 2 to another CTA.  The nodes it must have decomposed
+// since it last split shrink with the square of the waiting share: a split
+// costs about a node on either side, which is nothing while most warps wait,
+// and too much once few do (20x10 and 20x20 milliseconds: 1.0 and 56; with a
+// linear rule 1.5 and 57, and with a limit of 16 nodes whatever waits 1.1 and
+// 59).  With most CTAs asking, an empty SM is served before the warps of a
+// busy one, and splits go deeper.  A launch that is not `eager` (a short
+// window, whose caller may export the intervals) splits at the plain limit
+// only: every split leaves one more interval to export, and every exported
+// interval costs the resuming engine a path to bound again.  Lane 0 decides,
+// so that the warp never disagrees.
+__device__ __forceinline__ int share_wish(const DevSearch& srch, const CtaShare* H, long long since, int warps, int ctas,
+                                          int eager, bool& narrow)
 {
-    const unsigned long long cap = (unsigned long long)G.ivm.count;
-    for (int attempt = 0; attempt < 64; attempt++) {
-        unsigned long long pos = ld_volatile_u64(&G.ctl->q_tail);
-        const int cell = (int)(pos % cap);
-        const unsigned seq = ld_acquire_u32(G.ivm.qseq + cell);
-        const int dif = (int)(seq - (unsigned)pos);
-        if (dif == 0) {
-            if (atomicCAS(&G.ctl->q_tail, pos, pos + 1) == pos) {
-                G.ivm.qval[cell] = v;
-                st_release_u32(G.ivm.qseq + cell, (unsigned)(pos + 1));
-                return true;
-            }
-        } else if (dif < 0) {
-            return false;
-        }
+    int wish = 0;
+    if (lane_id() == 0) {
+        const int h = __popc(ld_shared(&H->hungry)), g = ld_shared(&H->asking);
+        const bool few_ctas = 2 * g > ctas;
+        const long long hh = eager ? h : 0, gg = eager ? PBB_WARPS_MAX * g / ctas : 0;
+        const bool far = g > 0 && since * (4 + gg * gg) >= 4ll * srch.share_after;
+        const bool near = h > 0 && since * (4 + hh * hh) >= 4ll * srch.share_after;
+        if (far && (few_ctas || h == 0)) wish = 2;
+        else if (near) wish = 1;
+        if (wish && (few_ctas || 2 * h > warps)) wish |= 4;
     }
-    return false;
+    wish = __shfl_sync(FULLMASK, wish, 0);
+    narrow = (wish & 4) != 0;
+    return wish & 3;
 }
 
-__device__ int queue_pop(const DevGroup& G)
+// Claim a waiting warp of this CTA; returns the explorer it offers, and the
+// warp in `to`, or -1.  One lane.
+__device__ __forceinline__ int claim_near(CtaShare* H, int wic, int& to)
 {
-    const unsigned long long cap = (unsigned long long)G.ivm.count;
-    for (int attempt = 0; attempt < 64; attempt++) {
-        unsigned long long pos = ld_volatile_u64(&G.ctl->q_head);
-        const int cell = (int)(pos % cap);
-        const unsigned seq = ld_acquire_u32(G.ivm.qseq + cell);
-        const int dif = (int)(seq - (unsigned)(pos + 1));
-        if (dif == 0) {
-            if (atomicCAS(&G.ctl->q_head, pos, pos + 1) == pos) {
-                const int v = __ldcg(G.ivm.qval + cell);
-                st_release_u32(G.ivm.qseq + cell, (unsigned)(pos + cap));
-                return v;
-            }
-        } else if (dif < 0) {
-            return -1;
+    int* offer = reinterpret_cast<int*>(H + 1);
+    for (int attempt = 0; attempt < 4; attempt++) {
+        const unsigned h = ld_shared(&H->hungry);
+        if (h == 0) return -1;
+        const unsigned above = h & ~((2u << wic) - 1u);      // the next waiting warp after this one
+        const unsigned bit = above ? (above & (0u - above)) : (h & (0u - h));
+        if (atomicAnd(&H->hungry, ~bit) & bit) {
+            to = __ffs(bit) - 1;
+            __threadfence_block();
+            return ld_shared(offer + to);
         }
     }
     return -1;
 }
 
-// Split the explorer's interval with a queued idle explorer
+// Claim an asking CTA of the group, searching from the one after this; returns
+// the explorer it offers or -1.  All lanes.
+__device__ __forceinline__ int claim_far(const DevGroup& G, int cta)
+{
+    // a CTA asks only with an explorer of its own: never more CTAs than explorers
+    const int words = (min(G.ctas, G.ivm.count) + 31) >> 5;
+    int id = -1;
+    const int w0 = ((cta + 1) >> 5) % words;
+    for (int q = 0; q < words && id < 0; q++) {
+        const int w = w0 + q < words ? w0 + q : w0 + q - words;
+        if (lane_id() == 0) {
+            unsigned v = ld_volatile_u32(G.ivm.ask + w);
+            for (int attempt = 0; attempt < 4 && v && id < 0; attempt++) {
+                const int from = (cta + 1) & 31;
+                const unsigned above = v & (0xffffffffu << from);
+                const unsigned bit = above ? (above & (0u - above)) : (v & (0u - v));
+                v = atomicAnd(G.ivm.ask + w, ~bit);
+                if (v & bit) {
+                    atomicSub(&G.ctl->asking, 1);
+                    __threadfence();
+                    id = __ldcg(G.ivm.askid + w * 32 + __ffs(bit) - 1);
+                }
+            }
+        }
+        id = __shfl_sync(FULLMASK, id, 0);
+    }
+    return id;
+}
+
+// Split the explorer's interval with a waiting explorer
 // (bbthread::shareWork multicore/src/bbthread.cpp:40-72 and
 // ivm::cuttingPosition multicore/src/ivm.cpp:199-237): the first level l where
-// pos and end differ (not below the current line, not deeper than n-10) is
-// cut so that the donor keeps half of the explorable cells after pos[l]; the
-// receiver gets row l, the path vectors of level l and the right part, and
-// continues with next() without an uncounted unfold, so decomposed-node counts
-// do not depend on how the work was shared.
+// pos and end differ (not below the current line, not deeper than
+// n - split_depth) is cut so that the donor keeps half of the explorable cells
+// after pos[l]; the receiver gets row l, the path vectors of level l and the
+// right part, and continues with next() without an uncounted unfold, so
+// decomposed-node counts do not depend on how the work was shared.  `wish` is
+// share_wish's answer; returns 1 when work was handed over, 2 when the donor
+// only dropped pruned cells from its interval.
 template <int NW>
-__device__ __forceinline__ int try_share(const DevGroup& G, int id, Ivm<NW>& R)
+__device__ __forceinline__ int try_share(const DevGroup& G, CtaShare* H, int wic, int id, Ivm<NW>& R, int wish,
+                                         bool narrow)
 {
     const int n = G.inst.n;
-    // cheap emptiness test of the queue first (one lane reads, all follow)
-    int empty = 0;
-    if (lane_id() == 0) empty = ld_volatile_u64(&G.ctl->q_tail) == ld_volatile_u64(&G.ctl->q_head);
-    if (__shfl_sync(FULLMASK, empty, 0)) return 0;
     int f = n;
 #pragma unroll
     for (int w = NW - 1; w >= 0; w--) {
@@ -481,7 +530,7 @@ __device__ __forceinline__ int try_share(const DevGroup& G, int id, Ivm<NW>& R)
         const unsigned d = __ballot_sync(FULLMASK, lv < n && R.pos[w] != R.end[w]);
         if (d) f = w * 32 + __ffs(d) - 1;
     }
-    const int lcap = max(n - G.search.split_depth, 0);
+    const int lcap = max(n - (narrow ? G.search.split_narrow : G.search.split_depth), 0);
     int l = f;
     if (l > R.line) l = R.line;
     if (l > lcap) l = lcap;
@@ -517,9 +566,13 @@ __device__ __forceinline__ int try_share(const DevGroup& G, int id, Ivm<NW>& R)
         }
         return 2;
     }
-    int thief = -1;
-    if (lane_id() == 0) thief = queue_pop(G);
-    thief = __shfl_sync(FULLMASK, thief, 0);
+    int thief = -1, to = -1;
+    if (wish == 1) {
+        if (lane_id() == 0) thief = claim_near(H, wic, to);
+        thief = __shfl_sync(FULLMASK, thief, 0);
+    } else {
+        thief = claim_far(G, (int)blockIdx.x - G.first_cta);
+    }
     if (thief < 0) return 0;
     const int keep = expl / 2;
     int cut = pl + 1;
@@ -575,9 +628,67 @@ __device__ __forceinline__ int try_share(const DevGroup& G, int id, Ivm<NW>& R)
         atomicAdd(&G.ctl->active, 1);
         atomicAdd(&G.ctl->steals, 1ull);
         st_release(G.ivm.state + thief, IVM_ACTIVE);
+        if (to >= 0) {
+            int* mail = reinterpret_cast<int*>(H + 1) + (blockDim.x >> 5);
+            __threadfence();
+            *reinterpret_cast<volatile int*>(mail + to) = thief;
+        }
     }
     __syncwarp();
     return 1;
+}
+
+// One look of a warp without work (lane 0; the other lanes follow the
+// returned code): offers `spare` to the CTA, then, after waiting `pause` looks
+// or at once when nobody in the CTA works, to the other CTAs.  `wait`: 0
+// nothing offered, 1 to the CTA, 2 to the group.  Returns 1 when `spare` has
+// been filled.
+__device__ __forceinline__ int seek_work(const DevGroup& G, CtaShare* H, int wic, int warps, int spare, int& wait,
+                                         int& looks, bool tier)
+{
+    int* offer = reinterpret_cast<int*>(H + 1);
+    int* mail = offer + warps;
+    const unsigned bit = 1u << wic;
+    const int cta = (int)blockIdx.x - G.first_cta;
+    if (wait == 0) {
+        if (spare < 0 || !tier) return 0;
+        *reinterpret_cast<volatile int*>(mail + wic) = -1;
+        *reinterpret_cast<volatile int*>(offer + wic) = spare;
+        __threadfence_block();
+        atomicOr(&H->hungry, bit);
+        wait = 1;
+        looks = 0;
+        return 0;
+    }
+    if (wait == 1) {
+        if (ld_shared(mail + wic) >= 0) {
+            __threadfence();
+            wait = 0;
+            return 1;
+        }
+        if (++looks >= 8 || ld_shared(&H->working) == 0) {
+            if (ld_shared(&H->asker) == 0 && atomicCAS(&H->asker, 0, wic + 1) == 0) {
+                if (atomicAnd(&H->hungry, ~bit) & bit) {
+                    // withdrawn from the CTA: ask the group
+                    *reinterpret_cast<volatile int*>(G.ivm.askid + cta) = spare;
+                    __threadfence();
+                    atomicOr(G.ivm.ask + (cta >> 5), 1u << (cta & 31));
+                    atomicAdd(&G.ctl->asking, 1);
+                    wait = 2;
+                } else {
+                    // a warp of this CTA is already filling the offer
+                    atomicExch(&H->asker, 0);
+                }
+            }
+        }
+        return 0;
+    }
+    if (ld_acquire(G.ivm.state + spare) == IVM_ACTIVE) {
+        atomicExch(&H->asker, 0);
+        wait = 0;
+        return 1;
+    }
+    return 0;
 }
 
 __device__ __forceinline__ int group_of_cta(const DevGroup* groups, int ngroups)
@@ -607,7 +718,7 @@ __global__ void pbb_reset_kernel(const DevGroup* groups, int ngroups, const int*
             G.ivm.state[id] = IVM_IDLE;
             G.ivm.line[id] = 0;
             G.ivm.bestcost[id] = 0x7fffffff;
-            G.ivm.qseq[id] = (unsigned)id;
+            G.ivm.ask[id >> 5] = 0u;
             const size_t b = (size_t)id * G.ivm.npad;
             for (int e = 0; e < G.ivm.npad; e++) {
                 G.ivm.pos[b + e] = 0;
@@ -622,7 +733,7 @@ __global__ void pbb_reset_kernel(const DevGroup* groups, int ngroups, const int*
             c->best_key = ((unsigned long long)(unsigned)ub[g] << 32) | 0xffffffffull;
             c->active = 0; c->found = 0; c->status = 0;
             c->decomposed = c->johnson_bounds = c->simple_bounds = c->leaves = c->root_simple = 0;
-            c->q_head = c->q_tail = 0; c->steals = 0;
+            c->asking = 0; c->steals = 0;
             c->jsweeps = c->jfree = c->jchild = 0;
             c->jdirect = c->jdirect_free = 0;
         }
@@ -737,7 +848,7 @@ __global__ void pbb_root_kernel(const DevGroup* groups, int ngroups, const int* 
 template <int NW, int VAR>
 __global__ void __launch_bounds__(32 * PBB_WARPS_MAX, 1)
 pbb_explore_kernel(const DevGroup* groups, const int* ngroups_d, int warps_per_cta, unsigned long long budget_ns,
-                   int max_rounds, int select_budget)
+                   int max_rounds, int select_budget, int eager)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     // the group count lives in device memory so that a captured launch
@@ -751,7 +862,8 @@ pbb_explore_kernel(const DevGroup* groups, const int* ngroups_d, int warps_per_c
     // gave the room for them (the host sizes the launch with them if they fit)
     unsigned dyn_smem;
     asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn_smem));
-    const int fm = G.inst.posj != nullptr &&
+    // (the one-machine bound alone has no use for them)
+    const int fm = G.inst.posj != nullptr && G.search.bound_mode != 0 &&
                    pbb_smem_plan(G.inst.n, G.inst.m, G.inst.Ppad, warps_per_cta, 1).total <= (int)dyn_smem;
     if (VAR == 3 && !fm) {
         // the fixed build relies on the masks; the host launches it only
@@ -762,6 +874,17 @@ pbb_explore_kernel(const DevGroup* groups, const int* ngroups_d, int warps_per_c
     const SmemPlan sp = pbb_smem_plan(G.inst.n, G.inst.m, G.inst.Ppad, warps_per_cta, fm);
     CtaTables T;
     load_tables(G.inst, smem, sp, T);
+    CtaShare* H = reinterpret_cast<CtaShare*>(smem + sp.share_off);
+    if (threadIdx.x == 0) {
+        H->hungry = 0u;
+        H->working = 0;
+        H->asker = 0;
+        H->stop = 0;
+        H->active = ld_volatile_s32(&G.ctl->active);
+        H->best = (int)(ld_volatile_u64(&G.ctl->best_key) >> 32);
+        H->asking = 0;
+        H->poll_ns = (unsigned)globaltimer_ns();
+    }
     __syncthreads();
     const int wic = threadIdx.x >> 5;
     const WarpScratch S = warp_scratch(smem + sp.warp_off + wic * sp.warp_bytes, sp, T.n, T.m, T.Ppad);
@@ -774,110 +897,146 @@ pbb_explore_kernel(const DevGroup* groups, const int* ngroups_d, int warps_per_c
     Ivm<NW> R;
     int cached = -1;                   // explorer whose state is held in registers
     int since = 0;                     // nodes it decomposed since it got work or gave some away
+    int scan = wid;                    // this warp's explorers from here on are not looked at yet
+    int spare = -1;                    // an idle explorer of this warp
+    int wait = 0, looks = 0;           // what it is offered to (seek_work), looks since (lane 0)
     // explorers holding work once the first core_warps warps of every CTA
     // are busy (no more than that share of the explorers can be)
     const int core_warps = G.search.core_warps;
     const int core_active = min(core_warps * G.ctas, (int)((long long)G.ivm.count * core_warps / warps_per_cta));
     const bool core_warp = wic < core_warps;   // this warp always asks for work
-    unsigned idle_ns = 500;            // back-off of a warp that found nothing to do
-    int best = 0;
-    if (lane_id() == 0) best = (int)(ld_volatile_u64(&G.ctl->best_key) >> 32);
-    best = __shfl_sync(FULLMASK, best, 0);
+    unsigned idle_ns = 100;            // pause of a warp that found nothing to do
+    int best = ld_shared(&H->best);
 
     for (int round = 0; round < max_rounds; round++) {
-        // loop control is decided by lane 0 and broadcast, so that the warp
-        // never splits on values read at slightly different times
-        int stop = 0, active = 0;
-        if (lane_id() == 0) {
-            active = ld_volatile_s32(&G.ctl->active);
-            stop = active == 0 || globaltimer_ns() - t0 > budget_ns;
-        }
-        if (__shfl_sync(FULLMASK, stop, 0)) break;
-        bool worked = false;
-        bool busy = false;          // an explorer of this warp is active or offered
-        int spare = -1;             // an idle explorer of this warp
         int id = cached;
-        if (id >= 0) {
-            // the explorer held in registers is ACTIVE, and only this warp can
-            // change that: keep stepping it without polling
-            busy = true;
-        } else {
-            for (int base = wid; base < G.ivm.count && id < 0; base += 32 * W) {
-                // the states of up to 32 of this warp's explorers in one load
-                // (lane j: explorer base + jW)
-                const int mine = base + lane_id() * W;
-                const int st_l = mine < G.ivm.count ? ld_volatile_s32(G.ivm.state + mine) : -1;
-                const unsigned act = __ballot_sync(FULLMASK, st_l == IVM_ACTIVE);
-                const unsigned idl = __ballot_sync(FULLMASK, st_l == IVM_IDLE);
-                if (act || __any_sync(FULLMASK, st_l == IVM_QUEUED)) busy = true;
-                if (spare < 0 && idl) spare = base + (__ffs(idl) - 1) * W;
-                if (act) id = base + (__ffs(act) - 1) * W;
+        if (id < 0) {
+            // ---- no work: this warp's own explorers first, each looked at
+            // once per launch (it becomes active later only where this warp
+            // offered it), the states of up to 32 in one load
+            if (scan < G.ivm.count) {
+                const int mine = scan + lane_id() * W;
+                const int st = mine < G.ivm.count ? ld_volatile_s32(G.ivm.state + mine) : -1;
+                const unsigned act = __ballot_sync(FULLMASK, st == IVM_ACTIVE);
+                const unsigned idl = __ballot_sync(FULLMASK, st == IVM_IDLE);
+                const int next = __ffs(act) - 1;
+                if (spare < 0 && idl) spare = scan + (__ffs(idl) - 1) * W;
+                if (act) {
+                    id = scan + next * W;
+                    scan = id + W;
+                    // it held work before this launch: it may split at once
+                    // (unless splits are as good as forbidden)
+                    since = min(G.search.share_after, 4096);
+                } else {
+                    scan += 32 * W;
+                }
+            } else {
+                // loop control is decided by lane 0 and broadcast, so that the
+                // warp never splits on values read at slightly different times
+                int code = 0;
+                if (lane_id() == 0) {
+                    const unsigned long long now = globaltimer_ns();
+                    if (ld_shared(&H->stop) || now - t0 > budget_ns) {
+                        code = 2;
+                    } else {
+                        // one warp of the CTA at a time reads the group's
+                        // counts, about every two microseconds
+                        if ((unsigned)now - ld_shared(&H->poll_ns) > 2000u) {
+                            *reinterpret_cast<volatile unsigned*>(&H->poll_ns) = (unsigned)now;
+                            const int a = ld_volatile_s32(&G.ctl->active);
+                            *reinterpret_cast<volatile int*>(&H->active) = a;
+                            if (a == 0) *reinterpret_cast<volatile int*>(&H->stop) = 1;
+                        }
+                        // The first core_warps warps of every CTA always take
+                        // part; the others join once that many explorers per
+                        // CTA hold work, so a narrow search is not cut into
+                        // pieces for warps that share an SM with busy ones,
+                        // and a wide one still gets every warp.
+                        const bool tier = core_warp || ld_shared(&H->active) >= core_active;
+                        code = seek_work(G, H, wic, warps_per_cta, spare, wait, looks, tier);
+                    }
+                }
+                code = __shfl_sync(FULLMASK, code, 0);
+                if (code == 2) break;
+                if (code == 1) {
+                    id = spare;
+                    spare = -1;
+                    since = 0;
+                }
             }
             if (id >= 0) {
-                int st = 0;
-                if (lane_id() == 0) st = ld_acquire(G.ivm.state + id);   // orders the reads of its image
-                st = __shfl_sync(FULLMASK, st, 0);
-                if (st == IVM_ACTIVE) {
-                    load_ivm<NW>(G.ivm, id, R);
-                    cached = id;
-                    since = 0;
-                    if (S.fmask) fmask_build<NW>(T, S, R.row, T.n - R.line);
-                } else {
-                    id = -1;
+                __syncwarp();
+                load_ivm<NW>(G.ivm, id, R);
+                cached = id;
+                idle_ns = 100;
+                if (S.fmask) fmask_build<NW>(T, S, R.row, T.n - R.line);
+                if (lane_id() == 0) atomicAdd(&H->working, 1);
+            } else {
+                if (scan >= G.ivm.count) {
+                    // waiting warps look at shared memory only, so the pause
+                    // is short; a warp that asked other CTAs looks at L2
+                    __nanosleep(idle_ns);
+                    idle_ns = idle_ns < 800u ? 2 * idle_ns : idle_ns;
                 }
+                continue;
             }
         }
-        if (id >= 0) {
+        // ---- one step of the explorer held in registers: it is ACTIVE, and
+        // only this warp can change that
+        if ((round & 3) == 0) {
+            // the window's clock, the incumbent and the waiting CTAs
+            int stop = 0;
+            if (lane_id() == 0) {
+                stop = globaltimer_ns() - t0 > budget_ns;
+                const int gb = (int)(ld_volatile_u64(&G.ctl->best_key) >> 32);
+                *reinterpret_cast<volatile int*>(&H->asking) = ld_volatile_s32(&G.ctl->asking);
+                atomicMin(&H->best, gb);
+            }
+            if (__shfl_sync(FULLMASK, stop, 0)) break;
+        }
+        {
             int gb = 0;
-            if (lane_id() == 0) gb = (int)(ld_volatile_u64(&G.ctl->best_key) >> 32);
+            if (lane_id() == 0) gb = ld_shared(&H->best);
             gb = __shfl_sync(FULLMASK, gb, 0);
             if (gb < best) best = gb;
-            // an explorer offers work once it has decomposed share_after nodes
-            // since it got its interval or last split it: in a narrow tree,
-            // splitting at every step hands out pieces that end before they
-            // pay for the split, and keeps the donors splitting instead of
-            // exploring
-            if (since >= G.search.share_after && try_share<NW>(G, id, R) == 1) since = 0;
-            const int r = select_node<NW, (VAR == 3)>(G, T, S, id, R, best, C, select_budget);
-            if (r == 1) since++;
-            if (r == 1)
-                bound_current<NW, (VAR == 1 || VAR == 2), (VAR == 2), (VAR == 3 ? 3 : 0)>(G, T, S, id, R, mode, best, C);
-            worked = true;
-            if (C.decomposed >= (1u << 20)) flush_counters(G, C);
-            if (r == 0) {
-                // interval exhausted: leave the pool of busy explorers (the
-                // registers need not go back: nobody resumes this interval)
-                __syncwarp();
-                cached = -1;
-                if (lane_id() == 0) {
-                    st_release(G.ivm.state + id, IVM_IDLE);
-                    atomicSub(&G.ctl->active, 1);
-                }
-                __syncwarp();
+        }
+        bool narrow;
+        const int wish = share_wish(G.search, H, since, warps_per_cta, G.ctas, eager, narrow);
+        if (wish && try_share<NW>(G, H, wic, id, R, wish, narrow) == 1) since = 0;
+        const int known = best;
+        const int r = select_node<NW, (VAR == 3)>(G, T, S, id, R, best, C, select_budget);
+        if (best < known && lane_id() == 0) atomicMin(&H->best, best);
+        if (r == 1) {
+            since++;
+            bound_current<NW, (VAR == 1 || VAR == 2), (VAR == 2), (VAR == 3 ? 3 : 0)>(G, T, S, id, R, mode, best, C);
+        }
+        if (C.decomposed >= (1u << 20)) flush_counters(G, C);
+        if (r == 0) {
+            // interval exhausted: leave the pool of busy explorers (the
+            // registers need not go back: nobody resumes this interval)
+            __syncwarp();
+            cached = -1;
+            if (spare < 0) spare = id;
+            if (lane_id() == 0) {
+                atomicSub(&H->working, 1);
+                st_release(G.ivm.state + id, IVM_IDLE);
+                atomicSub(&G.ctl->active, 1);
             }
-        }
-        // A warp with nothing to do offers ONE of its idle explorers to the
-        // donors: work is only split towards warps that would otherwise wait,
-        // never towards a warp that is busy with another explorer.  The first
-        // core_warps warps of every CTA always take part; the others join
-        // once that many explorers per CTA hold work, so a narrow search is
-        // not cut into pieces for warps it cannot feed, and a wide one still
-        // gets every warp.
-        const bool tier = core_warp || active >= core_active;
-        if (!busy && spare >= 0 && lane_id() == 0 && tier) {
-            st_release(G.ivm.state + spare, IVM_QUEUED);
-            if (!queue_push(G, spare)) st_release(G.ivm.state + spare, IVM_IDLE);
-        }
-        __syncwarp();
-        // idle warps back off (0.5 us doubling to 32 us): their polling
-        // competes with the working warps for issue slots and L2
-        if (!worked) {
-            __nanosleep(idle_ns);
-            idle_ns = idle_ns < 32000u ? 2 * idle_ns : idle_ns;
-        } else {
-            idle_ns = 500;
+            __syncwarp();
         }
     }
+    // offers end with the launch; one that a donor has claimed is filled and
+    // marked active, and the next launch finds it
+    if (lane_id() == 0) {
+        if (wait == 1) atomicAnd(&H->hungry, ~(1u << wic));
+        if (wait == 2) {
+            const int cta = (int)blockIdx.x - G.first_cta;
+            const unsigned b = 1u << (cta & 31);
+            if (atomicAnd(G.ivm.ask + (cta >> 5), ~b) & b) atomicSub(&G.ctl->asking, 1);
+            atomicExch(&H->asker, 0);
+        }
+    }
+    __syncwarp();
     if (cached >= 0) store_ivm<NW>(G.ivm, cached, R);
     flush_counters(G, C);
 }
@@ -1132,20 +1291,21 @@ cudaError_t launch_lower_ub(const DevGroup* groups, int g, int ub, cudaStream_t 
 
 template <int NW, int VAR>
 cudaError_t explore_launch(const DevGroup* groups, const int* ngroups_d, int ctas, int warps_per_cta, int smem,
-                           unsigned long long budget_ns, int max_rounds, int select_budget, cudaStream_t st)
+                           unsigned long long budget_ns, int max_rounds, int select_budget, int eager,
+                           cudaStream_t st)
 {
     cudaFuncSetAttribute(pbb_explore_kernel<NW, VAR>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     pbb_explore_kernel<NW, VAR><<<ctas, 32 * warps_per_cta, smem, st>>>(groups, ngroups_d, warps_per_cta, budget_ns,
-                                                                         max_rounds, select_budget);
+                                                                         max_rounds, select_budget, eager);
     return cudaGetLastError();
 }
 
 cudaError_t launch_explore(int nw, const DevGroup* groups, const int* ngroups_d, int ctas, int warps_per_cta, int smem,
                            unsigned long long budget_ns, int max_rounds, int select_budget, cudaStream_t st,
-                           int variant)
+                           int variant, int eager)
 {
 #define PBB_EXPLORE(NW_, VAR_) \
-    explore_launch<NW_, VAR_>(groups, ngroups_d, ctas, warps_per_cta, smem, budget_ns, max_rounds, select_budget, st)
+    explore_launch<NW_, VAR_>(groups, ngroups_d, ctas, warps_per_cta, smem, budget_ns, max_rounds, select_budget, eager, st)
     if (nw == 1) {
         switch (variant) {
         case 1: return PBB_EXPLORE(1, 1);

@@ -106,6 +106,7 @@ struct pbb_pool {
     int grid = 0;               // CTAs of a window launch (all the CTAs of this shape the GPU holds)
     int tail_warps = 0, tail_grid = 0, tail_smem = 0;   // the tail's block shape (0 warps: none)
     int core_warps = PBB_CORE_WARPS, split_depth = PBB_SPLIT_DEPTH, share_after = PBB_SHARE_AFTER;
+    int split_narrow = PBB_SPLIT_NARROW;
     int Ppad_max = 0;
     size_t table_stride = 0;
     size_t off_je = 0, off_p = 0, off_pm = 0, off_mt = 0, off_posj = 0;
@@ -183,7 +184,7 @@ size_t explorer_block_bytes(int E, int npad)
 {
     size_t b = align256((size_t)E * npad * npad);     // mat
     b += 5 * align256((size_t)E * npad);              // pos end dir pj bestperm
-    b += 5 * align256((size_t)E * 4);                 // line state bestcost qseq qval
+    b += 5 * align256((size_t)E * 4);                 // line state bestcost ask askid
     b += align256((size_t)E * npad * PBB_PATH_INTS * 4);   // path levels
     return b;
 }
@@ -202,8 +203,8 @@ void carve_explorers(unsigned char* base, int E, int npad, DevIvms& V)
     V.line = reinterpret_cast<int*>(base + o); o += align256((size_t)E * 4);
     V.state = reinterpret_cast<int*>(base + o); o += align256((size_t)E * 4);
     V.bestcost = reinterpret_cast<int*>(base + o); o += align256((size_t)E * 4);
-    V.qseq = reinterpret_cast<unsigned*>(base + o); o += align256((size_t)E * 4);
-    V.qval = reinterpret_cast<int*>(base + o); o += align256((size_t)E * 4);
+    V.ask = reinterpret_cast<unsigned*>(base + o); o += align256((size_t)E * 4);
+    V.askid = reinterpret_cast<int*>(base + o); o += align256((size_t)E * 4);
     V.path = reinterpret_cast<int*>(base + o);
 }
 
@@ -238,6 +239,7 @@ int pool_create(const pbb_pool_config* in, pbb_pool* P)
     P->epw = c.explorers_per_instance;
     P->core_warps = c.core_warps > 0 ? c.core_warps : PBB_CORE_WARPS;
     P->split_depth = c.split_depth > 0 ? c.split_depth : PBB_SPLIT_DEPTH;
+    P->split_narrow = c.split_depth > 0 ? c.split_depth : PBB_SPLIT_NARROW;
     P->share_after = c.share_after > 0 ? c.share_after : (c.share_after < 0 ? 0 : PBB_SHARE_AFTER);
     const int Pmax = c.max_machines * (c.max_machines - 1) / 2;
     P->Ppad_max = (Pmax + 31) / 32 * 32;
@@ -464,6 +466,7 @@ int admit(pbb_pool* P, std::vector<int>& admitted)
         g.search.early_stop = 0;
         g.search.core_warps = P->core_warps;
         g.search.split_depth = P->split_depth;
+        g.search.split_narrow = P->split_narrow;
         g.search.share_after = P->share_after;
         carve_explorers(P->arena + off, E, P->npad, g.ivm);
         g.ctl = P->ctl + s;

@@ -5,13 +5,13 @@
 #define PBB_MAX_N 64          // jobs per instance (int8 IVM cells, two 32-bit mask words)
 #define PBB_MAX_M 32          // machines per instance (one machine per lane in recurrences)
 #define PBB_WARPS_MAX 20      // explorer warps per CTA (96 registers a thread)
-#define PBB_CORE_WARPS 8      // default of DevSearch::core_warps
+#define PBB_CORE_WARPS PBB_WARPS_MAX   // default of DevSearch::core_warps
 #define PBB_SPLIT_DEPTH 10    // default of DevSearch::split_depth
 #define PBB_SHARE_AFTER 64    // default of DevSearch::share_after
+#define PBB_SPLIT_NARROW 4    // default of DevSearch::split_narrow
 
 // IVM life cycle (per explorer, in global memory)
 #define IVM_IDLE 0            // no interval
-#define IVM_QUEUED 1          // registered in the idle queue, waiting for a donor
 #define IVM_ACTIVE 2          // holds a non-empty interval
 
 // status bits written by kernels (never traps)
@@ -53,19 +53,20 @@ struct DevSearch {
     int early_stop;    // [bb] earlyStopJohnson: a child's Johnson scan may stop once it exceeds the incumbent
     int core_warps;    // warps per CTA that ask for work whatever the search's width (1..warps per CTA)
     int split_depth;   // work is not split at levels deeper than n - split_depth
-    int share_after;   // an explorer offers work only after decomposing this many nodes since it got
-                       // its interval or last gave part of it away (0 = at every step)
+    int split_narrow;  // the same limit while most warps of the CTA, or most CTAs, wait for work
+    int share_after;   // an explorer gives work away only after decomposing this many nodes since it
+                       // got its interval or last gave part of it away, fewer the more warps wait
+                       // (0 = at every step)
 };
 
 // Per-group control block (device memory).
-// The fields every warp polls or updates under contention each sit on their
-// own 128-byte line, so that reads of the incumbent and of the active count
-// do not queue behind the idle-queue atomics (and the other way round).
+// The incumbent and the count of waiting CTAs are read together by every
+// working warp; the active count, which every start and end of an interval
+// updates, sits on a line of its own.
 struct GroupCtl {
     alignas(128) unsigned long long best_key;   // (cost << 32) | ivm id of the slot holding the permutation
+    int asking;                                 // CTAs asking other CTAs for work
     alignas(128) int active;                    // explorers holding work
-    alignas(128) unsigned long long q_head;     // idle-explorer queue cursors
-    alignas(128) unsigned long long q_tail;
     alignas(128) int found;                     // leaves that improved (or matched, with findAll) the bound
     unsigned int status;                        // PBB_ST_* bits
     unsigned long long decomposed, johnson_bounds, simple_bounds, leaves, root_simple;
@@ -90,8 +91,8 @@ struct DevIvms {
     int* state;            // [count]
     int* bestcost;         // [count]
     signed char* bestperm; // [count][npad]
-    unsigned int* qseq;    // [count] Vyukov queue cell sequence numbers
-    int* qval;             // [count] queued explorer ids
+    unsigned int* ask;     // [(count + 31) / 32] bit c: CTA c of the group asks for work
+    int* askid;            // [count] explorer that asking CTA c offers for it
     int* path;             // [count][npad levels][3][32] heads / tails / free loads of the path nodes
 };
 
@@ -135,9 +136,25 @@ struct BoundExtra {
     int* strong_idle = nullptr;  // [count]
 };
 
+// Work sharing inside one CTA (shared memory): a warp without work sets its
+// bit in `hungry` after writing the explorer it offers; a working warp that
+// splits its interval clears a bit, fills that explorer and posts its id in
+// the waiting warp's mail.
+struct CtaShare {
+    unsigned hungry;       // warps waiting for work
+    int working;           // warps holding work
+    int asker;             // 1 + the warp that asks other CTAs for this one (0: none)
+    int stop;              // the group's search has ended
+    int active;            // last value read of the group's active count
+    int best;              // last value read of the incumbent
+    int asking;            // last value read of the group's waiting CTAs
+    unsigned poll_ns;      // when the group's active count was last read (low word of the timer)
+    // int offer[warps], mail[warps] follow
+};
+
 // Dynamic shared memory layout of one CTA (host and device agree).
 struct SmemPlan {
-    int je_off, p_off, pm0_off, pm1_off, marr_off, mdep_off, posj_off, warp_off, warp_bytes, total;
+    int je_off, p_off, pm0_off, pm1_off, marr_off, mdep_off, posj_off, share_off, warp_off, warp_bytes, total;
     int fmask;             // 1: each warp keeps its explorer's free-position masks (explorer only)
 };
 
@@ -161,6 +178,7 @@ __host__ __device__ inline SmemPlan pbb_smem_plan(int n, int m, int Ppad, int wa
     s.marr_off = off; off += pbb_align(m * 4, 16);
     s.mdep_off = off; off += pbb_align(m * 4, 16);
     s.posj_off = off; off += pbb_align(n * Ppad, 16);
+    s.share_off = off; off += pbb_align((int)sizeof(CtaShare) + 8 * warps, 16);
     s.warp_off = off;
     s.fmask = fmask;
     s.warp_bytes = pbb_warp_bytes(n, m, Ppad, fmask);
