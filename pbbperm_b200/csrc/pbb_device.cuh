@@ -15,13 +15,9 @@
 
 #define FULLMASK 0xffffffffu
 #define NEG_INF (-(1 << 28))
-// direct scans walk at most this many children together
+// direct scans walk at most this many children together; nodes with more
+// Johnson children use the max-plus sweeps
 #define PBB_DIRECT_MAX 4
-// nodes with at most this many Johnson children use direct scans (by groups
-// of PBB_DIRECT_MAX), more children use the max-plus sweeps
-#ifndef PBB_DIRECT_LIMIT
-#define PBB_DIRECT_LIMIT 4
-#endif
 // a lone child gets its own one-chain direct scan (instead of two chains, one
 // repeating the other)
 #ifndef PBB_DIRECT_ONE
@@ -117,14 +113,15 @@ __device__ __forceinline__ int next_open_cell(const int (&row)[NW], int from, in
 // shared-memory views
 // ---------------------------------------------------------------------------
 struct CtaTables {
-    const unsigned long long* je;  // [n][Ppad]
-    const int* p;                  // [m][n]
+    const unsigned long long* je;  // [n][je_stride]
+    const int* pt;                 // [n][mp] processing times, 0 past the last machine
+    const int* pre;                // [n][mp] their prefix sums, or NULL
     const unsigned char* pm0;
     const unsigned char* pm1;
     const int* min_arr;
     const int* min_dep;
     const unsigned char* posj;     // [n][Ppad] or NULL
-    int n, m, P, Ppad;
+    int n, m, P, Ppad, mp, je_stride;
 };
 
 struct WarpScratch {
@@ -146,29 +143,44 @@ struct WarpScratch {
     // explorer this warp holds (bit t = position t), kept up to date by the
     // explorer as it moves; NULL outside the explorer or when it does not fit
     unsigned long long* fmask;
+    // kept pair bounds only (PBB_SCRATCH_PAIRS)
+    int* pairs;             // two buffers of Ppad pair bounds
+    int4* child;            // [32] by machine: the child's head, its job's time (twice), the child's tail
 };
 
 __device__ __forceinline__ WarpScratch warp_scratch(unsigned char* base, const SmemPlan& sp, int n, int m, int Ppad)
 {
     WarpScratch s;
     s.fmask = nullptr;
-    if (sp.fmask) {
-        s.fmask = reinterpret_cast<unsigned long long*>(base);
-        base += Ppad * 8;
-    }
+    s.pairs = nullptr;
+    s.child = nullptr;
     int* ip = reinterpret_cast<int*>(base);
-    s.lbF = ip; ip += n;
-    s.lbB = ip; ip += n;
-    s.frontZ = ip; ip += 32;
-    s.backZ = ip; ip += 32;
     s.Fb = ip; ip += 32;
     s.Bb = ip; ip += 32;
-    s.rem = ip; ip += 32;
     s.RB = ip; ip += 32;
     s.FR = ip; ip += 32;
+    s.frontZ = ip; ip += 32;
+    s.backZ = ip; ip += 32;
+    s.rem = ip; ip += 32;
+    const bool pairs = sp.fmask == PBB_SCRATCH_PAIRS;
+    if (pairs) {
+        s.child = reinterpret_cast<int4*>(ip); ip += 128;
+        s.pairs = ip; ip += 2 * Ppad;
+        s.lbF = s.lbB = nullptr;
+        s.dF = s.dB = nullptr;
+    } else {
+        if (sp.fmask) {
+            s.fmask = reinterpret_cast<unsigned long long*>(ip);
+            ip += 2 * Ppad;
+        }
+        s.lbF = ip; ip += n;
+        s.lbB = ip; ip += n;
+    }
     short* sp2 = reinterpret_cast<short*>(ip);
-    s.dF = sp2; sp2 += n * m;
-    s.dB = sp2; sp2 += n * m;
+    if (!pairs) {
+        s.dF = sp2; sp2 += n * m;
+        s.dB = sp2; sp2 += n * m;
+    }
     unsigned char* bp = reinterpret_cast<unsigned char*>(sp2);
     s.fjob = bp; bp += n;
     s.bjob = bp; bp += n;
@@ -198,19 +210,19 @@ __device__ __forceinline__ void partial_schedule(const CtaTables& T, const WarpS
         if (lane == 0) upf = 0;
         if (lane == m - 1) dnb = 0;
         int i = s - lane;
-        if (lane < m && i >= 0 && i < f) cf = max(cf, upf) + T.p[lane * n + S.fjob[i]];
+        if (lane < m && i >= 0 && i < f) cf = max(cf, upf) + T.pt[S.fjob[i] * T.mp + lane];
         int ib = s - ib0;
-        if (lane < m && ib >= 0 && ib < b) cb = max(cb, dnb) + T.p[lane * n + S.bjob[ib]];
+        if (lane < m && ib >= 0 && ib < b) cb = max(cb, dnb) + T.pt[S.bjob[ib] * T.mp + lane];
     }
     if (lane < m) {
         // loads of the free jobs: sum the shorter of the free / fixed lists
         int r = 0;
         if (k <= n - k) {
-            for (int i = 0; i < k; i++) r += T.p[lane * n + S.rowj[i]];
+            for (int i = 0; i < k; i++) r += T.pt[S.rowj[i] * T.mp + lane];
         } else {
-            for (int j = 0; j < n; j++) r += T.p[lane * n + j];
-            for (int i = 0; i < f; i++) r -= T.p[lane * n + S.fjob[i]];
-            for (int i = 0; i < b; i++) r -= T.p[lane * n + S.bjob[i]];
+            for (int j = 0; j < n; j++) r += T.pt[j * T.mp + lane];
+            for (int i = 0; i < f; i++) r -= T.pt[S.fjob[i] * T.mp + lane];
+            for (int i = 0; i < b; i++) r -= T.pt[S.bjob[i] * T.mp + lane];
         }
         int fb = (f == 0) ? T.min_arr[lane] : cf;
         int bb = (b == 0) ? T.min_dep[lane] : cb;
@@ -221,6 +233,12 @@ __device__ __forceinline__ void partial_schedule(const CtaTables& T, const WarpS
         S.rem[lane] = r;
         S.RB[lane] = r + bb;
         S.FR[lane] = fb + r;
+    } else {
+        // past the last machine: nothing raises a bound (weak_children)
+        S.Fb[lane] = 0;
+        S.Bb[lane] = 0;
+        S.RB[lane] = NEG_INF;
+        S.FR[lane] = NEG_INF;
     }
     __syncwarp();
 }
@@ -238,7 +256,7 @@ __device__ __forceinline__ void partial_schedule(const CtaTables& T, const WarpS
 __device__ __forceinline__ int append_front(const CtaTables& T, int hf, int u)
 {
     const int lane = lane_id();
-    const int pu = lane < T.m ? T.p[lane * T.n + u] : 0;
+    const int pu = lane < T.m ? T.pt[u * T.mp + lane] : 0;
     int P = pu;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -261,7 +279,7 @@ __device__ __forceinline__ int prepend_back(const CtaTables& T, int hb, int u)
 {
     const int lane = lane_id();
     const bool on = lane < T.m;
-    const int pu = on ? T.p[lane * T.n + u] : 0;
+    const int pu = on ? T.pt[u * T.mp + lane] : 0;
     int Q = pu;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -275,6 +293,38 @@ __device__ __forceinline__ int prepend_back(const CtaTables& T, int hb, int u)
         if (lane + o < 32) x = max(x, t);
     }
     return Q + x;
+}
+
+// the same with the prefix sums P of p(u) from a table: one scan instead of two
+__device__ __forceinline__ int append_front_pre(const CtaTables& T, int hf, int u)
+{
+    const int lane = lane_id();
+    const bool on = lane < T.m;
+    const int at = u * T.mp + (on ? lane : 0);
+    const int P = T.pre[at];
+    int x = hf - P + T.pt[at];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(FULLMASK, x, o);
+        if (lane >= o) x = max(x, t);
+    }
+    return on ? P + x : 0;
+}
+
+// t_k = p_k(u) - P_k + max_{j>=k}(hb_j + P_j), since Q_{j+1} = P_{m-1} - P_j
+__device__ __forceinline__ int prepend_back_pre(const CtaTables& T, int hb, int u)
+{
+    const int lane = lane_id();
+    const bool on = lane < T.m;
+    const int at = u * T.mp + (on ? lane : 0);
+    const int P = T.pre[at];
+    int x = on ? hb + P : NEG_INF;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_down_sync(FULLMASK, x, o);
+        if (lane + o < 32) x = max(x, t);
+    }
+    return on ? T.pt[at] - P + x : 0;
 }
 
 // the bound-side arrays of the scratch from the path registers (what
@@ -293,6 +343,11 @@ __device__ __forceinline__ void partial_from_path(const CtaTables& T, const Warp
         S.rem[lane] = hr;
         S.RB[lane] = hr + bb;
         S.FR[lane] = fb + hr;
+    } else {
+        S.Fb[lane] = 0;
+        S.Bb[lane] = 0;
+        S.RB[lane] = NEG_INF;
+        S.FR[lane] = NEG_INF;
     }
     __syncwarp();
 }
@@ -311,47 +366,89 @@ __device__ __forceinline__ int weak_node_lb(const CtaTables& T, const WarpScratc
     return lb;
 }
 
-// weak LB of child u appended at the front (bound_fsp_weak.cpp:134-161)
-__device__ __forceinline__ int weak_front(const CtaTables& T, const WarpScratch& S, int u)
+// Weak LBs of the row's children, one job per lane and word: appended at the
+// front (bound_fsp_weak.cpp:134-161), and with `both` prepended at the back
+// (:164-191).  Bound by issue: a rolled step per machine cost nine
+// instructions for four of arithmetic, so four machines are taken at a time by
+// 16-byte loads (the node's vectors uniform, the job's times from its own row)
+// and both words of a row share the node's (18x20 searched with this bound
+// alone, 8.8 M nodes: 13.4 -> 11.2 ms).
+template <int NW>
+__device__ __forceinline__ void weak_children(const CtaTables& T, const WarpScratch& S, const int (&row)[NW],
+                                              const bool (&valid)[NW], int k, bool both, int (&cb)[NW], int (&ce)[NW])
 {
-    const int n = T.n;
-    int t0 = S.Fb[0] + T.p[u];
-    int lb = S.Fb[0] + S.RB[0];
-    PBB_ROLLED
-    for (int k = 1; k < T.m; k++) {
-        int t1 = max(S.Fb[k], t0);
-        lb = max(lb, t1 + S.RB[k]);
-        t0 = t1 + T.p[k * n + u];
+    const int chunks = (T.m + 3) >> 2;
+    const int words = NW > 1 && k <= 32 ? 1 : NW;
+    const int4* pr[NW];
+    int t[NW], lb[NW];
+#pragma unroll
+    for (int w = 0; w < NW; w++) {
+        pr[w] = reinterpret_cast<const int4*>(T.pt + (valid[w] ? cell_job(row[w]) : 0) * T.mp);
+        t[w] = 0;
+        lb[w] = 0;
+        cb[w] = 0;
+        ce[w] = 0;
     }
-    return lb;
-}
-
-// weak LB of child u prepended at the back (bound_fsp_weak.cpp:164-191)
-__device__ __forceinline__ int weak_back(const CtaTables& T, const WarpScratch& S, int u)
-{
-    const int n = T.n, m = T.m;
-    int t0 = S.Bb[m - 1] + T.p[(m - 1) * n + u];
-    int lb = S.FR[m - 1] + S.Bb[m - 1];
     PBB_ROLLED
-    for (int k = m - 2; k >= 0; k--) {
-        int t1 = max(t0, S.Bb[k]);
-        lb = max(lb, S.FR[k] + t1);
-        t0 = t1 + T.p[k * n + u];
+    for (int c = 0; c < chunks; c++) {
+        const int4 f = reinterpret_cast<const int4*>(S.Fb)[c];
+        const int4 r = reinterpret_cast<const int4*>(S.RB)[c];
+#pragma unroll
+        for (int w = 0; w < NW; w++) {
+            if (w >= words) break;
+            const int4 p = pr[w][c];
+            int x = max(t[w], f.x);
+            lb[w] = max(lb[w], x + r.x);
+            x = max(x + p.x, f.y);
+            lb[w] = max(lb[w], x + r.y);
+            x = max(x + p.y, f.z);
+            lb[w] = max(lb[w], x + r.z);
+            x = max(x + p.z, f.w);
+            lb[w] = max(lb[w], x + r.w);
+            t[w] = x + p.w;
+        }
     }
-    return lb;
+#pragma unroll
+    for (int w = 0; w < NW; w++) {
+        if (valid[w]) cb[w] = lb[w];
+        t[w] = 0;
+        lb[w] = 0;
+    }
+    if (!both) return;
+    PBB_ROLLED
+    for (int c = chunks - 1; c >= 0; c--) {
+        const int4 d = reinterpret_cast<const int4*>(S.Bb)[c];
+        const int4 r = reinterpret_cast<const int4*>(S.FR)[c];
+#pragma unroll
+        for (int w = 0; w < NW; w++) {
+            if (w >= words) break;
+            const int4 p = pr[w][c];
+            int x = max(t[w], d.w);
+            lb[w] = max(lb[w], x + r.w);
+            x = max(x + p.w, d.z);
+            lb[w] = max(lb[w], x + r.z);
+            x = max(x + p.z, d.y);
+            lb[w] = max(lb[w], x + r.y);
+            x = max(x + p.y, d.x);
+            lb[w] = max(lb[w], x + r.x);
+            t[w] = x + p.x;
+        }
+    }
+#pragma unroll
+    for (int w = 0; w < NW; w++)
+        if (valid[w]) ce[w] = lb[w];
 }
 
 // idle-time priority of child u appended at the front: the sum over machines
 // k >= 1 of |completion of u on k-1 - front_k| (bound_fsp_weak.cpp:140-146)
 __device__ __forceinline__ int weak_front_idle(const CtaTables& T, const WarpScratch& S, int u)
 {
-    const int n = T.n;
-    int t0 = S.Fb[0] + T.p[u];
+    int t0 = S.Fb[0] + T.pt[u * T.mp];
     int pr = 0;
     PBB_ROLLED
     for (int k = 1; k < T.m; k++) {
         pr += abs(t0 - S.Fb[k]);
-        t0 = max(S.Fb[k], t0) + T.p[k * n + u];
+        t0 = max(S.Fb[k], t0) + T.pt[u * T.mp + k];
     }
     return pr;
 }
@@ -359,13 +456,13 @@ __device__ __forceinline__ int weak_front_idle(const CtaTables& T, const WarpScr
 // the same for child u prepended at the back (bound_fsp_weak.cpp:172-178)
 __device__ __forceinline__ int weak_back_idle(const CtaTables& T, const WarpScratch& S, int u)
 {
-    const int n = T.n, m = T.m;
-    int t0 = S.Bb[m - 1] + T.p[(m - 1) * n + u];
+    const int m = T.m;
+    int t0 = S.Bb[m - 1] + T.pt[u * T.mp + m - 1];
     int pr = 0;
     PBB_ROLLED
     for (int k = m - 2; k >= 0; k--) {
         pr += abs(t0 - S.Bb[k]);
-        t0 = max(t0, S.Bb[k]) + T.p[k * n + u];
+        t0 = max(t0, S.Bb[k]) + T.pt[u * T.mp + k];
     }
     return pr;
 }
@@ -374,13 +471,12 @@ __device__ __forceinline__ int weak_back_idle(const CtaTables& T, const WarpScra
 // as max over machines of head + tail at the split
 __device__ __forceinline__ int makespan_split(const CtaTables& T, const WarpScratch& S, int x, int y)
 {
-    const int n = T.n;
     int h1 = 0, h2 = 0, best = 0;
     PBB_ROLLED
     for (int k = 0; k < T.m; k++) {
-        h1 = max(h1, S.frontZ[k]) + T.p[k * n + x];
+        h1 = max(h1, S.frontZ[k]) + T.pt[x * T.mp + k];
         int h = h1;
-        if (y >= 0) { h2 = max(h2, h1) + T.p[k * n + y]; h = h2; }
+        if (y >= 0) { h2 = max(h2, h1) + T.pt[y * T.mp + k]; h = h2; }
         best = max(best, h + S.backZ[k]);
     }
     return best;
@@ -608,14 +704,12 @@ __device__ __forceinline__ void fmask_flip(const CtaTables& T, const WarpScratch
     __syncwarp();
 }
 
-// the free-position mask of pair i for the node being bounded (FM: the
-// warp's masks are known to be there)
-template <int NW, int FM = 0>
+// the free-position mask of pair i for the node being bounded
+template <int NW>
 __device__ __forceinline__ typename PosMask<NW>::type node_positions(const CtaTables& T, const WarpScratch& S, int k,
                                                                      int i)
 {
     typedef typename PosMask<NW>::type M;
-    if (FM) return (M)S.fmask[i];
     return S.fmask ? (M)S.fmask[i] : free_positions<NW>(T, S, k, i);
 }
 
@@ -649,7 +743,7 @@ __device__ __forceinline__ void direct_start(const CtaTables& T, const WarpScrat
 // running maximum exceeds `stop` the remaining passes are skipped; such a
 // child is pruned whatever its remaining pairs give, so only the value of a
 // pruned child changes (INT_MAX = no early exit).
-template <int C, int NW, int FM = 0>
+template <int C, int NW>
 __device__ __forceinline__ void johnson_direct_chains(const CtaTables& T, const WarpScratch& S, int k, int nc,
                                                       const int (&cjob)[4], const int (&cside)[4], int stop)
 {
@@ -676,7 +770,7 @@ __device__ __forceinline__ void johnson_direct_chains(const CtaTables& T, const 
                 direct_start(T, S, u[c], sd[c], m0, m1, t0[c], t1[c], B0[c], B1[c]);
                 px[c] = T.posj[u[c] * T.Ppad + i];
             }
-            M pm = node_positions<NW, FM>(T, S, k, i);
+            M pm = node_positions<NW>(T, S, k, i);
             const unsigned long long* col = T.je + i;
             while (pm) {
                 const int t = low_pos(pm);
@@ -713,23 +807,23 @@ __device__ __forceinline__ void johnson_direct_chains(const CtaTables& T, const 
     __syncwarp();
 }
 
-template <int NW, int FM = 0>
+template <int NW>
 __device__ __forceinline__ void johnson_direct_masked(const CtaTables& T, const WarpScratch& S, int k, int nc,
                                                       const int (&cjob)[4], const int (&cside)[4], int stop)
 {
     static_assert(PBB_DIRECT_MAX <= 4, "direct scans walk at most four children together");
     if (nc <= 0) return;
 #if PBB_DIRECT_ONE
-    if (nc == 1) johnson_direct_chains<1, NW, FM>(T, S, k, nc, cjob, cside, stop);
+    if (nc == 1) johnson_direct_chains<1, NW>(T, S, k, nc, cjob, cside, stop);
     else
 #endif
-    if (nc <= 2) johnson_direct_chains<2, NW, FM>(T, S, k, nc, cjob, cside, stop);
-    else johnson_direct_chains<4, NW, FM>(T, S, k, nc, cjob, cside, stop);
+    if (nc <= 2) johnson_direct_chains<2, NW>(T, S, k, nc, cjob, cside, stop);
+    else johnson_direct_chains<4, NW>(T, S, k, nc, cjob, cside, stop);
 }
 
 // johnson_children (forward + backward max-plus sweeps) over the free
 // positions only (needs T.posj); same results, O(P k) instead of O(P n).
-template <int NW, int FM = 0>
+template <int NW>
 __device__ __forceinline__ void johnson_sweep_masked(const CtaTables& T, const WarpScratch& S, int k,
                                                      bool doF,
                                                      const unsigned (&sF)[NW], bool doB, const unsigned (&sB)[NW])
@@ -749,7 +843,7 @@ __device__ __forceinline__ void johnson_sweep_masked(const CtaTables& T, const W
             const int cB3 = S.Fb[m0] + Asum + S.backZ[m0];
             const unsigned long long* col = T.je + i;
             typedef typename PosMask<NW>::type M;
-            const M pm = node_positions<NW, FM>(T, S, k, i);
+            const M pm = node_positions<NW>(T, S, k, i);
             int Apre = 0, Bpre = 0, PMx = NEG_INF;
             M fwd = pm;
             while (fwd) {
@@ -806,7 +900,7 @@ template <int NW>
 __device__ __forceinline__ void child_tables(const CtaTables& T, const WarpScratch& S, const int (&row)[NW], int k,
                                              bool doF, const unsigned (&sF)[NW], bool doB, const unsigned (&sB)[NW])
 {
-    const int n = T.n, m = T.m;
+    const int m = T.m;
 #pragma unroll
     for (int w = 0; w < NW; w++) {
         const int idx = w * 32 + lane_id();
@@ -822,7 +916,7 @@ __device__ __forceinline__ void child_tables(const CtaTables& T, const WarpScrat
                 PBB_ROLLED
                 for (int kk = 0; kk < m; kk++) {
                     const int z = S.frontZ[kk];
-                    h = max(h, z) + T.p[kk * n + u];
+                    h = max(h, z) + T.pt[u * T.mp + kk];
                     S.dF[u * m + kk] = (short)(h - z);
                 }
             }
@@ -831,7 +925,7 @@ __device__ __forceinline__ void child_tables(const CtaTables& T, const WarpScrat
                 PBB_ROLLED
                 for (int kk = m - 1; kk >= 0; kk--) {
                     const int z = S.backZ[kk];
-                    t = max(t, z) + T.p[kk * n + u];
+                    t = max(t, z) + T.pt[u * T.mp + kk];
                     S.dB[u * m + kk] = (short)(t - z);
                 }
             }
@@ -943,12 +1037,62 @@ __device__ __noinline__ void sort_cells(unsigned char* out, int k, unsigned long
     __syncwarp();
 }
 
+// sortedDFS >= 1: eliminateJobs sorts the row (ivm_bound.cpp:338-370) by the
+// chosen side's first cost, then (2, 4) by the sibling priority
+// chooseChildrenSet set (:506-544), or (3) by the priority alone.  cb, ce: the
+// costs the side was chosen from; the row's cells are flagged already.
+template <int NW>
+__device__ __forceinline__ void sort_row(const CtaTables& T, const WarpScratch& S, const DevSearch& srch,
+                                         int (&row)[NW], const bool (&valid)[NW], int k, int dir, const int (&cb)[NW],
+                                         const int (&ce)[NW])
+{
+    unsigned long long key[NW];
+#pragma unroll
+    for (int w = 0; w < NW; w++) {
+        const int mine = dir ? ce[w] : cb[w];
+        int prio = 0;
+        if (srch.sort_nodes >= 2) {
+            const int other = dir ? cb[w] : ce[w];
+            if (srch.sort_crit == 1) prio = mine;
+            else if (srch.sort_crit == 2) prio = mine - other;
+            else if (mine <= 0) prio = 99999;
+            else if (valid[w]) {
+                // the row is flagged already (pruned cells hold -j-1): the
+                // reference sorts before pruning, so take the job itself
+                const int u = cell_job(row[w]);
+                prio = dir ? weak_back_idle(T, S, u) : weak_front_idle(T, S, u);
+            }
+        }
+        const unsigned long long lo = (unsigned)prio ^ 0x80000000u;   // signed order as unsigned
+        key[w] = srch.sort_nodes == 3 ? lo : ((unsigned long long)(unsigned)mine << 32) | lo;
+    }
+    sort_cells(S.rowj, k, key[0], NW > 1 ? key[NW - 1] : 0ull, row[0], NW > 1 ? row[NW - 1] : 0);
+#pragma unroll
+    for (int w = 0; w < NW; w++)
+        if (valid[w]) row[w] = (signed char)S.rowj[w * 32 + lane_id()];
+    __syncwarp();
+}
+
+// reverse the row when the side changes from the previous level (:620-636)
+template <int NW>
+__device__ __forceinline__ void reverse_row(int (&row)[NW], int k)
+{
+    int nr[NW];
+#pragma unroll
+    for (int w = 0; w < NW; w++) {
+        const int idx = w * 32 + lane_id();
+        const int src = k - 1 - idx;
+        const int v = vgather<NW>(row, src < 0 ? 0 : src);
+        nr[w] = (idx < k) ? v : row[w];
+    }
+#pragma unroll
+    for (int w = 0; w < NW; w++) row[w] = nr[w];
+}
+
 // Returns the side chosen for this level.  SAMPLE = 1 with `rec` set writes
 // the children's bounds, as computed and before pruning, into a node record
 // (SampleBuf layout: schedule at rec + PBB_SAMPLE_HDR, then four arrays of n).
-// RULE != 0 fixes the branching rule at compile time (the caller then passes
-// a constant mode too), so the hot explorer carries no code for the others.
-template <int NW, int SORT = 1, int SAMPLE = 0, int RULE = 0>
+template <int NW, int SORT = 1, int SAMPLE = 0>
 __device__ __forceinline__ int bound_and_prune(const CtaTables& T, const WarpScratch& S, const DevSearch& srch,
                                                int mode, int (&row)[NW], int k, int f, int b, int line,
                                                int prev_dir, int best, NodeCounters& cnt, bool partial_ready = false,
@@ -964,26 +1108,18 @@ __device__ __forceinline__ int bound_and_prune(const CtaTables& T, const WarpScr
     __syncwarp();
     if (!partial_ready) partial_schedule(T, S, f, b, k);
 
-    // the fixed build (RULE != 0) serves searches without findAll, with the
-    // position tables present and the warp's free-position masks kept
-    const bool both = (RULE ? RULE : srch.branch_mode) > 0;
-    const bool fa = RULE ? false : srch.find_all != 0;
-    const bool masked = RULE || T.posj;
+    const bool both = srch.branch_mode > 0;
+    const bool fa = srch.find_all != 0;
+    const bool masked = T.posj != nullptr;
     int cbw[NW], cew[NW], cbs[NW], ces[NW];
 #pragma unroll
     for (int w = 0; w < NW; w++) { cbw[w] = 0; cew[w] = 0; cbs[w] = 0; ces[w] = 0; }
 
     int dir;
     if (mode != 1) {
-#pragma unroll
-        for (int w = 0; w < NW; w++) {
-            if (valid[w]) {
-                cbw[w] = weak_front(T, S, row[w]);
-                if (both) cew[w] = weak_back(T, S, row[w]);
-            }
-        }
+        weak_children<NW>(T, S, row, valid, k, both, cbw, cew);
         cnt.simple += both ? 2 * k : k;
-        dir = choose_dir<NW>(RULE ? RULE : srch.branch_mode, line, best, cbw, cew, valid);
+        dir = choose_dir<NW>(srch.branch_mode, line, best, cbw, cew, valid);
     }
 
     if (mode != 0) {
@@ -1027,44 +1163,7 @@ __device__ __forceinline__ int bound_and_prune(const CtaTables& T, const WarpScr
                     if (w * 32 + lane < T.n) { S.lbF[w * 32 + lane] = 0; S.lbB[w * 32 + lane] = 0; }
                 }
                 child_tables<NW>(T, S, row, k, nF > 0, sF, nB > 0, sB);
-                if (nF + nB <= PBB_DIRECT_LIMIT) {
-#if PBB_DIRECT_LIMIT > PBB_DIRECT_MAX
-                    // list the children (front side first, job order), then
-                    // scan them by groups of at most PBB_DIRECT_MAX
-                    int list[PBB_DIRECT_LIMIT];
-                    int nc = 0;
-#pragma unroll
-                    for (int side = 0; side < 2; side++) {
-#pragma unroll
-                        for (int q = 0; q < NW; q++) {
-                            unsigned msk = side ? sB[q] : sF[q];
-                            while (msk) {
-                                const int j = q * 32 + __ffs(msk) - 1;
-                                msk &= msk - 1;
-#pragma unroll
-                                for (int c = 0; c < PBB_DIRECT_LIMIT; c++)
-                                    if (nc == c) list[c] = j | (side << 8);
-                                nc++;
-                            }
-                        }
-                    }
-                    // the early exit lives in the runtime-options build only (SORT = 1):
-                    // the default explorer passes a constant and keeps no trace of it
-                    const int stop = (SORT && srch.early_stop) ? best : INT_MAX;
-                    PBB_ROLLED
-                    for (int g = 0; g < nc; g += PBB_DIRECT_MAX) {
-                        int cjob[4] = {0, 0, 0, 0}, cside[4] = {0, 0, 0, 0};
-#pragma unroll
-                        for (int c = 0; c < 4; c++) {
-#pragma unroll
-                            for (int e = 0; e < PBB_DIRECT_LIMIT; e++)
-                                if (e == g + c) { cjob[c] = list[e] & 0xff; cside[c] = list[e] >> 8; }
-                        }
-                        const int gn = min(nc - g, PBB_DIRECT_MAX);
-                        if (T.posj) johnson_direct_masked<NW>(T, S, k, gn, cjob, cside, stop);
-                        else johnson_direct<NW>(T, S, um, gn, cjob, cside);
-                    }
-#else
+                if (nF + nB <= PBB_DIRECT_MAX) {
                     // list the children (front side first, job order)
                     int cjob[4] = {0, 0, 0, 0}, cside[4] = {0, 0, 0, 0};
                     int nc = 0;
@@ -1084,18 +1183,15 @@ __device__ __forceinline__ int bound_and_prune(const CtaTables& T, const WarpScr
                         }
                     }
                     // early exit: in the runtime-options build (SORT = 1) when
-                    // earlyStopJohnson asks for it; in the default search's build
-                    // (RULE != 0) always -- it only changes the values of
-                    // children that are pruned anyway, which that build never
-                    // reports; the general hot build keeps no trace of it
-                    const int stop = RULE ? best : ((SORT && srch.early_stop) ? best : INT_MAX);
-                    if (masked) johnson_direct_masked<NW, (RULE != 0)>(T, S, k, nc, cjob, cside, stop);
+                    // earlyStopJohnson asks for it; the general hot build keeps
+                    // no trace of it
+                    const int stop = (SORT && srch.early_stop) ? best : INT_MAX;
+                    if (masked) johnson_direct_masked<NW>(T, S, k, nc, cjob, cside, stop);
                     else johnson_direct<NW>(T, S, um, nc, cjob, cside);
-#endif
                     cnt.direct_children += nc;
-                    cnt.direct_free += (unsigned)(nc * k);
+                    cnt.direct_free += (unsigned)(nc * k * T.P);
                 } else {
-                    if (masked) johnson_sweep_masked<NW, (RULE != 0)>(T, S, k, nF > 0, sF, nB > 0, sB);
+                    if (masked) johnson_sweep_masked<NW>(T, S, k, nF > 0, sF, nB > 0, sB);
                     else johnson_children<NW>(T, S, um, nF > 0, sF, nB > 0, sB, nullptr);
                     cnt.sweeps++;
                     cnt.free_jobs += k;
@@ -1108,7 +1204,7 @@ __device__ __forceinline__ int bound_and_prune(const CtaTables& T, const WarpScr
                 }
             }
         }
-        if (mode == 1) dir = choose_dir<NW>(RULE ? RULE : srch.branch_mode, line, best, cbs, ces, valid);
+        if (mode == 1) dir = choose_dir<NW>(srch.branch_mode, line, best, cbs, ces, valid);
     }
 
     if (SAMPLE && rec) {
@@ -1140,49 +1236,276 @@ __device__ __forceinline__ int bound_and_prune(const CtaTables& T, const WarpScr
         if (valid[w] && cut) row[w] = cell_flag(row[w]);
     }
     if (SORT && srch.sort_nodes) {
-        // sortedDFS >= 1: eliminateJobs sorts the row (ivm_bound.cpp:338-370)
-        // by the chosen side's first cost, then (2, 4) by the sibling
-        // priority chooseChildrenSet set (:506-544), or (3) by the priority
-        // alone; out of line to keep the hot loop small.  The first cost is
-        // also the cost the side was chosen from (weak, or Johnson in mode 1).
-        unsigned long long key[NW];
+        // the first cost is the cost the side was chosen from (weak, or Johnson in mode 1)
+        if (mode == 1) sort_row<NW>(T, S, srch, row, valid, k, dir, cbs, ces);
+        else sort_row<NW>(T, S, srch, row, valid, k, dir, cbw, cew);
+    } else if (prev_dir != dir) {
+        reverse_row<NW>(row, k);
+    }
+    return dir;
+}
+
+// ---------------------------------------------------------------------------
+// Bounding mode 2 by kept pair bounds
+// ---------------------------------------------------------------------------
+//
+// In mode 2 the weak bound chooses the side and orders the row, so the search
+// only asks which children the Johnson bound prunes.  For machine
+// pair i with machines (m0, m1) and a child with heads h, tails t and free jobs
+// V, the pair's bound is the largest of two one-machine terms, which are no
+// larger than the child's weak bound and so below the incumbent already, and
+//   h[m0] + C_i(V) + t[m1],  C_i(V) = max_s (sum a up to s + lag_s + sum b from s)
+// over the jobs s of V in the pair's Johnson order.  Taking job q away from a
+// set lowers every term by a_q or by b_q (or removes it), so
+//   C_i(V \ q) <= C_i(V) - min(a_q, b_q):
+// one value per pair, kept from the parent and lowered by the job that led
+// here, proves for most pairs in a few instructions that they prune nothing.
+// Over 9 in 10 Johnson children of a 50x20 search survive, and about five of
+// the 190 pairs of a child need more: those are scanned by the whole warp, a
+// Johnson position per lane, which gives C_i of the node's free jobs (it
+// replaces the kept value, for the children to come and the levels below) and
+// of the child's.  Only comparisons are decided this way: the children pruned,
+// and so the node counts, are those of the full bound.  Kept values of the
+// levels above are stored per warp in device memory; those a warp does not
+// have (it just took the explorer) are scanned when it first comes back to
+// their level.  Explorer milliseconds, scans of every pair / this: 50x20
+// 503 / 194, 20x20 57 / 39, 16x20 3.6 / 2.3, 20x10 1.02 / 0.90.
+struct PairBounds {
+    int* cur;       // [Ppad] values of the node at level `level`
+    int* nxt;       // [Ppad] values of the node being bounded
+    int* stack;     // [n][Ppad] values of the levels of the current path (device memory, this warp's)
+    int level;      // level whose values `cur` holds, -1: none
+    int from;       // lowest level whose values `stack` holds
+};
+
+// Values of the parent (level L - 1) of a node with free jobs `um` that was
+// reached by fixing job u, into B.cur.
+template <int NW>
+__device__ __forceinline__ void pairs_of_parent(const CtaTables& T, PairBounds& B, int L, int u,
+                                                const unsigned (&um)[NW])
+{
+    int* lvl = B.stack + (size_t)(L - 1) * T.Ppad;
+    if (L - 1 >= B.from) {
+        PBB_ROLLED
+        for (int i = lane_id(); i < T.P; i += 32) B.cur[i] = __ldcg(lvl + i);
+    } else {
+        // a pair per lane: every pair is wanted here
+        PBB_ROLLED
+        for (int i = lane_id(); i < T.P; i += 32) {
+            const unsigned long long* col = T.je + i;
+            int t0 = 0, t1 = NEG_INF;
+            PBB_ROLLED
+            for (int t = 0; t < T.n; t++) {
+                const unsigned long long e = col[t * T.je_stride];
+                const int j = JE_JOB(e);
+                unsigned uw = um[0];
 #pragma unroll
-        for (int w = 0; w < NW; w++) {
-            const int mine = (mode == 1) ? (dir ? ces[w] : cbs[w]) : (dir ? cew[w] : cbw[w]);
-            int prio = 0;
-            if (srch.sort_nodes >= 2) {
-                const int other = (mode == 1) ? (dir ? cbs[w] : ces[w]) : (dir ? cbw[w] : cew[w]);
-                if (srch.sort_crit == 1) prio = mine;
-                else if (srch.sort_crit == 2) prio = mine - other;
-                else if (mine <= 0) prio = 99999;
-                else if (valid[w]) {
-                    // the row is flagged already (pruned cells hold -j-1): the
-                    // reference sorts before pruning, so take the job itself
-                    const int u = cell_job(row[w]);
-                    prio = dir ? weak_back_idle(T, S, u) : weak_front_idle(T, S, u);
+                for (int w = 1; w < NW; w++)
+                    if ((j >> 5) == w) uw = um[w];
+                if (((uw >> (j & 31)) & 1u) || j == u) {
+                    t0 += JE_A(e);
+                    t1 = max(t1, t0 + JE_C(e)) + JE_B(e);
                 }
             }
-            const unsigned long long lo = (unsigned)prio ^ 0x80000000u;   // signed order as unsigned
-            key[w] = srch.sort_nodes == 3 ? lo : ((unsigned long long)(unsigned)mine << 32) | lo;
+            B.cur[i] = t1;
+            __stcg(lvl + i, t1);
         }
-        sort_cells(S.rowj, k, key[0], NW > 1 ? key[NW - 1] : 0ull, row[0], NW > 1 ? row[NW - 1] : 0);
+        B.from = L - 1;
+    }
+    B.level = L - 1;
+    __syncwarp();
+}
+
+// C_i of the free jobs `um`, and of them without job v (times av, bv on the
+// pair's machines), a Johnson position per lane and word.  bsum: the free
+// jobs' load on the pair's second machine.
+template <int NW>
+__device__ __forceinline__ void pair_scan(const CtaTables& T, int i, const unsigned (&um)[NW], int v, int av, int bv,
+                                          int bsum, int& all, int& rest)
+{
+    const int lane = lane_id();
+    int W[NW], D[NW], job[NW];
+    bool fr[NW];
 #pragma unroll
-        for (int w = 0; w < NW; w++)
-            if (valid[w]) row[w] = (signed char)S.rowj[w * 32 + lane];
-        __syncwarp();
-    } else if (prev_dir != dir) {
-        // reverse the row when the side changes from the previous level (:620-636)
-        int nr[NW];
+    for (int w = 0; w < NW; w++) {
+        const int t = w * 32 + lane;
+        const bool in = t < T.n;
+        const unsigned long long e = T.je[(in ? t : 0) * T.je_stride + i];
+        job[w] = JE_JOB(e);
+        unsigned uw = um[0];
+#pragma unroll
+        for (int q = 1; q < NW; q++)
+            if ((job[w] >> 5) == q) uw = um[q];
+        fr[w] = in && ((uw >> (job[w] & 31)) & 1u);
+        D[w] = fr[w] ? JE_A(e) - JE_B(e) : 0;
+        W[w] = JE_B(e) + JE_C(e);
+    }
+    // prefix sums of a - b over the free positions
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
 #pragma unroll
         for (int w = 0; w < NW; w++) {
-            int idx = w * 32 + lane;
-            int src = k - 1 - idx;
-            int v = vgather<NW>(row, src < 0 ? 0 : src);
-            nr[w] = (idx < k) ? v : row[w];
+            const int x = __shfl_up_sync(FULLMASK, D[w], o);
+            if (lane >= o) D[w] += x;
         }
-#pragma unroll
-        for (int w = 0; w < NW; w++) row[w] = nr[w];
     }
+    int before = 0;
+    unsigned at[NW];
+#pragma unroll
+    for (int w = 0; w < NW; w++) {
+        W[w] = fr[w] ? W[w] + D[w] + before : NEG_INF;
+        if (w + 1 < NW) before += __shfl_sync(FULLMASK, D[w], 31);
+        at[w] = __ballot_sync(FULLMASK, fr[w] && job[w] == v);
+    }
+    int x = NEG_INF, y = NEG_INF;
+    bool past = false;      // v stands in an earlier word
+#pragma unroll
+    for (int w = 0; w < NW; w++) {
+        x = max(x, W[w]);
+        // a term before v loses b_v, one after it a_v
+        const bool ahead = !past && (at[w] == 0 || (at[w] & lanemask_lt()) == 0);
+        if (!((at[w] >> lane) & 1u)) y = max(y, W[w] - (ahead ? bv : av));
+        past = past || at[w] != 0;
+    }
+    all = bsum + __reduce_max_sync(FULLMASK, x);
+    rest = bsum + __reduce_max_sync(FULLMASK, y);
+}
+
+// Children of the node at level L (reached by fixing job u) kept by the
+// weak bound -- cells keep[w], all on side `side` -- that the Johnson bound
+// prunes too: their lanes' flags are set in cut[w].  k >= 3 free jobs; hf, hb:
+// the node's heads and tails, lane = machine.
+template <int NW>
+__device__ __forceinline__ void johnson_prune(const CtaTables& T, const WarpScratch& S, PairBounds& B,
+                                              const int (&row)[NW], const bool (&valid)[NW], const unsigned (&keep)[NW],
+                                              int side, int L, int u, int hf, int hb, int best, bool (&cut)[NW],
+                                              NodeCounters& cnt, int k)
+{
+    const int lane = lane_id();
+    unsigned um[NW];
+    job_mask<NW>(um, row, valid);
+    if (B.level != L - 1) pairs_of_parent<NW>(T, B, L, u, um);
+    const int* pu = T.pt + u * T.mp;
+    PBB_ROLLED
+    for (int i = lane; i < T.P; i += 32) B.nxt[i] = B.cur[i] - min(pu[T.pm0[i]], pu[T.pm1[i]]);
+    unsigned left[NW];
+    bool open = false;
+#pragma unroll
+    for (int w = 0; w < NW; w++) left[w] = keep[w];
+    const int2* ends = reinterpret_cast<const int2*>(S.child);
+    while (true) {
+        int cell = -1;
+#pragma unroll
+        for (int w = NW - 1; w >= 0; w--)
+            if (left[w]) cell = w * 32 + __ffs(left[w]) - 1;
+        if (cell < 0) break;
+#pragma unroll
+        for (int w = 0; w < NW; w++)
+            if ((cell >> 5) == w) left[w] &= left[w] - 1;
+        const int v = vget<NW>(row, cell);
+        {
+            const int x = side ? prepend_back_pre(T, hb, v) : append_front_pre(T, hf, v);
+            const int p = lane < T.m ? T.pt[v * T.mp + lane] : 0;
+            const int h = side ? S.Fb[lane] : x, t = side ? x : S.Bb[lane];
+            __syncwarp();
+            S.child[lane] = make_int4(h, p, p, t);
+            __syncwarp();
+        }
+        bool over = false;
+        PBB_ROLLED
+        for (int base = 0; base < T.P && !over; base += 32) {
+            const int i = base + lane;
+            bool fail = false;
+            if (i < T.P) {
+                const int2 c0 = ends[2 * T.pm0[i]], c1 = ends[2 * T.pm1[i] + 1];   // (head, a) and (b, tail)
+                fail = c0.x + c1.y + B.nxt[i] - min(c0.y, c1.x) >= best;
+            }
+            unsigned fb = __ballot_sync(FULLMASK, fail);
+            while (fb && !over) {
+                const int j = base + __ffs(fb) - 1;
+                fb &= fb - 1;
+                const int m1 = T.pm1[j];
+                const int2 c0 = ends[2 * T.pm0[j]], c1 = ends[2 * m1 + 1];
+                int all, rest;
+                pair_scan<NW>(T, j, um, v, c0.y, c1.x, S.rem[m1], all, rest);
+                if (lane == 0) B.nxt[j] = all;
+                over = c0.x + c1.y + rest >= best;
+                cnt.direct_free += 2 * k;
+            }
+        }
+        cnt.direct_children++;
+#pragma unroll
+        for (int w = 0; w < NW; w++)
+            if ((cell >> 5) == w && lane == (cell & 31)) cut[w] = over;
+        open = open || !over;
+    }
+    __syncwarp();
+    if (open) {
+        // the search goes below this node: its values are the parent's next
+        int* lvl = B.stack + (size_t)L * T.Ppad;
+        PBB_ROLLED
+        for (int i = lane; i < T.P; i += 32) __stcg(lvl + i, B.nxt[i]);
+        int* t = B.cur;
+        B.cur = B.nxt;
+        B.nxt = t;
+        B.level = L;
+    }
+}
+
+// bound_and_prune for bounding mode 2 with a rule that computes the weak bound
+// of the side it chooses (all but the fixed back sides): the same row and side,
+// the Johnson values compared instead of computed (see above).  GEN = 0: MinMin,
+// no findAll, no sorted rows, compiled in; GEN = 1: the search's settings.
+template <int NW, int GEN>
+__device__ __forceinline__ int bound_pairs(const CtaTables& T, const WarpScratch& S, PairBounds& B,
+                                           const DevSearch& srch, int (&row)[NW], int k, int line, int u, int hf,
+                                           int hb, int prev_dir, int best, NodeCounters& cnt)
+{
+    const int lane = lane_id();
+    bool valid[NW];
+    int cbw[NW], cew[NW];
+#pragma unroll
+    for (int w = 0; w < NW; w++) valid[w] = (w * 32 + lane) < k;
+    const bool both = GEN ? srch.branch_mode > 0 : true;
+    weak_children<NW>(T, S, row, valid, k, both, cbw, cew);
+    cnt.simple += both ? 2 * k : k;
+    const int dir = choose_dir<NW>(GEN ? srch.branch_mode : 3, line, best, cbw, cew, valid);
+    // a child goes when a bound reaches the incumbent, or exceeds it with findAll
+    const int limit = GEN && srch.find_all && best < INT_MAX ? best + 1 : best;
+    // children the weak bound keeps get the Johnson bound (ivm_bound.cpp:168)
+    bool cut[NW];
+    unsigned keep[NW];
+    int nk = 0;
+#pragma unroll
+    for (int w = 0; w < NW; w++) {
+        cut[w] = valid[w] && (dir ? cew[w] : cbw[w]) >= limit;
+        keep[w] = __ballot_sync(FULLMASK, valid[w] && !cut[w]);
+        nk += __popc(keep[w]);
+    }
+    cnt.johnson += nk;
+    if (nk > 0) {
+        if (k <= 2) {
+            // each child has at most one free job left: exact makespan
+            // (bound_fsp_strong.cpp:543-546)
+            const int x = vget<NW>(row, 0);
+            const int y = k == 2 ? vget<NW>(row, 1) : -1;
+            int mk = 0;
+            if (lane < 2) mk = makespan_split(T, S, lane == 0 ? x : y, lane == 0 ? y : x);
+            const int mxy = __shfl_sync(FULLMASK, mk, 0);
+            const int myx = __shfl_sync(FULLMASK, mk, 1);
+#pragma unroll
+            for (int w = 0; w < NW; w++)
+                if (valid[w] && !cut[w]) cut[w] = (((row[w] == x) == (dir == 0)) ? mxy : myx) >= limit;
+        } else {
+            johnson_prune<NW>(T, S, B, row, valid, keep, dir, line, u, hf, hb, limit, cut, cnt, k);
+        }
+    }
+    // prune (eliminateJobs :338-410)
+#pragma unroll
+    for (int w = 0; w < NW; w++)
+        if (valid[w] && cut[w]) row[w] = cell_flag(row[w]);
+    if (GEN && srch.sort_nodes) sort_row<NW>(T, S, srch, row, valid, k, dir, cbw, cew);
+    else if (prev_dir != dir) reverse_row<NW>(row, k);
     return dir;
 }
 

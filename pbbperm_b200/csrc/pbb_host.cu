@@ -130,6 +130,9 @@ struct pbb_engine {
     cudaStream_t st = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     int nw = 2, warps = 0, ctas = 0, smem = 0, root_smem = 0;
+    // the launch with kept pair bounds (explorer variants 3 and 4), pair_warps 0: not used
+    int pair_variant = 0, pair_warps = 0, pair_smem = 0, pair_stride = 0;
+    int* pair_stack = nullptr;
     DeviceInstance di;
     signed char *mat = nullptr, *vec = nullptr, *bestperm = nullptr;
     int* path = nullptr;   // per explorer and level: heads, tails, free loads
@@ -283,6 +286,7 @@ int pbb_engine_destroy(pbb_engine* e)
     if (e->st) cudaStreamSynchronize(e->st);
     e->di.release();
     cudaFree(e->mat); cudaFree(e->vec); cudaFree(e->bestperm); cudaFree(e->path);
+    cudaFree(e->pair_stack);
     cudaFree(e->line); cudaFree(e->state); cudaFree(e->bestcost); cudaFree(e->askid); cudaFree(e->ask);
     cudaFree(e->ub_d); cudaFree(e->root_d); cudaFree(e->ival_d); cudaFree(e->ctl); cudaFree(e->group_d);
     cudaFree(e->ngroups_d);
@@ -318,6 +322,22 @@ static int engine_create(const pbb_instance* inst, const pbb_config* cfg, pbb_en
     int sms = 0;
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, e->dev));
     e->ctas = cfg->ctas > 0 ? cfg->ctas : sms;
+    e->pair_variant = pbbl::pairs_variant(cfg->bounding_mode, cfg->branching_mode, cfg->find_all, cfg->sorted_dfs);
+    if (e->pair_variant) {
+        // earlyStopJohnson changes the values of pruned children only, which
+        // these builds do not compute: they serve both settings
+        const int cap = max_smem_optin(e->dev);
+        int w = e->warps;
+        while (w > 1 && pbbl::smem_bytes(H.n, H.m, H.Ppad, w, PBB_SCRATCH_PAIRS) > cap) w--;
+        e->pair_smem = pbbl::smem_bytes(H.n, H.m, H.Ppad, w, PBB_SCRATCH_PAIRS);
+        e->pair_stride = H.n * H.Ppad;
+        if (e->pair_smem <= cap) {
+            if (cudaMalloc(&e->pair_stack, sizeof(int) * (size_t)e->ctas * w * e->pair_stride) == cudaSuccess)
+                e->pair_warps = w;
+            else
+                cudaGetLastError();   // no room: the general build needs none
+        }
+    }
     rc = e->di.upload(H, e->st);
     if (rc) return rc;
     const int B = cfg->nb_ivms;
@@ -683,12 +703,11 @@ static int explore_window(pbb_engine* e, double seconds, int32_t* done, int eage
         const unsigned long long budget = (unsigned long long)(win * 1e9);
         CK(cudaEventRecord(e->ev0, e->st));
         int variant = e->sample_d ? 2 : ((e->cfg.sorted_dfs || e->cfg.early_stop_johnson) ? 1 : 0);
-        // the fixed build also needs the per-warp masks in the launch
-        const bool masks = e->smem == pbbl::smem_bytes(e->H.n, e->H.m, e->H.Ppad, e->warps, 1);
-        if (variant == 0 && e->cfg.bounding_mode == 2 && e->cfg.branching_mode == 3 && !e->cfg.find_all && masks)
-            variant = 3;
-        CK(pbbl::launch_explore(e->nw, e->group_d, e->ngroups_d, e->ctas, e->warps, e->smem, budget, e->max_rounds,
-                                e->select_budget, e->st, variant, eager));
+        if (variant != 2 && e->pair_warps > 0) variant = e->pair_variant;
+        const bool pairs = variant >= 3;
+        CK(pbbl::launch_explore(e->nw, e->group_d, e->ngroups_d, e->ctas, pairs ? e->pair_warps : e->warps,
+                                pairs ? e->pair_smem : e->smem, budget, e->max_rounds, e->select_budget, e->st,
+                                variant, eager, e->pair_stack, e->pair_stride));
         CK(cudaEventRecord(e->ev1, e->st));
         rc = wait_event(e->ev1, e->wait_limit_s < 0 ? win + 60.0 : e->wait_limit_s);
         if (rc == PBB_E_TIMEOUT) {
@@ -927,9 +946,9 @@ int pbb_work_counters(pbb_engine* e, pbb_work* out)
     out->sweep_free_jobs = c.jfree;
     out->sweep_children = c.jchild;
     out->direct_children = c.jdirect;
-    out->direct_free_jobs = c.jdirect_free;
+    out->direct_free_jobs = e->H.P > 0 ? c.jdirect_free / e->H.P : 0;   // counted per machine pair
     out->explorers = e->cfg.nb_ivms;
-    out->warps = e->warps * e->ctas;
+    out->warps = (e->pair_warps > 0 ? e->pair_warps : e->warps) * e->ctas;
     out->status = (int32_t)c.status;
     return PBB_OK;
 }

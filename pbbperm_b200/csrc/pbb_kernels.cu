@@ -59,20 +59,43 @@ __device__ __forceinline__ void load_tables(const DevInstance& I, unsigned char*
 {
     const int tid = threadIdx.x, nt = blockDim.x;
     unsigned long long* je = reinterpret_cast<unsigned long long*>(smem + sp.je_off);
-    int* p = reinterpret_cast<int*>(smem + sp.p_off);
-    unsigned char* pm0 = smem + sp.pm0_off;
-    unsigned char* pm1 = smem + sp.pm1_off;
+    int* pt = reinterpret_cast<int*>(smem + sp.p_off);
+    unsigned char* pm0 = smem + sp.pm_off;
+    unsigned char* pm1 = pm0 + I.Ppad;
     int* marr = reinterpret_cast<int*>(smem + sp.marr_off);
     int* mdep = reinterpret_cast<int*>(smem + sp.mdep_off);
-    for (int i = tid; i < I.n * I.Ppad; i += nt) je[i] = I.je[i];
-    for (int i = tid; i < I.n * I.m; i += nt) p[i] = I.p[i];
+    const int mp = pbb_machine_pad(I.m);
+    if (sp.je_stride == I.Ppad) {
+        for (int i = tid; i < I.n * I.Ppad; i += nt) je[i] = I.je[i];
+    } else {
+        for (int t = tid / 32; t < I.n; t += nt / 32)
+            for (int i = tid & 31; i < I.Ppad; i += 32) je[t * sp.je_stride + i] = I.je[t * I.Ppad + i];
+    }
+    for (int i = tid; i < I.n * mp; i += nt) {
+        const int j = i / mp, k = i - j * mp;
+        pt[i] = k < I.m ? I.p[k * I.n + j] : 0;
+    }
+    if (sp.fmask == PBB_SCRATCH_PAIRS) {
+        int* pre = reinterpret_cast<int*>(smem + sp.pre_off);
+        for (int i = tid; i < I.n * mp; i += nt) {
+            const int j = i / mp, k = min(i - j * mp, I.m - 1);
+            int sum = 0;
+            for (int q = 0; q <= k; q++) sum += I.p[q * I.n + j];
+            pre[i] = sum;
+        }
+        T.pre = pre;
+    } else {
+        T.pre = nullptr;
+    }
     for (int i = tid; i < I.Ppad; i += nt) { pm0[i] = I.pm0[i]; pm1[i] = I.pm1[i]; }
     for (int i = tid; i < I.m; i += nt) { marr[i] = I.min_arr[i]; mdep[i] = I.min_dep[i]; }
+    const bool posj_here = I.posj && sp.fmask != PBB_SCRATCH_PAIRS;
     unsigned char* posj = smem + sp.posj_off;
-    if (I.posj)
+    if (posj_here)
         for (int i = tid; i < I.n * I.Ppad; i += nt) posj[i] = I.posj[i];
-    T.je = je; T.p = p; T.pm0 = pm0; T.pm1 = pm1; T.min_arr = marr; T.min_dep = mdep;
-    T.posj = I.posj ? posj : nullptr;
+    T.je = je; T.pt = pt; T.mp = mp; T.pm0 = pm0; T.pm1 = pm1; T.min_arr = marr; T.min_dep = mdep;
+    T.posj = posj_here ? posj : nullptr;
+    T.je_stride = sp.je_stride;
     T.n = I.n; T.m = I.m; T.P = I.P; T.Ppad = I.Ppad;
 }
 
@@ -110,12 +133,13 @@ __device__ __forceinline__ void store_path(const DevIvms& V, int id, int l, cons
 }
 
 // path vectors of level L+1 from those of level L, job u fixed on side dir
-template <int NW>
+// (PRE: by the prefix sums of the processing times)
+template <int NW, int PRE = 0>
 __device__ __forceinline__ void path_down(const CtaTables& T, Ivm<NW>& R, int u, int dir)
 {
-    if (dir == 0) R.hf = append_front(T, R.hf, u);
-    else R.hb = prepend_back(T, R.hb, u);
-    if (lane_id() < T.m) R.hr -= T.p[lane_id() * T.n + u];
+    if (dir == 0) R.hf = PRE ? append_front_pre(T, R.hf, u) : append_front(T, R.hf, u);
+    else R.hb = PRE ? prepend_back_pre(T, R.hb, u) : prepend_back(T, R.hb, u);
+    if (lane_id() < T.m) R.hr -= T.pt[u * T.mp + lane_id()];
 }
 
 // jobs fixed in front among the levels above L
@@ -204,7 +228,9 @@ __device__ __forceinline__ void build_lists(const WarpScratch& S, const Ivm<NW>&
 }
 
 // 32-bit per warp (fewer live registers in the explorer loop), added to the
-// group's 64-bit counters at least every 2^20 decomposed nodes
+// group's 64-bit counters every 2^13 decomposed nodes (direct_free grows by at
+// most 2 x 64 x 496 x 64 a node: well under 2^32 in that many for any search
+// met, and it only feeds the work statistics)
 struct WarpCounters {
     unsigned decomposed, simple, johnson, leaves;
     unsigned sweeps, free_jobs, swept_children, direct_children, direct_free;
@@ -255,7 +281,7 @@ __device__ __forceinline__ void record_solution(const DevGroup& G, const WarpScr
 // advance to the next unpruned node of the interval, evaluating leaves on the
 // way.  Returns 1 with a node to bound at R.line, 0 when the interval is
 // exhausted, 2 when the selection budget ran out (state stays consistent).
-template <int NW, int FM = 0>
+template <int NW, int PAIRS = 0>
 __device__ __forceinline__ int select_node(const DevGroup& G, const CtaTables& T, const WarpScratch& S, int id, Ivm<NW>& R,
                            int& best, WarpCounters& C, int budget)
 {
@@ -271,7 +297,7 @@ __device__ __forceinline__ int select_node(const DevGroup& G, const CtaTables& T
                 vset<NW>(R.pos, L, 0);
                 L--;
                 R.line = L;
-                if (FM || S.fmask) fmask_flip(T, S, vget<NW>(R.pj, L));   // its job is free again
+                if (!PAIRS && S.fmask) fmask_flip(T, S, vget<NW>(R.pj, L));   // its job is free again
                 load_row<NW>(G.ivm, id, L, R.row);
                 load_path<NW>(G.ivm, id, L, R);
                 const int pp = vget<NW>(R.pos, L);
@@ -300,8 +326,8 @@ __device__ __forceinline__ int select_node(const DevGroup& G, const CtaTables& T
         C.decomposed++;
         const int u = vget<NW>(R.row, q);
         vset<NW>(R.pj, L, u);
-        if (FM || S.fmask) fmask_flip(T, S, u);                  // u is fixed below this level
-        path_down<NW>(T, R, u, vget<NW>(R.dir, L));
+        if (!PAIRS && S.fmask) fmask_flip(T, S, u);                    // u is fixed below this level
+        path_down<NW, PAIRS>(T, R, u, vget<NW>(R.dir, L));
         int nr[NW];
 #pragma unroll
         for (int w = 0; w < NW; w++) {
@@ -388,9 +414,10 @@ __device__ __forceinline__ int* sample_slot(const DevGroup& G, const WarpScratch
 }
 
 // Bound and prune the node selected at R.line and write its row back.
-template <int NW, int SORT, int SAMPLE, int RULE>
-__device__ __forceinline__ void bound_current(const DevGroup& G, const CtaTables& T, const WarpScratch& S, int id,
-                                              Ivm<NW>& R, int mode, int best, WarpCounters& C)
+// PAIRS: 0 full Johnson values, 1 + GEN of bound_pairs.
+template <int NW, int SORT, int SAMPLE, int PAIRS>
+__device__ __forceinline__ void bound_current(const DevGroup& G, const CtaTables& T, const WarpScratch& S,
+                                              PairBounds& B, int id, Ivm<NW>& R, int mode, int best, WarpCounters& C)
 {
     const int L = R.line;
     const int f = front_count<NW>(R, L), b = L - f;
@@ -399,8 +426,11 @@ __device__ __forceinline__ void bound_current(const DevGroup& G, const CtaTables
     int* rec = nullptr;
     if (SAMPLE) rec = sample_slot<NW>(G, S, R, id, f, b, best, C.decomposed);
     NodeCounters nc = {0, 0, 0, 0, 0};
-    const int d = bound_and_prune<NW, SORT, SAMPLE, RULE>(T, S, G.search, mode, R.row, T.n - L, f, b, L, prev, best, nc,
-                                                    true, rec);
+    int d;
+    if (PAIRS)
+        d = bound_pairs<NW, (PAIRS == 2)>(T, S, B, G.search, R.row, T.n - L, L, vget<NW>(R.pj, L - 1), R.hf, R.hb, prev, best, nc);
+    else
+        d = bound_and_prune<NW, SORT, SAMPLE>(T, S, G.search, mode, R.row, T.n - L, f, b, L, prev, best, nc, true, rec);
     vset<NW>(R.dir, L, d);
     store_row<NW>(G.ivm, id, L, R.row);
     C.simple += (unsigned)nc.simple;
@@ -788,7 +818,7 @@ __global__ void pbb_root_kernel(const DevGroup* groups, int ngroups, const int* 
     R.hb = 0;
     R.hr = 0;
     if (lane_id() < T.m)
-        for (int j = 0; j < n; j++) R.hr += T.p[lane_id() * n + j];
+        for (int j = 0; j < n; j++) R.hr += T.pt[j * T.mp + lane_id()];
     store_path<NW>(G.ivm, id, 0, R);
     NodeCounters nc = {0, 0, 0, 0, 0};
     const int mode = G.search.bound_mode;
@@ -838,17 +868,17 @@ __global__ void pbb_root_kernel(const DevGroup* groups, int ngroups, const int* 
 
 // Persistent explorer loop.  Warp w of a group serves explorers w, w+W, ...
 // (W = warps of the group).  Runs until no explorer of the group holds work,
-// or `budget_ns` of device time has passed, or `max_rounds` rounds.  VAR = 3
-// is VAR 0 for boundingMode 2 with MinMin branching and no findAll (the
-// default search), compiled in as constants; VAR = 0
+// or `budget_ns` of device time has passed, or `max_rounds` rounds.  VAR = 0
 // compiles the sortedDFS row sorts, the early Johnson exit and node sampling
 // out of the hot loop; VAR = 1 follows each group's sortedDFS and
 // earlyStopJohnson settings; VAR = 2 also records sampled nodes into the
-// group's SampleBuf.
+// group's SampleBuf.  VAR = 3 and 4 bound in mode 2 by kept pair bounds: 3 the
+// default search (MinMin, no findAll, rows not sorted, compiled in), 4 every
+// other search of that mode whose rule bounds the side it chooses.
 template <int NW, int VAR>
 __global__ void __launch_bounds__(32 * PBB_WARPS_MAX, 1)
 pbb_explore_kernel(const DevGroup* groups, const int* ngroups_d, int warps_per_cta, unsigned long long budget_ns,
-                   int max_rounds, int select_budget, int eager)
+                   int max_rounds, int select_budget, int eager, int* pair_stack, int pair_stride)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     // the group count lives in device memory so that a captured launch
@@ -863,13 +893,18 @@ pbb_explore_kernel(const DevGroup* groups, const int* ngroups_d, int warps_per_c
     unsigned dyn_smem;
     asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn_smem));
     // (the one-machine bound alone has no use for them)
-    const int fm = G.inst.posj != nullptr && G.search.bound_mode != 0 &&
-                   pbb_smem_plan(G.inst.n, G.inst.m, G.inst.Ppad, warps_per_cta, 1).total <= (int)dyn_smem;
-    if (VAR == 3 && !fm) {
-        // the fixed build relies on the masks; the host launches it only
-        // with room for them
-        if (threadIdx.x == 0) atomicOr(&G.ctl->status, PBB_ST_BADINPUT);
-        return;
+    int fm = PBB_SCRATCH_PLAIN;
+    if (VAR >= 3) {
+        // the host launches this build only with room for its scratch
+        fm = PBB_SCRATCH_PAIRS;
+        if (!pair_stack || G.inst.n * G.inst.Ppad > pair_stride ||
+            pbb_smem_plan(G.inst.n, G.inst.m, G.inst.Ppad, warps_per_cta, fm).total > (int)dyn_smem) {
+            if (threadIdx.x == 0) atomicOr(&G.ctl->status, PBB_ST_BADINPUT);
+            return;
+        }
+    } else if (G.inst.posj && G.search.bound_mode != 0 &&
+               pbb_smem_plan(G.inst.n, G.inst.m, G.inst.Ppad, warps_per_cta, PBB_SCRATCH_MASKS).total <= (int)dyn_smem) {
+        fm = PBB_SCRATCH_MASKS;
     }
     const SmemPlan sp = pbb_smem_plan(G.inst.n, G.inst.m, G.inst.Ppad, warps_per_cta, fm);
     CtaTables T;
@@ -890,10 +925,16 @@ pbb_explore_kernel(const DevGroup* groups, const int* ngroups_d, int warps_per_c
     const WarpScratch S = warp_scratch(smem + sp.warp_off + wic * sp.warp_bytes, sp, T.n, T.m, T.Ppad);
     const int W = G.ctas * warps_per_cta;
     const int wid = (blockIdx.x - G.first_cta) * warps_per_cta + wic;
-    const int mode = VAR == 3 ? 2 : G.search.bound_mode;
+    const int mode = VAR >= 3 ? 2 : G.search.bound_mode;
     const unsigned long long t0 = globaltimer_ns();
 
     WarpCounters C = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+    PairBounds B;
+    B.cur = S.pairs;
+    B.nxt = S.pairs + T.Ppad;
+    B.stack = VAR >= 3 ? pair_stack + (size_t)(blockIdx.x * warps_per_cta + wic) * pair_stride : nullptr;
+    B.level = -1;
+    B.from = 0;
     Ivm<NW> R;
     int cached = -1;                   // explorer whose state is held in registers
     int since = 0;                     // nodes it decomposed since it got work or gave some away
@@ -968,8 +1009,10 @@ pbb_explore_kernel(const DevGroup* groups, const int* ngroups_d, int warps_per_c
                 __syncwarp();
                 load_ivm<NW>(G.ivm, id, R);
                 cached = id;
+                B.level = -1;
+                B.from = R.line + 1;
                 idle_ns = 100;
-                if (S.fmask) fmask_build<NW>(T, S, R.row, T.n - R.line);
+                if (VAR < 3 && S.fmask) fmask_build<NW>(T, S, R.row, T.n - R.line);
                 if (lane_id() == 0) atomicAdd(&H->working, 1);
             } else {
                 if (scan >= G.ivm.count) {
@@ -1004,13 +1047,13 @@ pbb_explore_kernel(const DevGroup* groups, const int* ngroups_d, int warps_per_c
         const int wish = share_wish(G.search, H, since, warps_per_cta, G.ctas, eager, narrow);
         if (wish && try_share<NW>(G, H, wic, id, R, wish, narrow) == 1) since = 0;
         const int known = best;
-        const int r = select_node<NW, (VAR == 3)>(G, T, S, id, R, best, C, select_budget);
+        const int r = select_node<NW, (VAR >= 3)>(G, T, S, id, R, best, C, select_budget);
         if (best < known && lane_id() == 0) atomicMin(&H->best, best);
         if (r == 1) {
             since++;
-            bound_current<NW, (VAR == 1 || VAR == 2), (VAR == 2), (VAR == 3 ? 3 : 0)>(G, T, S, id, R, mode, best, C);
+            bound_current<NW, (VAR == 1 || VAR == 2), (VAR == 2), (VAR >= 3 ? VAR - 2 : 0)>(G, T, S, B, id, R, mode, best, C);
         }
-        if (C.decomposed >= (1u << 20)) flush_counters(G, C);
+        if (C.decomposed >= (1u << 13)) flush_counters(G, C);
         if (r == 0) {
             // interval exhausted: leave the pool of busy explorers (the
             // registers need not go back: nobody resumes this interval)
@@ -1093,11 +1136,13 @@ __global__ void pbb_bound_kernel(DevInstance I, int count, const int* sched, con
         int* ose = se + (size_t)node * n;
         for (int i = lane; i < n; i += 32) { owb[i] = 0; owe[i] = 0; osb[i] = 0; ose[i] = 0; }
         __syncwarp();
+        int wf[NW], wk[NW];
+        weak_children<NW>(T, S, row, valid, k, true, wf, wk);
 #pragma unroll
         for (int w = 0; w < NW; w++) {
             if (valid[w]) {
-                owb[row[w]] = weak_front(T, S, row[w]);
-                owe[row[w]] = weak_back(T, S, row[w]);
+                owb[row[w]] = wf[w];
+                owe[row[w]] = wk[w];
             }
         }
         if (X.prio_begin) {
@@ -1126,18 +1171,18 @@ __global__ void pbb_bound_kernel(DevInstance I, int count, const int* sched, con
                 for (int q = 0; q < T.m; q++) { fr[q] = 0; bk[q] = 0; }
                 for (int i = 0; i < f; i++) {
                     const int j = S.fjob[i];
-                    fr[0] += T.p[j];
+                    fr[0] += T.pt[j * T.mp];
                     for (int q = 1; q < T.m; q++) {
                         idle += max(0, fr[q - 1] - fr[q]);
-                        fr[q] = max(fr[q], fr[q - 1]) + T.p[q * n + j];
+                        fr[q] = max(fr[q], fr[q - 1]) + T.pt[j * T.mp + q];
                     }
                 }
                 for (int i = 0; i < b; i++) {
                     const int j = S.bjob[i];
-                    bk[T.m - 1] += T.p[(T.m - 1) * n + j];
+                    bk[T.m - 1] += T.pt[j * T.mp + T.m - 1];
                     for (int q = T.m - 2; q >= 0; q--) {
                         idle += max(0, bk[q + 1] - bk[q]);
-                        bk[q] = max(bk[q], bk[q + 1]) + T.p[q * n + j];
+                        bk[q] = max(bk[q], bk[q + 1]) + T.pt[j * T.mp + q];
                     }
                 }
             }
@@ -1251,6 +1296,7 @@ int explore_ctas_per_sm(int nw, int warps_per_cta, int smem, int variant)
         case 1: return explore_occupancy<1, 1>(warps_per_cta, smem);
         case 2: return explore_occupancy<1, 2>(warps_per_cta, smem);
         case 3: return explore_occupancy<1, 3>(warps_per_cta, smem);
+        case 4: return explore_occupancy<1, 4>(warps_per_cta, smem);
         default: return explore_occupancy<1, 0>(warps_per_cta, smem);
         }
     }
@@ -1258,6 +1304,7 @@ int explore_ctas_per_sm(int nw, int warps_per_cta, int smem, int variant)
     case 1: return explore_occupancy<2, 1>(warps_per_cta, smem);
     case 2: return explore_occupancy<2, 2>(warps_per_cta, smem);
     case 3: return explore_occupancy<2, 3>(warps_per_cta, smem);
+    case 4: return explore_occupancy<2, 4>(warps_per_cta, smem);
     default: return explore_occupancy<2, 0>(warps_per_cta, smem);
     }
 }
@@ -1292,25 +1339,27 @@ cudaError_t launch_lower_ub(const DevGroup* groups, int g, int ub, cudaStream_t 
 template <int NW, int VAR>
 cudaError_t explore_launch(const DevGroup* groups, const int* ngroups_d, int ctas, int warps_per_cta, int smem,
                            unsigned long long budget_ns, int max_rounds, int select_budget, int eager,
-                           cudaStream_t st)
+                           int* pair_stack, int pair_stride, cudaStream_t st)
 {
     cudaFuncSetAttribute(pbb_explore_kernel<NW, VAR>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     pbb_explore_kernel<NW, VAR><<<ctas, 32 * warps_per_cta, smem, st>>>(groups, ngroups_d, warps_per_cta, budget_ns,
-                                                                         max_rounds, select_budget, eager);
+                                                                         max_rounds, select_budget, eager, pair_stack, pair_stride);
     return cudaGetLastError();
 }
 
 cudaError_t launch_explore(int nw, const DevGroup* groups, const int* ngroups_d, int ctas, int warps_per_cta, int smem,
                            unsigned long long budget_ns, int max_rounds, int select_budget, cudaStream_t st,
-                           int variant, int eager)
+                           int variant, int eager, int* pair_stack, int pair_stride)
 {
 #define PBB_EXPLORE(NW_, VAR_) \
-    explore_launch<NW_, VAR_>(groups, ngroups_d, ctas, warps_per_cta, smem, budget_ns, max_rounds, select_budget, eager, st)
+    explore_launch<NW_, VAR_>(groups, ngroups_d, ctas, warps_per_cta, smem, budget_ns, max_rounds, select_budget, eager, pair_stack, \
+                              pair_stride, st)
     if (nw == 1) {
         switch (variant) {
         case 1: return PBB_EXPLORE(1, 1);
         case 2: return PBB_EXPLORE(1, 2);
         case 3: return PBB_EXPLORE(1, 3);
+        case 4: return PBB_EXPLORE(1, 4);
         default: return PBB_EXPLORE(1, 0);
         }
     }
@@ -1318,6 +1367,7 @@ cudaError_t launch_explore(int nw, const DevGroup* groups, const int* ngroups_d,
     case 1: return PBB_EXPLORE(2, 1);
     case 2: return PBB_EXPLORE(2, 2);
     case 3: return PBB_EXPLORE(2, 3);
+    case 4: return PBB_EXPLORE(2, 4);
     default: return PBB_EXPLORE(2, 0);
     }
 #undef PBB_EXPLORE

@@ -4,8 +4,16 @@
 #include "pbb_types.h"
 
 namespace pbbl {
-// dynamic shared memory of a CTA; fmask = 1 adds the explorer's per-warp
-// free-position masks
+// The explorer variant with kept pair bounds for a search's settings, 0 when
+// there is none: mode 2 with a rule that bounds the side it chooses (-2 and -3
+// choose the back side without its weak bound, so Johnson values stand alone).
+inline int pairs_variant(int bound_mode, int branch_mode, int find_all, int sort_nodes)
+{
+    if (bound_mode != 2 || branch_mode < -1) return 0;
+    return branch_mode == 3 && !find_all && !sort_nodes ? 3 : 4;
+}
+
+// dynamic shared memory of a CTA; fmask: the per-warp scratch (PBB_SCRATCH_*)
 int smem_bytes(int n, int m, int Ppad, int warps, int fmask = 0);
 cudaError_t launch_reset(const DevGroup* groups, int ngroups, const int* ub, cudaStream_t st);
 // reset must run first; interval b = g * per_group + j starts explorer j of
@@ -13,15 +21,16 @@ cudaError_t launch_reset(const DevGroup* groups, int ngroups, const int* ub, cud
 cudaError_t launch_root(int nw, const DevGroup* groups, int ngroups, const int* roots, const int* ivals,
                         int root_stride, int smem, cudaStream_t st, int per_group = 1, const int* ids = nullptr);
 cudaError_t launch_lower_ub(const DevGroup* groups, int g, int ub, cudaStream_t st);
-// variant: 0 = no row sort, no early Johnson exit, no sampling (the hot
-// path); 1 = each group's sortedDFS / earlyStopJohnson settings; 2 = as 1 and
-// record sampled nodes (groups' SampleBuf); 3 = as 0 for groups that all
-// bound in mode 2 with MinMin branching, without findAll, with position
-// tables (all compiled in); eager = 0: a short window, which splits work only
-// as often as share_after says, however many warps wait
+// variant: 0 = no row sort, no early Johnson exit, no sampling; 1 = each
+// group's sortedDFS / earlyStopJohnson settings; 2 = as 1 and record sampled
+// nodes (groups' SampleBuf); 3 and 4 = kept pair bounds (pairs_variant), launched
+// with the PBB_SCRATCH_PAIRS shared memory and with pair_stack, pair_stride
+// ints for each warp of the grid (at least jobs x padded machine pairs).
+// eager = 0: a short window, which splits work only as often as share_after
+// says, however many warps wait
 cudaError_t launch_explore(int nw, const DevGroup* groups, const int* ngroups_d, int ctas, int warps_per_cta, int smem,
                            unsigned long long budget_ns, int max_rounds, int select_budget, cudaStream_t st,
-                           int variant = 0, int eager = 1);
+                           int variant = 0, int eager = 1, int* pair_stack = nullptr, int pair_stride = 0);
 int explore_ctas_per_sm(int nw, int warps_per_cta, int smem, int variant = 0);
 cudaError_t launch_bound(int nw, const DevInstance& I, int count, const int* sched, const int* l1, const int* l2,
                          int* wb, int* we, int* sb, int* se, int* nweak, int* nstrong, unsigned int* status, int ctas,

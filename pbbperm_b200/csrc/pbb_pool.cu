@@ -123,10 +123,13 @@ struct pbb_pool {
     int* ivals_d = nullptr;
     int* neh_d = nullptr;         // per slot: device NEH permutation [64] and makespan
     NehTask* neh_tasks_d = nullptr;
-    cudaGraphExec_t window = nullptr;
-    cudaGraphExec_t window_tail = nullptr;   // the same window with the tail's block shape
-    cudaGraphExec_t window_fixed = nullptr, window_tail_fixed = nullptr;   // boundingMode 2 + MinMin builds
-    bool masks = false, tail_masks = false;   // launches sized with the per-warp free-position masks
+    // window graphs by block shape (bulk, tail) and explorer build (0: any
+    // settings, 1 and 2: variants 3 and 4), captured when first needed
+    cudaGraphExec_t window[2][3] = {{nullptr, nullptr, nullptr}, {nullptr, nullptr, nullptr}};
+    // the default search's build: scratch of its launches (0: not used) and
+    // the pair bounds of every warp of the wider grid
+    int pair_smem = 0, tail_pair_smem = 0, pair_stride = 0;
+    int* pair_stack = nullptr;
     std::vector<Slot> slots;
     // the FIFO and the finished results are shared with submitting and
     // polling threads; everything else belongs to the thread driving step()
@@ -157,12 +160,12 @@ extern "C" int pbb_pool_destroy(pbb_pool* P)
     pbbh::DeviceGuard keep_callers_device;
     cudaSetDevice(P->dev);
     if (P->st) cudaStreamSynchronize(P->st);
-    if (P->window) cudaGraphExecDestroy(P->window);
-    if (P->window_tail) cudaGraphExecDestroy(P->window_tail);
-    if (P->window_fixed) cudaGraphExecDestroy(P->window_fixed);
-    if (P->window_tail_fixed) cudaGraphExecDestroy(P->window_tail_fixed);
+    for (auto& shape : P->window)
+        for (cudaGraphExec_t g : shape)
+            if (g) cudaGraphExecDestroy(g);
     cudaFree(P->arena);
     cudaFree(P->tables);
+    cudaFree(P->pair_stack);
     cudaFree(P->ctl);
     cudaFreeHost(P->ctl_h);
     cudaFree(P->groups_d);
@@ -256,8 +259,9 @@ int pool_create(const pbb_pool_config* in, pbb_pool* P)
         const int ms = pbbl::smem_bytes(c.max_jobs, c.max_machines, P->Ppad_max, P->warps, 1);
         if (ms <= optin && pbbl::explore_ctas_per_sm(P->nw, P->warps, ms) >= per_sm) {
             P->smem = ms;
-            P->masks = true;
         }
+        const int ps = pbbl::smem_bytes(c.max_jobs, c.max_machines, P->Ppad_max, P->warps, PBB_SCRATCH_PAIRS);
+        if (ps <= optin && pbbl::explore_ctas_per_sm(P->nw, P->warps, ps, 3) >= per_sm) P->pair_smem = ps;
     }
     // every window launches all the CTAs the GPU holds at once and spreads
     // them over the resident instances
@@ -271,16 +275,13 @@ int pool_create(const pbb_pool_config* in, pbb_pool* P)
         int ts = pbbl::smem_bytes(c.max_jobs, c.max_machines, P->Ppad_max, tw);
         const int tper = ts <= optin ? pbbl::explore_ctas_per_sm(P->nw, tw, ts) : 0;
         const int tms = pbbl::smem_bytes(c.max_jobs, c.max_machines, P->Ppad_max, tw, 1);
-        bool tm = false;
-        if (tper >= 1 && tms <= optin && pbbl::explore_ctas_per_sm(P->nw, tw, tms) >= tper) {
-            ts = tms;
-            tm = true;
-        }
+        if (tper >= 1 && tms <= optin && pbbl::explore_ctas_per_sm(P->nw, tw, tms) >= tper) ts = tms;
         if (tper >= 1) {
             P->tail_warps = tw;
             P->tail_smem = ts;
             P->tail_grid = sms * tper;
-            P->tail_masks = tm;
+            const int ps = pbbl::smem_bytes(c.max_jobs, c.max_machines, P->Ppad_max, tw, PBB_SCRATCH_PAIRS);
+            if (ps <= optin && pbbl::explore_ctas_per_sm(P->nw, tw, ps, 3) >= tper) P->tail_pair_smem = ps;
         }
     }
     // default explorer count: every warp of the widest grid owns one, so that
@@ -309,6 +310,15 @@ int pool_create(const pbb_pool_config* in, pbb_pool* P)
     PCK(cudaMalloc(&P->ivals_d, sizeof(int) * S * 2 * PBB_MAX_N), "intervals");
     PCK(cudaMalloc(&P->neh_d, sizeof(int) * S * (PBB_MAX_N + 1)), "heuristic results");
     PCK(cudaMalloc(&P->neh_tasks_d, sizeof(NehTask) * S), "heuristic tasks");
+    if (P->pair_smem || P->tail_pair_smem) {
+        const size_t w = std::max((size_t)P->grid * P->warps, (size_t)P->tail_grid * P->tail_warps);
+        P->pair_stride = c.max_jobs * P->Ppad_max;
+        if (cudaMalloc(&P->pair_stack, sizeof(int) * w * P->pair_stride) != cudaSuccess) {
+            cudaGetLastError();       // no room: the general build needs none
+            P->pair_stack = nullptr;
+            P->pair_smem = P->tail_pair_smem = 0;
+        }
+    }
     P->arena_bytes = (size_t)c.explorer_bytes;
     const int E = P->epw;
     if (explorer_block_bytes(E, P->npad) > P->arena_bytes)
@@ -316,20 +326,25 @@ int pool_create(const pbb_pool_config* in, pbb_pool* P)
     PCK(cudaMalloc(&P->arena, P->arena_bytes), "explorer memory");
     P->alloc.init(P->arena_bytes);
     P->slots.assign(S, Slot());
-    // the window: explorer kernel and control read-back, as one graph; one
-    // graph per block shape (bulk, tail) and explorer build (the general one,
-    // and the one with boundingMode 2 and MinMin compiled in, used while every
-    // resident instance searches that way)
-    const unsigned long long budget = (unsigned long long)(c.window_s * 1e9);
-    // the tail's windows last at least 20 ms: its few long searches gain
-    // nothing from frequent admissions
-    const unsigned long long tail_budget = std::max(budget, 20000000ull);
-    auto capture = [&](int grid, int warps, int smem, unsigned long long win, int variant,
-                       cudaGraphExec_t* out) -> int {
+    return PBB_OK;
+}
+
+// The window as one graph: explorer kernel and control read-back.  `build`: 0
+// the general explorer, 1 and 2 its variants 3 and 4.
+int window_graph(pbb_pool* P, bool tail, int build, cudaGraphExec_t* out)
+{
+    cudaGraphExec_t& exec = P->window[tail ? 1 : 0][build];
+    if (!exec) {
+        unsigned long long budget = (unsigned long long)(P->cfg.window_s * 1e9);
+        // the tail's windows last at least 20 ms: its few long searches gain
+        // nothing from frequent admissions
+        if (tail) budget = std::max(budget, 20000000ull);
+        const int smem = tail ? (build ? P->tail_pair_smem : P->tail_smem) : (build ? P->pair_smem : P->smem);
         cudaGraph_t graph = nullptr;
         PCK(cudaStreamBeginCapture(P->st, cudaStreamCaptureModeRelaxed), "graph capture");
-        cudaError_t e1 = pbbl::launch_explore(P->nw, P->groups_d, P->ngroups_d, grid, warps, smem, win, INT_MAX, 4096,
-                                              P->st, variant);
+        cudaError_t e1 = pbbl::launch_explore(P->nw, P->groups_d, P->ngroups_d, tail ? P->tail_grid : P->grid,
+                                              tail ? P->tail_warps : P->warps, smem, budget, INT_MAX, 4096, P->st,
+                                              build ? build + 2 : 0, 1, P->pair_stack, P->pair_stride);
         cudaError_t e3 = cudaMemcpyAsync(P->ctl_h, P->ctl, sizeof(GroupCtl) * P->slots.size(),
                                          cudaMemcpyDeviceToHost, P->st);
         cudaError_t e4 = cudaStreamEndCapture(P->st, &graph);
@@ -337,19 +352,14 @@ int pool_create(const pbb_pool_config* in, pbb_pool* P)
             if (graph) cudaGraphDestroy(graph);
             return pfail(PBB_E_CUDA, "capturing a window graph failed");
         }
-        cudaError_t e5 = cudaGraphInstantiate(out, graph, 0);
+        cudaError_t e5 = cudaGraphInstantiate(&exec, graph, 0);
         cudaGraphDestroy(graph);
-        if (e5) return pfail(PBB_E_CUDA, "instantiating a window graph failed");
-        return PBB_OK;
-    };
-    int rc = capture(P->grid, P->warps, P->smem, budget, 0, &P->window);
-    if (!rc && P->masks) rc = capture(P->grid, P->warps, P->smem, budget, 3, &P->window_fixed);
-    if (!rc && P->tail_warps > 0) {
-        rc = capture(P->tail_grid, P->tail_warps, P->tail_smem, tail_budget, 0, &P->window_tail);
-        if (!rc && P->tail_masks)
-            rc = capture(P->tail_grid, P->tail_warps, P->tail_smem, tail_budget, 3, &P->window_tail_fixed);
+        if (e5) {
+            exec = nullptr;
+            return pfail(PBB_E_CUDA, "instantiating a window graph failed");
+        }
     }
-    if (rc) return rc;
+    *out = exec;
     return PBB_OK;
 }
 
@@ -570,13 +580,20 @@ extern "C" int pbb_pool_step(pbb_pool* P, int32_t* resident, int32_t* queued)
             "upload");
     }
     PCK(cudaMemcpyAsync(P->ngroups_d, &nact, sizeof(int), cudaMemcpyHostToDevice, P->st), "upload");
-    bool fixed = true;
-    for (int i = 0; i < nact; i++)
-        fixed = fixed && act[i].search.bound_mode == 2 && act[i].search.branch_mode == 3 && !act[i].search.find_all &&
-                act[i].inst.posj != nullptr;
-    cudaGraphExec_t win = tail ? P->window_tail : P->window;
-    if (fixed && tail && P->window_tail_fixed) win = P->window_tail_fixed;
-    if (fixed && !tail && P->window_fixed) win = P->window_fixed;
+    // kept pair bounds while every resident instance searches in a way they
+    // serve; the default search's build while all of them search that way
+    int build = (tail ? P->tail_pair_smem : P->pair_smem) > 0 ? 1 : 0;
+    for (int i = 0; i < nact; i++) {
+        const DevSearch& q = act[i].search;
+        const int v = pbbl::pairs_variant(q.bound_mode, q.branch_mode, q.find_all, q.sort_nodes);
+        if (v == 0) build = 0;
+        else if (build) build = std::max(build, v - 2);
+    }
+    cudaGraphExec_t win = nullptr;
+    if (nact > 0) {
+        rc = window_graph(P, tail, build, &win);
+        if (rc) return rc;
+    }
     if (nact > 0) PCK(cudaGraphLaunch(win, P->st), "window launch");
     PCK(cudaStreamSynchronize(P->st), "window");
     // retire the finished instances

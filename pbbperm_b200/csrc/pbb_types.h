@@ -74,7 +74,8 @@ struct GroupCtl {
     // work of the Johnson sweeps: nodes swept, free jobs summed over them,
     // children evaluated by them (roofline accounting)
     unsigned long long jsweeps, jfree, jchild;
-    // children bounded by direct scans, and their free jobs summed
+    // children bounded by direct scans, and free jobs summed over the machine
+    // pairs scanned for them
     unsigned long long jdirect, jdirect_free;
 };
 
@@ -154,30 +155,50 @@ struct CtaShare {
 
 // Dynamic shared memory layout of one CTA (host and device agree).
 struct SmemPlan {
-    int je_off, p_off, pm0_off, pm1_off, marr_off, mdep_off, posj_off, share_off, warp_off, warp_bytes, total;
-    int fmask;             // 1: each warp keeps its explorer's free-position masks (explorer only)
+    int je_off, p_off, pre_off, pm_off, marr_off, mdep_off, posj_off, share_off, warp_off, warp_bytes, total;
+    int je_stride;         // entries between rows of the Johnson table
+    int fmask;             // PBB_SCRATCH_*
 };
+
+// Per-warp scratch of the kernels
+#define PBB_SCRATCH_PLAIN 0   // no free-position masks
+#define PBB_SCRATCH_MASKS 1   // with the masks of the explorer the warp holds
+#define PBB_SCRATCH_PAIRS 2   // kept pair bounds (bounding mode 2), no per-child tables
 
 __host__ __device__ inline int pbb_align(int x, int a) { return (x + a - 1) / a * a; }
 
-// per-warp scratch: [fmask: u64 fmask[Ppad]] ints lbF[n] lbB[n] frontZ backZ
-// Fb Bb rem RB FR [32 each]; shorts dF[n*m] dB[n*m]; bytes fjob[n] bjob[n] row[n]
+// Row stride (ints) of the processing times kept job by job in shared memory:
+// machines rounded up to an odd number of 16-byte words, so that the lanes of
+// a warp read four machines of 32 different jobs without bank conflicts.
+__host__ __device__ inline int pbb_machine_pad(int m) { return ((m + 3) / 4 | 1) * 4; }
+
+// per-warp scratch: ints Fb Bb RB FR frontZ backZ rem [32 each], then
+// [fmask: u64 fmask[Ppad]] ints lbF[n] lbB[n]; shorts dF[n*m] dB[n*m]; bytes
+// fjob[n] bjob[n] row[n].  PBB_SCRATCH_PAIRS has, in place of fmask lbF lbB dF
+// dB: ints the child's vectors [128], two pair-bound buffers [Ppad each]
 __host__ __device__ inline int pbb_warp_bytes(int n, int m, int Ppad, int fmask)
 {
+    if (fmask == PBB_SCRATCH_PAIRS) return pbb_align((7 * 32 + 128 + 2 * Ppad) * 4 + 3 * n, 16);
     return pbb_align((fmask ? Ppad * 8 : 0) + (2 * n + 7 * 32) * 4 + 2 * n * m * 2 + 3 * n, 16);
 }
 
+// PBB_SCRATCH_PAIRS keeps no position table, but the prefix sums of the
+// processing times, and an odd row stride of the Johnson entries, so that a
+// warp can read one pair's column as well as 32 pairs' rows.
 __host__ __device__ inline SmemPlan pbb_smem_plan(int n, int m, int Ppad, int warps, int fmask = 0)
 {
+    const bool pairs = fmask == PBB_SCRATCH_PAIRS;
+    const int times = n * pbb_machine_pad(m) * 4;
     SmemPlan s;
     int off = 0;
-    s.je_off = off;   off += n * Ppad * 8;
-    s.p_off = off;    off += pbb_align(m * n * 4, 16);
-    s.pm0_off = off;  off += pbb_align(Ppad, 16);
-    s.pm1_off = off;  off += pbb_align(Ppad, 16);
+    s.je_stride = pairs ? Ppad + 1 : Ppad;
+    s.je_off = off;   off += pbb_align(n * s.je_stride * 8, 16);
+    s.p_off = off;    off += times;
+    s.pre_off = off;  off += pairs ? times : 0;
+    s.pm_off = off;   off += pbb_align(Ppad * 2, 16);
     s.marr_off = off; off += pbb_align(m * 4, 16);
     s.mdep_off = off; off += pbb_align(m * 4, 16);
-    s.posj_off = off; off += pbb_align(n * Ppad, 16);
+    s.posj_off = off; off += pairs ? 0 : pbb_align(n * Ppad, 16);
     s.share_off = off; off += pbb_align((int)sizeof(CtaShare) + 8 * warps, 16);
     s.warp_off = off;
     s.fmask = fmask;
