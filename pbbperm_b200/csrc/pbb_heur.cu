@@ -8,10 +8,15 @@
 // findBestPos restated): with e the heads of the sequence and q its tails,
 // inserting x at position i gives the makespan
 //   max_k ( f_k + q_i,k ),  f_k = max(f_{k-1}, e_{i-1,k}) + p_k(x),
-// exactly the makespan of the sequence with x at i.  Heads and tails are
-// max-plus prefix / suffix scans over the machines (one machine per lane), the
-// insertion costs one position per lane.  Integer only: the result equals the
-// host restatement pbb_neh job for job.
+// exactly the makespan of the sequence with x at i.  Heads and tails run as
+// one diagonal wavefront (one machine per lane), the insertion costs one
+// position per lane.  Integer only: the result equals the host restatement
+// pbb_neh job for job.
+//
+// What bounds these kernels is the serial chain of one instance, not the GPU's
+// throughput: a wavefront step is one shuffle, one max and one add for every
+// machine, where a max-plus scan per job took ten shuffles (NEH of 64
+// instances of 50 x 20, whole call with 0.9 ms of host work: 1.9 -> 1.25 ms).
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <string.h>
@@ -30,100 +35,112 @@ namespace {
 
 __device__ __forceinline__ int hlane() { return threadIdx.x & 31; }
 
-// heads after appending a job with times pu (lane = machine, m lanes used):
-// h_k = max(h_{k-1}, prev_k) + pu_k, h_{-1} = 0
-__device__ __forceinline__ int scan_append(int prev, int pu)
+// Heads of `la` jobs appended to a sequence whose heads are h0 (job r:
+// ahead[r]), and tails of `lb` jobs put before one whose tails are t0 (job r:
+// behind[-r]), lane = machine, as one wavefront; row r of the results at
+// E + r * PBB_HEUR_ROW and Q + r * qstep.  m lanes used.
+__device__ __forceinline__ void wavefront(const int* pt, int mp, int m, int h0, const int* ahead, int la, int* E,
+                                          int t0, const int* behind, int lb, int* Q, int qstep)
 {
     const int lane = hlane();
-    int P = pu;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int t = __shfl_up_sync(HEUR_FULL, P, o);
-        if (lane >= o) P += t;
+    const int steps = max(la, lb) + m - 1;
+    const int back = m - 1 - lane;         // the last machine leads the tails
+    int cf = h0, cb = t0;
+    for (int s = 0; s < steps; s++) {
+        int up = __shfl_up_sync(HEUR_FULL, cf, 1), dn = __shfl_down_sync(HEUR_FULL, cb, 1);
+        if (lane == 0) up = 0;
+        if (lane == m - 1) dn = 0;
+        const int i = s - lane, j = s - back;
+        if (lane < m && i >= 0 && i < la) {
+            cf = max(cf, up) + pt[ahead[i] * mp + lane];
+            E[i * PBB_HEUR_ROW + lane] = cf;
+        }
+        if (lane < m && j >= 0 && j < lb) {
+            cb = max(cb, dn) + pt[behind[-j] * mp + lane];
+            Q[j * qstep + lane] = cb;
+        }
     }
-    int x = prev - (P - pu);
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int t = __shfl_up_sync(HEUR_FULL, x, o);
-        if (lane >= o) x = max(x, t);
-    }
-    return P + max(x, 0);
 }
-
-// tails after putting a job first: t_k = max(t_{k+1}, prev_k) + pu_k, t_m = 0
-// (lanes >= m carry pu = 0 and prev = 0, so they add nothing)
-__device__ __forceinline__ int scan_prepend(int prev, int pu)
-{
-    const int lane = hlane();
-    int Q = pu;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int t = __shfl_down_sync(HEUR_FULL, Q, o);
-        if (lane + o < 32) Q += t;
-    }
-    int x = prev - (Q - pu);
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int t = __shfl_down_sync(HEUR_FULL, x, o);
-        if (lane + o < 32) x = max(x, t);
-    }
-    return Q + max(x, 0);
-}
-
-// makespan of seq[0..len) (lane = machine), read by every lane
-__device__ __forceinline__ int seq_makespan(const int* p, int n, int m, const int* seq, int len)
-{
-    const int lane = hlane();
-    int h = 0;
-    for (int i = 0; i < len; i++) h = scan_append(h, lane < m ? p[lane * n + seq[i]] : 0);
-    return __shfl_sync(HEUR_FULL, h, m - 1);
-}
-
-}  // namespace
-
-namespace {
 
 // Heads E[i] (positions 0..len-1) and tails Q[i] (0..len, Q[len] = 0) of
 // seq[0..len), one machine per lane, stored by position.
-__device__ __forceinline__ void heads_tails(const int* p, int n, int m, const int* seq, int len, int* E, int* Q)
+__device__ __forceinline__ void heads_tails(const int* pt, int mp, int m, const int* seq, int len, int* E, int* Q)
 {
-    const int lane = hlane();
-    int h = 0;
-    for (int i = 0; i < len; i++) {
-        h = scan_append(h, lane < m ? p[lane * n + seq[i]] : 0);
-        E[i * 32 + lane] = h;
-    }
-    int q = 0;
-    Q[len * 32 + lane] = 0;
-    for (int i = len - 1; i >= 0; i--) {
-        q = scan_prepend(q, lane < m ? p[lane * n + seq[i]] : 0);
-        Q[i * 32 + lane] = q;
-    }
+    Q[len * PBB_HEUR_ROW + hlane()] = 0;
+    wavefront(pt, mp, m, 0, seq, len, E, 0, seq + len - 1, len, Q + (len - 1) * PBB_HEUR_ROW, -PBB_HEUR_ROW);
     __syncwarp();
 }
 
-// Makespan of x inserted at the best position in [lo, hi] of the sequence
+// makespan of jobs a then b, read by every lane
+__device__ __forceinline__ int pair_makespan(const int* pt, int mp, int m, int a, int b)
+{
+    int h1 = 0, h2 = 0;
+    for (int k = 0; k < m; k++) {
+        h1 += pt[a * mp + k];
+        h2 = max(h1, h2) + pt[b * mp + k];
+    }
+    return h2;
+}
+
+// makespan of job x between the heads e (NULL: none) and the tails q
+__device__ __forceinline__ int insert_cost(const int* pt, int mp, int m, const int* e, const int* q, int x)
+{
+    const int* px = pt + x * mp;
+    int f = 0, c = 0;
+#pragma unroll 4
+    for (int k = 0; k < m; k++) {
+        f = max(f, e ? e[k] : 0) + px[k];
+        c = max(c, f + q[k]);
+    }
+    return c;
+}
+
+// smallest (makespan << 32) | position over the lanes
+__device__ __forceinline__ unsigned long long least_key(unsigned long long best)
+{
+    const unsigned hi = __reduce_min_sync(HEUR_FULL, (unsigned)(best >> 32));
+    const unsigned lo = __reduce_min_sync(HEUR_FULL, (unsigned)(best >> 32) == hi ? (unsigned)best : 0xffffffffu);
+    return ((unsigned long long)hi << 32) | lo;
+}
+
+// Makespan of x inserted at the best position of the sequence of `len` jobs
 // whose heads and tails are E, Q (fastNEH.cpp:120-178): the first position
 // of least makespan.  Returns (makespan << 32) | position, on every lane.
-__device__ __forceinline__ unsigned long long best_insert(const int* p, int n, int m, const int* E, const int* Q,
-                                                          int x, int lo, int hi)
+__device__ __forceinline__ unsigned long long best_insert(const int* pt, int mp, int m, const int* E, const int* Q,
+                                                          int x, int len)
 {
     unsigned long long best = ~0ull;
-    for (int i = lo + hlane(); i <= hi; i += 32) {
-        int f = 0, c = 0;
-        for (int k = 0; k < m; k++) {
-            f = max(f, i > 0 ? E[(i - 1) * 32 + k] : 0) + p[k * n + x];
-            c = max(c, f + Q[i * 32 + k]);
-        }
+    for (int i = hlane(); i <= len; i += 32) {
+        const int c = insert_cost(pt, mp, m, i > 0 ? E + (i - 1) * PBB_HEUR_ROW : nullptr, Q + i * PBB_HEUR_ROW, x);
         const unsigned long long key = ((unsigned long long)(unsigned)c << 32) | (unsigned)i;
         best = key < best ? key : best;
     }
-#pragma unroll
-    for (int o = 16; o; o >>= 1) {
-        const unsigned long long other = __shfl_xor_sync(HEUR_FULL, best, o);
-        best = other < best ? other : best;
+    return least_key(best);
+}
+
+// The same for the job at position i of the whole sequence seq[0..n), taken
+// out and put back within `reach` places; E, Q: heads and tails of the whole
+// sequence.  Without the job, heads before i and tails behind it stay as they
+// are, so only the rows between i and the reach are computed, into Er and Qr:
+// a probe costs 2 x reach jobs instead of two passes over the sequence.
+__device__ __forceinline__ unsigned long long probe_move(const int* pt, int mp, int n, int m, const int* seq,
+                                                         const int* E, const int* Q, int i, int reach, int* Er, int* Qr)
+{
+    const int lane = hlane();
+    const int lo = max(0, i - reach), hi = min(n - 1, i + reach);
+    const int h0 = i > 0 && lane < m ? E[(i - 1) * PBB_HEUR_ROW + lane] : 0;
+    const int t0 = lane < m ? Q[(i + 1) * PBB_HEUR_ROW + lane] : 0;
+    __syncwarp();
+    wavefront(pt, mp, m, h0, seq + i + 1, hi - i, Er, t0, seq + i - 1, i - lo, Qr, PBB_HEUR_ROW);
+    __syncwarp();
+    unsigned long long best = ~0ull;
+    const int q = lo + lane;               // at most 2 x 8 + 1 positions
+    if (q <= hi) {
+        const int* e = q == 0 ? nullptr : (q - 1 < i ? E + (q - 1) * PBB_HEUR_ROW : Er + (q - 1 - i) * PBB_HEUR_ROW);
+        const int* t = q >= i ? Q + (q + 1) * PBB_HEUR_ROW : Qr + (i - 1 - q) * PBB_HEUR_ROW;
+        best = ((unsigned long long)(unsigned)insert_cost(pt, mp, m, e, t, seq[i]) << 32) | (unsigned)q;
     }
-    return best;
+    return least_key(best);
 }
 
 // seq[0..len) -> seq[0..len] with x at position pos
@@ -164,33 +181,46 @@ __device__ __forceinline__ int remove_at(int* seq, int len, int pos)
 }
 
 struct HeurSmem {
-    int *p, *E, *Q, *seq, *order, *tot, *cur, *best, *vo;
+    int *pt, *E, *Q, *seq, *order, *tot, *cur, *best, *vo, *probe;
+    int mp;                                     // row stride of pt
 };
 
-__device__ __forceinline__ HeurSmem heur_smem(int* hs)
+__device__ __forceinline__ HeurSmem heur_smem(int* hs, int m)
 {
     HeurSmem S;
-    S.p = hs;                                   // [m][n]
-    S.E = S.p + PBB_MAX_N * PBB_MAX_M;          // [PBB_MAX_N][32] heads by position
-    S.Q = S.E + PBB_MAX_N * 32;                 // [PBB_MAX_N + 1][32] tails by position
-    S.seq = S.Q + (PBB_MAX_N + 1) * 32;         // [PBB_MAX_N] each of the following
+    S.pt = hs;                                  // [n][mp]
+    S.E = S.pt + PBB_MAX_N * 36;                // [PBB_MAX_N] rows: heads by position
+    S.Q = S.E + PBB_MAX_N * PBB_HEUR_ROW;       // [PBB_MAX_N + 1] rows: tails by position
+    S.seq = S.Q + (PBB_MAX_N + 1) * PBB_HEUR_ROW;   // [PBB_MAX_N] each of the following
     S.order = S.seq + PBB_MAX_N;
     S.tot = S.order + PBB_MAX_N;
     S.cur = S.tot + PBB_MAX_N;
     S.best = S.cur + PBB_MAX_N;
     S.vo = S.best + PBB_MAX_N;
+    S.probe = S.vo + PBB_MAX_N;                 // iterated greedy: two sets of rows per warp
+    S.mp = pbb_machine_pad(m);
     return S;
+}
+
+// the instance's times, job by job
+__device__ __forceinline__ void load_times(const HeurSmem& S, const int* p, int n, int m)
+{
+    for (int i = threadIdx.x; i < n * m; i += blockDim.x) {
+        const int k = i / n, j = i - k * n;
+        S.pt[j * S.mp + k] = p[i];
+    }
 }
 
 // NEH into S.seq; returns the makespan (every lane)
 __device__ int neh_warp(const HeurSmem& S, int n, int m)
 {
     const int lane = hlane();
-    const int* p = S.p;
+    const int* pt = S.pt;
+    const int mp = S.mp;
     // total time per job, then the jobs by decreasing total (ties: lower id first)
     for (int j = lane; j < n; j += 32) {
         int s = 0;
-        for (int k = 0; k < m; k++) s += p[k * n + j];
+        for (int k = 0; k < m; k++) s += pt[j * mp + k];
         S.tot[j] = s;
     }
     __syncwarp();
@@ -200,31 +230,29 @@ __device__ int neh_warp(const HeurSmem& S, int n, int m)
         S.order[r] = j;
     }
     __syncwarp();
-    int len;
     if (n == 1) {
         if (lane == 0) S.seq[0] = S.order[0];
         __syncwarp();
-        len = 1;
-    } else {
-        // the first two keep the swapped order unless the original one is
-        // strictly better (fastNEH.cpp:233-236)
-        if (lane == 0) { S.seq[0] = S.order[0]; S.seq[1] = S.order[1]; }
-        __syncwarp();
-        const int ca = seq_makespan(p, n, m, S.seq, 2);
-        if (lane == 0) { S.seq[0] = S.order[1]; S.seq[1] = S.order[0]; }
-        __syncwarp();
-        const int cb = seq_makespan(p, n, m, S.seq, 2);
-        if (ca < cb && lane == 0) { S.seq[0] = S.order[0]; S.seq[1] = S.order[1]; }
-        __syncwarp();
-        len = 2;
+        return S.tot[0];
     }
-    for (; len < n; len++) {
+    // the first two keep the swapped order unless the original one is
+    // strictly better (fastNEH.cpp:233-236)
+    const int a = S.order[0], b = S.order[1];
+    const int ca = pair_makespan(pt, mp, m, a, b), cb = pair_makespan(pt, mp, m, b, a);
+    if (lane == 0) {
+        S.seq[0] = ca < cb ? a : b;
+        S.seq[1] = ca < cb ? b : a;
+    }
+    __syncwarp();
+    int cost = min(ca, cb);
+    for (int len = 2; len < n; len++) {
         const int x = S.order[len];
-        heads_tails(p, n, m, S.seq, len, S.E, S.Q);
-        const unsigned long long b = best_insert(p, n, m, S.E, S.Q, x, 0, len);
-        insert_at(S.seq, len, (int)(b & 0xffffffffu), x);
+        heads_tails(pt, mp, m, S.seq, len, S.E, S.Q);
+        const unsigned long long key = best_insert(pt, mp, m, S.E, S.Q, x, len);
+        insert_at(S.seq, len, (int)(key & 0xffffffffu), x);
+        cost = (int)(key >> 32);
     }
-    return seq_makespan(p, n, m, S.seq, n);
+    return cost;
 }
 
 // splitmix64 step (the project's generator), lane 0 only
@@ -253,8 +281,8 @@ __global__ void __launch_bounds__(32) pbb_neh_kernel(const NehTask* tasks, int c
     if (t >= count) return;
     const NehTask T = tasks[t];
     const int n = T.n, m = T.m, lane = hlane();
-    const HeurSmem S = heur_smem(hs);
-    for (int i = lane; i < n * m; i += 32) S.p[i] = T.p[i];
+    const HeurSmem S = heur_smem(hs, m);
+    load_times(S, T.p, n, m);
     __syncwarp();
     const int cost = neh_warp(S, n, m);
     for (int i = lane; i < n; i += 32) T.perm[i] = S.seq[i];
@@ -266,107 +294,142 @@ __global__ void __launch_bounds__(32) pbb_neh_kernel(const NehTask* tasks, int c
 
 // Iterated greedy from the NEH schedule (heuristic/src/IG.cpp:341-416 runIG,
 // destruction :120-160, construction :229-255, localSearchKI :567-612,
-// acceptance :258-274), one warp per task.  Every random decision is drawn by
-// lane 0 from the task's splitmix64 stream (seed + task index), in this
+// acceptance :258-274), one block per task.  Every random decision is drawn by
+// thread 0 from the task's splitmix64 stream (seed + task index), in this
 // order per round: the destruction's window r, its shuffle, then the
 // acceptance draw; a worse schedule is kept with probability T / (T + delta),
 // T = 0.2 x mean processing time / 10 (the reference's temperature, with the
 // exponential replaced by a rational of the same shape so that the test is
 // integer arithmetic).  The host restatement in the test oracle follows the
 // same stream.
-__global__ void __launch_bounds__(32) pbb_ig_kernel(const NehTask* tasks, int count, IgParams prm)
+//
+// The local search takes nearly all of the time: a probe per job, the first
+// improvement taken.  The block's warps probe the next jobs of the visit order
+// at once, and the first in that order that improves is taken, which is the
+// one a single warp would have come to; a pass computes the whole sequence's
+// heads and tails once for all its probes.  64 instances of 50 x 20, five
+// rounds, whole call: 23.7 ms with one warp and two whole passes per probe,
+// 2.4 ms so (NEH alone 1.2); 1500 mixed instances, three rounds: 17 and 7.
+__global__ void __launch_bounds__(32 * PBB_IG_WARPS) pbb_ig_kernel(const NehTask* tasks, int count, IgParams prm)
 {
     extern __shared__ __align__(16) int hs[];
     const int t = blockIdx.x;
     if (t >= count) return;
     const NehTask T = tasks[t];
     const int n = T.n, m = T.m, lane = hlane();
-    const HeurSmem S = heur_smem(hs);
+    const int warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    const HeurSmem S = heur_smem(hs, m);
     __shared__ int removed[PBB_MAX_N];
-    for (int i = lane; i < n * m; i += 32) S.p[i] = T.p[i];
-    __syncwarp();
-    int cur_cost = neh_warp(S, n, m);
+    __shared__ unsigned long long found[PBB_IG_WARPS];
+    __shared__ int sh_cost, sh_accept;
+    load_times(S, T.p, n, m);
+    __syncthreads();
+    if (warp == 0) {
+        const int c = neh_warp(S, n, m);
+        if (lane == 0) sh_cost = c;
+        // visit order: the middle position first, then alternately right and left (IG.cpp:33-45)
+        if (lane == 0) {
+            const int start = n / 2;
+            int ind = 0;
+            for (int i = start; i < n; i++) { S.vo[ind] = i; ind += 2; }
+            ind = 1;
+            for (int i = start - 1; i >= 0; i--) { S.vo[ind] = i; ind += 2; }
+        }
+        __syncwarp();
+        for (int i = lane; i < n; i += 32) { S.cur[i] = S.seq[i]; S.best[i] = S.seq[i]; }
+    }
+    __syncthreads();
+    int cur_cost = sh_cost;
     int best_cost = cur_cost;
     long long sum = 0;
-    for (int i = 0; i < n * m; i++) sum += S.p[i];
+    for (int j = 0; j < n; j++) sum += S.tot[j];                // the jobs' total times, left by NEH
     const long long temp1000 = 20 * sum / ((long long)n * m);   // 1000 x 0.2 x mean / 10
-    for (int i = lane; i < n; i += 32) { S.cur[i] = S.seq[i]; S.best[i] = S.seq[i]; }
-    // visit order: the middle position first, then alternately right and left (IG.cpp:33-45)
-    if (lane == 0) {
-        const int start = n / 2;
-        int ind = 0;
-        for (int i = start; i < n; i++) { S.vo[ind] = i; ind += 2; }
-        ind = 1;
-        for (int i = start - 1; i >= 0; i--) { S.vo[ind] = i; ind += 2; }
-    }
-    __syncwarp();
+    __syncthreads();
     int kmax = 1;
     while ((kmax + 1) * (kmax + 1) <= n) kmax++;   // integer square root
+    int* Er = S.probe + warp * 2 * PBB_HEUR_REACH * PBB_HEUR_ROW;
+    int* Qr = Er + PBB_HEUR_REACH * PBB_HEUR_ROW;
     unsigned long long rs = prm.seed + (unsigned long long)t;
     int perturb = prm.destruct;
     for (int it = 0; it < prm.iterations && n >= 3; it++) {
-        const int d = min(perturb, n - 1);
-        for (int i = lane; i < n; i += 32) S.seq[i] = S.cur[i];
-        __syncwarp();
-        // destruction: d positions from a shuffled prefix of the visit order
-        if (lane == 0) {
-            const int r = rng_range(rs, d, n);
-            for (int i = 0; i < r; i++) S.order[i] = S.vo[i];
-            for (int i = 0; i < r - 1; i++) {
-                const int j = rng_range(rs, i, r - 1);
-                const int tmp = S.order[i]; S.order[i] = S.order[j]; S.order[j] = tmp;
+        if (warp == 0) {
+            const int d = min(perturb, n - 1);
+            for (int i = lane; i < n; i += 32) S.seq[i] = S.cur[i];
+            __syncwarp();
+            // destruction: d positions from a shuffled prefix of the visit order
+            if (lane == 0) {
+                const int r = rng_range(rs, d, n);
+                for (int i = 0; i < r; i++) S.order[i] = S.vo[i];
+                for (int i = 0; i < r - 1; i++) {
+                    const int j = rng_range(rs, i, r - 1);
+                    const int tmp = S.order[i]; S.order[i] = S.order[j]; S.order[j] = tmp;
+                }
+                // remove the chosen positions, highest first, keeping their jobs in draw order
+                for (int i = 0; i < d; i++) removed[i] = S.seq[S.order[i]];
+                for (int i = 0; i < n; i++) S.tot[i] = 0;
+                for (int i = 0; i < d; i++) S.tot[S.order[i]] = 1;
+                int w = 0;
+                for (int i = 0; i < n; i++)
+                    if (!S.tot[i]) S.seq[w++] = S.seq[i];
             }
-            // remove the chosen positions, highest first, keeping their jobs in draw order
-            for (int i = 0; i < d; i++) removed[i] = S.seq[S.order[i]];
-            for (int i = 0; i < n; i++) S.tot[i] = 0;
-            for (int i = 0; i < d; i++) S.tot[S.order[i]] = 1;
-            int w = 0;
-            for (int i = 0; i < n; i++)
-                if (!S.tot[i]) S.seq[w++] = S.seq[i];
+            __syncwarp();
+            // construction: each removed job at its best position
+            int len = n - d, c = 0;
+            for (int i = 0; i < d; i++) {
+                const int x = removed[i];
+                heads_tails(S.pt, S.mp, m, S.seq, len, S.E, S.Q);
+                const unsigned long long key = best_insert(S.pt, S.mp, m, S.E, S.Q, x, len);
+                insert_at(S.seq, len, (int)(key & 0xffffffffu), x);
+                c = (int)(key >> 32);
+                len++;
+            }
+            if (lane == 0) sh_cost = c;
         }
-        __syncwarp();
-        // construction: each removed job at its best position
-        int len = n - d;
-        for (int i = 0; i < d; i++) {
-            const int x = removed[i];
-            heads_tails(S.p, n, m, S.seq, len, S.E, S.Q);
-            const unsigned long long b = best_insert(S.p, n, m, S.E, S.Q, x, 0, len);
-            insert_at(S.seq, len, (int)(b & 0xffffffffu), x);
-            len++;
-        }
+        __syncthreads();
+        int cost = sh_cost;
         // local search: move the job at each visited position to the best
         // place within kmax of it, first improvement, until a pass finds none
-        int cost = seq_makespan(S.p, n, m, S.seq, n);
         for (int pass = 0; pass < prm.ls_passes; pass++) {
-            bool improved = false;
-            for (int j = 0; j < n && !improved; j++) {
-                const int i = S.vo[j];
-                const int x = remove_at(S.seq, n, i);
-                heads_tails(S.p, n, m, S.seq, n - 1, S.E, S.Q);
-                const unsigned long long b =
-                    best_insert(S.p, n, m, S.E, S.Q, x, max(0, i - kmax), min(n - 1, i + kmax));
-                const int c = (int)(b >> 32);
-                if (c < cost) {
-                    insert_at(S.seq, n - 1, (int)(b & 0xffffffffu), x);
-                    cost = c;
-                    improved = true;
-                } else {
-                    insert_at(S.seq, n - 1, i, x);
+            if (warp == 0) heads_tails(S.pt, S.mp, m, S.seq, n, S.E, S.Q);
+            __syncthreads();
+            int taken = -1;
+            unsigned long long key = 0;
+            for (int base = 0; base < n && taken < 0; base += warps) {
+                const int j = base + warp;
+                if (j < n) {
+                    const unsigned long long b =
+                        probe_move(S.pt, S.mp, n, m, S.seq, S.E, S.Q, S.vo[j], kmax, Er, Qr);
+                    if (lane == 0) found[warp] = b;
                 }
+                __syncthreads();
+                for (int w = 0; w < warps && base + w < n && taken < 0; w++) {
+                    if ((int)(found[w] >> 32) < cost) {
+                        taken = base + w;
+                        key = found[w];
+                    }
+                }
+                __syncthreads();
             }
-            if (!improved) break;
+            if (taken < 0) break;
+            cost = (int)(key >> 32);
+            if (warp == 0) {
+                const int i = S.vo[taken];
+                const int x = remove_at(S.seq, n, i);
+                insert_at(S.seq, n - 1, (int)(key & 0xffffffffu), x);
+            }
+            __syncthreads();
         }
         // acceptance: one draw per round; not worse, or u / 2^32 < T / (T + delta)
-        int accept = 0;
-        if (lane == 0) {
+        if (threadIdx.x == 0) {
             const long long delta = (long long)cost - cur_cost;
             const unsigned long long u = rng_next(rs) >> 32;
-            accept = (delta <= 0 ||
-                      u < ((unsigned long long)temp1000 << 32) / (unsigned long long)(temp1000 + 1000 * delta)) ? 1 : 0;
+            sh_accept = (delta <= 0 || u < ((unsigned long long)temp1000 << 32) /
+                                               (unsigned long long)(temp1000 + 1000 * delta)) ? 1 : 0;
         }
-        accept = __shfl_sync(HEUR_FULL, accept, 0);
-        if (accept) {
-            for (int i = lane; i < n; i += 32) S.cur[i] = S.seq[i];
+        __syncthreads();
+        if (sh_accept) {
+            if (warp == 0)
+                for (int i = lane; i < n; i += 32) S.cur[i] = S.seq[i];
             cur_cost = cost;
             perturb = prm.destruct;
         } else {
@@ -374,12 +437,13 @@ __global__ void __launch_bounds__(32) pbb_ig_kernel(const NehTask* tasks, int co
         }
         if (cost < best_cost) {
             best_cost = cost;
-            for (int i = lane; i < n; i += 32) S.best[i] = S.seq[i];
+            if (warp == 0)
+                for (int i = lane; i < n; i += 32) S.best[i] = S.seq[i];
         }
-        __syncwarp();
+        __syncthreads();
     }
-    for (int i = lane; i < n; i += 32) T.perm[i] = S.best[i];
-    if (lane == 0) {
+    for (int i = threadIdx.x; i < n; i += blockDim.x) T.perm[i] = S.best[i];
+    if (threadIdx.x == 0) {
         if (T.cost) *T.cost = best_cost;
         if (T.ub) *T.ub = best_cost;
     }
@@ -398,8 +462,12 @@ cudaError_t launch_neh(const NehTask* tasks_d, int count, cudaStream_t st)
 cudaError_t launch_ig(const NehTask* tasks_d, int count, const IgParams& prm, cudaStream_t st)
 {
     if (count <= 0) return cudaSuccess;
-    cudaFuncSetAttribute(pbb_ig_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PBB_HEUR_SMEM);
-    pbb_ig_kernel<<<count, 32, PBB_HEUR_SMEM, st>>>(tasks_d, count, prm);
+    // eight warps an instance while the GPU holds them all at once; past that
+    // the probes made for nothing would cost other instances their turn
+    const int warps = count <= 512 ? PBB_IG_WARPS : 2;
+    const int smem = PBB_HEUR_SMEM + warps * PBB_IG_WARP_SMEM;
+    cudaFuncSetAttribute(pbb_ig_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    pbb_ig_kernel<<<count, 32 * warps, smem, st>>>(tasks_d, count, prm);
     return cudaGetLastError();
 }
 

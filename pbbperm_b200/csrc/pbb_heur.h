@@ -23,8 +23,16 @@ struct IgParams {
     unsigned long long seed;
 };
 
-// shared memory of one heuristic block: p, heads, tails, and per-job arrays
-#define PBB_HEUR_SMEM (int)(sizeof(int) * (PBB_MAX_N * PBB_MAX_M + PBB_MAX_N * 32 + (PBB_MAX_N + 1) * 32 + 6 * PBB_MAX_N))
+// Row stride of the heads and tails kept by position: with 34 ints neither the
+// wavefront's diagonal stores nor the reads of one machine at many positions
+// meet on a bank more than twice.
+#define PBB_HEUR_ROW 34
+#define PBB_HEUR_REACH 8          // local-search moves reach at most sqrt(64) places
+#define PBB_IG_WARPS 8            // warps of an iterated-greedy block at most
+// shared memory of one heuristic block: p, heads, tails, and per-job arrays;
+// and of each local-search warp: the rows its probe computes anew
+#define PBB_HEUR_SMEM (int)(sizeof(int) * (PBB_MAX_N * 36 + (2 * PBB_MAX_N + 1) * PBB_HEUR_ROW + 6 * PBB_MAX_N))
+#define PBB_IG_WARP_SMEM (int)(sizeof(int) * 2 * PBB_HEUR_REACH * PBB_HEUR_ROW)
 
 namespace pbbl {
 cudaError_t launch_neh(const NehTask* tasks_d, int count, cudaStream_t st);

@@ -86,3 +86,15 @@ def test_device_ig_equals_its_restatement(iterations):
         assert O.eval(perm) == cost
         assert cost <= pb.neh(p)[0]
         assert sorted(perm.tolist()) == list(range(p.shape[1]))
+
+
+@pytest.mark.parametrize("copies", [1, 70])
+def test_device_ig_at_the_edges_of_its_block_shapes(copies):
+    """Sizes at the reach of a probe, one and 32 machines' worth of lanes, and
+    enough instances (8 x 70 > 512) for the narrow blocks."""
+    shapes = [(2, 2), (3, 2), (4, 3), (9, 32), (17, 31), (32, 4), (33, 5), (64, 2)]
+    insts = [synthetic_instance(60 + i, n, m) for _ in range(copies) for i, (n, m) in enumerate(shapes)]
+    got = pb.ig_batch(insts, iterations=4, seed=77)
+    for t in list(range(8)) + list(range(len(insts) - 8, len(insts))):
+        hc, hp = Oracle(insts[t]).ig(4, 77 + t)
+        assert got[t][0] == hc and (got[t][1] == hp).all(), (t, insts[t].shape)
