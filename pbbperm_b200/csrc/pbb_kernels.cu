@@ -1075,8 +1075,9 @@ pbb_explore_kernel(const DevGroup* groups, const int* ngroups_d, int warps_per_c
         if (wait == 2) {
             const int cta = (int)blockIdx.x - G.first_cta;
             const unsigned b = 1u << (cta & 31);
+            // the CTA asks no more in this launch: a donor that has just
+            // claimed this request still has to read which explorer it offers
             if (atomicAnd(G.ivm.ask + (cta >> 5), ~b) & b) atomicSub(&G.ctl->asking, 1);
-            atomicExch(&H->asker, 0);
         }
     }
     __syncwarp();
