@@ -191,8 +191,8 @@ int pbb_get_result(pbb_engine* e, pbb_result* out);
  * for every resident instance inside one launch per window.
  *
  * Instances wait in a FIFO until a slot and enough explorer memory are free
- * (footprint per instance = explorers x (row stride^2 + 5 x row stride + 20
- * + 384 x row stride) bytes, row stride 32 for n <= 32 jobs, else 64).  Each pbb_pool_step
+ * (footprint per instance = explorers x (max_jobs x (row stride + 384) + 5 x
+ * row stride + 20) bytes, row stride 32 for max_jobs <= 32, else 64).  Each pbb_pool_step
  * admits what fits, runs one exploration window of `window_s` device seconds
  * over all resident instances (one captured CUDA graph: explorer kernel,
  * status read-back), and retires the finished ones, whose results

@@ -172,6 +172,21 @@ def _instance(p):
     return inst, p
 
 
+# layout of pbb_instance, filled for many instances at once
+_INSTANCE_DTYPE = np.dtype([("n_jobs", np.int32), ("n_machines", np.int32), ("p", np.uint64)])
+
+
+def _instance_array(instances):
+    """pbb_instance array of a list of (machines x jobs) matrices, and what
+    has to stay alive while it is used."""
+    keep = [np.ascontiguousarray(p, dtype=np.int32) for p in instances]
+    arr = np.empty(len(keep), _INSTANCE_DTYPE)
+    arr["n_jobs"] = [p.shape[1] for p in keep]
+    arr["n_machines"] = [p.shape[0] for p in keep]
+    arr["p"] = [p.__array_interface__["data"][0] for p in keep]
+    return arr.ctypes.data_as(ctypes.POINTER(_Instance)), (keep, arr)
+
+
 class Config:
     """Search settings, named after the reference ini keys."""
 
@@ -448,24 +463,22 @@ def neh_batch(instances, device=0):
     """NEH of many instances on the device (one warp each): list of
     (cost, permutation), equal to neh() for each."""
     cnt = len(instances)
-    keep = [np.ascontiguousarray(p, dtype=np.int32) for p in instances]
-    arr = (_Instance * cnt)(*[_Instance(p.shape[1], p.shape[0], _ptr(p)) for p in keep])
+    arr, keep = _instance_array(instances)
     perms = np.zeros((cnt, MAX_JOBS), np.int32)
     costs = np.zeros(cnt, np.int32)
     _check(lib().pbb_neh_batch(arr, cnt, int(device), _ptr(perms), _ptr(costs)))
-    return [(int(costs[i]), perms[i, :keep[i].shape[1]].copy()) for i in range(cnt)]
+    return [(c, row[:p.shape[1]].copy()) for c, row, p in zip(costs.tolist(), perms, keep[0])]
 
 
 def ig_batch(instances, iterations=100, seed=0, device=0):
     """Seeded iterated greedy from NEH on the device (one warp per instance):
     list of (cost, permutation); instance i draws from seed + i."""
     cnt = len(instances)
-    keep = [np.ascontiguousarray(p, dtype=np.int32) for p in instances]
-    arr = (_Instance * cnt)(*[_Instance(p.shape[1], p.shape[0], _ptr(p)) for p in keep])
+    arr, keep = _instance_array(instances)
     perms = np.zeros((cnt, MAX_JOBS), np.int32)
     costs = np.zeros(cnt, np.int32)
     _check(lib().pbb_ig_batch(arr, cnt, int(device), int(iterations), int(seed), _ptr(perms), _ptr(costs)))
-    return [(int(costs[i]), perms[i, :keep[i].shape[1]].copy()) for i in range(cnt)]
+    return [(c, row[:p.shape[1]].copy()) for c, row, p in zip(costs.tolist(), perms, keep[0])]
 
 
 class PoolConfig:
@@ -549,8 +562,7 @@ class Pool:
 def batch_solve(instances, ubs=None, config=None, pool_config=None):
     """Solve many instances through one resident pool (pbb_batch_solve)."""
     cnt = len(instances)
-    keep = [np.ascontiguousarray(p, dtype=np.int32) for p in instances]
-    arr = (_Instance * cnt)(*[_Instance(p.shape[1], p.shape[0], _ptr(p)) for p in keep])
+    arr, keep = _instance_array(instances)
     cfg = (config or Config())._c()
     u = None if ubs is None else np.ascontiguousarray(ubs, dtype=np.int32)
     res = (_Result * cnt)()

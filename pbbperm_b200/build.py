@@ -17,9 +17,9 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVFLAGS = ARCH + ["-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC"]
 
 LIB_SOURCES = ["pbb_kernels.cu", "pbb_host.cu", "pbb_diag.cu", "pbb_noalloc.cu", "pbb_pool.cu", "pbb_heur.cu",
-               "pbb_ckpt.cu"]
+               "pbb_ckpt.cu", "pbb_mem.cu"]
 LIB_DEPS = LIB_SOURCES + ["pbb_types.h", "pbb_device.cuh", "pbb_launch.h", "pbb_tables.h", "pbb_heur.h",
-                          "pbb_devguard.h"]
+                          "pbb_devguard.h", "pbb_mem.h"]
 HEADERS = ["pbbperm.h", "pbbperm_diag.h"]
 
 

@@ -26,6 +26,7 @@
 #include "pbb_types.h"
 #include "pbb_heur.h"
 #include "pbb_devguard.h"
+#include "pbb_mem.h"
 #include "pbb_tables.h"
 #include "../../include/pbbperm.h"
 
@@ -493,28 +494,28 @@ int heur_batch(const pbb_instance* inst, int32_t count, int32_t device, const Ig
     pbbh::DeviceGuard keep_callers_device;
     if (cudaSetDevice(device) != cudaSuccess) return pbbt::fail(PBB_E_CUDA, "cudaSetDevice failed");
     cudaStream_t st = nullptr;
-    int* buf = nullptr;
-    NehTask* tasks_d = nullptr;
+    if (pbbh::stream_take(&st, device) != cudaSuccess) return pbbt::fail(PBB_E_CUDA, "stream creation failed");
+    unsigned char* d = nullptr;
     int rc = PBB_OK;
     do {
-        if (cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess) {
-            rc = pbbt::fail(PBB_E_CUDA, "stream creation failed");
-            break;
-        }
         const size_t out_words = (size_t)count * (PBB_MAX_JOBS + 1);
-        if (cudaMalloc(&buf, sizeof(int) * (words + out_words)) != cudaSuccess ||
-            cudaMalloc(&tasks_d, sizeof(NehTask) * count) != cudaSuccess) {
+        pbbh::Carver C;
+        const size_t o_tasks = C.take(sizeof(NehTask) * count), o_p = C.take(sizeof(int) * words);
+        const size_t filled = C.bytes;
+        const size_t o_out = C.take(sizeof(int) * out_words);
+        if (pbbh::mem_alloc((void**)&d, C.bytes, device, st) != cudaSuccess) {
             rc = pbbt::fail(PBB_E_NOMEM, "device allocation failed");
             break;
         }
-        std::vector<int> host(words);
-        std::vector<NehTask> tasks(count);
+        std::vector<unsigned char> host(filled);
+        NehTask* tasks = reinterpret_cast<NehTask*>(host.data() + o_tasks);
+        int* times = reinterpret_cast<int*>(host.data() + o_p);
+        int* out = reinterpret_cast<int*>(d + o_out);
         size_t off = 0;
-        int* out = buf + words;
         for (int i = 0; i < count; i++) {
             const int n = inst[i].n_jobs, m = inst[i].n_machines;
-            memcpy(host.data() + off, inst[i].p, sizeof(int) * n * m);
-            tasks[i].p = buf + off;
+            memcpy(times + off, inst[i].p, sizeof(int) * n * m);
+            tasks[i].p = reinterpret_cast<int*>(d + o_p) + off;
             tasks[i].n = n;
             tasks[i].m = m;
             tasks[i].perm = out + (size_t)i * (PBB_MAX_JOBS + 1);
@@ -522,8 +523,8 @@ int heur_batch(const pbb_instance* inst, int32_t count, int32_t device, const Ig
             tasks[i].ub = nullptr;
             off += (size_t)n * m;
         }
-        cudaError_t ce = cudaMemcpyAsync(buf, host.data(), sizeof(int) * words, cudaMemcpyHostToDevice, st);
-        if (!ce) ce = cudaMemcpyAsync(tasks_d, tasks.data(), sizeof(NehTask) * count, cudaMemcpyHostToDevice, st);
+        const NehTask* tasks_d = reinterpret_cast<const NehTask*>(d + o_tasks);
+        cudaError_t ce = cudaMemcpyAsync(d, host.data(), filled, cudaMemcpyHostToDevice, st);
         if (!ce) ce = ig ? pbbl::launch_ig(tasks_d, count, *ig, st) : pbbl::launch_neh(tasks_d, count, st);
         std::vector<int> res(out_words);
         if (!ce) ce = cudaMemcpyAsync(res.data(), out, sizeof(int) * out_words, cudaMemcpyDeviceToHost, st);
@@ -533,14 +534,17 @@ int heur_batch(const pbb_instance* inst, int32_t count, int32_t device, const Ig
             break;
         }
         for (int i = 0; i < count; i++) {
-            for (int j = 0; j < PBB_MAX_JOBS; j++)
-                perms[(size_t)i * PBB_MAX_JOBS + j] = j < inst[i].n_jobs ? res[(size_t)i * (PBB_MAX_JOBS + 1) + j] : 0;
-            costs[i] = res[(size_t)i * (PBB_MAX_JOBS + 1) + PBB_MAX_JOBS];
+            const int* row = res.data() + (size_t)i * (PBB_MAX_JOBS + 1);
+            const int n = inst[i].n_jobs;
+            int32_t* to = perms + (size_t)i * PBB_MAX_JOBS;
+            memcpy(to, row, sizeof(int) * n);
+            memset(to + n, 0, sizeof(int) * (PBB_MAX_JOBS - n));
+            costs[i] = row[PBB_MAX_JOBS];
         }
     } while (0);
-    cudaFree(buf);
-    cudaFree(tasks_d);
-    if (st) cudaStreamDestroy(st);
+    cudaStreamSynchronize(st);
+    pbbh::mem_free(d, st);
+    pbbh::stream_give(st, device);
     return rc;
 }
 

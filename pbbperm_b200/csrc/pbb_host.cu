@@ -16,6 +16,7 @@
 #include "pbb_launch.h"
 #include "pbb_tables.h"
 #include "pbb_heur.h"
+#include "pbb_mem.h"
 #include "../../include/pbbperm.h"
 #include "../../include/pbbperm_diag.h"
 
@@ -44,38 +45,39 @@ int cuda_fail(cudaError_t e, const char* where)
         if (e_ != cudaSuccess) return cuda_fail(e_, #call); \
     } while (0)
 
-struct DeviceInstance {
-    int* p = nullptr;
-    unsigned long long* je = nullptr;
-    unsigned char* pm = nullptr;
-    unsigned char* posj = nullptr;
-    int* mt = nullptr;
-    DevInstance view{};
-
-    int upload(const HostTables& H, cudaStream_t st)
+// An instance's tables as one block, laid out on the host and uploaded by one
+// copy.
+struct InstanceBlock {
+    size_t je, posj, p, pm, mt;       // offsets
+    explicit InstanceBlock(const HostTables& H, pbbh::Carver& C)
     {
-        CK(cudaMalloc(&p, sizeof(int) * H.n * H.m));
-        CK(cudaMalloc(&je, sizeof(unsigned long long) * H.je.size()));
-        CK(cudaMalloc(&pm, 2 * H.Ppad));
-        CK(cudaMalloc(&posj, H.posj.size()));
-        CK(cudaMalloc(&mt, sizeof(int) * 2 * H.m));
-        CK(cudaMemcpyAsync(p, H.p.data(), sizeof(int) * H.n * H.m, cudaMemcpyHostToDevice, st));
-        CK(cudaMemcpyAsync(je, H.je.data(), sizeof(unsigned long long) * H.je.size(), cudaMemcpyHostToDevice, st));
-        CK(cudaMemcpyAsync(pm, H.pm0.data(), H.Ppad, cudaMemcpyHostToDevice, st));
-        CK(cudaMemcpyAsync(posj, H.posj.data(), H.posj.size(), cudaMemcpyHostToDevice, st));
-        CK(cudaMemcpyAsync(pm + H.Ppad, H.pm1.data(), H.Ppad, cudaMemcpyHostToDevice, st));
-        CK(cudaMemcpyAsync(mt, H.min_arr.data(), sizeof(int) * H.m, cudaMemcpyHostToDevice, st));
-        CK(cudaMemcpyAsync(mt + H.m, H.min_dep.data(), sizeof(int) * H.m, cudaMemcpyHostToDevice, st));
-        view.n = H.n; view.m = H.m; view.P = H.P; view.Ppad = H.Ppad;
-        view.p = p; view.je = je; view.pm0 = pm; view.pm1 = pm + H.Ppad;
-        view.min_arr = mt; view.min_dep = mt + H.m;
-        view.posj = posj;
-        return PBB_OK;
+        je = C.take(sizeof(unsigned long long) * H.je.size());
+        posj = C.take(H.posj.size());
+        p = C.take(sizeof(int) * H.n * H.m);
+        pm = C.take(2 * H.Ppad);
+        mt = C.take(sizeof(int) * 2 * H.m);
     }
-    void release()
+    void fill(const HostTables& H, unsigned char* host) const
     {
-        cudaFree(p); cudaFree(je); cudaFree(pm); cudaFree(mt); cudaFree(posj);
-        p = nullptr; je = nullptr; pm = nullptr; mt = nullptr; posj = nullptr;
+        memcpy(host + je, H.je.data(), sizeof(unsigned long long) * H.je.size());
+        memcpy(host + posj, H.posj.data(), H.posj.size());
+        memcpy(host + p, H.p.data(), sizeof(int) * H.n * H.m);
+        memcpy(host + pm, H.pm0.data(), H.Ppad);
+        memcpy(host + pm + H.Ppad, H.pm1.data(), H.Ppad);
+        memcpy(host + mt, H.min_arr.data(), sizeof(int) * H.m);
+        memcpy(host + mt + sizeof(int) * H.m, H.min_dep.data(), sizeof(int) * H.m);
+    }
+    DevInstance view(const HostTables& H, unsigned char* dev) const
+    {
+        DevInstance v{};
+        v.n = H.n; v.m = H.m; v.P = H.P; v.Ppad = H.Ppad;
+        v.je = reinterpret_cast<const unsigned long long*>(dev + je);
+        v.posj = dev + posj;
+        v.p = reinterpret_cast<const int*>(dev + p);
+        v.pm0 = dev + pm; v.pm1 = dev + pm + H.Ppad;
+        v.min_arr = reinterpret_cast<const int*>(dev + mt);
+        v.min_dep = v.min_arr + H.m;
+        return v;
     }
 };
 
@@ -133,12 +135,11 @@ struct pbb_engine {
     // the launch with kept pair bounds (explorer variants 3 and 4), pair_warps 0: not used
     int pair_variant = 0, pair_warps = 0, pair_smem = 0, pair_stride = 0;
     int* pair_stack = nullptr;
-    DeviceInstance di;
-    signed char *mat = nullptr, *vec = nullptr, *bestperm = nullptr;
-    int* path = nullptr;   // per explorer and level: heads, tails, free loads
-    int *line = nullptr, *state = nullptr, *bestcost = nullptr, *askid = nullptr, *ub_d = nullptr, *root_d = nullptr;
+    unsigned char* block = nullptr;   // everything below but the pair bounds and samples
+    int npad = 32;                    // row stride
+    signed char* bestperm = nullptr;
+    int *state = nullptr, *ub_d = nullptr, *root_d = nullptr;
     int* ival_d = nullptr;   // [2][64] interval start / end vectors
-    unsigned* ask = nullptr;
     GroupCtl* ctl = nullptr;
     DevGroup* group_d = nullptr;
     int* ngroups_d = nullptr;     // device copy of the group count (1)
@@ -180,15 +181,16 @@ int wait_event(cudaEvent_t ev, double limit_s)
         return PBB_OK;
     }
     const auto t0 = std::chrono::steady_clock::now();
-    unsigned sleep_us = 20;
     while (true) {
         const cudaError_t q = cudaEventQuery(ev);
         if (q == cudaSuccess) return PBB_OK;
         if (q != cudaErrorNotReady) return cuda_fail(q, "exploration window");
         const double el = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
         if (el > limit_s) return PBB_E_TIMEOUT;
-        std::this_thread::sleep_for(std::chrono::microseconds(sleep_us));
-        sleep_us = std::min(2 * sleep_us, 500u);
+        // small searches end within a fraction of a millisecond; later on the
+        // pause is a sixteenth of the time waited
+        if (el < 5e-4) std::this_thread::yield();
+        else std::this_thread::sleep_for(std::chrono::microseconds((int)std::min(el * 1e6 / 16, 500.0)));
     }
 }
 
@@ -284,19 +286,13 @@ int pbb_engine_destroy(pbb_engine* e)
     pbbh::DeviceGuard keep_callers_device;
     cudaSetDevice(e->dev);
     if (e->st) cudaStreamSynchronize(e->st);
-    e->di.release();
-    cudaFree(e->mat); cudaFree(e->vec); cudaFree(e->bestperm); cudaFree(e->path);
-    cudaFree(e->pair_stack);
-    cudaFree(e->line); cudaFree(e->state); cudaFree(e->bestcost); cudaFree(e->askid); cudaFree(e->ask);
-    cudaFree(e->ub_d); cudaFree(e->root_d); cudaFree(e->ival_d); cudaFree(e->ctl); cudaFree(e->group_d);
-    cudaFree(e->ngroups_d);
+    pbbh::mem_free(e->block, e->st);
+    pbbh::mem_free(e->pair_stack, e->st);
     cudaFree(e->sample_d);
     cudaFree(e->sample_rec);
-    cudaFree(e->neh_d);
-    cudaFree(e->neh_task_d);
     if (e->ev0) cudaEventDestroy(e->ev0);
     if (e->ev1) cudaEventDestroy(e->ev1);
-    if (e->st) cudaStreamDestroy(e->st);
+    pbbh::stream_give(e->st, e->dev);
     delete e;
     return PBB_OK;
 }
@@ -311,7 +307,7 @@ static int engine_create(const pbb_instance* inst, const pbb_config* cfg, pbb_en
     e->dev = cfg->device;
     pbbh::DeviceGuard keep_callers_device;
     CK(cudaSetDevice(e->dev));
-    CK(cudaStreamCreateWithFlags(&e->st, cudaStreamNonBlocking));
+    CK(pbbh::stream_take(&e->st, e->dev));
     CK(cudaEventCreate(&e->ev0));
     CK(cudaEventCreate(&e->ev1));
     const HostTables& H = e->H;
@@ -332,50 +328,42 @@ static int engine_create(const pbb_instance* inst, const pbb_config* cfg, pbb_en
         e->pair_smem = pbbl::smem_bytes(H.n, H.m, H.Ppad, w, PBB_SCRATCH_PAIRS);
         e->pair_stride = H.n * H.Ppad;
         if (e->pair_smem <= cap) {
-            if (cudaMalloc(&e->pair_stack, sizeof(int) * (size_t)e->ctas * w * e->pair_stride) == cudaSuccess)
+            if (pbbh::mem_alloc((void**)&e->pair_stack, sizeof(int) * (size_t)e->ctas * w * e->pair_stride, e->dev,
+                                e->st) == cudaSuccess)
                 e->pair_warps = w;
             else
                 cudaGetLastError();   // no room: the general build needs none
         }
     }
-    rc = e->di.upload(H, e->st);
-    if (rc) return rc;
-    const int B = cfg->nb_ivms;
-    const int npad = PBB_MAX_N;
-    CK(cudaMalloc(&e->mat, (size_t)B * npad * npad));
-    CK(cudaMalloc(&e->vec, (size_t)B * npad * 4));
-    CK(cudaMalloc(&e->path, (size_t)B * npad * PBB_PATH_INTS * sizeof(int)));
-    CK(cudaMalloc(&e->bestperm, (size_t)B * npad));
-    CK(cudaMalloc(&e->line, sizeof(int) * B));
-    CK(cudaMalloc(&e->state, sizeof(int) * B));
-    CK(cudaMalloc(&e->bestcost, sizeof(int) * B));
-    CK(cudaMalloc(&e->askid, sizeof(int) * B));
-    CK(cudaMalloc(&e->ask, sizeof(unsigned) * B));
-    CK(cudaMalloc(&e->ub_d, sizeof(int)));
-    CK(cudaMalloc(&e->root_d, sizeof(int) * PBB_MAX_N));
-    CK(cudaMalloc(&e->neh_d, sizeof(int) * (PBB_MAX_N + 1)));
-    CK(cudaMalloc(&e->neh_task_d, sizeof(NehTask)));
-    {
-        NehTask t;
-        t.p = e->di.p;
-        t.n = H.n;
-        t.m = H.m;
-        t.perm = e->neh_d;
-        t.cost = e->neh_d + PBB_MAX_N;
-        t.ub = e->ub_d;
-        CK(cudaMemcpyAsync(e->neh_task_d, &t, sizeof(t), cudaMemcpyHostToDevice, e->st));
-    }
-    CK(cudaMalloc(&e->ival_d, sizeof(int) * 2 * PBB_MAX_N));
-    CK(cudaMalloc(&e->ctl, sizeof(GroupCtl)));
-    CK(cudaMalloc(&e->group_d, sizeof(DevGroup)));
-    CK(cudaMalloc(&e->ngroups_d, sizeof(int)));
-    {
-        const int one = 1;
-        CK(cudaMemcpyAsync(e->ngroups_d, &one, sizeof(int), cudaMemcpyHostToDevice, e->st));
-    }
-    CK(cudaMemsetAsync(e->mat, 0, (size_t)B * npad * npad, e->st));
+    // one block: what the host fills first (one upload), then the explorers
+    const size_t B = (size_t)cfg->nb_ivms;
+    const size_t npad = e->npad = 32 * e->nw, levels = H.n;
+    pbbh::Carver C;
+    const InstanceBlock tables(H, C);
+    const size_t o_group = C.take(sizeof(DevGroup)), o_one = C.take(sizeof(int)), o_task = C.take(sizeof(NehTask));
+    const size_t filled = C.bytes;
+    const size_t o_ub = C.take(sizeof(int)), o_root = C.take(sizeof(int) * PBB_MAX_N);
+    const size_t o_ival = C.take(sizeof(int) * 2 * PBB_MAX_N), o_neh = C.take(sizeof(int) * (PBB_MAX_N + 1));
+    const size_t o_ctl = C.take(sizeof(GroupCtl));
+    const size_t o_line = C.take(sizeof(int) * B), o_state = C.take(sizeof(int) * B);
+    const size_t o_cost = C.take(sizeof(int) * B), o_askid = C.take(sizeof(int) * B);
+    const size_t o_ask = C.take(sizeof(unsigned) * ((B + 31) / 32));
+    const size_t o_vec = C.take(4 * B * npad), o_perm = C.take(B * npad);
+    const size_t o_mat = C.take(B * levels * npad), o_path = C.take(B * levels * PBB_PATH_INTS * sizeof(int));
+    CK(pbbh::mem_alloc((void**)&e->block, C.bytes, e->dev, e->st));
+    unsigned char* d = e->block;
+    e->ub_d = reinterpret_cast<int*>(d + o_ub);
+    e->root_d = reinterpret_cast<int*>(d + o_root);
+    e->ival_d = reinterpret_cast<int*>(d + o_ival);
+    e->neh_d = reinterpret_cast<int*>(d + o_neh);
+    e->neh_task_d = reinterpret_cast<NehTask*>(d + o_task);
+    e->ctl = reinterpret_cast<GroupCtl*>(d + o_ctl);
+    e->group_d = reinterpret_cast<DevGroup*>(d + o_group);
+    e->ngroups_d = reinterpret_cast<int*>(d + o_one);
+    e->state = reinterpret_cast<int*>(d + o_state);
+    e->bestperm = reinterpret_cast<signed char*>(d + o_perm);
     DevGroup& g = e->group;
-    g.inst = e->di.view;
+    g.inst = tables.view(H, d);
     g.search.bound_mode = cfg->bounding_mode;
     g.search.branch_mode = cfg->branching_mode;
     g.search.find_all = cfg->find_all ? 1 : 0;
@@ -386,24 +374,39 @@ static int engine_create(const pbb_instance* inst, const pbb_config* cfg, pbb_en
     g.search.split_narrow = cfg->split_depth > 0 ? cfg->split_depth : PBB_SPLIT_NARROW;
     g.search.share_after = cfg->share_after > 0 ? cfg->share_after : (cfg->share_after < 0 ? 0 : PBB_SHARE_AFTER);
     g.search.early_stop = cfg->early_stop_johnson ? 1 : 0;
-    g.ivm.count = B;
-    g.ivm.npad = npad;
-    g.ivm.mat = e->mat;
-    g.ivm.pos = e->vec;
-    g.ivm.end = e->vec + (size_t)B * npad;
-    g.ivm.dir = e->vec + (size_t)2 * B * npad;
-    g.ivm.pj = e->vec + (size_t)3 * B * npad;
-    g.ivm.line = e->line;
+    g.ivm.count = cfg->nb_ivms;
+    g.ivm.npad = e->npad;
+    g.ivm.levels = H.n;
+    g.ivm.mat = reinterpret_cast<signed char*>(d + o_mat);
+    g.ivm.pos = reinterpret_cast<signed char*>(d + o_vec);
+    g.ivm.end = g.ivm.pos + B * npad;
+    g.ivm.dir = g.ivm.end + B * npad;
+    g.ivm.pj = g.ivm.dir + B * npad;
+    g.ivm.line = reinterpret_cast<int*>(d + o_line);
     g.ivm.state = e->state;
-    g.ivm.bestcost = e->bestcost;
+    g.ivm.bestcost = reinterpret_cast<int*>(d + o_cost);
     g.ivm.bestperm = e->bestperm;
-    g.ivm.ask = e->ask;
-    g.ivm.askid = e->askid;
-    g.ivm.path = e->path;
+    g.ivm.ask = reinterpret_cast<unsigned*>(d + o_ask);
+    g.ivm.askid = reinterpret_cast<int*>(d + o_askid);
+    g.ivm.path = reinterpret_cast<int*>(d + o_path);
     g.ctl = e->ctl;
     g.first_cta = 0;
     g.ctas = e->ctas;
-    CK(cudaMemcpyAsync(e->group_d, &g, sizeof(DevGroup), cudaMemcpyHostToDevice, e->st));
+    g.sample = nullptr;
+    NehTask t;
+    t.p = g.inst.p;
+    t.n = H.n;
+    t.m = H.m;
+    t.perm = e->neh_d;
+    t.cost = e->neh_d + PBB_MAX_N;
+    t.ub = e->ub_d;
+    const int one = 1;
+    std::vector<unsigned char> host(filled);
+    tables.fill(H, host.data());
+    memcpy(host.data() + o_group, &g, sizeof(g));
+    memcpy(host.data() + o_one, &one, sizeof(one));
+    memcpy(host.data() + o_task, &t, sizeof(t));
+    CK(cudaMemcpyAsync(d, host.data(), filled, cudaMemcpyHostToDevice, e->st));
     CK(cudaStreamSynchronize(e->st));
     return PBB_OK;
 }
@@ -514,11 +517,11 @@ int pbb_init_from_fac(pbb_engine* e, int32_t ub, const int32_t* root_perm, int32
             iv[(size_t)(2 * k + 1) * PBB_MAX_N + i] = q;
         }
     }
+    const size_t iv_bytes = sizeof(int) * iv.size(), id_bytes = sizeof(int) * nb_intervals;
     int* ival_d = nullptr;
-    int* ids_d = nullptr;
-    CK(cudaMalloc(&ival_d, sizeof(int) * iv.size()));
-    cudaError_t err = cudaMalloc(&ids_d, sizeof(int) * nb_intervals);
-    if (!err) err = cudaMemcpyAsync(ival_d, iv.data(), sizeof(int) * iv.size(), cudaMemcpyHostToDevice, e->st);
+    CK(pbbh::mem_alloc((void**)&ival_d, iv_bytes + id_bytes, e->dev, e->st));
+    int* ids_d = ival_d + iv.size();
+    cudaError_t err = cudaMemcpyAsync(ival_d, iv.data(), iv_bytes, cudaMemcpyHostToDevice, e->st);
     if (!err) err = cudaMemcpyAsync(ids_d, id.data(), sizeof(int) * nb_intervals, cudaMemcpyHostToDevice, e->st);
     if (!err) err = cudaMemcpyAsync(e->ub_d, &ub, sizeof(int), cudaMemcpyHostToDevice, e->st);
     if (!err && ub == PBB_UB_NEH) err = pbbl::launch_neh(e->neh_task_d, 1, e->st);
@@ -529,8 +532,7 @@ int pbb_init_from_fac(pbb_engine* e, int32_t ub, const int32_t* root_perm, int32
                                 nb_intervals, ids_d);
     if (!err) err = cudaStreamSynchronize(e->st);
     if (!err) e->pending = false;
-    cudaFree(ival_d);
-    cudaFree(ids_d);
+    pbbh::mem_free(ival_d, e->st);
     if (err) return fail(PBB_E_CUDA, std::string("init_from_fac: ") + cudaGetErrorString(err));
     GroupCtl c;
     CK(cudaMemcpy(&c, e->ctl, sizeof(c), cudaMemcpyDeviceToHost));
@@ -557,9 +559,9 @@ int pbb_get_intervals(pbb_engine* e, int32_t max_intervals, int32_t* pos, int32_
         if (rs) return rs;
     }
     CK(cudaStreamSynchronize(e->st));
-    const int B = e->cfg.nb_ivms, n = e->H.n;
+    const int B = e->cfg.nb_ivms, n = e->H.n, npad = e->npad;
     std::vector<int> st(B);
-    std::vector<signed char> ps((size_t)B * PBB_MAX_N), es((size_t)B * PBB_MAX_N);
+    std::vector<signed char> ps((size_t)B * npad), es((size_t)B * npad);
     CK(cudaMemcpy(st.data(), e->state, sizeof(int) * B, cudaMemcpyDeviceToHost));
     CK(cudaMemcpy(ps.data(), e->group.ivm.pos, ps.size(), cudaMemcpyDeviceToHost));
     CK(cudaMemcpy(es.data(), e->group.ivm.end, es.size(), cudaMemcpyDeviceToHost));
@@ -574,8 +576,8 @@ int pbb_get_intervals(pbb_engine* e, int32_t max_intervals, int32_t* pos, int32_
         int* a = &pv[(size_t)k * n];
         int* z = &ev[(size_t)k * n];
         for (int i = 0; i < n; i++) {
-            a[i] = ps[(size_t)k * PBB_MAX_N + i];
-            z[i] = es[(size_t)k * PBB_MAX_N + i];
+            a[i] = ps[(size_t)k * npad + i];
+            z[i] = es[(size_t)k * npad + i];
         }
         for (int l = n - 1; l > 0; l--)
             if (a[l] >= n - l) { a[l] = 0; a[l - 1]++; }
@@ -767,7 +769,7 @@ int pbb_get_result(pbb_engine* e, pbb_result* out)
         const unsigned id = (unsigned)(c.best_key & 0xffffffffull);
         if (id >= (unsigned)e->cfg.nb_ivms) return fail(PBB_E_CUDA, "corrupt best key");
         signed char buf[PBB_MAX_N];
-        CK(cudaMemcpy(buf, e->bestperm + (size_t)id * PBB_MAX_N, PBB_MAX_N, cudaMemcpyDeviceToHost));
+        CK(cudaMemcpy(buf, e->bestperm + (size_t)id * e->npad, e->H.n, cudaMemcpyDeviceToHost));
         for (int i = 0; i < e->H.n; i++) out->perm[i] = buf[i];
         out->has_perm = 1;
     } else if (e->from_neh && out->cost == e->ub) {
@@ -851,46 +853,52 @@ static int bound_children_impl(const pbb_instance* inst, int32_t johnson_mode, i
     const int n = H.n;
     for (int i = 0; i < count; i++) {
         if (limit1[i] < -1 || limit2[i] > n || limit1[i] >= limit2[i]) return fail(PBB_E_INVAL, "bad limits");
-        std::vector<int> seen(n, 0);
+        unsigned long long seen = 0ull;
         for (int t = 0; t < n; t++) {
             const int j = sched[(size_t)i * n + t];
-            if (j < 0 || j >= n || seen[j]) return fail(PBB_E_INVAL, "schedule is not a permutation");
-            seen[j] = 1;
+            if (j < 0 || j >= n || ((seen >> j) & 1ull)) return fail(PBB_E_INVAL, "schedule is not a permutation");
+            seen |= 1ull << j;
         }
     }
     pbbh::DeviceGuard keep_callers_device;
     CK(cudaSetDevice(device));
-    cudaStream_t st;
-    CK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
-    DeviceInstance di;
-    rc = di.upload(H, st);
-    int* buf = nullptr;
-    unsigned* status = nullptr;
-    const size_t cn = (size_t)count * n;
+    cudaStream_t st = nullptr;
+    CK(pbbh::stream_take(&st, device));
+    const size_t cn = (size_t)count * n * sizeof(int), c1 = (size_t)count * sizeof(int);
     const bool want_prio = prio_begin || prio_end;
-    const size_t words = cn * 5 + (size_t)count * 4 + (want_prio ? 2 * cn : 0) + (strong_idle ? count : 0);
+    // one block: tables, status and inputs, then the outputs.  Up to
+    // PACKED_BYTES of inputs go up in one copy with the tables, and as many of
+    // outputs come back in one.
+    const size_t PACKED_BYTES = 256 * 1024;
+    pbbh::Carver C;
+    const InstanceBlock tables(H, C);
+    const size_t o_status = C.take(sizeof(unsigned));
+    const size_t o_tables_end = C.bytes;
+    const size_t o_s = C.take(cn), o_l1 = C.take(c1), o_l2 = C.take(c1);
+    const size_t o_inputs_end = C.bytes;
+    struct Out { int32_t* host; size_t off, bytes; };
+    Out out[9] = {{weak_begin, 0, cn}, {weak_end, 0, cn}, {strong_begin, 0, cn}, {strong_end, 0, cn},
+                  {node_weak, 0, c1}, {node_strong, 0, c1}, {prio_begin, 0, cn}, {prio_end, 0, cn},
+                  {strong_idle, 0, c1}};
+    for (int q = 0; q < 9; q++)
+        if (q < 6 || (q < 8 && want_prio) || (q == 8 && strong_idle)) out[q].off = C.take(out[q].bytes);
+    unsigned char* d = nullptr;
     do {
-        if (rc) break;
-        cudaError_t ce = cudaMalloc(&buf, sizeof(int) * words);
-        if (ce == cudaSuccess) ce = cudaMalloc(&status, sizeof(unsigned));
+        cudaError_t ce = pbbh::mem_alloc((void**)&d, C.bytes, device, st);
         if (ce != cudaSuccess) { rc = cuda_fail(ce, "cudaMalloc"); break; }
-        int* d_s = buf;
-        int* d_wb = d_s + cn;
-        int* d_we = d_wb + cn;
-        int* d_sb = d_we + cn;
-        int* d_se = d_sb + cn;
-        int* d_l1 = d_se + cn;
-        int* d_l2 = d_l1 + count;
-        int* d_nw = d_l2 + count;
-        int* d_ns = d_nw + count;
-        BoundExtra X;
-        int* tail = d_ns + count;
-        if (want_prio) { X.prio_begin = tail; X.prio_end = tail + cn; tail += 2 * cn; }
-        if (strong_idle) X.strong_idle = tail;
-        cudaMemcpyAsync(d_s, sched, sizeof(int) * cn, cudaMemcpyHostToDevice, st);
-        cudaMemcpyAsync(d_l1, limit1, sizeof(int) * count, cudaMemcpyHostToDevice, st);
-        cudaMemcpyAsync(d_l2, limit2, sizeof(int) * count, cudaMemcpyHostToDevice, st);
-        cudaMemsetAsync(status, 0, sizeof(unsigned), st);
+        const bool packed_in = o_inputs_end - o_tables_end <= PACKED_BYTES;
+        std::vector<unsigned char> host(packed_in ? o_inputs_end : o_tables_end, 0);
+        tables.fill(H, host.data());
+        if (packed_in) {
+            memcpy(host.data() + o_s, sched, cn);
+            memcpy(host.data() + o_l1, limit1, c1);
+            memcpy(host.data() + o_l2, limit2, c1);
+        } else {
+            cudaMemcpyAsync(d + o_s, sched, cn, cudaMemcpyHostToDevice, st);
+            cudaMemcpyAsync(d + o_l1, limit1, c1, cudaMemcpyHostToDevice, st);
+            cudaMemcpyAsync(d + o_l2, limit2, c1, cudaMemcpyHostToDevice, st);
+        }
+        cudaMemcpyAsync(d, host.data(), host.size(), cudaMemcpyHostToDevice, st);
         int smem = 0;
         const int warps = pick_warps(H, 8, device, smem);
         if (warps < 1) { rc = fail(PBB_E_INVAL, "instance tables do not fit in shared memory"); break; }
@@ -898,28 +906,35 @@ static int bound_children_impl(const pbb_instance* inst, int32_t johnson_mode, i
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
         int ctas = (count + warps - 1) / warps;
         ctas = std::min(ctas, sms * 4);
-        ce = pbbl::launch_bound(n <= 32 ? 1 : 2, di.view, count, d_s, d_l1, d_l2, d_wb, d_we, d_sb, d_se, d_nw, d_ns,
-                                status, ctas, warps, smem, st, method, X);
+        auto dev = [&](size_t off) { return reinterpret_cast<int*>(d + off); };
+        BoundExtra X;
+        if (want_prio) { X.prio_begin = dev(out[6].off); X.prio_end = dev(out[7].off); }
+        if (strong_idle) X.strong_idle = dev(out[8].off);
+        unsigned* status = reinterpret_cast<unsigned*>(d + o_status);
+        ce = pbbl::launch_bound(n <= 32 ? 1 : 2, tables.view(H, d), count, dev(o_s), dev(o_l1), dev(o_l2),
+                                dev(out[0].off), dev(out[1].off), dev(out[2].off), dev(out[3].off), dev(out[4].off),
+                                dev(out[5].off), status, ctas, warps, smem, st, method, X);
         if (ce != cudaSuccess) { rc = cuda_fail(ce, "pbb_bound_kernel launch"); break; }
-        if (weak_begin) cudaMemcpyAsync(weak_begin, d_wb, sizeof(int) * cn, cudaMemcpyDeviceToHost, st);
-        if (weak_end) cudaMemcpyAsync(weak_end, d_we, sizeof(int) * cn, cudaMemcpyDeviceToHost, st);
-        if (strong_begin) cudaMemcpyAsync(strong_begin, d_sb, sizeof(int) * cn, cudaMemcpyDeviceToHost, st);
-        if (strong_end) cudaMemcpyAsync(strong_end, d_se, sizeof(int) * cn, cudaMemcpyDeviceToHost, st);
-        if (node_weak) cudaMemcpyAsync(node_weak, d_nw, sizeof(int) * count, cudaMemcpyDeviceToHost, st);
-        if (node_strong) cudaMemcpyAsync(node_strong, d_ns, sizeof(int) * count, cudaMemcpyDeviceToHost, st);
-        if (prio_begin) cudaMemcpyAsync(prio_begin, X.prio_begin, sizeof(int) * cn, cudaMemcpyDeviceToHost, st);
-        if (prio_end) cudaMemcpyAsync(prio_end, X.prio_end, sizeof(int) * cn, cudaMemcpyDeviceToHost, st);
-        if (strong_idle) cudaMemcpyAsync(strong_idle, X.strong_idle, sizeof(int) * count, cudaMemcpyDeviceToHost, st);
         unsigned hs = 0;
         cudaMemcpyAsync(&hs, status, sizeof(unsigned), cudaMemcpyDeviceToHost, st);
+        const size_t back = C.bytes - o_inputs_end;
+        std::vector<unsigned char> packed(back <= PACKED_BYTES ? back : 0);
+        if (!packed.empty()) {
+            cudaMemcpyAsync(packed.data(), d + o_inputs_end, back, cudaMemcpyDeviceToHost, st);
+        } else {
+            for (const Out& o : out)
+                if (o.host && o.off) cudaMemcpyAsync(o.host, d + o.off, o.bytes, cudaMemcpyDeviceToHost, st);
+        }
         ce = cudaStreamSynchronize(st);
         if (ce != cudaSuccess) { rc = cuda_fail(ce, "pbb_bound_kernel"); break; }
-        if (hs & PBB_ST_BADINPUT) rc = fail(PBB_E_INVAL, "device rejected a node");
+        if (hs & PBB_ST_BADINPUT) { rc = fail(PBB_E_INVAL, "device rejected a node"); break; }
+        if (!packed.empty())
+            for (const Out& o : out)
+                if (o.host && o.off) memcpy(o.host, packed.data() + (o.off - o_inputs_end), o.bytes);
     } while (0);
-    cudaFree(buf);
-    cudaFree(status);
-    di.release();
-    cudaStreamDestroy(st);
+    cudaStreamSynchronize(st);
+    pbbh::mem_free(d, st);
+    pbbh::stream_give(st, device);
     return rc;
 }
 

@@ -111,7 +111,7 @@ struct Ivm {
 
 __device__ __forceinline__ int* path_level(const DevIvms& V, int id, int l)
 {
-    return V.path + ((size_t)id * V.npad + l) * PBB_PATH_INTS;
+    return V.path + ((size_t)id * V.levels + l) * PBB_PATH_INTS;
 }
 
 template <int NW>
@@ -157,7 +157,7 @@ __device__ __forceinline__ int front_count(const Ivm<NW>& R, int L)
 
 __device__ __forceinline__ signed char* mat_row(const DevIvms& V, int id, int l)
 {
-    return V.mat + ((size_t)id * V.npad + l) * V.npad;
+    return V.mat + ((size_t)id * V.levels + l) * V.npad;
 }
 
 template <int NW>
@@ -738,25 +738,18 @@ __device__ __forceinline__ int group_of_cta(const DevGroup* groups, int ngroups)
 // kernels
 // ---------------------------------------------------------------------------
 
-// Empty every explorer of every group; clear counters and queues.
+// Empty every explorer of every group; clear counters and requests.  An
+// explorer without work has no image: whoever starts one (the root kernel, a
+// donor) writes all of it that is read.
 __global__ void pbb_reset_kernel(const DevGroup* groups, int ngroups, const int* ub)
 {
     for (int g = blockIdx.y; g < ngroups; g += gridDim.y) {
-        const DevGroup G = groups[g];
-        const int n = G.inst.n;
+        const DevGroup& G = groups[g];
         for (int id = blockIdx.x * blockDim.x + threadIdx.x; id < G.ivm.count; id += gridDim.x * blockDim.x) {
             G.ivm.state[id] = IVM_IDLE;
             G.ivm.line[id] = 0;
             G.ivm.bestcost[id] = 0x7fffffff;
-            G.ivm.ask[id >> 5] = 0u;
-            const size_t b = (size_t)id * G.ivm.npad;
-            for (int e = 0; e < G.ivm.npad; e++) {
-                G.ivm.pos[b + e] = 0;
-                G.ivm.end[b + e] = 0;
-                G.ivm.dir[b + e] = 0;
-                G.ivm.pj[b + e] = 0;
-            }
-            G.ivm.pos[b] = (signed char)n;   // empty interval (ivm.cpp:36-49)
+            if ((id & 31) == 0) G.ivm.ask[id >> 5] = 0u;
         }
         if (blockIdx.x == 0 && threadIdx.x == 0) {
             GroupCtl* c = G.ctl;

@@ -20,6 +20,7 @@
 #include "pbb_launch.h"
 #include "pbb_tables.h"
 #include "pbb_heur.h"
+#include "pbb_mem.h"
 #include "../../include/pbbperm.h"
 
 namespace {
@@ -111,6 +112,7 @@ struct pbb_pool {
     size_t table_stride = 0;
     size_t off_je = 0, off_p = 0, off_pm = 0, off_mt = 0, off_posj = 0;
     unsigned char* arena = nullptr;
+    unsigned char* block = nullptr;   // tables and the lists below
     size_t arena_bytes = 0;
     unsigned char* tables = nullptr;
     GroupCtl* ctl = nullptr;
@@ -163,41 +165,33 @@ extern "C" int pbb_pool_destroy(pbb_pool* P)
     for (auto& shape : P->window)
         for (cudaGraphExec_t g : shape)
             if (g) cudaGraphExecDestroy(g);
-    cudaFree(P->arena);
-    cudaFree(P->tables);
-    cudaFree(P->pair_stack);
-    cudaFree(P->ctl);
+    pbbh::mem_free(P->arena, P->st);
+    pbbh::mem_free(P->block, P->st);
+    pbbh::mem_free(P->pair_stack, P->st);
     cudaFreeHost(P->ctl_h);
-    cudaFree(P->groups_d);
-    cudaFree(P->ngroups_d);
-    cudaFree(P->new_d);
-    cudaFree(P->ub_d);
-    cudaFree(P->roots_d);
-    cudaFree(P->ivals_d);
-    cudaFree(P->neh_d);
-    cudaFree(P->neh_tasks_d);
-    if (P->st) cudaStreamDestroy(P->st);
+    pbbh::stream_give(P->st, P->dev);
     delete P;
     return PBB_OK;
 }
 
 namespace {
 
-size_t explorer_block_bytes(int E, int npad)
+size_t explorer_block_bytes(int E, int npad, int levels)
 {
-    size_t b = align256((size_t)E * npad * npad);     // mat
+    size_t b = align256((size_t)E * levels * npad);   // mat
     b += 5 * align256((size_t)E * npad);              // pos end dir pj bestperm
     b += 5 * align256((size_t)E * 4);                 // line state bestcost ask askid
-    b += align256((size_t)E * npad * PBB_PATH_INTS * 4);   // path levels
+    b += align256((size_t)E * levels * PBB_PATH_INTS * 4);   // path levels
     return b;
 }
 
-void carve_explorers(unsigned char* base, int E, int npad, DevIvms& V)
+void carve_explorers(unsigned char* base, int E, int npad, int levels, DevIvms& V)
 {
     size_t o = 0;
     V.count = E;
     V.npad = npad;
-    V.mat = reinterpret_cast<signed char*>(base + o); o += align256((size_t)E * npad * npad);
+    V.levels = levels;
+    V.mat = reinterpret_cast<signed char*>(base + o); o += align256((size_t)E * levels * npad);
     V.pos = reinterpret_cast<signed char*>(base + o); o += align256((size_t)E * npad);
     V.end = reinterpret_cast<signed char*>(base + o); o += align256((size_t)E * npad);
     V.dir = reinterpret_cast<signed char*>(base + o); o += align256((size_t)E * npad);
@@ -211,7 +205,9 @@ void carve_explorers(unsigned char* base, int E, int npad, DevIvms& V)
     V.path = reinterpret_cast<int*>(base + o);
 }
 
-int pool_create(const pbb_pool_config* in, pbb_pool* P)
+// `most`: instances the pool will ever hold (a batch knows), so that it is not
+// made larger than they need
+int pool_create(const pbb_pool_config* in, pbb_pool* P, int most)
 {
     pbb_pool_config c;
     pbb_pool_config_default(&c);
@@ -234,7 +230,7 @@ int pool_create(const pbb_pool_config* in, pbb_pool* P)
     P->dev = c.device;
     pbbh::DeviceGuard keep_callers_device;
     PCK(cudaSetDevice(P->dev), "cudaSetDevice failed");
-    PCK(cudaStreamCreateWithFlags(&P->st, cudaStreamNonBlocking), "stream creation failed");
+    PCK(pbbh::stream_take(&P->st, P->dev), "stream creation failed");
     P->nw = c.max_jobs <= 32 ? 1 : 2;
     P->npad = 32 * P->nw;
     P->warps = c.warps_per_cta;
@@ -287,7 +283,7 @@ int pool_create(const pbb_pool_config* in, pbb_pool* P)
     // default explorer count: every warp of the widest grid owns one, so that
     // an instance left alone at the end of a batch can keep the whole GPU busy
     if (P->epw <= 0) P->epw = std::max(P->grid * P->warps, P->tail_grid * P->tail_warps);
-    P->max_slots = c.max_resident > 0 ? std::min(c.max_resident, capacity) : capacity;
+    P->max_slots = std::min(c.max_resident > 0 ? std::min(c.max_resident, capacity) : capacity, std::max(1, most));
     // per-slot instance tables
     P->off_je = 0;
     P->off_p = align256(P->off_je + (size_t)c.max_jobs * P->Ppad_max * 8);
@@ -296,24 +292,33 @@ int pool_create(const pbb_pool_config* in, pbb_pool* P)
     P->off_posj = align256(P->off_mt + 2 * (size_t)c.max_machines * 4);
     P->table_stride = align256(P->off_posj + (size_t)c.max_jobs * P->Ppad_max);
     const int S = P->max_slots;
-    PCK(cudaMalloc(&P->tables, P->table_stride * S), "table memory");
-    PCK(cudaMalloc(&P->ctl, sizeof(GroupCtl) * S), "control blocks");
-    PCK(cudaMemset(P->ctl, 0, sizeof(GroupCtl) * S), "control blocks");
+    {
+        pbbh::Carver C;
+        const size_t o_tables = C.take(P->table_stride * S), o_ctl = C.take(sizeof(GroupCtl) * S);
+        const size_t o_groups = C.take(sizeof(DevGroup) * S), o_new = C.take(sizeof(DevGroup) * S);
+        const size_t o_n = C.take(sizeof(int)), o_ub = C.take(sizeof(int) * S);
+        const size_t o_roots = C.take(sizeof(int) * S * PBB_MAX_N), o_ivals = C.take(sizeof(int) * S * 2 * PBB_MAX_N);
+        const size_t o_neh = C.take(sizeof(int) * S * (PBB_MAX_N + 1)), o_tasks = C.take(sizeof(NehTask) * S);
+        PCK(pbbh::mem_alloc((void**)&P->block, C.bytes, P->dev, P->st), "table memory");
+        P->tables = P->block + o_tables;
+        P->ctl = reinterpret_cast<GroupCtl*>(P->block + o_ctl);
+        P->groups_d = reinterpret_cast<DevGroup*>(P->block + o_groups);
+        P->new_d = reinterpret_cast<DevGroup*>(P->block + o_new);
+        P->ngroups_d = reinterpret_cast<int*>(P->block + o_n);
+        P->ub_d = reinterpret_cast<int*>(P->block + o_ub);
+        P->roots_d = reinterpret_cast<int*>(P->block + o_roots);
+        P->ivals_d = reinterpret_cast<int*>(P->block + o_ivals);
+        P->neh_d = reinterpret_cast<int*>(P->block + o_neh);
+        P->neh_tasks_d = reinterpret_cast<NehTask*>(P->block + o_tasks);
+    }
+    PCK(cudaMemsetAsync(P->ctl, 0, sizeof(GroupCtl) * S, P->st), "control blocks");
+    PCK(cudaMemsetAsync(P->ngroups_d, 0, sizeof(int), P->st), "group count");
     PCK(cudaMallocHost(&P->ctl_h, sizeof(GroupCtl) * S), "pinned control mirror");
     memset(P->ctl_h, 0, sizeof(GroupCtl) * S);
-    PCK(cudaMalloc(&P->groups_d, sizeof(DevGroup) * S), "group list");
-    PCK(cudaMalloc(&P->new_d, sizeof(DevGroup) * S), "group list");
-    PCK(cudaMalloc(&P->ngroups_d, sizeof(int)), "group count");
-    PCK(cudaMemset(P->ngroups_d, 0, sizeof(int)), "group count");
-    PCK(cudaMalloc(&P->ub_d, sizeof(int) * S), "bounds");
-    PCK(cudaMalloc(&P->roots_d, sizeof(int) * S * PBB_MAX_N), "roots");
-    PCK(cudaMalloc(&P->ivals_d, sizeof(int) * S * 2 * PBB_MAX_N), "intervals");
-    PCK(cudaMalloc(&P->neh_d, sizeof(int) * S * (PBB_MAX_N + 1)), "heuristic results");
-    PCK(cudaMalloc(&P->neh_tasks_d, sizeof(NehTask) * S), "heuristic tasks");
     if (P->pair_smem || P->tail_pair_smem) {
         const size_t w = std::max((size_t)P->grid * P->warps, (size_t)P->tail_grid * P->tail_warps);
         P->pair_stride = c.max_jobs * P->Ppad_max;
-        if (cudaMalloc(&P->pair_stack, sizeof(int) * w * P->pair_stride) != cudaSuccess) {
+        if (pbbh::mem_alloc((void**)&P->pair_stack, sizeof(int) * w * P->pair_stride, P->dev, P->st) != cudaSuccess) {
             cudaGetLastError();       // no room: the general build needs none
             P->pair_stack = nullptr;
             P->pair_smem = P->tail_pair_smem = 0;
@@ -321,9 +326,10 @@ int pool_create(const pbb_pool_config* in, pbb_pool* P)
     }
     P->arena_bytes = (size_t)c.explorer_bytes;
     const int E = P->epw;
-    if (explorer_block_bytes(E, P->npad) > P->arena_bytes)
+    if (explorer_block_bytes(E, P->npad, P->cfg.max_jobs) > P->arena_bytes)
         return pfail(PBB_E_INVAL, "explorer_bytes is smaller than one instance's footprint");
-    PCK(cudaMalloc(&P->arena, P->arena_bytes), "explorer memory");
+    P->arena_bytes = std::min(P->arena_bytes, explorer_block_bytes(E, P->npad, c.max_jobs) * (size_t)P->max_slots);
+    PCK(pbbh::mem_alloc((void**)&P->arena, P->arena_bytes, P->dev, P->st), "explorer memory");
     P->alloc.init(P->arena_bytes);
     P->slots.assign(S, Slot());
     return PBB_OK;
@@ -365,18 +371,23 @@ int window_graph(pbb_pool* P, bool tail, int build, cudaGraphExec_t* out)
 
 }  // namespace
 
-extern "C" int pbb_pool_create(const pbb_pool_config* cfg, pbb_pool** out)
+static int new_pool(const pbb_pool_config* cfg, pbb_pool** out, int most)
 {
-    if (!out) return pfail(PBB_E_INVAL, "out is NULL");
     *out = nullptr;
     pbb_pool* P = new pbb_pool();
-    const int rc = pool_create(cfg, P);
+    const int rc = pool_create(cfg, P, most);
     if (rc) {
         pbb_pool_destroy(P);
         return rc;
     }
     *out = P;
     return PBB_OK;
+}
+
+extern "C" int pbb_pool_create(const pbb_pool_config* cfg, pbb_pool** out)
+{
+    if (!out) return pfail(PBB_E_INVAL, "out is NULL");
+    return new_pool(cfg, out, INT_MAX);
 }
 
 extern "C" int pbb_pool_submit(pbb_pool* P, const pbb_instance* inst, const pbb_config* search, int32_t ub,
@@ -420,7 +431,7 @@ namespace {
 int admit(pbb_pool* P, std::vector<int>& admitted)
 {
     const int E = P->epw;
-    const size_t bytes = explorer_block_bytes(E, P->npad);
+    const size_t bytes = explorer_block_bytes(E, P->npad, P->cfg.max_jobs);
     while (true) {
         int s = -1;
         for (int i = 0; i < P->max_slots; i++)
@@ -478,7 +489,7 @@ int admit(pbb_pool* P, std::vector<int>& admitted)
         g.search.split_depth = P->split_depth;
         g.search.split_narrow = P->split_narrow;
         g.search.share_after = P->share_after;
-        carve_explorers(P->arena + off, E, P->npad, g.ivm);
+        carve_explorers(P->arena + off, E, P->npad, P->cfg.max_jobs, g.ivm);
         g.ctl = P->ctl + s;
         admitted.push_back(s);
         P->pending_ub.push_back(r.ub);
@@ -682,7 +693,7 @@ extern "C" int pbb_batch_solve(const pbb_instance* inst, int32_t count, const pb
         c.window_s = 0.02;
     }
     pbb_pool* P = nullptr;
-    int rc = pbb_pool_create(&c, &P);
+    int rc = new_pool(&c, &P, count);
     if (rc) return rc;
     // The whole batch is known: admit the largest instances first (jobs, then
     // machines), so that the long searches start early and overlap with the

@@ -82,8 +82,9 @@ struct GroupCtl {
 // Explorer storage of a group (device memory, structure of arrays).
 struct DevIvms {
     int count;             // explorers in the group
-    int npad;              // row stride (64)
-    signed char* mat;      // [count][npad][npad]
+    int npad;              // row stride (32 for up to 32 jobs, else 64)
+    int levels;            // levels kept of each explorer (at least the jobs)
+    signed char* mat;      // [count][levels][npad]
     signed char* pos;      // [count][npad]
     signed char* end;      // [count][npad]
     signed char* dir;      // [count][npad]
@@ -94,7 +95,7 @@ struct DevIvms {
     signed char* bestperm; // [count][npad]
     unsigned int* ask;     // [(count + 31) / 32] bit c: CTA c of the group asks for work
     int* askid;            // [count] explorer that asking CTA c offers for it
-    int* path;             // [count][npad levels][3][32] heads / tails / free loads of the path nodes
+    int* path;             // [count][levels][3][32] heads / tails / free loads of the path nodes
 };
 
 #define PBB_PATH_INTS 96   // ints per path level: heads, tails, free loads, 32 machines each

@@ -33,7 +33,7 @@ def test_counts_equal_the_oracle(n, m, jmode, seed, ub, opt):
     ub -= 1 if opt.get("findAll") else 0
     want = Oracle(p, jmode).solve(ub, bound_mode=2, branch_mode=rule, find_all=opt.get("findAll", False),
                                   sorted_dfs=opt.get("sortedDFS", 0),
-                                  sorting_criterion=opt.get("sortingCriterion", 1), node_limit=400000)
+                                  sorting_criterion=opt.get("sortingCriterion", 1), node_limit=60000)
     if not want["complete"]:
         pytest.skip("the tree is too large for the oracle")
     assert not want["found"]
