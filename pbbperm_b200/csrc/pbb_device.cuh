@@ -68,6 +68,13 @@ __device__ __forceinline__ int vgather(const int (&x)[NW], int s)
     return r;
 }
 
+// element `s` (per lane, below 32) of a lane-distributed vector
+template <int NW>
+__device__ __forceinline__ int vget_lane(const int (&x)[NW], int s)
+{
+    return __shfl_sync(FULLMASK, x[0], s);
+}
+
 template <int NW>
 __device__ __forceinline__ void vset(int (&x)[NW], int idx, int val)
 {
@@ -120,8 +127,8 @@ struct CtaTables {
     const unsigned char* pm1;
     const int* min_arr;
     const int* min_dep;
-    const unsigned char* posj;     // [n][Ppad] or NULL
-    int n, m, P, Ppad, mp, je_stride;
+    const unsigned char* posj;     // [n][posj_stride] or NULL
+    int n, m, P, Ppad, mp, je_stride, posj_stride;
 };
 
 struct WarpScratch {
@@ -146,6 +153,9 @@ struct WarpScratch {
     // kept pair bounds only (PBB_SCRATCH_PAIRS)
     int* pairs;             // two buffers of Ppad pair bounds
     int4* child;            // [32] by machine: the child's head, its job's time (twice), the child's tail
+    // every child's Johnson value only (PBB_SCRATCH_ALL)
+    int4* pass;             // [32] the pass's pairs: end terms of front and back children, m0 and m1 rows of dF and dB
+    int* vals;              // [n][33] their values without the job at each position
 };
 
 __device__ __forceinline__ WarpScratch warp_scratch(unsigned char* base, const SmemPlan& sp, int n, int m, int Ppad)
@@ -154,6 +164,8 @@ __device__ __forceinline__ WarpScratch warp_scratch(unsigned char* base, const S
     s.fmask = nullptr;
     s.pairs = nullptr;
     s.child = nullptr;
+    s.pass = nullptr;
+    s.vals = nullptr;
     int* ip = reinterpret_cast<int*>(base);
     s.Fb = ip; ip += 32;
     s.Bb = ip; ip += 32;
@@ -162,8 +174,12 @@ __device__ __forceinline__ WarpScratch warp_scratch(unsigned char* base, const S
     s.frontZ = ip; ip += 32;
     s.backZ = ip; ip += 32;
     s.rem = ip; ip += 32;
-    const bool pairs = sp.fmask == PBB_SCRATCH_PAIRS;
-    if (pairs) {
+    const bool pairs = sp.fmask == PBB_SCRATCH_PAIRS, all = sp.fmask == PBB_SCRATCH_ALL;
+    if (all) {
+        s.pass = reinterpret_cast<int4*>(ip); ip += 128;
+        s.vals = ip; ip += n * 33;
+        s.lbF = s.lbB = nullptr;
+    } else if (pairs) {
         s.child = reinterpret_cast<int4*>(ip); ip += 128;
         s.pairs = ip; ip += 2 * Ppad;
         s.lbF = s.lbB = nullptr;
@@ -177,7 +193,10 @@ __device__ __forceinline__ WarpScratch warp_scratch(unsigned char* base, const S
         s.lbB = ip; ip += n;
     }
     short* sp2 = reinterpret_cast<short*>(ip);
-    if (!pairs) {
+    if (all) {
+        s.dF = sp2; sp2 += m * (n <= 32 ? 32 : 64);
+        s.dB = sp2; sp2 += m * (n <= 32 ? 32 : 64);
+    } else if (!pairs) {
         s.dF = sp2; sp2 += n * m;
         s.dB = sp2; sp2 += n * m;
     }
@@ -892,6 +911,191 @@ __device__ __forceinline__ void johnson_sweep_masked(const CtaTables& T, const W
         }
     }
     __syncwarp();
+}
+
+// ---------------------------------------------------------------------------
+// Johnson values of every child of both sides
+// ---------------------------------------------------------------------------
+// A child's value is the largest over its one-machine terms and, per pair,
+//   front: h_q[m0] + C_{-q} + Bb[m1],  back: Fb[m0] + C_{-q} + t_q[m1],
+// with C_{-q} the pair's value without the child's job (johnson_children).
+// C_{-q} does not depend on the side, so it is computed once per pair and job,
+// a pair per lane by walks from both ends of the positions, and
+// left in shared memory by position; then the lanes turn to the children, read
+// the pair's value at their job's position and keep both sides' maxima in
+// registers.  Small rows put two (k <= 16) or four (k <= 8) pairs side by side
+// in a warp.  Before, every pair's every child went through a shared atomic.
+// Whole call on device buffers, 0.6 ms of it host work at 50x20: 50,000 nodes
+// of 50x20 4.46 -> 3.12 ms, of 20x20 1.50 -> 1.02, of 12x10 0.38 -> 0.30.
+// What bounds it now is latency: the values by position leave room for 10
+// warps an SM at 50x20 (16 at 32 jobs and fewer).
+
+// head and tail deltas of every child by machine (dF, dB: [m][32 NW]), and the
+// largest one-machine term of each child's Johnson value
+template <int NW>
+__device__ __forceinline__ void all_child_tables(const CtaTables& T, const WarpScratch& S, const int (&row)[NW],
+                                                 const bool (&valid)[NW], int (&lbF)[NW], int (&lbB)[NW])
+{
+    const int m = T.m;
+#pragma unroll
+    for (int w = 0; w < NW; w++) {
+        lbF[w] = 0;
+        lbB[w] = 0;
+        if (!valid[w]) continue;
+        const int at = w * 32 + lane_id();
+        const int* p = T.pt + row[w] * T.mp;
+        int h = 0;
+        PBB_ROLLED
+        for (int q = 0; q < m; q++) {
+            const int z = S.frontZ[q], x = max(h, z);
+            lbF[w] = max(lbF[w], x + S.rem[q] + S.Bb[q]);
+            h = x + p[q];
+            S.dF[q * 32 * NW + at] = (short)(h - z);
+        }
+        int t = 0;
+        PBB_ROLLED
+        for (int q = m - 1; q >= 0; q--) {
+            const int z = S.backZ[q], x = max(t, z);
+            lbB[w] = max(lbB[w], x + S.rem[q] + S.Fb[q]);
+            t = x + p[q];
+            S.dB[q * 32 * NW + at] = (short)(t - z);
+        }
+    }
+    __syncwarp();
+}
+
+template <int NW>
+__device__ __forceinline__ bool job_free(const unsigned (&um)[NW], int j)
+{
+    unsigned uw = um[0];
+#pragma unroll
+    for (int w = 1; w < NW; w++)
+        if ((j >> 5) == w) uw = um[w];
+    return (uw >> (j & 31)) & 1u;
+}
+
+// k >= 2 free jobs `row` (mask um); kids: children wanted (k >= 3).  lbF, lbB
+// by cell; returns the node's own Johnson value.
+template <int NW>
+__device__ __forceinline__ int johnson_all(const CtaTables& T, const WarpScratch& S, const int (&row)[NW],
+                                           const bool (&valid)[NW], const unsigned (&um)[NW], int k, bool kids,
+                                           int (&lbF)[NW], int (&lbB)[NW])
+{
+    const int lane = lane_id(), n = T.n;
+    if (kids) all_child_tables<NW>(T, S, row, valid, lbF, lbB);
+    // children of small rows: `side` pairs at a time, each on `group` lanes
+    const int group = k > 16 ? 32 : (k > 8 ? 16 : 8);
+    const int slot = lane & (group - 1), part = lane / group, side = 32 / group;
+    int job[NW], aF[NW], aB[NW];
+    bool on[NW];
+#pragma unroll
+    for (int w = 0; w < NW; w++) {
+        job[w] = group == 32 ? row[w] : vget_lane<NW>(row, slot);
+        on[w] = group == 32 ? valid[w] : (w == 0 && slot < k);
+        aF[w] = 0;
+        aB[w] = 0;
+        if (!on[w]) job[w] = 0;
+    }
+    int node = 0;
+    for (int base = 0; base < T.P; base += 32) {
+        const int i = base + lane;
+        if (i < T.P) {
+            const int m0 = T.pm0[i], m1 = T.pm1[i];
+            const int Asum = S.rem[m0], Bsum = S.rem[m1];
+            // forward walk from the first position, backward from the last, in
+            // one loop: two independent chains.  Up to the middle each leaves
+            // its term, past it each raises what the other left.
+            int Apre = 0, Bpre = Bsum, PM = NEG_INF;     // Bpre: the load from this position on
+            int Aup = Asum, Bsuf = 0, SM = NEG_INF;      // Aup: the load up to this position
+            const unsigned long long* fw = T.je + i;
+            const unsigned long long* bw = fw + (n - 1) * T.je_stride;
+            int* vf = S.vals + lane;
+            int* vb = vf + (n - 1) * 33;
+            const int half = n >> 1;
+#pragma unroll 2
+            for (int t = 0; t < half; t++) {
+                const unsigned long long e = *fw, g = *bw;
+                fw += T.je_stride;
+                bw -= T.je_stride;
+                const int b = JE_B(e), a = JE_A(g);
+                if (job_free<NW>(um, JE_JOB(e))) {
+                    *vf = PM - b;
+                    Apre += JE_A(e);
+                    PM = max(PM, Apre + Bpre + JE_C(e));
+                    Bpre -= b;
+                }
+                if (job_free<NW>(um, JE_JOB(g))) {
+                    *vb = SM - a;
+                    Bsuf += JE_B(g);
+                    SM = max(SM, Aup + Bsuf + JE_C(g));
+                    Aup -= a;
+                }
+                vf += 33;
+                vb -= 33;
+            }
+            if (n & 1) {
+                // the middle position: the forward term, raised by the
+                // backward one in the loop below
+                *vf = NEG_INF;
+            }
+#pragma unroll 2
+            for (int t = half; t < n; t++) {
+                const unsigned long long e = *fw, g = *bw;
+                fw += T.je_stride;
+                bw -= T.je_stride;
+                const int b = JE_B(e), a = JE_A(g);
+                if (job_free<NW>(um, JE_JOB(e))) {
+                    *vf = max(*vf, PM - b);
+                    Apre += JE_A(e);
+                    PM = max(PM, Apre + Bpre + JE_C(e));
+                    Bpre -= b;
+                }
+                if (job_free<NW>(um, JE_JOB(g))) {
+                    *vb = max(*vb, SM - a);
+                    Bsuf += JE_B(g);
+                    SM = max(SM, Aup + Bsuf + JE_C(g));
+                    Aup -= a;
+                }
+                vf += 33;
+                vb -= 33;
+            }
+            node = max(node, max(S.Fb[m1] + Bsum + S.Bb[m1], S.Fb[m0] + PM + S.Bb[m1]));
+            node = max(node, S.Fb[m0] + Asum + S.Bb[m0]);
+            if (kids)
+                S.pass[lane] = make_int4(S.frontZ[m0] + S.Bb[m1], S.Fb[m0] + S.backZ[m1], m0 * 32 * NW, m1 * 32 * NW);
+        }
+        __syncwarp();
+        if (kids) {
+            const int last = min(32, T.P - base);
+            PBB_ROLLED
+            for (int c = part; c < last; c += side) {
+                const int4 u = S.pass[c];
+#pragma unroll
+                for (int w = 0; w < NW; w++) {
+                    if (NW > 1 && w > 0 && k <= 32) break;
+                    if (on[w]) {
+                        const int at = (group == 32 ? w * 32 + lane : slot);
+                        const int v = S.vals[T.posj[job[w] * T.posj_stride + base + c] * 33 + c];
+                        aF[w] = max(aF[w], v + u.x + S.dF[u.z + at]);
+                        aB[w] = max(aB[w], v + u.y + S.dB[u.w + at]);
+                    }
+                }
+            }
+            __syncwarp();
+        }
+    }
+    if (kids) {
+        for (int o = 16; o >= group; o >>= 1) {
+            aF[0] = max(aF[0], __shfl_xor_sync(FULLMASK, aF[0], o));
+            aB[0] = max(aB[0], __shfl_xor_sync(FULLMASK, aB[0], o));
+        }
+#pragma unroll
+        for (int w = 0; w < NW; w++) {
+            lbF[w] = max(lbF[w], aF[w]);
+            lbB[w] = max(lbB[w], aB[w]);
+        }
+    }
+    return __reduce_max_sync(FULLMASK, node);
 }
 
 // Per-child head/tail deltas used by johnson_children (front child u: heads of

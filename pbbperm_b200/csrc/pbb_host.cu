@@ -815,7 +815,7 @@ int pbb_bound_children(const pbb_instance* inst, int32_t johnson_mode, int32_t d
                        int32_t* weak_end, int32_t* strong_begin, int32_t* strong_end, int32_t* node_weak,
                        int32_t* node_strong)
 {
-    return bound_children_impl(inst, johnson_mode, device, 0, count, sched, limit1, limit2, weak_begin, weak_end,
+    return bound_children_impl(inst, johnson_mode, device, -1, count, sched, limit1, limit2, weak_begin, weak_end,
                                strong_begin, strong_end, node_weak, node_strong);
 }
 
@@ -823,7 +823,7 @@ int pbb_bound_children_ex(const pbb_instance* inst, int32_t johnson_mode, int32_
                           const int32_t* sched, const int32_t* limit1, const int32_t* limit2, const pbb_bound_out* out)
 {
     if (!out) return fail(PBB_E_INVAL, "out is NULL");
-    return bound_children_impl(inst, johnson_mode, device, 0, count, sched, limit1, limit2, out->weak_begin,
+    return bound_children_impl(inst, johnson_mode, device, -1, count, sched, limit1, limit2, out->weak_begin,
                                out->weak_end, out->strong_begin, out->strong_end, out->node_weak, out->node_strong,
                                out->prio_begin, out->prio_end, out->strong_idle);
 }
@@ -899,21 +899,28 @@ static int bound_children_impl(const pbb_instance* inst, int32_t johnson_mode, i
             cudaMemcpyAsync(d + o_l2, limit2, c1, cudaMemcpyHostToDevice, st);
         }
         cudaMemcpyAsync(d, host.data(), host.size(), cudaMemcpyHostToDevice, st);
-        int smem = 0;
-        const int warps = pick_warps(H, 8, device, smem);
-        if (warps < 1) { rc = fail(PBB_E_INVAL, "instance tables do not fit in shared memory"); break; }
         int sms = 0;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-        int ctas = (count + warps - 1) / warps;
-        ctas = std::min(ctas, sms * 4);
+        const pbbl::BoundShape shape = pbbl::bound_shape(n, H.m, H.Ppad, count, sms, max_smem_optin(device));
+        if (shape.warps < 1) { rc = fail(PBB_E_INVAL, "instance tables do not fit in shared memory"); break; }
         auto dev = [&](size_t off) { return reinterpret_cast<int*>(d + off); };
         BoundExtra X;
         if (want_prio) { X.prio_begin = dev(out[6].off); X.prio_end = dev(out[7].off); }
         if (strong_idle) X.strong_idle = dev(out[8].off);
         unsigned* status = reinterpret_cast<unsigned*>(d + o_status);
-        ce = pbbl::launch_bound(n <= 32 ? 1 : 2, tables.view(H, d), count, dev(o_s), dev(o_l1), dev(o_l2),
-                                dev(out[0].off), dev(out[1].off), dev(out[2].off), dev(out[3].off), dev(out[4].off),
-                                dev(out[5].off), status, ctas, warps, smem, st, method, X);
+        const int nw = n <= 32 ? 1 : 2;
+        if (method < 0) {
+            ce = pbbl::launch_bound_all(nw, tables.view(H, d), count, dev(o_s), dev(o_l1), dev(o_l2), dev(out[0].off),
+                                        dev(out[1].off), dev(out[2].off), dev(out[3].off), dev(out[4].off),
+                                        dev(out[5].off), status, shape, st, X);
+        } else {
+            int smem = 0;
+            const int warps = pick_warps(H, 8, device, smem);
+            const int ctas = std::min((count + warps - 1) / warps, sms * 4);
+            ce = pbbl::launch_bound(nw, tables.view(H, d), count, dev(o_s), dev(o_l1), dev(o_l2), dev(out[0].off),
+                                    dev(out[1].off), dev(out[2].off), dev(out[3].off), dev(out[4].off),
+                                    dev(out[5].off), status, ctas, warps, smem, st, method, X);
+        }
         if (ce != cudaSuccess) { rc = cuda_fail(ce, "pbb_bound_kernel launch"); break; }
         unsigned hs = 0;
         cudaMemcpyAsync(&hs, status, sizeof(unsigned), cudaMemcpyDeviceToHost, st);

@@ -89,13 +89,19 @@ __device__ __forceinline__ void load_tables(const DevInstance& I, unsigned char*
     }
     for (int i = tid; i < I.Ppad; i += nt) { pm0[i] = I.pm0[i]; pm1[i] = I.pm1[i]; }
     for (int i = tid; i < I.m; i += nt) { marr[i] = I.min_arr[i]; mdep[i] = I.min_dep[i]; }
-    const bool posj_here = I.posj && sp.fmask != PBB_SCRATCH_PAIRS;
+    const bool all = sp.fmask == PBB_SCRATCH_ALL;
+    const bool posj_here = all || (I.posj && sp.fmask != PBB_SCRATCH_PAIRS);
     unsigned char* posj = smem + sp.posj_off;
-    if (posj_here)
+    if (all) {
+        for (int t = tid / 32; t < I.n; t += nt / 32)
+            for (int i = tid & 31; i < I.P; i += 32)
+                posj[JE_JOB(I.je[t * I.Ppad + i]) * sp.posj_stride + i] = (unsigned char)t;
+    } else if (posj_here)
         for (int i = tid; i < I.n * I.Ppad; i += nt) posj[i] = I.posj[i];
     T.je = je; T.pt = pt; T.mp = mp; T.pm0 = pm0; T.pm1 = pm1; T.min_arr = marr; T.min_dep = mdep;
     T.posj = posj_here ? posj : nullptr;
     T.je_stride = sp.je_stride;
+    T.posj_stride = sp.posj_stride;
     T.n = I.n; T.m = I.m; T.P = I.P; T.Ppad = I.Ppad;
 }
 
@@ -1084,6 +1090,37 @@ __global__ void pbb_lower_ub_kernel(const DevGroup* groups, int g, int ub)
     atomicMin(&groups[g].ctl->best_key, ((unsigned long long)(unsigned)ub << 32) | 0xffffffffull);
 }
 
+// couts[1] of bound_fsp_strong::bornes_calculer: idle time of the fixed jobs'
+// schedules (scheduleFront :457-478, scheduleBack :490-509): 0 with nothing
+// fixed in front for the front part, and 0 altogether when nothing is fixed at
+// the back; 0 as well with at most one free job (the reference leaves it unset
+// there).  One lane.
+__device__ __noinline__ int fixed_idle(const CtaTables& T, const WarpScratch& S, int f, int b, int k)
+{
+    int idle = 0;
+    if (k > 1 && b > 0) {
+        int fr[PBB_MAX_M], bk[PBB_MAX_M];
+        for (int q = 0; q < T.m; q++) { fr[q] = 0; bk[q] = 0; }
+        for (int i = 0; i < f; i++) {
+            const int* p = T.pt + S.fjob[i] * T.mp;
+            fr[0] += p[0];
+            for (int q = 1; q < T.m; q++) {
+                idle += max(0, fr[q - 1] - fr[q]);
+                fr[q] = max(fr[q], fr[q - 1]) + p[q];
+            }
+        }
+        for (int i = 0; i < b; i++) {
+            const int* p = T.pt + S.bjob[i] * T.mp;
+            bk[T.m - 1] += p[T.m - 1];
+            for (int q = T.m - 2; q >= 0; q--) {
+                idle += max(0, bk[q + 1] - bk[q]);
+                bk[q] = max(bk[q], bk[q + 1]) + p[q];
+            }
+        }
+    }
+    return idle;
+}
+
 // Children bounds of `count` nodes (warp per node): weak LBs of every free job
 // appended at the front / back (bound_fsp_weak::boundChildren), Johnson LBs
 // of the same children (bound_fsp_strong::bornes_calculer on the child), the
@@ -1153,35 +1190,7 @@ __global__ void pbb_bound_kernel(DevInstance I, int count, const int* sched, con
                 }
             }
         }
-        if (X.strong_idle && lane == 0) {
-            // couts[1] of bound_fsp_strong::bornes_calculer: idle time of the
-            // fixed jobs' schedules (scheduleFront :457-478, scheduleBack
-            // :490-509): 0 with nothing fixed in front for the front part, and
-            // 0 altogether when nothing is fixed at the back; 0 as well with at
-            // most one free job (the reference leaves it unset there)
-            int idle = 0;
-            if (k > 1 && b > 0) {
-                int fr[PBB_MAX_M], bk[PBB_MAX_M];
-                for (int q = 0; q < T.m; q++) { fr[q] = 0; bk[q] = 0; }
-                for (int i = 0; i < f; i++) {
-                    const int j = S.fjob[i];
-                    fr[0] += T.pt[j * T.mp];
-                    for (int q = 1; q < T.m; q++) {
-                        idle += max(0, fr[q - 1] - fr[q]);
-                        fr[q] = max(fr[q], fr[q - 1]) + T.pt[j * T.mp + q];
-                    }
-                }
-                for (int i = 0; i < b; i++) {
-                    const int j = S.bjob[i];
-                    bk[T.m - 1] += T.pt[j * T.mp + T.m - 1];
-                    for (int q = T.m - 2; q >= 0; q--) {
-                        idle += max(0, bk[q + 1] - bk[q]);
-                        bk[q] = max(bk[q], bk[q + 1]) + T.pt[j * T.mp + q];
-                    }
-                }
-            }
-            X.strong_idle[node] = idle;
-        }
+        if (X.strong_idle && lane == 0) X.strong_idle[node] = fixed_idle(T, S, f, b, k);
         const int wn = weak_node_lb(T, S);
         // node Johnson LB and children Johnson LBs
         int snode = 0;
@@ -1259,6 +1268,114 @@ __global__ void pbb_bound_kernel(DevInstance I, int count, const int* sched, con
                 }
             }
         }
+        if (lane == 0) {
+            node_weak[node] = wn;
+            node_strong[node] = snode;
+        }
+        __syncwarp();
+    }
+}
+
+// The same outputs with the Johnson values of johnson_all: what the bound entry
+// points run wherever its scratch fits.  Node w * grid + b goes to warp w of
+// block b first, so that a handful of nodes spreads over the SMs and every
+// block's warps share in loading its tables.
+template <int NW>
+__global__ void __launch_bounds__(32 * PBB_BOUND_WARPS(NW))
+pbb_bound_all_kernel(DevInstance I, int count, const int* sched, const int* l1s, const int* l2s,
+                                     int* wb, int* we, int* sb, int* se, int* node_weak, int* node_strong,
+                                     unsigned int* status, int warps_per_cta, BoundExtra X)
+{
+    extern __shared__ __align__(16) unsigned char smem[];
+    const SmemPlan sp = pbb_smem_plan(I.n, I.m, I.Ppad, warps_per_cta, PBB_SCRATCH_ALL);
+    CtaTables T;
+    load_tables(I, smem, sp, T);
+    __syncthreads();
+    const int wic = threadIdx.x >> 5;
+    const WarpScratch S = warp_scratch(smem + sp.warp_off + wic * sp.warp_bytes, sp, T.n, T.m, T.Ppad);
+    const int n = T.n;
+    const int lane = lane_id();
+    for (int node = wic * gridDim.x + blockIdx.x; node < count; node += gridDim.x * warps_per_cta) {
+        const int* s = sched + (size_t)node * n;
+        const int l1 = l1s[node], l2 = l2s[node];
+        if (!(l1 >= -1 && l2 <= n && l1 < l2)) {
+            if (lane == 0) atomicOr(status, PBB_ST_BADINPUT);
+            continue;
+        }
+        const int f = l1 + 1, b = n - l2, k = l2 - l1 - 1;
+        for (int i = lane; i < f; i += 32) S.fjob[i] = (unsigned char)s[i];
+        for (int i = lane; i < b; i += 32) S.bjob[i] = (unsigned char)s[n - 1 - i];
+        int row[NW], sF[NW], sB[NW], wF[NW], wB[NW];
+        bool valid[NW];
+#pragma unroll
+        for (int w = 0; w < NW; w++) {
+            const int idx = w * 32 + lane;
+            valid[w] = idx < k;
+            row[w] = valid[w] ? s[l1 + 1 + idx] : 0;
+            if (valid[w]) S.rowj[idx] = (unsigned char)row[w];
+            sF[w] = 0;
+            sB[w] = 0;
+        }
+        __syncwarp();
+        partial_schedule(T, S, f, b, k);
+        weak_children<NW>(T, S, row, valid, k, true, wF, wB);
+        const int wn = weak_node_lb(T, S);
+        int snode = 0;
+        if (k <= 1) {
+            // at most one free job: the reference evaluates the full permutation
+            const int x0 = vget<NW>(row, 0);
+            int v = 0;
+            if (lane == 0) {
+                if (k == 1) v = makespan_split(T, S, x0, -1);
+                else
+                    for (int q = 0; q < T.m; q++) v = max(v, S.frontZ[q] + S.backZ[q]);
+            }
+            snode = __shfl_sync(FULLMASK, v, 0);
+            // the one child on either side completes the permutation: its makespan
+            sF[0] = snode;
+            sB[0] = snode;
+        } else {
+            unsigned um[NW];
+            job_mask<NW>(um, row, valid);
+            snode = johnson_all<NW>(T, S, row, valid, um, k, k >= 3, sF, sB);
+            if (k == 2) {
+                const int x0 = vget<NW>(row, 0), x1 = vget<NW>(row, 1);
+                int mk = 0;
+                if (lane < 2) mk = makespan_split(T, S, lane == 0 ? x0 : x1, lane == 0 ? x1 : x0);
+                const int mxy = __shfl_sync(FULLMASK, mk, 0), myx = __shfl_sync(FULLMASK, mk, 1);
+                sF[0] = lane == 0 ? mxy : myx;
+                sB[0] = lane == 0 ? myx : mxy;
+            }
+        }
+        const size_t at = (size_t)node * n;
+        // by job id, 0 for the fixed jobs
+        for (int i = lane; i < f + b; i += 32) {
+            const int j = i < f ? S.fjob[i] : S.bjob[i - f];
+            wb[at + j] = 0; we[at + j] = 0; sb[at + j] = 0; se[at + j] = 0;
+        }
+#pragma unroll
+        for (int w = 0; w < NW; w++) {
+            if (valid[w]) {
+                const size_t o = at + row[w];
+                wb[o] = wF[w]; we[o] = wB[w]; sb[o] = sF[w]; se[o] = sB[w];
+            }
+        }
+        if (X.prio_begin) {
+            // idle-time priorities of the children (bound_fsp_weak.cpp:140-146, 172-178)
+            for (int i = lane; i < f + b; i += 32) {
+                const int j = i < f ? S.fjob[i] : S.bjob[i - f];
+                X.prio_begin[at + j] = 0;
+                X.prio_end[at + j] = 0;
+            }
+#pragma unroll
+            for (int w = 0; w < NW; w++) {
+                if (valid[w]) {
+                    X.prio_begin[at + row[w]] = weak_front_idle(T, S, row[w]);
+                    X.prio_end[at + row[w]] = weak_back_idle(T, S, row[w]);
+                }
+            }
+        }
+        if (X.strong_idle && lane == 0) X.strong_idle[node] = fixed_idle(T, S, f, b, k);
         if (lane == 0) {
             node_weak[node] = wn;
             node_strong[node] = snode;
@@ -1365,6 +1482,42 @@ cudaError_t launch_explore(int nw, const DevGroup* groups, const int* ngroups_d,
     default: return PBB_EXPLORE(2, 0);
     }
 #undef PBB_EXPLORE
+}
+
+BoundShape bound_shape(int n, int m, int Ppad, int count, int sms, int optin)
+{
+    BoundShape b;
+    // as many warps as the tables and the larger scratch leave room for; where
+    // that is under a quarter of what the plain scratch holds, the plain kernel
+    // with its shared atomics is no slower
+    int plain = 8, all = PBB_BOUND_WARPS(n <= 32 ? 1 : 2);
+    while (plain > 0 && smem_bytes(n, m, Ppad, plain) > optin) plain--;
+    while (all > 0 && smem_bytes(n, m, Ppad, all, PBB_SCRATCH_ALL) > optin) all--;
+    b.all = all > 0 && 4 * all >= plain;
+    b.warps = b.all ? all : plain;
+    b.smem = b.warps > 0 ? smem_bytes(n, m, Ppad, b.warps, b.all ? PBB_SCRATCH_ALL : PBB_SCRATCH_PLAIN) : 0;
+    if (b.all) b.ctas = count < sms ? count : sms;
+    else if (b.warps > 0) b.ctas = (count + b.warps - 1) / b.warps < sms * 4 ? (count + b.warps - 1) / b.warps : sms * 4;
+    return b;
+}
+
+cudaError_t launch_bound_all(int nw, const DevInstance& I, int count, const int* sched, const int* l1, const int* l2,
+                             int* wb, int* we, int* sb, int* se, int* nweak, int* nstrong, unsigned int* status,
+                             const BoundShape& b, cudaStream_t st, BoundExtra extra)
+{
+    if (!b.all)
+        return launch_bound(nw, I, count, sched, l1, l2, wb, we, sb, se, nweak, nstrong, status, b.ctas, b.warps, b.smem,
+                            st, 0, extra);
+    if (nw == 1) {
+        cudaFuncSetAttribute(pbb_bound_all_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, b.smem);
+        pbb_bound_all_kernel<1><<<b.ctas, 32 * b.warps, b.smem, st>>>(I, count, sched, l1, l2, wb, we, sb, se, nweak,
+                                                                      nstrong, status, b.warps, extra);
+    } else {
+        cudaFuncSetAttribute(pbb_bound_all_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, b.smem);
+        pbb_bound_all_kernel<2><<<b.ctas, 32 * b.warps, b.smem, st>>>(I, count, sched, l1, l2, wb, we, sb, se, nweak,
+                                                                      nstrong, status, b.warps, extra);
+    }
+    return cudaGetLastError();
 }
 
 cudaError_t launch_bound(int nw, const DevInstance& I, int count, const int* sched, const int* l1, const int* l2,

@@ -32,6 +32,17 @@ cudaError_t launch_explore(int nw, const DevGroup* groups, const int* ngroups_d,
                            unsigned long long budget_ns, int max_rounds, int select_budget, cudaStream_t st,
                            int variant = 0, int eager = 1, int* pair_stack = nullptr, int pair_stride = 0);
 int explore_ctas_per_sm(int nw, int warps_per_cta, int smem, int variant = 0);
+// The launch of a batch of `count` nodes: kernel and block shape that fit
+// `optin` bytes of shared memory (warps 0: none does)
+struct BoundShape {
+    bool all = false;      // pbb_bound_all_kernel
+    int warps = 0, ctas = 1, smem = 0;
+};
+BoundShape bound_shape(int n, int m, int Ppad, int count, int sms, int optin);
+cudaError_t launch_bound_all(int nw, const DevInstance& I, int count, const int* sched, const int* l1, const int* l2,
+                             int* wb, int* we, int* sb, int* se, int* nweak, int* nstrong, unsigned int* status,
+                             const BoundShape& b, cudaStream_t st, BoundExtra extra = BoundExtra());
+// method (diagnostic): 0 sweeps over all positions, 1 direct scans, 2 sweeps over the free positions
 cudaError_t launch_bound(int nw, const DevInstance& I, int count, const int* sched, const int* l1, const int* l2,
                          int* wb, int* we, int* sb, int* se, int* nweak, int* nstrong, unsigned int* status, int ctas,
                          int warps_per_cta, int smem, cudaStream_t st, int method = 0, BoundExtra extra = BoundExtra());

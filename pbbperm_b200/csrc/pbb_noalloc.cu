@@ -21,7 +21,7 @@
 //     callers and waits for its stream before returning;
 //   * the calling thread's current device is the same after the call as
 //     before it (the call selects `device` only while it runs);
-//   * the block shape shrinks (8 warps down to 1) until the tables fit the
+//   * the block shape shrinks (16 warps down to 1) until the tables fit the
 //     device's per-block shared memory; if even one warp does not fit, the
 //     call returns PBB_E_INVAL.
 #include <cuda_runtime.h>
@@ -157,11 +157,11 @@ extern "C" int pbb_bound_children_noalloc(const pbb_instance* inst, int32_t john
               "device query failed");
         g_scratch_addr[device] = base;
     }
-    // block shape: the most warps (up to 8) whose tables and scratch fit the
-    // device's per-block shared memory
-    int warps = 8, smem = pbbl::smem_bytes(n, m, Ppad, warps);
-    while (warps > 1 && smem > g_smem_optin[device]) smem = pbbl::smem_bytes(n, m, Ppad, --warps);
-    if (smem > g_smem_optin[device])
+    // kernel and block shape that fit the device's per-block shared memory
+    int sms = 0;
+    NA_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device), "device query failed");
+    const pbbl::BoundShape shape = pbbl::bound_shape(n, m, Ppad, count, sms, g_smem_optin[device]);
+    if (shape.warps < 1)
         return na_fail(PBB_E_INVAL, "instance tables do not fit in this device's shared memory");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     unsigned* status = reinterpret_cast<unsigned*>(base + NA_STATUS_OFF);
@@ -190,13 +190,9 @@ extern "C" int pbb_bound_children_noalloc(const pbb_instance* inst, int32_t john
     I.n = n; I.m = m; I.P = P; I.Ppad = Ppad;
     I.p = pd; I.je = je; I.pm0 = pm; I.pm1 = pm + Ppad;
     I.min_arr = mt; I.min_dep = mt + m;
-    I.posj = nullptr;   // method 0 (sweeps over all positions) needs no position table
-    int sms = 0;
-    NA_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device), "device query failed");
-    int ctas = (count + warps - 1) / warps;
-    if (ctas > sms * 4) ctas = sms * 4;
-    NA_CK(pbbl::launch_bound(n <= 32 ? 1 : 2, I, count, sched, limit1, limit2, weak_begin, weak_end, strong_begin,
-                             strong_end, node_weak, node_strong, status, ctas, warps, smem, st),
+    I.posj = nullptr;   // the bound kernel builds its position table from the Johnson entries
+    NA_CK(pbbl::launch_bound_all(n <= 32 ? 1 : 2, I, count, sched, limit1, limit2, weak_begin, weak_end, strong_begin,
+                                 strong_end, node_weak, node_strong, status, shape, st),
           "bound kernel launch failed");
     NA_CK(cudaMemcpyAsync(&hs, status, sizeof(unsigned), cudaMemcpyDeviceToHost, st), "status read failed");
     NA_CK(cudaStreamSynchronize(st), "bound kernel failed");

@@ -5,6 +5,9 @@
 #define PBB_MAX_N 64          // jobs per instance (int8 IVM cells, two 32-bit mask words)
 #define PBB_MAX_M 32          // machines per instance (one machine per lane in recurrences)
 #define PBB_WARPS_MAX 20      // explorer warps per CTA (96 registers a thread)
+// warps of a bound kernel's CTA at most, by the 32-job words of a row: two
+// words leave shared memory for fewer, and want more registers
+#define PBB_BOUND_WARPS(nw) ((nw) == 1 ? 16 : 12)
 #define PBB_CORE_WARPS PBB_WARPS_MAX   // default of DevSearch::core_warps
 #define PBB_SPLIT_DEPTH 10    // default of DevSearch::split_depth
 #define PBB_SHARE_AFTER 64    // default of DevSearch::share_after
@@ -158,6 +161,7 @@ struct CtaShare {
 struct SmemPlan {
     int je_off, p_off, pre_off, pm_off, marr_off, mdep_off, posj_off, share_off, warp_off, warp_bytes, total;
     int je_stride;         // entries between rows of the Johnson table
+    int posj_stride;       // bytes between rows of the position table
     int fmask;             // PBB_SCRATCH_*
 };
 
@@ -165,6 +169,7 @@ struct SmemPlan {
 #define PBB_SCRATCH_PLAIN 0   // no free-position masks
 #define PBB_SCRATCH_MASKS 1   // with the masks of the explorer the warp holds
 #define PBB_SCRATCH_PAIRS 2   // kept pair bounds (bounding mode 2), no per-child tables
+#define PBB_SCRATCH_ALL 3     // Johnson values of every child of both sides (bound kernel)
 
 __host__ __device__ inline int pbb_align(int x, int a) { return (x + a - 1) / a * a; }
 
@@ -176,10 +181,14 @@ __host__ __device__ inline int pbb_machine_pad(int m) { return ((m + 3) / 4 | 1)
 // per-warp scratch: ints Fb Bb RB FR frontZ backZ rem [32 each], then
 // [fmask: u64 fmask[Ppad]] ints lbF[n] lbB[n]; shorts dF[n*m] dB[n*m]; bytes
 // fjob[n] bjob[n] row[n].  PBB_SCRATCH_PAIRS has, in place of fmask lbF lbB dF
-// dB: ints the child's vectors [128], two pair-bound buffers [Ppad each]
+// dB: ints the child's vectors [128], two pair-bound buffers [Ppad each];
+// PBB_SCRATCH_ALL: ints a warp pass's pairs [128], their values by position
+// [n][33]; shorts dF dB [m][32 or 64 children each]
 __host__ __device__ inline int pbb_warp_bytes(int n, int m, int Ppad, int fmask)
 {
     if (fmask == PBB_SCRATCH_PAIRS) return pbb_align((7 * 32 + 128 + 2 * Ppad) * 4 + 3 * n, 16);
+    if (fmask == PBB_SCRATCH_ALL)
+        return pbb_align((7 * 32 + 128 + n * 33) * 4 + 2 * m * (n <= 32 ? 32 : 64) * 2 + 3 * n, 16);
     return pbb_align((fmask ? Ppad * 8 : 0) + (2 * n + 7 * 32) * 4 + 2 * n * m * 2 + 3 * n, 16);
 }
 
@@ -199,7 +208,10 @@ __host__ __device__ inline SmemPlan pbb_smem_plan(int n, int m, int Ppad, int wa
     s.pm_off = off;   off += pbb_align(Ppad * 2, 16);
     s.marr_off = off; off += pbb_align(m * 4, 16);
     s.mdep_off = off; off += pbb_align(m * 4, 16);
-    s.posj_off = off; off += pairs ? 0 : pbb_align(n * Ppad, 16);
+    // an odd number of words between the rows of the position table lets the
+    // lanes read one pair's positions of 32 jobs without bank conflicts
+    s.posj_stride = fmask == PBB_SCRATCH_ALL ? Ppad + 4 : Ppad;
+    s.posj_off = off; off += pairs ? 0 : pbb_align(n * s.posj_stride, 16);
     s.share_off = off; off += pbb_align((int)sizeof(CtaShare) + 8 * warps, 16);
     s.warp_off = off;
     s.fmask = fmask;

@@ -113,3 +113,22 @@ def test_bound_children_ex_priorities_and_idle(n, m, seed):
             want = O.strong_node_idle(sched[i], l1[i], l2[i])
         assert g["strong_idle"][i] == want
         assert (g["weak_begin"][i] == O.weak_children(sched[i], l1[i], l2[i])[0]).all()
+
+
+@pytest.mark.parametrize("n,m,jmode", [(2, 2, 0), (3, 2, 0), (9, 3, 0), (17, 20, 0), (32, 9, 0), (33, 9, 0), (49, 20, 1),
+                                       (64, 20, 0), (64, 5, 2), (31, 32, 0), (46, 32, 0), (57, 29, 0)])
+def test_children_bounds_equal_the_direct_scans(n, m, jmode):
+    """The bound kernel's values against per-child scans, nodes of every depth
+    (each warp split of small rows, one and two words, odd and even middles,
+    and tables too large for its scratch), a handful and many at once."""
+    p = synthetic_instance(n * m, n, m)
+    rng = np.random.default_rng(n)
+    for count in (1, 5, 700):
+        sched = np.argsort(rng.random((count, n)), axis=1).astype(np.int32)
+        k = (np.arange(count) % (n + 1)).astype(np.int64) if count > 5 else rng.integers(1, n + 1, size=count)
+        front = (rng.random(count) * (n - k + 1)).astype(np.int64)
+        l1, l2 = (front - 1).astype(np.int32), (front + k).astype(np.int32)
+        got = pb.bound_children(p, sched, l1, l2, johnson_mode=jmode)
+        want = pb.bound_children(p, sched, l1, l2, johnson_mode=jmode, method=1)
+        for key in want:
+            assert (got[key] == want[key]).all(), (key, n, m)
