@@ -323,7 +323,11 @@ static int engine_create(const pbb_instance* inst, const pbb_config* cfg, pbb_en
         // earlyStopJohnson changes the values of pruned children only, which
         // these builds do not compute: they serve both settings
         const int cap = max_smem_optin(e->dev);
-        int w = e->warps;
+        // (instances whose tables hold the general build below its full CTA
+        // keep that count in every build: the work statistics report one)
+        const bool wide = cfg->warps_per_cta <= 0 && e->warps == PBB_WARPS_MAX && H.n * H.m > PBB_WIDE_FROM;
+        if (wide) e->pair_variant += 2;
+        int w = wide ? PBB_WIDE_WARPS : e->warps;
         while (w > 1 && pbbl::smem_bytes(H.n, H.m, H.Ppad, w, PBB_SCRATCH_PAIRS) > cap) w--;
         e->pair_smem = pbbl::smem_bytes(H.n, H.m, H.Ppad, w, PBB_SCRATCH_PAIRS);
         e->pair_stride = H.n * H.Ppad;

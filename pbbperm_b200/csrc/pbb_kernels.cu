@@ -873,9 +873,10 @@ __global__ void pbb_root_kernel(const DevGroup* groups, int ngroups, const int* 
 // earlyStopJohnson settings; VAR = 2 also records sampled nodes into the
 // group's SampleBuf.  VAR = 3 and 4 bound in mode 2 by kept pair bounds: 3 the
 // default search (MinMin, no findAll, rows not sorted, compiled in), 4 every
-// other search of that mode whose rule bounds the side it chooses.
+// other search of that mode whose rule bounds the side it chooses; 5 and 6 are
+// their builds for 32 warps a CTA.
 template <int NW, int VAR>
-__global__ void __launch_bounds__(32 * PBB_WARPS_MAX, 1)
+__global__ void __launch_bounds__(32 * PBB_EXPLORE_WARPS(VAR), 1)
 pbb_explore_kernel(const DevGroup* groups, const int* ngroups_d, int warps_per_cta, unsigned long long budget_ns,
                    int max_rounds, int select_budget, int eager, int* pair_stack, int pair_stride)
 {
@@ -1050,7 +1051,7 @@ pbb_explore_kernel(const DevGroup* groups, const int* ngroups_d, int warps_per_c
         if (best < known && lane_id() == 0) atomicMin(&H->best, best);
         if (r == 1) {
             since++;
-            bound_current<NW, (VAR == 1 || VAR == 2), (VAR == 2), (VAR >= 3 ? VAR - 2 : 0)>(G, T, S, B, id, R, mode, best, C);
+            bound_current<NW, (VAR == 1 || VAR == 2), (VAR == 2), (VAR >= 3 ? 2 - (VAR & 1) : 0)>(G, T, S, B, id, R, mode, best, C);
         }
         if (C.decomposed >= (1u << 13)) flush_counters(G, C);
         if (r == 0) {
@@ -1408,6 +1409,8 @@ int explore_ctas_per_sm(int nw, int warps_per_cta, int smem, int variant)
         case 2: return explore_occupancy<1, 2>(warps_per_cta, smem);
         case 3: return explore_occupancy<1, 3>(warps_per_cta, smem);
         case 4: return explore_occupancy<1, 4>(warps_per_cta, smem);
+        case 5: return explore_occupancy<1, 5>(warps_per_cta, smem);
+        case 6: return explore_occupancy<1, 6>(warps_per_cta, smem);
         default: return explore_occupancy<1, 0>(warps_per_cta, smem);
         }
     }
@@ -1416,6 +1419,8 @@ int explore_ctas_per_sm(int nw, int warps_per_cta, int smem, int variant)
     case 2: return explore_occupancy<2, 2>(warps_per_cta, smem);
     case 3: return explore_occupancy<2, 3>(warps_per_cta, smem);
     case 4: return explore_occupancy<2, 4>(warps_per_cta, smem);
+    case 5: return explore_occupancy<2, 5>(warps_per_cta, smem);
+    case 6: return explore_occupancy<2, 6>(warps_per_cta, smem);
     default: return explore_occupancy<2, 0>(warps_per_cta, smem);
     }
 }
@@ -1471,6 +1476,8 @@ cudaError_t launch_explore(int nw, const DevGroup* groups, const int* ngroups_d,
         case 2: return PBB_EXPLORE(1, 2);
         case 3: return PBB_EXPLORE(1, 3);
         case 4: return PBB_EXPLORE(1, 4);
+        case 5: return PBB_EXPLORE(1, 5);
+        case 6: return PBB_EXPLORE(1, 6);
         default: return PBB_EXPLORE(1, 0);
         }
     }
@@ -1479,6 +1486,8 @@ cudaError_t launch_explore(int nw, const DevGroup* groups, const int* ngroups_d,
     case 2: return PBB_EXPLORE(2, 2);
     case 3: return PBB_EXPLORE(2, 3);
     case 4: return PBB_EXPLORE(2, 4);
+    case 5: return PBB_EXPLORE(2, 5);
+    case 6: return PBB_EXPLORE(2, 6);
     default: return PBB_EXPLORE(2, 0);
     }
 #undef PBB_EXPLORE

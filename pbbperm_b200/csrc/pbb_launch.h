@@ -23,7 +23,8 @@ cudaError_t launch_root(int nw, const DevGroup* groups, int ngroups, const int* 
 cudaError_t launch_lower_ub(const DevGroup* groups, int g, int ub, cudaStream_t st);
 // variant: 0 = no row sort, no early Johnson exit, no sampling; 1 = each
 // group's sortedDFS / earlyStopJohnson settings; 2 = as 1 and record sampled
-// nodes (groups' SampleBuf); 3 and 4 = kept pair bounds (pairs_variant), launched
+// nodes (groups' SampleBuf); 3 to 6 = kept pair bounds (pairs_variant; 5 and 6
+// for up to PBB_WIDE_WARPS a CTA), launched
 // with the PBB_SCRATCH_PAIRS shared memory and with pair_stack, pair_stride
 // ints for each warp of the grid (at least jobs x padded machine pairs).
 // eager = 0: a short window, which splits work only as often as share_after

@@ -5,6 +5,19 @@
 #define PBB_MAX_N 64          // jobs per instance (int8 IVM cells, two 32-bit mask words)
 #define PBB_MAX_M 32          // machines per instance (one machine per lane in recurrences)
 #define PBB_WARPS_MAX 20      // explorer warps per CTA (96 registers a thread)
+// Warps of an explorer CTA at most: 20 at 96 registers a thread, or 32 at 64
+// in the wide builds of the variants with kept pair bounds (5 and 6, of 3 and
+// 4), whose scratch leaves the room.
+#define PBB_WIDE_WARPS 32
+#define PBB_EXPLORE_WARPS(var) ((var) >= 5 ? PBB_WIDE_WARPS : PBB_WARPS_MAX)
+// The wide builds pay where a search is long enough to be bound by throughput;
+// below, where it is bound by the time one node takes and by how fast work
+// spreads, their spilled registers and additional warps cost a little.  The
+// tree is not known beforehand, so the line is drawn by the instance: measured
+// ms with 20 and with 32 warps, 50x20 (56 M nodes) 194 and 167, 20x20 (13 M)
+// 38.9 and 31.9, 16x20 (0.6 M) 2.35 and 2.51, 20x10 (0.12 M) 0.90 and 0.98,
+// 12x10 0.21 and 0.23.
+#define PBB_WIDE_FROM 320             // jobs x machines above which they are used
 // warps of a bound kernel's CTA at most, by the 32-job words of a row: two
 // words leave shared memory for fewer, and want more registers
 #define PBB_BOUND_WARPS(nw) ((nw) == 1 ? 16 : 12)
