@@ -9,7 +9,7 @@
 // in the wide builds of the variants with kept pair bounds (5 and 6, of 3 and
 // 4), whose scratch leaves the room.
 #define PBB_WIDE_WARPS 32
-#define PBB_EXPLORE_WARPS(var) ((var) >= 5 ? PBB_WIDE_WARPS : PBB_WARPS_MAX)
+#define PBB_EXPLORE_WARPS(var) ((var) == 5 || (var) == 6 ? PBB_WIDE_WARPS : PBB_WARPS_MAX)
 // The wide builds pay where a search is long enough to be bound by throughput;
 // below, where it is bound by the time one node takes and by how fast work
 // spreads, their spilled registers and additional warps cost a little.  The
@@ -182,7 +182,7 @@ struct SmemPlan {
 #define PBB_SCRATCH_PLAIN 0   // no free-position masks
 #define PBB_SCRATCH_MASKS 1   // with the masks of the explorer the warp holds
 #define PBB_SCRATCH_PAIRS 2   // kept pair bounds (bounding mode 2), no per-child tables
-#define PBB_SCRATCH_ALL 3     // Johnson values of every child of both sides (bound kernel)
+#define PBB_SCRATCH_ALL 3     // Johnson values of every child of both sides (bound kernel, bounding mode 1)
 
 __host__ __device__ inline int pbb_align(int x, int a) { return (x + a - 1) / a * a; }
 

@@ -56,3 +56,21 @@ def test_smallest_rows_from_no_bound(n, m):
     assert got["complete"] and got["cost"] == want["best"]
     for k in KEYS:
         assert got[k] == want[k], (k, got[k], want[k])
+
+
+@pytest.mark.parametrize("n,m,seed,ub", [(12, 10, 3, 1171), (13, 10, 3, 1277), (9, 20, 2, 1400), (32, 10, 3, 2110),
+                                         (33, 10, 3, 2070), (14, 32, 1, 2300)])
+@pytest.mark.parametrize("opt", [dict(), dict(adaptiveBranchingMode=2, sortedDFS=1), dict(adaptiveBranchingMode=1),
+                                 dict(adaptiveBranchingMode=-1, findAll=True)], ids=["0", "1", "2", "3"])
+def test_mode_1_counts_equal_the_oracle(n, m, seed, ub, opt):
+    """Bounding mode 1: rows of one word (values by position) and of two."""
+    p = synthetic_instance(seed, n, m)
+    want = Oracle(p).solve(ub, bound_mode=1, branch_mode=opt.get("adaptiveBranchingMode", 3),
+                           find_all=opt.get("findAll", False), sorted_dfs=opt.get("sortedDFS", 0), node_limit=20000)
+    if not want["complete"] or want["found"]:
+        pytest.skip("not a small proof")
+    with pb.Engine(p, pb.Config(boundingMode=1, nbIVMs=4096, **opt)) as e:
+        got = e.solve(ub=ub)
+    assert got["complete"] and not got["found"]
+    for k in KEYS:
+        assert got[k] == want[k], (k, got[k], want[k])
