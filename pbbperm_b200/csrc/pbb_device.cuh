@@ -544,7 +544,7 @@ __device__ __forceinline__ void johnson_children(const CtaTables& T, const WarpS
         int Apre = 0, Bpre = 0, PMx = NEG_INF;
         if (act) {
             for (int t = 0; t < n; t++) {
-                const unsigned long long e = col[t * T.Ppad];
+                const unsigned long long e = col[t * T.je_stride];
                 const int u = JE_JOB(e);
                 const unsigned bit = 1u << (u & 31);
                 unsigned uw = um[0], fw = sF[0], bw = sB[0];
@@ -579,7 +579,7 @@ __device__ __forceinline__ void johnson_children(const CtaTables& T, const WarpS
             }
             int Asuf = 0, Bsuf = 0, SMx = NEG_INF;
             for (int t = n - 1; t >= 0; t--) {
-                const unsigned long long e = col[t * T.Ppad];
+                const unsigned long long e = col[t * T.je_stride];
                 const int u = JE_JOB(e);
                 const unsigned bit = 1u << (u & 31);
                 unsigned uw = um[0], fw = sF[0], bw = sB[0];
@@ -652,7 +652,7 @@ __device__ __forceinline__ void johnson_direct(const CtaTables& T, const WarpScr
             const unsigned long long* col = T.je + i;
 #pragma unroll 2
             for (int t = 0; t < n; t++) {
-                const unsigned long long e = col[t * T.Ppad];
+                const unsigned long long e = col[t * T.je_stride];
                 const bool fr = (fm >> JE_JOB(e)) & 1ull;
                 const int t0n = t0 + JE_A(e);
                 const int t1n = max(t1, t0n + JE_C(e)) + JE_B(e);
@@ -794,7 +794,7 @@ __device__ __forceinline__ void johnson_direct_chains(const CtaTables& T, const 
             while (pm) {
                 const int t = low_pos(pm);
                 pm &= pm - 1;
-                const unsigned long long e = col[t * T.Ppad];
+                const unsigned long long e = col[t * T.je_stride];
                 const int a = JE_A(e), bb = JE_B(e), cc = JE_C(e);
 #pragma unroll
                 for (int c = 0; c < C; c++) {
@@ -868,7 +868,7 @@ __device__ __forceinline__ void johnson_sweep_masked(const CtaTables& T, const W
             while (fwd) {
                 const int t = low_pos(fwd);
                 fwd &= fwd - 1;
-                const unsigned long long e = col[t * T.Ppad];
+                const unsigned long long e = col[t * T.je_stride];
                 const int u = JE_JOB(e);
                 const unsigned bit = 1u << (u & 31);
                 unsigned fw = sF[0], bw = sB[0];
@@ -894,7 +894,7 @@ __device__ __forceinline__ void johnson_sweep_masked(const CtaTables& T, const W
             while (r) {
                 const int t = high_pos(r);
                 r &= ~((M)1 << t);
-                const unsigned long long e = col[t * T.Ppad];
+                const unsigned long long e = col[t * T.je_stride];
                 const int u = JE_JOB(e);
                 const unsigned bit = 1u << (u & 31);
                 unsigned fw = sF[0], bw = sB[0];

@@ -69,7 +69,7 @@ __device__ __forceinline__ void load_tables(const DevInstance& I, unsigned char*
         for (int i = tid; i < I.n * I.Ppad; i += nt) je[i] = I.je[i];
     } else {
         for (int t = tid / 32; t < I.n; t += nt / 32)
-            for (int i = tid & 31; i < I.Ppad; i += 32) je[t * sp.je_stride + i] = I.je[t * I.Ppad + i];
+            for (int i = tid & 31; i < I.P; i += 32) je[t * sp.je_stride + i] = I.je[t * I.Ppad + i];
     }
     for (int i = tid; i < I.n * mp; i += nt) {
         const int j = i / mp, k = i - j * mp;

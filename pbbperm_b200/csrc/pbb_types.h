@@ -214,7 +214,11 @@ __host__ __device__ inline SmemPlan pbb_smem_plan(int n, int m, int Ppad, int wa
     const int times = n * pbb_machine_pad(m) * 4;
     SmemPlan s;
     int off = 0;
-    s.je_stride = pairs ? Ppad + 1 : Ppad;
+    // without the padding past the last pair (whatever the Johnson mode, there
+    // are no more pairs than machine pairs): it pays for the padded rows of the
+    // processing times, so that no instance needs more than with tight rows
+    const int tight = m * (m - 1) / 2;
+    s.je_stride = pairs ? Ppad + 1 : (tight < Ppad ? tight : Ppad);
     s.je_off = off;   off += pbb_align(n * s.je_stride * 8, 16);
     s.p_off = off;    off += times;
     s.pre_off = off;  off += pairs ? times : 0;
