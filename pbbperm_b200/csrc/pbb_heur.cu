@@ -493,8 +493,9 @@ int heur_batch(const pbb_instance* inst, int32_t count, int32_t device, const Ig
     }
     pbbh::DeviceGuard keep_callers_device;
     if (cudaSetDevice(device) != cudaSuccess) return pbbt::fail(PBB_E_CUDA, "cudaSetDevice failed");
-    cudaStream_t st = nullptr;
-    if (pbbh::stream_take(&st, device) != cudaSuccess) return pbbt::fail(PBB_E_CUDA, "stream creation failed");
+    pbbh::Lease lease;
+    if (pbbh::stream_take(&lease, device) != cudaSuccess) return pbbt::fail(PBB_E_CUDA, "stream creation failed");
+    const cudaStream_t st = lease.st;
     unsigned char* d = nullptr;
     int rc = PBB_OK;
     do {
@@ -503,7 +504,7 @@ int heur_batch(const pbb_instance* inst, int32_t count, int32_t device, const Ig
         const size_t o_tasks = C.take(sizeof(NehTask) * count), o_p = C.take(sizeof(int) * words);
         const size_t filled = C.bytes;
         const size_t o_out = C.take(sizeof(int) * out_words);
-        if (pbbh::mem_alloc((void**)&d, C.bytes, device, st) != cudaSuccess) {
+        if (pbbh::mem_alloc((void**)&d, C.bytes, lease) != cudaSuccess) {
             rc = pbbt::fail(PBB_E_NOMEM, "device allocation failed");
             break;
         }
@@ -543,8 +544,8 @@ int heur_batch(const pbb_instance* inst, int32_t count, int32_t device, const Ig
         }
     } while (0);
     cudaStreamSynchronize(st);
-    pbbh::mem_free(d, st);
-    pbbh::stream_give(st, device);
+    pbbh::mem_free(d, lease);
+    pbbh::stream_give(lease);
     return rc;
 }
 

@@ -129,7 +129,8 @@ struct pbb_engine {
     pbb_config cfg{};
     HostTables H;
     int dev = 0;
-    cudaStream_t st = nullptr;
+    pbbh::Lease lease;
+    cudaStream_t st = nullptr;        // the lease's
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     int nw = 2, warps = 0, ctas = 0, smem = 0, root_smem = 0;
     // the launch of the explorer variants 3 to 7, pair_warps 0: not used
@@ -285,14 +286,16 @@ int pbb_engine_destroy(pbb_engine* e)
     if (!e) return PBB_OK;
     pbbh::DeviceGuard keep_callers_device;
     cudaSetDevice(e->dev);
-    if (e->st) cudaStreamSynchronize(e->st);
-    pbbh::mem_free(e->block, e->st);
-    pbbh::mem_free(e->pair_stack, e->st);
-    cudaFree(e->sample_d);
-    cudaFree(e->sample_rec);
-    if (e->ev0) cudaEventDestroy(e->ev0);
-    if (e->ev1) cudaEventDestroy(e->ev1);
-    pbbh::stream_give(e->st, e->dev);
+    if (pbbh::alive(e->lease)) {
+        cudaStreamSynchronize(e->st);
+        pbbh::mem_free(e->block, e->lease);
+        pbbh::mem_free(e->pair_stack, e->lease);
+        cudaFree(e->sample_d);
+        cudaFree(e->sample_rec);
+        if (e->ev0) cudaEventDestroy(e->ev0);
+        if (e->ev1) cudaEventDestroy(e->ev1);
+        pbbh::stream_give(e->lease);
+    }
     delete e;
     return PBB_OK;
 }
@@ -307,7 +310,8 @@ static int engine_create(const pbb_instance* inst, const pbb_config* cfg, pbb_en
     e->dev = cfg->device;
     pbbh::DeviceGuard keep_callers_device;
     CK(cudaSetDevice(e->dev));
-    CK(pbbh::stream_take(&e->st, e->dev));
+    CK(pbbh::stream_take(&e->lease, e->dev));
+    e->st = e->lease.st;
     CK(cudaEventCreate(&e->ev0));
     CK(cudaEventCreate(&e->ev1));
     const HostTables& H = e->H;
@@ -332,8 +336,8 @@ static int engine_create(const pbb_instance* inst, const pbb_config* cfg, pbb_en
         e->pair_smem = pbbl::smem_bytes(H.n, H.m, H.Ppad, w, PBB_SCRATCH_PAIRS);
         e->pair_stride = H.n * H.Ppad;
         if (e->pair_smem <= cap) {
-            if (pbbh::mem_alloc((void**)&e->pair_stack, sizeof(int) * (size_t)e->ctas * w * e->pair_stride, e->dev,
-                                e->st) == cudaSuccess)
+            if (pbbh::mem_alloc((void**)&e->pair_stack, sizeof(int) * (size_t)e->ctas * w * e->pair_stride,
+                                e->lease) == cudaSuccess)
                 e->pair_warps = w;
             else
                 cudaGetLastError();   // no room: the general build needs none
@@ -363,7 +367,7 @@ static int engine_create(const pbb_instance* inst, const pbb_config* cfg, pbb_en
     const size_t o_ask = C.take(sizeof(unsigned) * ((B + 31) / 32));
     const size_t o_vec = C.take(4 * B * npad), o_perm = C.take(B * npad);
     const size_t o_mat = C.take(B * levels * npad), o_path = C.take(B * levels * PBB_PATH_INTS * sizeof(int));
-    CK(pbbh::mem_alloc((void**)&e->block, C.bytes, e->dev, e->st));
+    CK(pbbh::mem_alloc((void**)&e->block, C.bytes, e->lease));
     unsigned char* d = e->block;
     e->ub_d = reinterpret_cast<int*>(d + o_ub);
     e->root_d = reinterpret_cast<int*>(d + o_root);
@@ -532,7 +536,7 @@ int pbb_init_from_fac(pbb_engine* e, int32_t ub, const int32_t* root_perm, int32
     }
     const size_t iv_bytes = sizeof(int) * iv.size(), id_bytes = sizeof(int) * nb_intervals;
     int* ival_d = nullptr;
-    CK(pbbh::mem_alloc((void**)&ival_d, iv_bytes + id_bytes, e->dev, e->st));
+    CK(pbbh::mem_alloc((void**)&ival_d, iv_bytes + id_bytes, e->lease));
     int* ids_d = ival_d + iv.size();
     cudaError_t err = cudaMemcpyAsync(ival_d, iv.data(), iv_bytes, cudaMemcpyHostToDevice, e->st);
     if (!err) err = cudaMemcpyAsync(ids_d, id.data(), sizeof(int) * nb_intervals, cudaMemcpyHostToDevice, e->st);
@@ -545,7 +549,7 @@ int pbb_init_from_fac(pbb_engine* e, int32_t ub, const int32_t* root_perm, int32
                                 nb_intervals, ids_d);
     if (!err) err = cudaStreamSynchronize(e->st);
     if (!err) e->pending = false;
-    pbbh::mem_free(ival_d, e->st);
+    pbbh::mem_free(ival_d, e->lease);
     if (err) return fail(PBB_E_CUDA, std::string("init_from_fac: ") + cudaGetErrorString(err));
     GroupCtl c;
     CK(cudaMemcpy(&c, e->ctl, sizeof(c), cudaMemcpyDeviceToHost));
@@ -875,8 +879,9 @@ static int bound_children_impl(const pbb_instance* inst, int32_t johnson_mode, i
     }
     pbbh::DeviceGuard keep_callers_device;
     CK(cudaSetDevice(device));
-    cudaStream_t st = nullptr;
-    CK(pbbh::stream_take(&st, device));
+    pbbh::Lease lease;
+    CK(pbbh::stream_take(&lease, device));
+    const cudaStream_t st = lease.st;
     const size_t cn = (size_t)count * n * sizeof(int), c1 = (size_t)count * sizeof(int);
     const bool want_prio = prio_begin || prio_end;
     // one block: tables, status and inputs, then the outputs.  Up to
@@ -897,7 +902,7 @@ static int bound_children_impl(const pbb_instance* inst, int32_t johnson_mode, i
         if (q < 6 || (q < 8 && want_prio) || (q == 8 && strong_idle)) out[q].off = C.take(out[q].bytes);
     unsigned char* d = nullptr;
     do {
-        cudaError_t ce = pbbh::mem_alloc((void**)&d, C.bytes, device, st);
+        cudaError_t ce = pbbh::mem_alloc((void**)&d, C.bytes, lease);
         if (ce != cudaSuccess) { rc = cuda_fail(ce, "cudaMalloc"); break; }
         const bool packed_in = o_inputs_end - o_tables_end <= PACKED_BYTES;
         std::vector<unsigned char> host(packed_in ? o_inputs_end : o_tables_end, 0);
@@ -953,8 +958,8 @@ static int bound_children_impl(const pbb_instance* inst, int32_t johnson_mode, i
                 if (o.host && o.off) memcpy(o.host, packed.data() + (o.off - o_inputs_end), o.bytes);
     } while (0);
     cudaStreamSynchronize(st);
-    pbbh::mem_free(d, st);
-    pbbh::stream_give(st, device);
+    pbbh::mem_free(d, lease);
+    pbbh::stream_give(lease);
     return rc;
 }
 

@@ -39,16 +39,18 @@ unsigned long long context_id()
     return get && get(nullptr, &id) == 0 ? id : 0;
 }
 
-// What is kept for a device belongs to its context: with another one current,
-// it is gone and forgotten.
+// What is known of a device belongs to its context: with another one current,
+// it is gone and forgotten, the blocks in use too.  What those are replaced by
+// may stand at the same addresses, so their owners are told apart by the
+// context of their lease, not by the address.
 unsigned long long g_context[PBB_MEM_DEVICES];
 
-void check_context(int device)
+unsigned long long check_context(int device)
 {
-    if (device < 0 || device >= PBB_MEM_DEVICES) return;
     const unsigned long long id = context_id();
+    if (device < 0 || device >= PBB_MEM_DEVICES) return id;
     std::lock_guard<std::mutex> lock(g_mem_mutex);
-    if (g_context[device] == id) return;
+    if (g_context[device] == id) return id;
     g_context[device] = id;
     g_pool[device] = nullptr;
     g_pool_tried[device] = false;
@@ -57,6 +59,11 @@ void check_context(int device)
         if (g_kept[i].device == device) g_kept.erase(g_kept.begin() + i);
         else i++;
     }
+    for (auto it = g_big.begin(); it != g_big.end();) {
+        if (it->second.device == device) it = g_big.erase(it);
+        else ++it;
+    }
+    return id;
 }
 
 // A kept block of at most a quarter more than asked for, or NULL.
@@ -114,10 +121,13 @@ cudaMemPool_t pool_of(int device)
 
 namespace pbbh {
 
-cudaError_t mem_alloc(void** out, size_t bytes, int device, cudaStream_t st)
+bool alive(const Lease& l) { return l.st && context_id() == l.context; }
+
+cudaError_t mem_alloc(void** out, size_t bytes, const Lease& l)
 {
     *out = nullptr;
-    check_context(device);
+    const int device = l.device;
+    if (check_context(device) != l.context) return cudaErrorInvalidResourceHandle;
     const bool big = bytes > PBB_BIG_BLOCK;
     cudaMemPool_t p = pool_of(device);
     cudaError_t rc = cudaErrorMemoryAllocation;
@@ -133,7 +143,7 @@ cudaError_t mem_alloc(void** out, size_t bytes, int device, cudaStream_t st)
             if ((*out = take_kept(bytes, device))) return cudaSuccess;
             rc = cudaMalloc(out, bytes);
         } else {
-            rc = p ? cudaMallocFromPoolAsync(out, bytes, p, st) : cudaMalloc(out, bytes);
+            rc = p ? cudaMallocFromPoolAsync(out, bytes, p, l.st) : cudaMalloc(out, bytes);
         }
     }
     if (rc == cudaSuccess && big) {
@@ -143,9 +153,9 @@ cudaError_t mem_alloc(void** out, size_t bytes, int device, cudaStream_t st)
     return rc;
 }
 
-void mem_free(void* p, cudaStream_t st)
+void mem_free(void* p, const Lease& l)
 {
-    if (!p) return;
+    if (!p || !alive(l)) return;
     bool big = false;
     {
         std::lock_guard<std::mutex> lock(g_mem_mutex);
@@ -164,34 +174,39 @@ void mem_free(void* p, cudaStream_t st)
         }
     }
     if (!big) {
-        if (cudaFreeAsync(p, st) == cudaSuccess) return;
+        if (cudaFreeAsync(p, l.st) == cudaSuccess) return;
         cudaGetLastError();
     }
     cudaFree(p);
 }
 
-cudaError_t stream_take(cudaStream_t* st, int device)
+cudaError_t stream_take(Lease* l, int device)
 {
-    check_context(device);
+    l->device = device;
+    l->context = check_context(device);
     if (device >= 0 && device < PBB_MEM_DEVICES) {
         std::lock_guard<std::mutex> lock(g_mem_mutex);
         while (!g_streams[device].empty()) {
-            *st = g_streams[device].back();
+            l->st = g_streams[device].back();
             g_streams[device].pop_back();
-            if (cudaStreamQuery(*st) == cudaSuccess) return cudaSuccess;
+            if (cudaStreamQuery(l->st) == cudaSuccess) return cudaSuccess;
             cudaGetLastError();
         }
     }
-    return cudaStreamCreateWithFlags(st, cudaStreamNonBlocking);
+    l->st = nullptr;
+    return cudaStreamCreateWithFlags(&l->st, cudaStreamNonBlocking);
 }
 
-void stream_give(cudaStream_t st, int device)
+void stream_give(Lease& l)
 {
-    if (!st) return;
-    if (device >= 0 && device < PBB_MEM_DEVICES) {
+    const cudaStream_t st = l.st;
+    const bool valid = alive(l);
+    l.st = nullptr;
+    if (!valid) return;
+    if (l.device >= 0 && l.device < PBB_MEM_DEVICES) {
         std::lock_guard<std::mutex> lock(g_mem_mutex);
-        if (g_streams[device].size() < PBB_STREAMS_KEPT) {
-            g_streams[device].push_back(st);
+        if (g_streams[l.device].size() < PBB_STREAMS_KEPT) {
+            g_streams[l.device].push_back(st);
             return;
         }
     }

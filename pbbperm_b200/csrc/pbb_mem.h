@@ -20,14 +20,24 @@
 #define PBB_STREAMS_KEPT 8
 
 namespace pbbh {
-// `device` is the current device; the memory belongs to stream `st`'s order
-cudaError_t mem_alloc(void** out, size_t bytes, int device, cudaStream_t st);
-// the work that used p has finished
-void mem_free(void* p, cudaStream_t st);
-// a non-blocking stream of the current device
-cudaError_t stream_take(cudaStream_t* st, int device);
-// `st` has no work left
-void stream_give(cudaStream_t st, int device);
+// A stream lent to an object or call.  The object's memory, events and graphs
+// are of the same context; they die with it when the device is reset.
+struct Lease {
+    cudaStream_t st = nullptr;
+    int device = 0;
+    unsigned long long context = 0;
+};
+// All of these: the lease's device is current.
+// a non-blocking stream
+cudaError_t stream_take(Lease* l, int device);
+// the context of the lease is the device's current one: its handles are valid
+bool alive(const Lease& l);
+// memory in the order of the lease's stream
+cudaError_t mem_alloc(void** out, size_t bytes, const Lease& l);
+// the work that used p has finished; nothing to do when the lease is not alive
+void mem_free(void* p, const Lease& l);
+// the stream has no work left but frees; forgotten when the lease is not alive
+void stream_give(Lease& l);
 
 // sub-buffers of one block, each on a 256-byte boundary
 struct Carver {

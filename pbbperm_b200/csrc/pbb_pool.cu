@@ -101,7 +101,8 @@ struct Arena {
 struct pbb_pool {
     pbb_pool_config cfg{};
     int dev = 0;
-    cudaStream_t st = nullptr;
+    pbbh::Lease lease;
+    cudaStream_t st = nullptr;  // the lease's
     int nw = 1, npad = 32, warps = 8, cpi = 1, epw = 1, smem = 0, root_smem = 0;
     int max_slots = 0;          // resident instances at most
     int grid = 0;               // CTAs of a window launch (all the CTAs of this shape the GPU holds)
@@ -161,15 +162,17 @@ extern "C" int pbb_pool_destroy(pbb_pool* P)
     if (!P) return PBB_OK;
     pbbh::DeviceGuard keep_callers_device;
     cudaSetDevice(P->dev);
-    if (P->st) cudaStreamSynchronize(P->st);
-    for (auto& shape : P->window)
-        for (cudaGraphExec_t g : shape)
-            if (g) cudaGraphExecDestroy(g);
-    pbbh::mem_free(P->arena, P->st);
-    pbbh::mem_free(P->block, P->st);
-    pbbh::mem_free(P->pair_stack, P->st);
-    cudaFreeHost(P->ctl_h);
-    pbbh::stream_give(P->st, P->dev);
+    if (pbbh::alive(P->lease)) {
+        cudaStreamSynchronize(P->st);
+        for (auto& shape : P->window)
+            for (cudaGraphExec_t g : shape)
+                if (g) cudaGraphExecDestroy(g);
+        pbbh::mem_free(P->arena, P->lease);
+        pbbh::mem_free(P->block, P->lease);
+        pbbh::mem_free(P->pair_stack, P->lease);
+        cudaFreeHost(P->ctl_h);
+        pbbh::stream_give(P->lease);
+    }
     delete P;
     return PBB_OK;
 }
@@ -230,7 +233,8 @@ int pool_create(const pbb_pool_config* in, pbb_pool* P, int most)
     P->dev = c.device;
     pbbh::DeviceGuard keep_callers_device;
     PCK(cudaSetDevice(P->dev), "cudaSetDevice failed");
-    PCK(pbbh::stream_take(&P->st, P->dev), "stream creation failed");
+    PCK(pbbh::stream_take(&P->lease, P->dev), "stream creation failed");
+    P->st = P->lease.st;
     P->nw = c.max_jobs <= 32 ? 1 : 2;
     P->npad = 32 * P->nw;
     P->warps = c.warps_per_cta;
@@ -299,7 +303,7 @@ int pool_create(const pbb_pool_config* in, pbb_pool* P, int most)
         const size_t o_n = C.take(sizeof(int)), o_ub = C.take(sizeof(int) * S);
         const size_t o_roots = C.take(sizeof(int) * S * PBB_MAX_N), o_ivals = C.take(sizeof(int) * S * 2 * PBB_MAX_N);
         const size_t o_neh = C.take(sizeof(int) * S * (PBB_MAX_N + 1)), o_tasks = C.take(sizeof(NehTask) * S);
-        PCK(pbbh::mem_alloc((void**)&P->block, C.bytes, P->dev, P->st), "table memory");
+        PCK(pbbh::mem_alloc((void**)&P->block, C.bytes, P->lease), "table memory");
         P->tables = P->block + o_tables;
         P->ctl = reinterpret_cast<GroupCtl*>(P->block + o_ctl);
         P->groups_d = reinterpret_cast<DevGroup*>(P->block + o_groups);
@@ -318,7 +322,7 @@ int pool_create(const pbb_pool_config* in, pbb_pool* P, int most)
     if (P->pair_smem || P->tail_pair_smem) {
         const size_t w = std::max((size_t)P->grid * P->warps, (size_t)P->tail_grid * P->tail_warps);
         P->pair_stride = c.max_jobs * P->Ppad_max;
-        if (pbbh::mem_alloc((void**)&P->pair_stack, sizeof(int) * w * P->pair_stride, P->dev, P->st) != cudaSuccess) {
+        if (pbbh::mem_alloc((void**)&P->pair_stack, sizeof(int) * w * P->pair_stride, P->lease) != cudaSuccess) {
             cudaGetLastError();       // no room: the general build needs none
             P->pair_stack = nullptr;
             P->pair_smem = P->tail_pair_smem = 0;
@@ -329,7 +333,7 @@ int pool_create(const pbb_pool_config* in, pbb_pool* P, int most)
     if (explorer_block_bytes(E, P->npad, P->cfg.max_jobs) > P->arena_bytes)
         return pfail(PBB_E_INVAL, "explorer_bytes is smaller than one instance's footprint");
     P->arena_bytes = std::min(P->arena_bytes, explorer_block_bytes(E, P->npad, c.max_jobs) * (size_t)P->max_slots);
-    PCK(pbbh::mem_alloc((void**)&P->arena, P->arena_bytes, P->dev, P->st), "explorer memory");
+    PCK(pbbh::mem_alloc((void**)&P->arena, P->arena_bytes, P->lease), "explorer memory");
     P->alloc.init(P->arena_bytes);
     P->slots.assign(S, Slot());
     return PBB_OK;

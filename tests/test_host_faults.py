@@ -1,0 +1,85 @@
+"""The library's host code on a fake CUDA runtime (tests/fake_cuda.cpp), where
+calls can be made to fail and a device can be reset without a GPU."""
+import ctypes
+import os
+import shutil
+import subprocess
+
+import numpy as np
+import pytest
+
+import pbbperm_b200 as pb
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+CSRC = os.path.join(ROOT, "pbbperm_b200", "csrc")
+i32p = ctypes.POINTER(ctypes.c_int32)
+
+
+@pytest.fixture(scope="session")
+def fake_so(tmp_path_factory):
+    so = str(tmp_path_factory.mktemp("fake") / "libfake.so")
+    # -Bsymbolic: the fake runtime is this library's alone
+    subprocess.check_call(["g++", "-w", "-shared", "-fPIC", "-O1", "-std=c++17", "-Wl,-Bsymbolic",
+                           "-I", "/usr/local/cuda/include", "-I", CSRC, "-o", so, "-x", "c++",
+                           os.path.join(CSRC, "pbb_host.cu"), os.path.join(CSRC, "pbb_mem.cu"),
+                           os.path.join(ROOT, "tests", "fake_cuda.cpp"), "-lpthread"])
+    return so
+
+
+@pytest.fixture
+def L(fake_so, tmp_path):
+    # a library of its own for every test: its state starts empty
+    so = str(tmp_path / "libfake.so")
+    shutil.copy(fake_so, so)
+    lib = ctypes.CDLL(so)
+    lib.fake_capacity.argtypes = [ctypes.c_size_t]
+    lib.fake_used.restype = ctypes.c_size_t
+    lib.pbb_last_error.restype = ctypes.c_char_p
+    lib.pbb_engine_destroy.argtypes = [ctypes.c_void_p]
+    lib.pbb_start.argtypes = [ctypes.c_void_p, ctypes.c_int32, ctypes.c_void_p]
+    lib.pbb_explore.argtypes = [ctypes.c_void_p, ctypes.c_double, ctypes.c_void_p]
+    return lib
+
+
+def instance(seed, n, m):
+    p = np.random.default_rng(seed).integers(1, 99, size=(m, n), dtype=np.int32)
+    return pb._instance(p)
+
+
+def create(L, n=50, m=20, seed=0, **cfg):
+    inst, keep = instance(seed, n, m)
+    e = ctypes.c_void_p()
+    rc = L.pbb_engine_create(ctypes.byref(inst), ctypes.byref(pb.Config(**cfg)._c()), ctypes.byref(e))
+    return rc, e
+
+
+def test_blocks_of_an_engine_that_outlives_its_context_are_not_handed_on(L):
+    """A device reset takes all handles with it: an engine destroyed after it
+    gives nothing back, and leaves the blocks and streams of engines made since
+    alone although they may stand at the same addresses."""
+    rc, old = create(L, nbIVMs=65536)                 # over 256 MiB: a block of its own
+    assert rc == 0
+    L.fake_reset()
+    rc, new = create(L, nbIVMs=65536)
+    assert rc == 0
+    L.pbb_engine_destroy(old)
+    rc, third = create(L, nbIVMs=65536)
+    assert rc == 0
+    assert L.pbb_start(new, 1000, None) == 0 and L.pbb_start(third, 1000, None) == 0
+    L.pbb_engine_destroy(new)
+    L.pbb_engine_destroy(third)
+    rc, again = create(L, nbIVMs=65536)               # from what was kept
+    assert rc == 0
+    L.pbb_engine_destroy(again)
+    assert L.fake_invalid() == 0
+
+
+def test_nothing_of_a_reset_device_is_used_by_an_engine_made_before(L):
+    rc, old = create(L, n=12, m=10, nbIVMs=64)
+    assert rc == 0
+    L.fake_reset()
+    L.pbb_engine_destroy(old)
+    rc, new = create(L, n=12, m=10, nbIVMs=64)
+    assert rc == 0 and L.pbb_start(new, 1000, None) == 0
+    L.pbb_engine_destroy(new)
+    assert L.fake_invalid() == 0
