@@ -186,11 +186,12 @@ cudaError_t stream_take(Lease* l, int device)
     l->context = check_context(device);
     if (device >= 0 && device < PBB_MEM_DEVICES) {
         std::lock_guard<std::mutex> lock(g_mem_mutex);
-        while (!g_streams[device].empty()) {
+        if (!g_streams[device].empty()) {
+            // its last user's frees may still be on it: they come before the
+            // next user's work, as any order of the stream does
             l->st = g_streams[device].back();
             g_streams[device].pop_back();
-            if (cudaStreamQuery(l->st) == cudaSuccess) return cudaSuccess;
-            cudaGetLastError();
+            return cudaSuccess;
         }
     }
     l->st = nullptr;

@@ -83,3 +83,15 @@ def test_nothing_of_a_reset_device_is_used_by_an_engine_made_before(L):
     assert rc == 0 and L.pbb_start(new, 1000, None) == 0
     L.pbb_engine_destroy(new)
     assert L.fake_invalid() == 0
+
+
+def test_streams_are_used_again(L):
+    """A stream comes back with its user's frees still on it, and serves the next."""
+    for _ in range(20):
+        rc, a = create(L, n=12, m=10, nbIVMs=64)
+        assert rc == 0
+        rc, b = create(L, n=12, m=10, nbIVMs=64)
+        assert rc == 0
+        L.pbb_engine_destroy(a)
+        L.pbb_engine_destroy(b)
+    assert L.fake_streams() == 2 and L.fake_invalid() == 0
