@@ -912,13 +912,14 @@ static int bound_children_impl(const pbb_instance* inst, int32_t johnson_mode, i
             memcpy(host.data() + o_l1, limit1, c1);
             memcpy(host.data() + o_l2, limit2, c1);
         } else {
-            cudaMemcpyAsync(d + o_s, sched, cn, cudaMemcpyHostToDevice, st);
-            cudaMemcpyAsync(d + o_l1, limit1, c1, cudaMemcpyHostToDevice, st);
-            cudaMemcpyAsync(d + o_l2, limit2, c1, cudaMemcpyHostToDevice, st);
+            ce = cudaMemcpyAsync(d + o_s, sched, cn, cudaMemcpyHostToDevice, st);
+            if (!ce) ce = cudaMemcpyAsync(d + o_l1, limit1, c1, cudaMemcpyHostToDevice, st);
+            if (!ce) ce = cudaMemcpyAsync(d + o_l2, limit2, c1, cudaMemcpyHostToDevice, st);
         }
-        cudaMemcpyAsync(d, host.data(), host.size(), cudaMemcpyHostToDevice, st);
+        if (!ce) ce = cudaMemcpyAsync(d, host.data(), host.size(), cudaMemcpyHostToDevice, st);
         int sms = 0;
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+        if (!ce) ce = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+        if (ce != cudaSuccess) { rc = cuda_fail(ce, "upload of the tables and nodes"); break; }
         const pbbl::BoundShape shape = pbbl::bound_shape(n, H.m, H.Ppad, count, sms, max_smem_optin(device));
         if (shape.warps < 1) { rc = fail(PBB_E_INVAL, "instance tables do not fit in shared memory"); break; }
         auto dev = [&](size_t off) { return reinterpret_cast<int*>(d + off); };
@@ -941,16 +942,18 @@ static int bound_children_impl(const pbb_instance* inst, int32_t johnson_mode, i
         }
         if (ce != cudaSuccess) { rc = cuda_fail(ce, "pbb_bound_kernel launch"); break; }
         unsigned hs = 0;
-        cudaMemcpyAsync(&hs, status, sizeof(unsigned), cudaMemcpyDeviceToHost, st);
+        ce = cudaMemcpyAsync(&hs, status, sizeof(unsigned), cudaMemcpyDeviceToHost, st);
         const size_t back = C.bytes - o_inputs_end;
         std::vector<unsigned char> packed(back <= PACKED_BYTES ? back : 0);
         if (!packed.empty()) {
-            cudaMemcpyAsync(packed.data(), d + o_inputs_end, back, cudaMemcpyDeviceToHost, st);
+            if (!ce) ce = cudaMemcpyAsync(packed.data(), d + o_inputs_end, back, cudaMemcpyDeviceToHost, st);
         } else {
             for (const Out& o : out)
-                if (o.host && o.off) cudaMemcpyAsync(o.host, d + o.off, o.bytes, cudaMemcpyDeviceToHost, st);
+                if (!ce && o.host && o.off) ce = cudaMemcpyAsync(o.host, d + o.off, o.bytes, cudaMemcpyDeviceToHost, st);
         }
-        ce = cudaStreamSynchronize(st);
+        // the copies under way read and write this frame's buffers
+        const cudaError_t end = cudaStreamSynchronize(st);
+        if (!ce) ce = end;
         if (ce != cudaSuccess) { rc = cuda_fail(ce, "pbb_bound_kernel"); break; }
         if (hs & PBB_ST_BADINPUT) { rc = fail(PBB_E_INVAL, "device rejected a node"); break; }
         if (!packed.empty())

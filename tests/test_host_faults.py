@@ -95,3 +95,35 @@ def test_streams_are_used_again(L):
         L.pbb_engine_destroy(a)
         L.pbb_engine_destroy(b)
     assert L.fake_streams() == 2 and L.fake_invalid() == 0
+
+
+def bound_call(L, seed, n, m, count, outs=9):
+    """pbb_bound_children_ex: (code, outputs)."""
+    inst, keep = instance(seed, n, m)
+    rng = np.random.default_rng(seed)
+    sched = np.argsort(rng.random((count, n)), axis=1).astype(np.int32)
+    l1 = rng.integers(-1, n // 2, size=count).astype(np.int32)
+    l2 = (l1 + 1 + rng.integers(1, n // 2, size=count)).astype(np.int32)
+    arrays = [np.full((count, n) if q < 4 or q in (6, 7) else count, -5, np.int32) for q in range(outs)]
+    ptrs = (i32p * 9)(*[a.ctypes.data_as(i32p) for a in arrays])
+    rc = L.pbb_bound_children_ex(ctypes.byref(inst), 0, 0, count, sched.ctypes.data_as(i32p), l1.ctypes.data_as(i32p),
+                                 l2.ctypes.data_as(i32p), ptrs)
+    return rc, arrays
+
+
+@pytest.mark.parametrize("count", [5, 4000])
+def test_every_failed_copy_of_a_bound_call_is_reported(L, count):
+    """Inputs that did not arrive are never bounded with what the last call left."""
+    L.fake_calls.restype = ctypes.c_int
+    assert bound_call(L, 1, 20, 10, count)[0] == 0
+    before = L.fake_calls(b"cudaMemcpyAsync")
+    rc, want = bound_call(L, 2, 20, 10, count)
+    copies = L.fake_calls(b"cudaMemcpyAsync") - before
+    assert rc == 0 and copies >= 3 and (want[0] != -5).all()
+    for k in range(1, copies + 1):
+        assert bound_call(L, 1, 20, 10, count)[0] == 0
+        L.fake_fail(b"cudaMemcpyAsync", k)
+        assert bound_call(L, 2, 20, 10, count)[0] == pb.PBB_E_CUDA, k
+    rc, got = bound_call(L, 2, 20, 10, count)
+    assert rc == 0 and all((a == b).all() for a, b in zip(got, want))
+    assert L.fake_invalid() == 0
