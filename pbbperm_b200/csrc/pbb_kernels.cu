@@ -234,9 +234,11 @@ __device__ __forceinline__ void build_lists(const WarpScratch& S, const Ivm<NW>&
 }
 
 // 32-bit per warp (fewer live registers in the explorer loop), added to the
-// group's 64-bit counters every 2^13 decomposed nodes (direct_free grows by at
-// most 2 x 64 x 496 x 64 a node: well under 2^32 in that many for any search
-// met, and it only feeds the work statistics)
+// group's 64-bit counters every PBB_FLUSH_NODES decomposed nodes.  direct_free
+// grows fastest: by two passes over the free jobs for every child and pair.
+static_assert((unsigned long long)PBB_FLUSH_NODES * (PBB_MAX_N - 1) * (PBB_MAX_M * (PBB_MAX_M - 1) / 2) * 2 *
+                      (PBB_MAX_N - 1) <= 0xffffffffull,
+              "a warp's 32-bit counters hold the work of PBB_FLUSH_NODES nodes");
 struct WarpCounters {
     unsigned decomposed, simple, johnson, leaves;
     unsigned sweeps, free_jobs, swept_children, direct_children, direct_free;
@@ -1062,7 +1064,7 @@ pbb_explore_kernel(const DevGroup* groups, const int* ngroups_d, int warps_per_c
             since++;
             bound_current<NW, (VAR == 1 || VAR == 2), (VAR == 2), (VAR == 7 ? 3 : VAR >= 3 ? 2 - (VAR & 1) : 0)>(G, T, S, B, id, R, mode, best, C);
         }
-        if (C.decomposed >= (1u << 13)) flush_counters(G, C);
+        if (C.decomposed >= PBB_FLUSH_NODES) flush_counters(G, C);
         if (r == 0) {
             // interval exhausted: leave the pool of busy explorers (the
             // registers need not go back: nobody resumes this interval)

@@ -25,6 +25,7 @@
 #define PBB_SPLIT_DEPTH 10    // default of DevSearch::split_depth
 #define PBB_SHARE_AFTER 64    // default of DevSearch::share_after
 #define PBB_SPLIT_NARROW 4    // default of DevSearch::split_narrow
+#define PBB_FLUSH_NODES (1u << 10)     // nodes after which a warp adds its counters to the group's
 
 // IVM life cycle (per explorer, in global memory)
 #define IVM_IDLE 0            // no interval
