@@ -1414,26 +1414,11 @@ int explore_occupancy(int warps_per_cta, int smem)
 
 int explore_ctas_per_sm(int nw, int warps_per_cta, int smem, int variant)
 {
-    if (nw == 1) {
-        switch (variant) {
-        case 1: return explore_occupancy<1, 1>(warps_per_cta, smem);
-        case 2: return explore_occupancy<1, 2>(warps_per_cta, smem);
-        case 3: return explore_occupancy<1, 3>(warps_per_cta, smem);
-        case 4: return explore_occupancy<1, 4>(warps_per_cta, smem);
-        case 5: return explore_occupancy<1, 5>(warps_per_cta, smem);
-        case 6: return explore_occupancy<1, 6>(warps_per_cta, smem);
-        case 7: return explore_occupancy<1, 7>(warps_per_cta, smem);
-        default: return explore_occupancy<1, 0>(warps_per_cta, smem);
-        }
-    }
     switch (variant) {
-    case 1: return explore_occupancy<2, 1>(warps_per_cta, smem);
-    case 2: return explore_occupancy<2, 2>(warps_per_cta, smem);
-    case 3: return explore_occupancy<2, 3>(warps_per_cta, smem);
-    case 4: return explore_occupancy<2, 4>(warps_per_cta, smem);
-    case 5: return explore_occupancy<2, 5>(warps_per_cta, smem);
-    case 6: return explore_occupancy<2, 6>(warps_per_cta, smem);
-    default: return explore_occupancy<2, 0>(warps_per_cta, smem);
+    case 0: return nw == 1 ? explore_occupancy<1, 0>(warps_per_cta, smem) : explore_occupancy<2, 0>(warps_per_cta, smem);
+    case 3: return nw == 1 ? explore_occupancy<1, 3>(warps_per_cta, smem) : explore_occupancy<2, 3>(warps_per_cta, smem);
+    case 4: return nw == 1 ? explore_occupancy<1, 4>(warps_per_cta, smem) : explore_occupancy<2, 4>(warps_per_cta, smem);
+    default: return 0;
     }
 }
 

@@ -34,6 +34,7 @@ cudaError_t launch_lower_ub(const DevGroup* groups, int g, int ub, cudaStream_t 
 cudaError_t launch_explore(int nw, const DevGroup* groups, const int* ngroups_d, int ctas, int warps_per_cta, int smem,
                            unsigned long long budget_ns, int max_rounds, int select_budget, cudaStream_t st,
                            int variant = 0, int eager = 1, int* pair_stack = nullptr, int pair_stride = 0);
+// resident CTAs of the variants a pool launches (0, 3, 4)
 int explore_ctas_per_sm(int nw, int warps_per_cta, int smem, int variant = 0);
 // The launch of a batch of `count` nodes: kernel and block shape that fit
 // `optin` bytes of shared memory (warps 0: none does)

@@ -129,8 +129,10 @@ struct pbb_pool {
     // window graphs by block shape (bulk, tail) and explorer build (0: any
     // settings, 1 and 2: variants 3 and 4), captured when first needed
     cudaGraphExec_t window[2][3] = {{nullptr, nullptr, nullptr}, {nullptr, nullptr, nullptr}};
-    // the default search's build: scratch of its launches (0: not used) and
-    // the pair bounds of every warp of the wider grid
+    // builds 1 and 2: how many of them the grid's CTAs are resident with (0
+    // with no room for their scratch), that scratch, and the pair bounds of
+    // every warp of the wider grid
+    int pair_builds = 0, tail_pair_builds = 0;
     int pair_smem = 0, tail_pair_smem = 0, pair_stride = 0;
     int* pair_stack = nullptr;
     std::vector<Slot> slots;
@@ -208,6 +210,15 @@ void carve_explorers(unsigned char* base, int E, int npad, int levels, DevIvms& 
     V.path = reinterpret_cast<int*>(base + o);
 }
 
+// how many of the builds with kept pair bounds have `per_sm` CTAs resident
+int pair_builds(int nw, int warps, int smem, int optin, int per_sm)
+{
+    if (smem > optin) return 0;
+    int b = 0;
+    while (b < 2 && pbbl::explore_ctas_per_sm(nw, warps, smem, 3 + b) >= per_sm) b++;
+    return b;
+}
+
 // `most`: instances the pool will ever hold (a batch knows), so that it is not
 // made larger than they need
 int pool_create(const pbb_pool_config* in, pbb_pool* P, int most)
@@ -260,8 +271,8 @@ int pool_create(const pbb_pool_config* in, pbb_pool* P, int most)
         if (ms <= optin && pbbl::explore_ctas_per_sm(P->nw, P->warps, ms) >= per_sm) {
             P->smem = ms;
         }
-        const int ps = pbbl::smem_bytes(c.max_jobs, c.max_machines, P->Ppad_max, P->warps, PBB_SCRATCH_PAIRS);
-        if (ps <= optin && pbbl::explore_ctas_per_sm(P->nw, P->warps, ps, 3) >= per_sm) P->pair_smem = ps;
+        P->pair_smem = pbbl::smem_bytes(c.max_jobs, c.max_machines, P->Ppad_max, P->warps, PBB_SCRATCH_PAIRS);
+        P->pair_builds = pair_builds(P->nw, P->warps, P->pair_smem, optin, per_sm);
     }
     // every window launches all the CTAs the GPU holds at once and spreads
     // them over the resident instances
@@ -280,8 +291,8 @@ int pool_create(const pbb_pool_config* in, pbb_pool* P, int most)
             P->tail_warps = tw;
             P->tail_smem = ts;
             P->tail_grid = sms * tper;
-            const int ps = pbbl::smem_bytes(c.max_jobs, c.max_machines, P->Ppad_max, tw, PBB_SCRATCH_PAIRS);
-            if (ps <= optin && pbbl::explore_ctas_per_sm(P->nw, tw, ps, 3) >= tper) P->tail_pair_smem = ps;
+            P->tail_pair_smem = pbbl::smem_bytes(c.max_jobs, c.max_machines, P->Ppad_max, tw, PBB_SCRATCH_PAIRS);
+            P->tail_pair_builds = pair_builds(P->nw, tw, P->tail_pair_smem, optin, tper);
         }
     }
     // default explorer count: every warp of the widest grid owns one, so that
@@ -319,13 +330,13 @@ int pool_create(const pbb_pool_config* in, pbb_pool* P, int most)
     PCK(cudaMemsetAsync(P->ngroups_d, 0, sizeof(int), P->st), "group count");
     PCK(cudaMallocHost(&P->ctl_h, sizeof(GroupCtl) * S), "pinned control mirror");
     memset(P->ctl_h, 0, sizeof(GroupCtl) * S);
-    if (P->pair_smem || P->tail_pair_smem) {
+    if (P->pair_builds || P->tail_pair_builds) {
         const size_t w = std::max((size_t)P->grid * P->warps, (size_t)P->tail_grid * P->tail_warps);
         P->pair_stride = c.max_jobs * P->Ppad_max;
         if (pbbh::mem_alloc((void**)&P->pair_stack, sizeof(int) * w * P->pair_stride, P->lease) != cudaSuccess) {
             cudaGetLastError();       // no room: the general build needs none
             P->pair_stack = nullptr;
-            P->pair_smem = P->tail_pair_smem = 0;
+            P->pair_builds = P->tail_pair_builds = 0;
         }
     }
     P->arena_bytes = (size_t)c.explorer_bytes;
@@ -597,13 +608,15 @@ extern "C" int pbb_pool_step(pbb_pool* P, int32_t* resident, int32_t* queued)
     PCK(cudaMemcpyAsync(P->ngroups_d, &nact, sizeof(int), cudaMemcpyHostToDevice, P->st), "upload");
     // kept pair bounds while every resident instance searches in a way they
     // serve; the default search's build while all of them search that way
-    int build = (tail ? P->tail_pair_smem : P->pair_smem) > 0 ? 1 : 0;
+    const int builds = tail ? P->tail_pair_builds : P->pair_builds;
+    int build = builds > 0 ? 1 : 0;
     for (int i = 0; i < nact; i++) {
         const DevSearch& q = act[i].search;
         const int v = pbbl::pairs_variant(q.bound_mode, q.branch_mode, q.find_all, q.sort_nodes);
         if (v == 0) build = 0;
         else if (build) build = std::max(build, v - 2);
     }
+    if (build > builds) build = 0;
     cudaGraphExec_t win = nullptr;
     if (nact > 0) {
         rc = window_graph(P, tail, build, &win);

@@ -1,5 +1,5 @@
 // A CUDA runtime on host memory, for the library's host code without a GPU
-// (tests/test_host_faults.py links it with pbb_host.cu and pbb_mem.cu): it
+// (tests/test_host_faults.py links it with the host files of the library): it
 // keeps account of blocks, streams and contexts, fails the calls it is told to
 // fail, and counts uses of handles that are not valid.  The kernel launches it
 // stands in for only move enough data to tell right from stale inputs.
@@ -38,6 +38,8 @@ std::map<std::string, int> g_fail, g_calls;
 size_t g_capacity = ~(size_t)0, g_used = 0, g_reserved = 0, g_threshold = 0;
 int g_invalid = 0;                         // uses of handles that are not valid
 int g_variant = -1;
+int g_per_sm[8] = {2, 2, 2, 2, 2, 2, 2, 2};   // resident CTAs an SM, by explorer variant
+int g_not_resident = 0;                    // explorer launches of more CTAs than are resident
 cudaError_t g_last = cudaSuccess;
 
 cudaError_t done(const char* name, cudaError_t rc = cudaSuccess)
@@ -121,6 +123,8 @@ void fake_reset()
     g_ctx++;
 }
 int fake_invalid() { Lock l(g_mu); return g_invalid; }
+void fake_per_sm(int variant, int ctas) { Lock l(g_mu); g_per_sm[variant] = ctas; }
+int fake_not_resident() { Lock l(g_mu); return g_not_resident; }
 int fake_variant() { Lock l(g_mu); return g_variant; }
 size_t fake_used() { Lock l(g_mu); return g_used + g_reserved; }
 int fake_calls(const char* name) { Lock l(g_mu); return g_calls[name]; }
@@ -244,23 +248,41 @@ cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaEventQuery(cudaEvent_t) { return cudaSuccess; }
 cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
 cudaError_t cudaEventElapsedTime(float* ms, cudaEvent_t, cudaEvent_t) { *ms = 1.f; return cudaSuccess; }
+cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) { *p = calloc(1, n); return cudaSuccess; }
+cudaError_t cudaFreeHost(void* p) { free(p); return cudaSuccess; }
+// a graph is the launches and copies of its capture: none here, the calls
+// made in it have had their effect
+cudaError_t cudaStreamBeginCapture(cudaStream_t, enum cudaStreamCaptureMode) { return cudaSuccess; }
+cudaError_t cudaStreamEndCapture(cudaStream_t, cudaGraph_t* g) { *g = reinterpret_cast<cudaGraph_t>(0x30); return cudaSuccess; }
+cudaError_t cudaGraphInstantiate(cudaGraphExec_t* e, cudaGraph_t, unsigned long long)
+{
+    Lock l(g_mu);
+    *e = reinterpret_cast<cudaGraphExec_t>(0x40);
+    return done("cudaGraphInstantiate");
+}
+cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaGraphDestroy(cudaGraph_t) { return cudaSuccess; }
+cudaError_t cudaGraphExecDestroy(cudaGraphExec_t) { return cudaSuccess; }
 }  // extern "C"
 
 // --- launches ---------------------------------------------------------------
 namespace pbbl {
 int smem_bytes(int n, int m, int Ppad, int warps, int fmask) { return pbb_smem_plan(n, m, Ppad, warps, fmask).total; }
 cudaError_t launch_reset(const DevGroup*, int, const int*, cudaStream_t) { return cudaSuccess; }
-cudaError_t launch_root(int, const DevGroup* g, int, const int*, const int*, int, int, cudaStream_t, int, const int*)
+int explore_ctas_per_sm(int, int, int, int variant) { return g_per_sm[variant]; }
+cudaError_t launch_root(int, const DevGroup* g, int count, const int*, const int*, int, int, cudaStream_t, int, const int*)
 {
-    g->ctl->active = 1;
+    for (int i = 0; i < count; i++) g[i].ctl->active = 1;
     return cudaSuccess;
 }
 cudaError_t launch_lower_ub(const DevGroup*, int, int, cudaStream_t) { return cudaSuccess; }
-cudaError_t launch_explore(int, const DevGroup* g, const int*, int, int, int, unsigned long long, int, int, cudaStream_t,
-                           int variant, int, int*, int)
+cudaError_t launch_explore(int, const DevGroup* g, const int* count, int ctas, int, int, unsigned long long, int, int,
+                           cudaStream_t, int variant, int, int*, int)
 {
+    Lock l(g_mu);
     g_variant = variant;
-    g->ctl->active = 0;
+    g_not_resident += ctas > 148 * g_per_sm[variant];
+    for (int i = 0; i < *count; i++) g[i].ctl->active = 0;
     return cudaSuccess;
 }
 cudaError_t launch_neh(const NehTask*, int, cudaStream_t) { return cudaSuccess; }

@@ -21,7 +21,7 @@ def fake_so(tmp_path_factory):
     # -Bsymbolic: the fake runtime is this library's alone
     subprocess.check_call(["g++", "-w", "-shared", "-fPIC", "-O1", "-std=c++17", "-Wl,-Bsymbolic",
                            "-I", "/usr/local/cuda/include", "-I", CSRC, "-o", so, "-x", "c++",
-                           os.path.join(CSRC, "pbb_host.cu"), os.path.join(CSRC, "pbb_mem.cu"),
+                           *[os.path.join(CSRC, f) for f in ("pbb_host.cu", "pbb_mem.cu", "pbb_pool.cu")],
                            os.path.join(ROOT, "tests", "fake_cuda.cpp"), "-lpthread"])
     return so
 
@@ -37,6 +37,10 @@ def L(fake_so, tmp_path):
     lib.pbb_last_error.restype = ctypes.c_char_p
     lib.pbb_engine_destroy.argtypes = [ctypes.c_void_p]
     lib.pbb_start.argtypes = [ctypes.c_void_p, ctypes.c_int32, ctypes.c_void_p]
+    lib.pbb_pool_submit.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int32, ctypes.c_void_p,
+                                    ctypes.c_int64]
+    lib.pbb_pool_step.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p]
+    lib.pbb_pool_destroy.argtypes = [ctypes.c_void_p]
     lib.pbb_explore.argtypes = [ctypes.c_void_p, ctypes.c_double, ctypes.c_void_p]
     return lib
 
@@ -127,3 +131,22 @@ def test_every_failed_copy_of_a_bound_call_is_reported(L, count):
     rc, got = bound_call(L, 2, 20, 10, count)
     assert rc == 0 and all((a == b).all() for a, b in zip(got, want))
     assert L.fake_invalid() == 0
+
+
+@pytest.mark.parametrize("per_sm,opt,variant", [
+    ({}, {}, 3), ({}, dict(adaptiveBranchingMode=2), 4),
+    ({4: 1}, {}, 3), ({4: 1}, dict(adaptiveBranchingMode=2), 0), ({3: 1}, {}, 0),
+])
+def test_pool_windows_launch_only_resident_ctas(L, per_sm, opt, variant):
+    """Every build a window launches holds all the CTAs of the pool's grid."""
+    for v, c in per_sm.items():
+        L.fake_per_sm(v, c)
+    inst, keep = instance(1, 12, 10)
+    pool = ctypes.c_void_p()
+    cfg = pb.PoolConfig(max_jobs=12, max_machines=10, max_resident=2, explorers_per_instance=64)._c()
+    assert L.pbb_pool_create(ctypes.byref(cfg), ctypes.byref(pool)) == 0, L.pbb_last_error()
+    search = pb.Config(**opt)._c()
+    assert L.pbb_pool_submit(pool, ctypes.byref(inst), ctypes.byref(search), 1000, None, 0) == 0
+    assert L.pbb_pool_step(pool, None, None) == 0, L.pbb_last_error()
+    assert L.fake_variant() == variant and L.fake_not_resident() == 0
+    L.pbb_pool_destroy(pool)
