@@ -335,13 +335,7 @@ static int engine_create(const pbb_instance* inst, const pbb_config* cfg, pbb_en
         while (w > 1 && pbbl::smem_bytes(H.n, H.m, H.Ppad, w, PBB_SCRATCH_PAIRS) > cap) w--;
         e->pair_smem = pbbl::smem_bytes(H.n, H.m, H.Ppad, w, PBB_SCRATCH_PAIRS);
         e->pair_stride = H.n * H.Ppad;
-        if (e->pair_smem <= cap) {
-            if (pbbh::mem_alloc((void**)&e->pair_stack, sizeof(int) * (size_t)e->ctas * w * e->pair_stride,
-                                e->lease) == cudaSuccess)
-                e->pair_warps = w;
-            else
-                cudaGetLastError();   // no room: the general build needs none
-        }
+        if (e->pair_smem <= cap) e->pair_warps = w;
     }
     // mode 1: the general build's shared atomics against values by position, at
     // the same warps (24 gain 7 % on 20x20 and lose 2 to 4 % on 18x20 to 30x10)
@@ -368,6 +362,13 @@ static int engine_create(const pbb_instance* inst, const pbb_config* cfg, pbb_en
     const size_t o_vec = C.take(4 * B * npad), o_perm = C.take(B * npad);
     const size_t o_mat = C.take(B * levels * npad), o_path = C.take(B * levels * PBB_PATH_INTS * sizeof(int));
     CK(pbbh::mem_alloc((void**)&e->block, C.bytes, e->lease));
+    // after what the engine cannot do without: the general build needs none
+    if (e->pair_variant && e->pair_variant != 7 && e->pair_warps > 0 &&
+        pbbh::mem_alloc((void**)&e->pair_stack, sizeof(int) * (size_t)e->ctas * e->pair_warps * e->pair_stride,
+                        e->lease) != cudaSuccess) {
+        cudaGetLastError();
+        e->pair_warps = 0;
+    }
     unsigned char* d = e->block;
     e->ub_d = reinterpret_cast<int*>(d + o_ub);
     e->root_d = reinterpret_cast<int*>(d + o_root);

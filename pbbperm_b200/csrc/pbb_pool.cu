@@ -330,21 +330,22 @@ int pool_create(const pbb_pool_config* in, pbb_pool* P, int most)
     PCK(cudaMemsetAsync(P->ngroups_d, 0, sizeof(int), P->st), "group count");
     PCK(cudaMallocHost(&P->ctl_h, sizeof(GroupCtl) * S), "pinned control mirror");
     memset(P->ctl_h, 0, sizeof(GroupCtl) * S);
-    if (P->pair_builds || P->tail_pair_builds) {
-        const size_t w = std::max((size_t)P->grid * P->warps, (size_t)P->tail_grid * P->tail_warps);
-        P->pair_stride = c.max_jobs * P->Ppad_max;
-        if (pbbh::mem_alloc((void**)&P->pair_stack, sizeof(int) * w * P->pair_stride, P->lease) != cudaSuccess) {
-            cudaGetLastError();       // no room: the general build needs none
-            P->pair_stack = nullptr;
-            P->pair_builds = P->tail_pair_builds = 0;
-        }
-    }
     P->arena_bytes = (size_t)c.explorer_bytes;
     const int E = P->epw;
     if (explorer_block_bytes(E, P->npad, P->cfg.max_jobs) > P->arena_bytes)
         return pfail(PBB_E_INVAL, "explorer_bytes is smaller than one instance's footprint");
     P->arena_bytes = std::min(P->arena_bytes, explorer_block_bytes(E, P->npad, c.max_jobs) * (size_t)P->max_slots);
     PCK(pbbh::mem_alloc((void**)&P->arena, P->arena_bytes, P->lease), "explorer memory");
+    // after what the pool cannot do without: the general build needs none
+    if (P->pair_builds || P->tail_pair_builds) {
+        const size_t w = std::max((size_t)P->grid * P->warps, (size_t)P->tail_grid * P->tail_warps);
+        P->pair_stride = c.max_jobs * P->Ppad_max;
+        if (pbbh::mem_alloc((void**)&P->pair_stack, sizeof(int) * w * P->pair_stride, P->lease) != cudaSuccess) {
+            cudaGetLastError();
+            P->pair_stack = nullptr;
+            P->pair_builds = P->tail_pair_builds = 0;
+        }
+    }
     P->alloc.init(P->arena_bytes);
     P->slots.assign(S, Slot());
     return PBB_OK;

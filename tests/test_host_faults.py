@@ -150,3 +150,42 @@ def test_pool_windows_launch_only_resident_ctas(L, per_sm, opt, variant):
     assert L.pbb_pool_step(pool, None, None) == 0, L.pbb_last_error()
     assert L.fake_variant() == variant and L.fake_not_resident() == 0
     L.pbb_pool_destroy(pool)
+
+
+def test_an_engine_does_without_pair_bounds_before_it_fails(L):
+    """50x20: 95 MB of explorers and 182 MB of pair bounds by level.  With room
+    for the explorers alone the general build runs; with less nothing does."""
+    L.fake_capacity(200 << 20)
+    rc, e = create(L, nbIVMs=4096)
+    assert rc == 0, L.pbb_last_error()
+    assert L.pbb_start(e, 1000, None) == 0 and L.pbb_explore(e, 1.0, None) == 0
+    assert L.fake_variant() == 0
+    L.pbb_engine_destroy(e)
+    L.fake_capacity(300 << 20)
+    rc, e = create(L, nbIVMs=4096)
+    assert rc == 0 and L.pbb_start(e, 1000, None) == 0 and L.pbb_explore(e, 1.0, None) == 0
+    assert L.fake_variant() == 5
+    L.pbb_engine_destroy(e)
+    L.fake_capacity(80 << 20)
+    assert create(L, nbIVMs=4096)[0] == pb.PBB_E_NOMEM
+    L.fake_capacity(300 << 20)
+    rc, e = create(L, nbIVMs=4096)
+    assert rc == 0
+    L.pbb_engine_destroy(e)
+    assert L.fake_invalid() == 0
+
+
+def test_a_pool_does_without_pair_bounds_before_it_fails(L):
+    """50x20, two slots: 186 MB of explorers, 91 MB of pair bounds for 2368 warps."""
+    inst, keep = instance(1, 50, 20)
+    for capacity, variant in ((240, 0), (400, 3)):
+        L.fake_capacity(capacity << 20)
+        pool = ctypes.c_void_p()
+        cfg = pb.PoolConfig(max_jobs=50, max_machines=20, max_resident=2, explorers_per_instance=4096, tail_warps=-1)._c()
+        assert L.pbb_pool_create(ctypes.byref(cfg), ctypes.byref(pool)) == 0, L.pbb_last_error()
+        search = pb.Config()._c()
+        assert L.pbb_pool_submit(pool, ctypes.byref(inst), ctypes.byref(search), 1000, None, 0) == 0
+        assert L.pbb_pool_step(pool, None, None) == 0, L.pbb_last_error()
+        assert L.fake_variant() == variant
+        L.pbb_pool_destroy(pool)
+    assert L.fake_invalid() == 0
