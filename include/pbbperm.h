@@ -119,6 +119,13 @@ typedef struct pbb_engine pbb_engine;
 void pbb_config_default(pbb_config* cfg);
 const char* pbb_last_error(void);
 
+/* The library keeps freed device memory and streams for its next engine, pool
+ * or call (at most 1 GiB of small blocks, 2 GiB of blocks over 256 MiB and
+ * eight streams per device), and gives all of it back to the driver before an
+ * allocation of its own fails.  This gives it back now, for other users of
+ * `device`'s memory; objects in use keep theirs. */
+int pbb_release_memory(int32_t device);
+
 int pbb_engine_create(const pbb_instance* inst, const pbb_config* cfg, pbb_engine** out);
 int pbb_engine_destroy(pbb_engine* e);
 

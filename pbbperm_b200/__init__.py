@@ -160,6 +160,12 @@ def _check(rc):
         raise PbbError(rc, lib().pbb_last_error().decode())
 
 
+def release_memory(device=0):
+    """Give the device memory the library keeps for its next engine, pool or
+    call back to the driver (pbb_release_memory)."""
+    _check(lib().pbb_release_memory(int(device)))
+
+
 def _ptr(a):
     return a.ctypes.data_as(_i32p) if a is not None else None
 

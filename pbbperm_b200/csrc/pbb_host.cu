@@ -232,6 +232,14 @@ void pbb_config_default(pbb_config* c)
 
 const char* pbb_last_error(void) { return g_err.c_str(); }
 
+int pbb_release_memory(int32_t device)
+{
+    pbbh::DeviceGuard keep_callers_device;
+    CK(cudaSetDevice(device));
+    pbbh::mem_release(device);
+    return PBB_OK;
+}
+
 }  // extern "C"
 
 namespace pbbh {
@@ -290,8 +298,8 @@ int pbb_engine_destroy(pbb_engine* e)
         cudaStreamSynchronize(e->st);
         pbbh::mem_free(e->block, e->lease);
         pbbh::mem_free(e->pair_stack, e->lease);
-        cudaFree(e->sample_d);
-        cudaFree(e->sample_rec);
+        pbbh::mem_free(e->sample_d, e->lease);
+        pbbh::mem_free(e->sample_rec, e->lease);
         if (e->ev0) cudaEventDestroy(e->ev0);
         if (e->ev1) cudaEventDestroy(e->ev1);
         pbbh::stream_give(e->lease);
@@ -661,16 +669,16 @@ int pbb_diag_sample_nodes(pbb_engine* e, int32_t capacity, int32_t rate_log2)
         if (rs) return rs;
     }
     CK(cudaStreamSynchronize(e->st));
-    cudaFree(e->sample_d);
-    cudaFree(e->sample_rec);
+    pbbh::mem_free(e->sample_d, e->lease);
+    pbbh::mem_free(e->sample_rec, e->lease);
     e->sample_d = nullptr;
     e->sample_rec = nullptr;
     e->group.sample = nullptr;
     if (capacity > 0) {
         e->sample_stride = PBB_SAMPLE_HDR + 5 * e->H.n;
         const size_t bytes = sizeof(int) * (size_t)capacity * e->sample_stride;
-        CK(cudaMalloc(&e->sample_rec, bytes));
-        CK(cudaMalloc(&e->sample_d, sizeof(SampleBuf)));
+        CK(pbbh::mem_alloc((void**)&e->sample_rec, bytes, e->lease));
+        CK(pbbh::mem_alloc((void**)&e->sample_d, sizeof(SampleBuf), e->lease));
         CK(cudaMemsetAsync(e->sample_rec, 0, bytes, e->st));
         SampleBuf sb;
         sb.count = 0;

@@ -121,6 +121,26 @@ cudaMemPool_t pool_of(int device)
 
 namespace pbbh {
 
+void mem_release(int device)
+{
+    check_context(device);
+    drop_kept(device);
+    cudaMemPool_t p = nullptr;
+    std::vector<cudaStream_t> streams;
+    if (device >= 0 && device < PBB_MEM_DEVICES) {
+        std::lock_guard<std::mutex> lock(g_mem_mutex);
+        p = g_pool[device];
+        streams.swap(g_streams[device]);
+    }
+    // frees still in a stream's order come before the pool can shrink
+    for (cudaStream_t st : streams) {
+        cudaStreamSynchronize(st);
+        cudaStreamDestroy(st);
+    }
+    if (p) cudaMemPoolTrimTo(p, 0);
+    cudaGetLastError();
+}
+
 bool alive(const Lease& l) { return l.st && context_id() == l.context; }
 
 cudaError_t mem_alloc(void** out, size_t bytes, const Lease& l)
@@ -135,9 +155,7 @@ cudaError_t mem_alloc(void** out, size_t bytes, const Lease& l)
         if (attempt == 1) {
             // what is kept goes back before an allocation fails
             cudaGetLastError();
-            drop_kept(device);
-            if (p) cudaMemPoolTrimTo(p, 0);
-            cudaGetLastError();
+            mem_release(device);
         }
         if (big) {
             if ((*out = take_kept(bytes, device))) return cudaSuccess;

@@ -8,8 +8,9 @@
 // PBB_POOL_KEEP bytes of freed memory, larger ones -- a pool grows by them ten
 // times slower than cudaMalloc does (1.6 GB: 40 ms and 3) -- in a list of freed
 // blocks of at most PBB_BIG_KEEP bytes.  More than that goes back to the driver
-// as it is freed, and all of it before an allocation fails.  Streams are kept
-// too, a few per device.  All of it is safe from any thread.
+// as it is freed, and all of it before an allocation fails or when the caller
+// asks for it (pbb_release_memory).  Streams are kept too, a few per device.
+// All of it is safe from any thread.
 #pragma once
 #include <cuda_runtime.h>
 #include <stddef.h>
@@ -38,6 +39,8 @@ cudaError_t mem_alloc(void** out, size_t bytes, const Lease& l);
 void mem_free(void* p, const Lease& l);
 // the stream has no work left but frees; forgotten when the lease is not alive
 void stream_give(Lease& l);
+// what is kept of the current device goes back to the driver
+void mem_release(int device);
 
 // sub-buffers of one block, each on a 256-byte boundary
 struct Carver {

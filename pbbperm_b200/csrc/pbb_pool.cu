@@ -375,6 +375,12 @@ int window_graph(pbb_pool* P, bool tail, int build, cudaGraphExec_t* out)
             return pfail(PBB_E_CUDA, "capturing a window graph failed");
         }
         cudaError_t e5 = cudaGraphInstantiate(&exec, graph, 0);
+        if (e5) {
+            // a graph takes device memory of its own
+            cudaGetLastError();
+            pbbh::mem_release(P->dev);
+            e5 = cudaGraphInstantiate(&exec, graph, 0);
+        }
         cudaGraphDestroy(graph);
         if (e5) {
             exec = nullptr;

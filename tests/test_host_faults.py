@@ -189,3 +189,42 @@ def test_a_pool_does_without_pair_bounds_before_it_fails(L):
         assert L.fake_variant() == variant
         L.pbb_pool_destroy(pool)
     assert L.fake_invalid() == 0
+
+
+def test_kept_memory_and_streams_are_released_when_asked_for(L):
+    for ivms in (64, 65536, 64):
+        rc, e = create(L, nbIVMs=ivms)
+        assert rc == 0
+        L.pbb_engine_destroy(e)
+    rc, e = create(L, nbIVMs=64)
+    assert rc == 0
+    kept = L.fake_used()
+    assert L.pbb_release_memory(0) == 0
+    assert 0 < L.fake_used() < kept and L.fake_streams() == 1       # the engine's own
+    assert L.pbb_start(e, 1000, None) == 0 and L.pbb_explore(e, 1.0, None) == 0
+    L.pbb_engine_destroy(e)
+    assert L.pbb_release_memory(0) == 0
+    assert L.fake_used() == 0 and L.fake_streams() == 0 and L.fake_invalid() == 0
+
+
+def test_kept_memory_goes_back_before_sampling_or_a_window_fails(L):
+    """Whatever of the library needs memory gets what the library only keeps."""
+    rc, old = create(L, nbIVMs=65536)
+    assert rc == 0
+    rc, e = create(L, n=12, m=10, nbIVMs=64)
+    assert rc == 0
+    L.pbb_engine_destroy(old)                         # 1.6 GB kept
+    L.fake_capacity(L.fake_used() + (1 << 20))
+    assert L.pbb_diag_sample_nodes(ctypes.c_void_p(e.value), 100000, 0) == 0, L.pbb_last_error()
+    L.pbb_engine_destroy(e)
+    L.fake_capacity(1 << 40)
+    inst, keep = instance(1, 12, 10)
+    pool = ctypes.c_void_p()
+    cfg = pb.PoolConfig(max_jobs=12, max_machines=10, max_resident=2, explorers_per_instance=64)._c()
+    assert L.pbb_pool_create(ctypes.byref(cfg), ctypes.byref(pool)) == 0, L.pbb_last_error()
+    search = pb.Config()._c()
+    assert L.pbb_pool_submit(pool, ctypes.byref(inst), ctypes.byref(search), 1000, None, 0) == 0
+    L.fake_fail(b"cudaGraphInstantiate", 1)
+    assert L.pbb_pool_step(pool, None, None) == 0, L.pbb_last_error()
+    L.pbb_pool_destroy(pool)
+    assert L.fake_invalid() == 0
