@@ -4,6 +4,7 @@ import ctypes
 import os
 import shutil
 import subprocess
+import threading
 
 import numpy as np
 import pytest
@@ -228,3 +229,31 @@ def test_kept_memory_goes_back_before_sampling_or_a_window_fails(L):
     assert L.pbb_pool_step(pool, None, None) == 0, L.pbb_last_error()
     L.pbb_pool_destroy(pool)
     assert L.fake_invalid() == 0
+
+
+def test_threads_share_what_is_kept(L):
+    """Engines and bound calls of several sizes from eight threads at once: no
+    block or stream is lent twice or after it went back."""
+    bad = []
+
+    def work(t):
+        for i in range(12):
+            rc, e = create(L, n=(12, 50)[(t + i) % 2], m=(10, 20)[(t + i) % 2], nbIVMs=(64, 12000)[(t + i) % 2])
+            if rc or L.pbb_start(e, 1000, None) or L.pbb_explore(e, 1.0, None):
+                bad.append((t, i))
+            rc, out = bound_call(L, t, 20, 10, (5, 3000)[i % 2])
+            want = bound_call(L, t, 20, 10, (5, 3000)[i % 2])[1]
+            if rc or any((a != b).any() for a, b in zip(out, want)):
+                bad.append((t, i, "bounds"))
+            L.pbb_engine_destroy(e)
+            if i == 6:
+                L.pbb_release_memory(0)
+
+    threads = [threading.Thread(target=work, args=(t,)) for t in range(8)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad and L.fake_invalid() == 0
+    assert L.pbb_release_memory(0) == 0
+    assert L.fake_used() == 0 and L.fake_streams() == 0
