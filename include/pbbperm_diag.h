@@ -64,8 +64,16 @@ int pbb_diag_set_step_limits(struct pbb_engine* e, int32_t select_budget, int32_
  *   then n ints of schedule (front jobs, free jobs, back jobs: the
  *   reference's node->schedule), then n each of weak LB front, weak LB back,
  *   Johnson LB front, Johnson LB back, by job id, exactly as the explorer
- *   computed them before pruning (0 = not evaluated). */
+ *   computed them before pruning (0 = not evaluated).
+ * The values are those of the search's own explorer build, except in bounding
+ * mode 2 with a rule of -1 to 3: that search compares kept pair bounds and
+ * computes no Johnson values, so the sampled windows run the general build,
+ * whose counts and decisions are the same. */
 int pbb_diag_sample_nodes(struct pbb_engine* e, int32_t capacity, int32_t rate_log2);
+/* The same in that search's own build, with what it decided by the kept pair
+ * bounds in place of the Johnson values: 0 = child not asked about, 1 = kept,
+ * 2 = pruned.  PBB_E_UNSUPPORTED for a search that does not run with them. */
+int pbb_diag_sample_decisions(struct pbb_engine* e, int32_t capacity, int32_t rate_log2);
 /* Copy up to max_records records; *count = records copied (max_records <= 0:
  * records available). */
 int pbb_diag_get_samples(struct pbb_engine* e, int32_t max_records, int32_t* out, int32_t* count);

@@ -134,6 +134,7 @@ def lib():
         L.pbb_decimal_to_fact.argtypes = [ctypes.c_int32, ctypes.c_char_p, _i32p]
         L.pbb_diag_set_step_limits.argtypes = [ctypes.c_void_p, ctypes.c_int32, ctypes.c_int32]
         L.pbb_diag_sample_nodes.argtypes = [ctypes.c_void_p, ctypes.c_int32, ctypes.c_int32]
+        L.pbb_diag_sample_decisions.argtypes = [ctypes.c_void_p, ctypes.c_int32, ctypes.c_int32]
         L.pbb_diag_get_samples.argtypes = [ctypes.c_void_p, ctypes.c_int32, _i32p, ctypes.POINTER(ctypes.c_int32)]
         L.pbb_work_counters.argtypes = [ctypes.c_void_p, ctypes.POINTER(_Work)]
         L.pbb_diag_bound_children.argtypes = [ctypes.POINTER(_Instance), ctypes.c_int32, ctypes.c_int32,
@@ -321,6 +322,11 @@ class Engine:
         explore() raises PbbError(PBB_E_TIMEOUT) when it runs out, and the
         next call accounts for the window."""
         _check(lib().pbb_set_wait_limit(self._h, float(seconds)))
+
+    def sample_decisions(self, capacity, rate_log2):
+        """Diagnostic: as sample_nodes, by the build with kept pair bounds; the
+        strong arrays hold what it decided (0 not asked, 1 kept, 2 pruned)."""
+        _check(lib().pbb_diag_sample_decisions(self._h, int(capacity), int(rate_log2)))
 
     def sample_nodes(self, capacity, rate_log2):
         """Diagnostic: from the next window on, record nodes the explorer

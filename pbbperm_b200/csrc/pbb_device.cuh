@@ -1293,9 +1293,32 @@ __device__ __forceinline__ void reverse_row(int (&row)[NW], int k)
     for (int w = 0; w < NW; w++) row[w] = nr[w];
 }
 
-// Returns the side chosen for this level.  SAMPLE = 1 with `rec` set writes
-// the children's bounds, as computed and before pruning, into a node record
+// The row and four values of each of its children into a node record
 // (SampleBuf layout: schedule at rec + PBB_SAMPLE_HDR, then four arrays of n).
+template <int NW>
+__device__ __forceinline__ void store_sample(int* rec, int n, const int (&row)[NW], const bool (&valid)[NW], int f, int dir,
+                                             const int (&v0)[NW], const int (&v1)[NW], const int (&v2)[NW],
+                                             const int (&v3)[NW])
+{
+    const int lane = lane_id();
+    int* sch = rec + PBB_SAMPLE_HDR;
+#pragma unroll
+    for (int w = 0; w < NW; w++) {
+        if (valid[w]) {
+            const int u = row[w];
+            sch[f + w * 32 + lane] = u;
+            sch[n + u] = v0[w];
+            sch[2 * n + u] = v1[w];
+            sch[3 * n + u] = v2[w];
+            sch[4 * n + u] = v3[w];
+        }
+    }
+    if (lane == 0) rec[4] = dir;
+    __syncwarp();
+}
+
+// Returns the side chosen for this level.  SAMPLE = 1 with `rec` set writes
+// the children's bounds, as computed and before pruning, into a node record.
 template <int NW, int SORT = 1, int SAMPLE = 0>
 __device__ __forceinline__ int bound_and_prune(const CtaTables& T, const WarpScratch& S, const DevSearch& srch,
                                                int mode, int (&row)[NW], int k, int f, int b, int line,
@@ -1411,23 +1434,7 @@ __device__ __forceinline__ int bound_and_prune(const CtaTables& T, const WarpScr
         if (mode == 1) dir = choose_dir<NW>(srch.branch_mode, line, best, cbs, ces, valid);
     }
 
-    if (SAMPLE && rec) {
-        const int n = T.n;
-        int* sch = rec + PBB_SAMPLE_HDR;
-#pragma unroll
-        for (int w = 0; w < NW; w++) {
-            if (valid[w]) {
-                const int u = row[w];
-                sch[f + w * 32 + lane] = u;
-                sch[n + u] = cbw[w];
-                sch[2 * n + u] = cew[w];
-                sch[3 * n + u] = cbs[w];
-                sch[4 * n + u] = ces[w];
-            }
-        }
-        if (lane == 0) rec[4] = dir;
-        __syncwarp();
-    }
+    if (SAMPLE && rec) store_sample<NW>(rec, T.n, row, valid, f, dir, cbw, cew, cbs, ces);
 
     // prune: mark children whose bound reaches the incumbent (eliminateJobs :338-410)
 #pragma unroll
@@ -1662,9 +1669,10 @@ __device__ __forceinline__ void johnson_prune(const CtaTables& T, const WarpScra
 // milliseconds, sweeps with shared atomics / this: 18x20 9.6 / 8.4, 20x20 144 /
 // 137, 30x10 2.05 / 1.70, 13x10 0.33 / 0.28; both are bound by the two walks
 // over all positions of every pair.
-template <int NW>
+template <int NW, int SAMPLE>
 __device__ __forceinline__ int bound_all(const CtaTables& T, const WarpScratch& S, const DevSearch& srch,
-                                         int (&row)[NW], int k, int line, int prev_dir, int best, NodeCounters& cnt)
+                                         int (&row)[NW], int k, int f, int line, int prev_dir, int best,
+                                         NodeCounters& cnt, int* rec)
 {
     const int lane = lane_id();
     bool valid[NW];
@@ -1693,6 +1701,12 @@ __device__ __forceinline__ int bound_all(const CtaTables& T, const WarpScratch& 
         cnt.swept_children += 2 * k;
     }
     const int dir = choose_dir<NW>(srch.branch_mode, line, best, cb, ce, valid);
+    if (SAMPLE && rec) {
+        int none[NW];
+#pragma unroll
+        for (int w = 0; w < NW; w++) none[w] = 0;
+        store_sample<NW>(rec, T.n, row, valid, f, dir, none, none, cb, ce);
+    }
     // prune (eliminateJobs :338-410)
 #pragma unroll
     for (int w = 0; w < NW; w++) {
@@ -1708,10 +1722,12 @@ __device__ __forceinline__ int bound_all(const CtaTables& T, const WarpScratch& 
 // of the side it chooses (all but the fixed back sides): the same row and side,
 // the Johnson values compared instead of computed (see above).  GEN = 0: MinMin,
 // no findAll, no sorted rows, compiled in; GEN = 1: the search's settings.
-template <int NW, int GEN>
+// SAMPLE = 1 with `rec` set: the one-machine bounds, and in place of Johnson
+// values what was decided on the side chosen (0 not asked, 1 kept, 2 pruned).
+template <int NW, int GEN, int SAMPLE>
 __device__ __forceinline__ int bound_pairs(const CtaTables& T, const WarpScratch& S, PairBounds& B,
-                                           const DevSearch& srch, int (&row)[NW], int k, int line, int u, int hf,
-                                           int hb, int prev_dir, int best, NodeCounters& cnt)
+                                           const DevSearch& srch, int (&row)[NW], int k, int f, int line, int u, int hf,
+                                           int hb, int prev_dir, int best, NodeCounters& cnt, int* rec)
 {
     const int lane = lane_id();
     bool valid[NW];
@@ -1751,6 +1767,16 @@ __device__ __forceinline__ int bound_pairs(const CtaTables& T, const WarpScratch
         } else {
             johnson_prune<NW>(T, S, B, row, valid, keep, dir, line, u, hf, hb, limit, cut, cnt, k);
         }
+    }
+    if (SAMPLE && rec) {
+        int front[NW], back[NW];
+#pragma unroll
+        for (int w = 0; w < NW; w++) {
+            const int said = !((keep[w] >> lane) & 1u) ? 0 : (cut[w] ? 2 : 1);
+            front[w] = dir ? 0 : said;
+            back[w] = dir ? said : 0;
+        }
+        store_sample<NW>(rec, T.n, row, valid, f, dir, cbw, cew, front, back);
     }
     // prune (eliminateJobs :338-410)
 #pragma unroll

@@ -159,6 +159,7 @@ struct pbb_engine {
     SampleBuf* sample_d = nullptr; // node sampling (diagnostic), NULL when off
     int* sample_rec = nullptr;
     int sample_stride = 0;
+    bool sample_decisions = false; // by the build with kept pair bounds
     double wait_limit_s = -1.0;    // host wait per window: < 0 window + 60 s, 0 unbounded
     bool pending = false;          // a window whose wait ran out is still on the stream
 };
@@ -658,9 +659,11 @@ int pbb_diag_set_step_limits(pbb_engine* e, int32_t select_budget, int32_t max_r
     return PBB_OK;
 }
 
-int pbb_diag_sample_nodes(pbb_engine* e, int32_t capacity, int32_t rate_log2)
+static int sample_nodes(pbb_engine* e, int32_t capacity, int32_t rate_log2, bool decisions)
 {
     if (!e) return fail(PBB_E_INVAL, "engine is NULL");
+    if (decisions && (e->pair_warps <= 0 || !PBB_VAR_PAIRS(e->pair_variant)))
+        return fail(PBB_E_UNSUPPORTED, "this search does not run with kept pair bounds");
     if (capacity < 0 || rate_log2 < 0 || rate_log2 > 30) return fail(PBB_E_INVAL, "bad sampling parameters");
     pbbh::DeviceGuard keep_callers_device;
     CK(cudaSetDevice(e->dev));
@@ -674,6 +677,7 @@ int pbb_diag_sample_nodes(pbb_engine* e, int32_t capacity, int32_t rate_log2)
     e->sample_d = nullptr;
     e->sample_rec = nullptr;
     e->group.sample = nullptr;
+    e->sample_decisions = decisions;
     if (capacity > 0) {
         e->sample_stride = PBB_SAMPLE_HDR + 5 * e->H.n;
         const size_t bytes = sizeof(int) * (size_t)capacity * e->sample_stride;
@@ -692,6 +696,16 @@ int pbb_diag_sample_nodes(pbb_engine* e, int32_t capacity, int32_t rate_log2)
     CK(cudaMemcpyAsync(e->group_d, &e->group, sizeof(DevGroup), cudaMemcpyHostToDevice, e->st));
     CK(cudaStreamSynchronize(e->st));
     return PBB_OK;
+}
+
+int pbb_diag_sample_nodes(pbb_engine* e, int32_t capacity, int32_t rate_log2)
+{
+    return sample_nodes(e, capacity, rate_log2, false);
+}
+
+int pbb_diag_sample_decisions(pbb_engine* e, int32_t capacity, int32_t rate_log2)
+{
+    return sample_nodes(e, capacity, rate_log2, true);
 }
 
 int pbb_diag_get_samples(pbb_engine* e, int32_t max_records, int32_t* out, int32_t* count)
@@ -730,11 +744,18 @@ static int explore_window(pbb_engine* e, double seconds, int32_t* done, int eage
         const double win = (seconds > 0 && seconds < 120.0) ? seconds : 120.0;
         const unsigned long long budget = (unsigned long long)(win * 1e9);
         CK(cudaEventRecord(e->ev0, e->st));
-        int variant = e->sample_d ? 2 : ((e->cfg.sorted_dfs || e->cfg.early_stop_johnson) ? 1 : 0);
-        if (variant != 2 && e->pair_warps > 0) variant = e->pair_variant;
-        const bool pairs = variant >= 3;
-        CK(pbbl::launch_explore(e->nw, e->group_d, e->ngroups_d, e->ctas, pairs ? e->pair_warps : e->warps,
-                                pairs ? e->pair_smem : e->smem, budget, e->max_rounds, e->select_budget, e->st,
+        int variant = (e->cfg.sorted_dfs || e->cfg.early_stop_johnson) ? 1 : 0;
+        if (e->pair_warps > 0) variant = e->pair_variant;
+        // sampling: by the search's own build, but for the Johnson values of a
+        // search with kept pair bounds, which computes none
+        if (e->sample_d) {
+            if (variant == 7) variant = 10;
+            else if (e->sample_decisions) variant = PBB_VAR_GEN(variant) ? 9 : 8;
+            else variant = 2;
+        }
+        const bool own = variant >= 3;
+        const int warps = std::min(own ? e->pair_warps : e->warps, PBB_EXPLORE_WARPS(variant));
+        CK(pbbl::launch_explore(e->nw, e->group_d, e->ngroups_d, e->ctas, warps, own ? e->pair_smem : e->smem, budget, e->max_rounds, e->select_budget, e->st,
                                 variant, eager, e->pair_stack, e->pair_stride));
         CK(cudaEventRecord(e->ev1, e->st));
         rc = wait_event(e->ev1, e->wait_limit_s < 0 ? win + 60.0 : e->wait_limit_s);

@@ -436,9 +436,10 @@ __device__ __forceinline__ void bound_current(const DevGroup& G, const CtaTables
     NodeCounters nc = {0, 0, 0, 0, 0};
     int d;
     if (PAIRS == 3)
-        d = bound_all<NW>(T, S, G.search, R.row, T.n - L, L, prev, best, nc);
+        d = bound_all<NW, SAMPLE>(T, S, G.search, R.row, T.n - L, f, L, prev, best, nc, rec);
     else if (PAIRS)
-        d = bound_pairs<NW, (PAIRS == 2)>(T, S, B, G.search, R.row, T.n - L, L, vget<NW>(R.pj, L - 1), R.hf, R.hb, prev, best, nc);
+        d = bound_pairs<NW, (PAIRS == 2), SAMPLE>(T, S, B, G.search, R.row, T.n - L, f, L, vget<NW>(R.pj, L - 1), R.hf, R.hb,
+                                                  prev, best, nc, rec);
     else
         d = bound_and_prune<NW, SORT, SAMPLE>(T, S, G.search, mode, R.row, T.n - L, f, b, L, prev, best, nc, true, rec);
     vset<NW>(R.dir, L, d);
@@ -879,7 +880,8 @@ __global__ void pbb_root_kernel(const DevGroup* groups, int ngroups, const int* 
 // default search (MinMin, no findAll, rows not sorted, compiled in), 4 every
 // other search of that mode whose rule bounds the side it chooses; 5 and 6 are
 // their builds for 32 warps a CTA.  VAR = 7 bounds in mode 1 by
-// johnson_all (rows of one word).
+// johnson_all (rows of one word).  VAR = 8, 9 and 10 are 3, 4 and 7 and record
+// sampled nodes.
 template <int NW, int VAR>
 __global__ void __launch_bounds__(32 * PBB_EXPLORE_WARPS(VAR), 1)
 pbb_explore_kernel(const DevGroup* groups, const int* ngroups_d, int warps_per_cta, unsigned long long budget_ns,
@@ -899,13 +901,13 @@ pbb_explore_kernel(const DevGroup* groups, const int* ngroups_d, int warps_per_c
     asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn_smem));
     // (the one-machine bound alone has no use for them)
     int fm = PBB_SCRATCH_PLAIN;
-    if (VAR == 7) {
+    if (PBB_VAR_ALL(VAR)) {
         fm = PBB_SCRATCH_ALL;
         if (pbb_smem_plan(G.inst.n, G.inst.m, G.inst.Ppad, warps_per_cta, fm).total > (int)dyn_smem) {
             if (threadIdx.x == 0) atomicOr(&G.ctl->status, PBB_ST_BADINPUT);
             return;
         }
-    } else if (VAR >= 3) {
+    } else if (PBB_VAR_PAIRS(VAR)) {
         // the host launches this build only with room for its scratch
         fm = PBB_SCRATCH_PAIRS;
         if (!pair_stack || G.inst.n * G.inst.Ppad > pair_stride ||
@@ -936,14 +938,14 @@ pbb_explore_kernel(const DevGroup* groups, const int* ngroups_d, int warps_per_c
     const WarpScratch S = warp_scratch(smem + sp.warp_off + wic * sp.warp_bytes, sp, T.n, T.m, T.Ppad);
     const int W = G.ctas * warps_per_cta;
     const int wid = (blockIdx.x - G.first_cta) * warps_per_cta + wic;
-    const int mode = VAR == 7 ? 1 : VAR >= 3 ? 2 : G.search.bound_mode;
+    const int mode = PBB_VAR_ALL(VAR) ? 1 : PBB_VAR_PAIRS(VAR) ? 2 : G.search.bound_mode;
     const unsigned long long t0 = globaltimer_ns();
 
     WarpCounters C = {0, 0, 0, 0, 0, 0, 0, 0, 0};
     PairBounds B;
     B.cur = S.pairs;
     B.nxt = S.pairs + T.Ppad;
-    B.stack = VAR >= 3 && VAR <= 6 ? pair_stack + (size_t)(blockIdx.x * warps_per_cta + wic) * pair_stride : nullptr;
+    B.stack = PBB_VAR_PAIRS(VAR) ? pair_stack + (size_t)(blockIdx.x * warps_per_cta + wic) * pair_stride : nullptr;
     B.level = -1;
     B.from = 0;
     Ivm<NW> R;
@@ -1058,11 +1060,13 @@ pbb_explore_kernel(const DevGroup* groups, const int* ngroups_d, int warps_per_c
         const int wish = share_wish(G.search, H, since, warps_per_cta, G.ctas, eager, narrow);
         if (wish && try_share<NW>(G, H, wic, id, R, wish, narrow) == 1) since = 0;
         const int known = best;
-        const int r = select_node<NW, (VAR >= 3 && VAR <= 6)>(G, T, S, id, R, best, C, select_budget);
+        const int r = select_node<NW, PBB_VAR_PAIRS(VAR)>(G, T, S, id, R, best, C, select_budget);
         if (best < known && lane_id() == 0) atomicMin(&H->best, best);
         if (r == 1) {
             since++;
-            bound_current<NW, (VAR == 1 || VAR == 2), (VAR == 2), (VAR == 7 ? 3 : VAR >= 3 ? 2 - (VAR & 1) : 0)>(G, T, S, B, id, R, mode, best, C);
+            bound_current<NW, (VAR == 1 || VAR == 2), PBB_VAR_SAMPLE(VAR),
+                          (PBB_VAR_ALL(VAR) ? 3 : PBB_VAR_PAIRS(VAR) ? 1 + PBB_VAR_GEN(VAR) : 0)>(G, T, S, B, id, R, mode, best,
+                                                                                            C);
         }
         if (C.decomposed >= PBB_FLUSH_NODES) flush_counters(G, C);
         if (r == 0) {
@@ -1476,6 +1480,9 @@ cudaError_t launch_explore(int nw, const DevGroup* groups, const int* ngroups_d,
         case 5: return PBB_EXPLORE(1, 5);
         case 6: return PBB_EXPLORE(1, 6);
         case 7: return PBB_EXPLORE(1, 7);
+        case 8: return PBB_EXPLORE(1, 8);
+        case 9: return PBB_EXPLORE(1, 9);
+        case 10: return PBB_EXPLORE(1, 10);
         default: return PBB_EXPLORE(1, 0);
         }
     }
@@ -1486,6 +1493,8 @@ cudaError_t launch_explore(int nw, const DevGroup* groups, const int* ngroups_d,
     case 4: return PBB_EXPLORE(2, 4);
     case 5: return PBB_EXPLORE(2, 5);
     case 6: return PBB_EXPLORE(2, 6);
+    case 8: return PBB_EXPLORE(2, 8);
+    case 9: return PBB_EXPLORE(2, 9);
     default: return PBB_EXPLORE(2, 0);
     }
 #undef PBB_EXPLORE

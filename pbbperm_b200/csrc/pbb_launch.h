@@ -28,7 +28,8 @@ cudaError_t launch_lower_ub(const DevGroup* groups, int g, int ub, cudaStream_t 
 // with the PBB_SCRATCH_PAIRS shared memory and with pair_stack, pair_stride
 // ints for each warp of the grid (at least jobs x padded machine pairs).
 // 7 = every child's Johnson value (mode 1, up to 32 jobs), launched with the
-// PBB_SCRATCH_ALL shared memory.
+// PBB_SCRATCH_ALL shared memory.  8, 9 and 10 = as 3, 4 and 7 and record sampled
+// nodes.
 // eager = 0: a short window, which splits work only as often as share_after
 // says, however many warps wait
 cudaError_t launch_explore(int nw, const DevGroup* groups, const int* ngroups_d, int ctas, int warps_per_cta, int smem,

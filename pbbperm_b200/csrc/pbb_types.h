@@ -10,6 +10,13 @@
 // 4), whose scratch leaves the room.
 #define PBB_WIDE_WARPS 32
 #define PBB_EXPLORE_WARPS(var) ((var) == 5 || (var) == 6 ? PBB_WIDE_WARPS : PBB_WARPS_MAX)
+// What an explorer variant bounds with (pbb_launch.h): kept pair bounds, with
+// the search's settings at run time, or every child's Johnson value; and
+// whether it records sampled nodes
+#define PBB_VAR_PAIRS(var) (((var) >= 3 && (var) <= 6) || (var) == 8 || (var) == 9)
+#define PBB_VAR_GEN(var) ((var) == 4 || (var) == 6 || (var) == 9)
+#define PBB_VAR_ALL(var) ((var) == 7 || (var) == 10)
+#define PBB_VAR_SAMPLE(var) ((var) == 2 || (var) >= 8)
 // The wide builds pay where a search is long enough to be bound by throughput;
 // below, where it is bound by the time one node takes and by how fast work
 // spreads, their spilled registers and additional warps cost a little.  The

@@ -1,18 +1,23 @@
-"""LB parity of the explorer's own bound code on nodes it actually bounded.
+"""Parity of the explorer's own bound code on nodes it actually bounded.
 
-The explorer does not bound through pbb_bound_children: it keeps heads and
-tails of the fixed jobs in a per-level path stack, scans the Johnson orders
-over the free positions only, walks up to four children's scans together and
-switches to max-plus sweeps for more children.  Here it records nodes as it
-bounds them (hash of explorer id and step, include/pbbperm_diag.h), and every
-recorded value is checked bit-exact against the reference's own bounds
-library (oracle/_ref/libref_bounds.so: bound_fsp_weak::boundChildren, and
-bound_fsp_strong::bornes_calculer on each child the explorer evaluated, as
-ivm_bound::computeStrongBounds calls it, multicore/src/ivm_bound.cpp:141-195).
-The side chosen and the set of Johnson-evaluated children are checked against
-the reference's rules: MinMin (ivm_bound.cpp:479-504) on the weak bounds with
-the incumbent as UB, and Johnson only for children the weak bound keeps on
-that side (ivm_bound.cpp:168)."""
+The explorer does not bound through pbb_bound_children.  It records nodes as it
+bounds them (hash of explorer id and step, include/pbbperm_diag.h), and:
+
+* in bounding mode 2 the general build -- heads and tails from a per-level path
+  stack, Johnson scans over the free positions, up to four children's scans
+  together, max-plus sweeps for more -- is checked value by value against the
+  reference's own bounds library (oracle/_ref/libref_bounds.so:
+  bound_fsp_weak::boundChildren, and bound_fsp_strong::bornes_calculer on each
+  child the explorer evaluated, as ivm_bound::computeStrongBounds calls it,
+  multicore/src/ivm_bound.cpp:141-195), with the side chosen and the set of
+  Johnson-evaluated children by the reference's rules: MinMin
+  (ivm_bound.cpp:479-504) on the weak bounds with the incumbent as UB, and
+  Johnson only for children the weak bound keeps on that side
+  (ivm_bound.cpp:168);
+* searches of that mode run a build that compares kept pair bounds and has no
+  Johnson values: what it decided about every child is checked against them;
+* in bounding mode 1 the values of the search's own build are checked: shared
+  maxima for rows of two words, values by position for rows of one."""
 import numpy as np
 import pytest
 
@@ -131,3 +136,96 @@ def test_explorer_sampled_nodes_johnson_only_mode():
         bad = idx[(got[idx] != want[idx]).any(axis=1)]
         assert len(bad) == 0, (name, len(bad), bad[:5].tolist())
     assert len(np.unique(s["line"])) >= 10
+
+
+def child_bounds(p, s, samples=200):
+    """Johnson bounds of the records' children by direct scans, checked by the
+    oracle on some of them."""
+    want = pb.bound_children(p, s["sched"], s["limit1"], s["limit2"], method=1)
+    O = Oracle(p)
+    cnt = len(s["k"])
+    for i in range(0, cnt, max(1, cnt // samples)):
+        for key, front in (("strong_begin", True), ("strong_end", False)):
+            assert (want[key][i] == O.strong_children(s["sched"][i], s["limit1"][i], s["limit2"][i], front)).all(), (i, key)
+    return want
+
+
+def free_mask(s, n):
+    free = np.zeros((len(s["k"]), n), bool)
+    for i in range(len(s["k"])):
+        free[i, s["sched"][i, s["limit1"][i] + 1:s["limit2"][i]]] = True
+    return free
+
+
+@pytest.mark.parametrize("n,m,seed,ub,ivms,cap,rate,warm,opt", [
+    (50, 20, 2, None, 65536, 50000, 6, 0.5, {}),          # 32 warps a CTA in the search itself
+    (20, 20, 1, 2352, 16384, 30000, 7, 0.0, {}),
+    (16, 12, 2, 1525, 4096, 20000, 0, 0.0, {}),
+    (64, 10, 4, 3777, 4096, 20000, 0, 0.0, {}),
+    (50, 20, 2, None, 65536, 50000, 6, 0.5, dict(adaptiveBranchingMode=2, findAll=True)),
+    (20, 20, 1, 2352, 16384, 30000, 7, 0.0, dict(adaptiveBranchingMode=1, sortedDFS=2, sortingCriterion=2)),
+    (16, 12, 2, 1525, 4096, 20000, 0, 0.0, dict(adaptiveBranchingMode=-1, earlyStopJohnson=True)),
+])
+def test_decisions_by_kept_pair_bounds(n, m, seed, ub, ivms, cap, rate, warm, opt):
+    p = synthetic_instance(seed, n, m)
+    ub = pb.neh(p)[0] if ub is None else ub
+    cfg = pb.Config(boundingMode=2, nbIVMs=ivms, **opt)
+    with pb.Engine(p, cfg) as e:
+        e.start(ub=ub)
+        done = e.explore(warm) if warm > 0 else False
+        e.sample_decisions(cap, rate)
+        for _ in range(4000):
+            if done or e.sample_count() >= cap:
+                break
+            done = e.explore(0.02)
+        s = e.samples()
+    cnt = len(s["k"])
+    assert cnt >= 1000, cnt
+    assert (np.sort(s["sched"], axis=1) == np.arange(n)).all()
+    assert ((s["limit1"] + 1) + (n - s["limit2"]) == s["line"]).all()
+    free = free_mask(s, n)
+    limit = (s["best"] + (1 if opt.get("findAll") else 0))[:, None]
+    asked = pruned = 0
+    want = child_bounds(p, s)
+    for side, weak, said, strong in ((0, "weak_begin", "strong_begin", "strong_begin"),
+                                     (1, "weak_end", "strong_end", "strong_end")):
+        on = (s["side"] == side)[:, None]
+        if opt.get("adaptiveBranchingMode", 3) > 0 or side == 0:
+            assert (np.where(free, s[weak] == want[weak], s[weak] == 0)).all()
+        keep = free & on & (s[weak] < limit)
+        assert ((s[said] != 0) == keep).all()
+        assert ((s[said] == 2) == (keep & (want[strong] >= limit))).all()
+        asked += keep.sum()
+        pruned += (s[said] == 2).sum()
+    if opt.get("adaptiveBranchingMode", 3) == 3:
+        assert (s["side"] == minmin_side(s["weak_begin"], s["weak_end"], s["best"])).all()
+    # both answers were given often enough to tell
+    assert pruned >= 100 and asked - pruned >= 100, (asked, pruned)
+
+
+@pytest.mark.parametrize("n,m,seed,ub,opt", [
+    (20, 20, 1, 2352, {}), (32, 10, 3, 2160, {}), (18, 20, 1, None, dict(adaptiveBranchingMode=2, findAll=True)),
+    (12, 10, 3, 1171, dict(adaptiveBranchingMode=1)),
+])
+def test_values_by_position_in_mode_1(n, m, seed, ub, opt):
+    """Rows of one word: every child's Johnson value on both sides."""
+    p = synthetic_instance(seed, n, m)
+    ub = int(pb.neh(p)[0] * 0.97) if ub is None else ub
+    with pb.Engine(p, pb.Config(boundingMode=1, nbIVMs=16384, **opt)) as e:
+        e.start(ub=ub)
+        e.sample_nodes(20000, 4 if n >= 18 else 0)
+        done = False
+        for _ in range(4000):
+            if done or e.sample_count() >= 20000:
+                break
+            done = e.explore(0.02)
+        s = e.samples()
+    cnt = len(s["k"])
+    assert cnt >= 1000, cnt
+    free = free_mask(s, n)
+    assert (s["weak_begin"] == 0).all() and (s["weak_end"] == 0).all()
+    want = child_bounds(p, s)
+    for key in ("strong_begin", "strong_end"):
+        assert (np.where(free, s[key] == want[key], s[key] == 0)).all(), key
+    if opt.get("adaptiveBranchingMode", 3) == 3:
+        assert (s["side"] == minmin_side(s["strong_begin"], s["strong_end"], s["best"])).all()
