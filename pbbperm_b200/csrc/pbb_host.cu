@@ -162,6 +162,7 @@ struct pbb_engine {
     bool sample_decisions = false; // by the build with kept pair bounds
     double wait_limit_s = -1.0;    // host wait per window: < 0 window + 60 s, 0 unbounded
     bool pending = false;          // a window whose wait ran out is still on the stream
+    bool exporting = true;         // the search has just started, or its intervals were exported since its last window
 };
 
 namespace pbbh {
@@ -497,6 +498,7 @@ static int start_impl(pbb_engine* e, int32_t ub, const int32_t* root_perm, const
     GroupCtl c;
     CK(cudaMemcpy(&c, e->ctl, sizeof(c), cudaMemcpyDeviceToHost));
     e->started = true;
+    e->exporting = true;
     e->done = (c.active == 0);
     e->dev_seconds = 0.0;
     return PBB_OK;
@@ -569,6 +571,7 @@ int pbb_init_from_fac(pbb_engine* e, int32_t ub, const int32_t* root_perm, int32
     e->root.assign(root.begin(), root.begin() + n);
     e->start_perm.clear();
     e->started = true;
+    e->exporting = true;
     e->done = (c.active == 0);
     e->dev_seconds = 0.0;
     return PBB_OK;
@@ -586,6 +589,7 @@ int pbb_get_intervals(pbb_engine* e, int32_t max_intervals, int32_t* pos, int32_
         if (rs) return rs;
     }
     CK(cudaStreamSynchronize(e->st));
+    e->exporting = true;
     const int B = e->cfg.nb_ivms, n = e->H.n, npad = e->npad;
     std::vector<int> st(B);
     std::vector<signed char> ps((size_t)B * npad), es((size_t)B * npad);
@@ -776,14 +780,23 @@ static int explore_window(pbb_engine* e, double seconds, int32_t* done, int eage
     return PBB_OK;
 }
 
-// A window this short serves a caller that looks at the search between
-// windows (exports, exchanges or saves its intervals): it is not cut into more
-// intervals than share_after allows.
-#define PBB_SHORT_WINDOW_S 0.01
+// A caller that exports intervals between windows pays for every one: the
+// engine that resumes it bounds its path again.  So the first window of a
+// search, and one after an export, keeps to share_after when it is shorter than
+// this, and a caller that comes back without having exported gets eager windows
+// from then on.  Intervals after a first window kept to share_after / an eager
+// one: 2 ms 20x20 15 / 2924, 16x20 16 / 2914, 24x10 84 / done; 5 ms 330 / 4700,
+// 383 / 2803, 552 / done; at 9 ms 2935 / 4692 and 2899 / done, not worth the
+// speed: device ms of whole searches 20x20 42 / 32, 16x20 14.4 / 6.1, 24x10
+// 10 / 1.6, 13x20 8.5 / 0.9.
+#define PBB_SHORT_WINDOW_S 0.005
 
 int pbb_explore(pbb_engine* e, double seconds, int32_t* done)
 {
-    return explore_window(e, seconds, done, !(seconds > 0 && seconds < PBB_SHORT_WINDOW_S));
+    if (!e || !e->started) return fail(PBB_E_INVAL, "engine not started");
+    const bool may_export = e->exporting && seconds > 0 && seconds < PBB_SHORT_WINDOW_S;
+    e->exporting = false;
+    return explore_window(e, seconds, done, !may_export);
 }
 
 int pbb_get_result(pbb_engine* e, pbb_result* out)

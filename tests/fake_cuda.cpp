@@ -37,7 +37,8 @@ std::vector<void*> g_spare;                // addresses of the contexts before, 
 std::map<std::string, int> g_fail, g_calls;
 size_t g_capacity = ~(size_t)0, g_used = 0, g_reserved = 0, g_threshold = 0;
 int g_invalid = 0;                         // uses of handles that are not valid
-int g_variant = -1;
+int g_variant = -1, g_eager = -1;
+int g_windows = 1;                         // windows a search takes
 int g_per_sm[8] = {2, 2, 2, 2, 2, 2, 2, 2};   // resident CTAs an SM, by explorer variant
 int g_not_resident = 0;                    // explorer launches of more CTAs than are resident
 cudaError_t g_last = cudaSuccess;
@@ -125,6 +126,8 @@ void fake_reset()
 int fake_invalid() { Lock l(g_mu); return g_invalid; }
 void fake_per_sm(int variant, int ctas) { Lock l(g_mu); g_per_sm[variant] = ctas; }
 int fake_not_resident() { Lock l(g_mu); return g_not_resident; }
+int fake_eager() { Lock l(g_mu); return g_eager; }
+void fake_windows(int n) { Lock l(g_mu); g_windows = n; }
 int fake_variant() { Lock l(g_mu); return g_variant; }
 size_t fake_used() { Lock l(g_mu); return g_used + g_reserved; }
 int fake_calls(const char* name) { Lock l(g_mu); return g_calls[name]; }
@@ -277,12 +280,14 @@ cudaError_t launch_root(int, const DevGroup* g, int count, const int*, const int
 }
 cudaError_t launch_lower_ub(const DevGroup*, int, int, cudaStream_t) { return cudaSuccess; }
 cudaError_t launch_explore(int, const DevGroup* g, const int* count, int ctas, int, int, unsigned long long, int, int,
-                           cudaStream_t, int variant, int, int*, int)
+                           cudaStream_t, int variant, int eager, int*, int)
 {
     Lock l(g_mu);
     g_variant = variant;
+    g_eager = eager;
     g_not_resident += ctas > 148 * g_per_sm[variant];
-    for (int i = 0; i < *count; i++) g[i].ctl->active = 0;
+    if (--g_windows <= 0)
+        for (int i = 0; i < *count; i++) g[i].ctl->active = 0;
     return cudaSuccess;
 }
 cudaError_t launch_neh(const NehTask*, int, cudaStream_t) { return cudaSuccess; }

@@ -42,6 +42,7 @@ def L(fake_so, tmp_path):
                                     ctypes.c_int64]
     lib.pbb_pool_step.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p]
     lib.pbb_pool_destroy.argtypes = [ctypes.c_void_p]
+    lib.pbb_get_intervals.argtypes = [ctypes.c_void_p, ctypes.c_int32, i32p, i32p, i32p, ctypes.c_void_p]
     lib.pbb_explore.argtypes = [ctypes.c_void_p, ctypes.c_double, ctypes.c_void_p]
     return lib
 
@@ -257,3 +258,27 @@ def test_threads_share_what_is_kept(L):
     assert not bad and L.fake_invalid() == 0
     assert L.pbb_release_memory(0) == 0
     assert L.fake_used() == 0 and L.fake_streams() == 0
+
+
+def test_short_windows_share_fully_unless_their_caller_exports(L):
+    """Under 5 ms, the first window and one after an export keep the number of
+    intervals down; other windows do not."""
+    L.fake_windows(100)
+    rc, e = create(L, n=12, m=10, nbIVMs=64)
+    assert rc == 0
+    pos, end, ids = (np.zeros(64 * 12, np.int32) for _ in range(3))
+    cnt = ctypes.c_int32()
+
+    def window(seconds):
+        assert L.pbb_explore(e, seconds, None) == 0
+        return L.fake_eager()
+
+    for _ in range(2):
+        assert L.pbb_start(e, 1000, None) == 0
+        assert [window(0.002), window(0.002), window(0.002)] == [0, 1, 1]
+        assert L.pbb_get_intervals(e, 64, pos.ctypes.data_as(i32p), end.ctypes.data_as(i32p), ids.ctypes.data_as(i32p),
+                                   ctypes.byref(cnt)) == 0
+        assert [window(0.002), window(0.002)] == [0, 1]
+        assert L.pbb_start(e, 1000, None) == 0
+        assert [window(0.006), window(0.001)] == [1, 1]
+    L.pbb_engine_destroy(e)
