@@ -311,8 +311,8 @@ int pbb_neh(const pbb_instance* inst, int32_t* perm, int32_t* cost);
  * stride of PBB_MAX_JOBS per instance. */
 int pbb_neh_batch(const pbb_instance* inst, int32_t count, int32_t device, int32_t* perms, int32_t* costs);
 
-/* Iterated greedy from the NEH schedule on the device, one warp per instance
- * (IG::runIG, heuristic/src/IG.cpp:341-416): per round, 2 to 5 jobs removed
+/* Iterated greedy from the NEH schedule on the device, eight warps per
+ * instance (IG::runIG, heuristic/src/IG.cpp:341-416): per round, 2 to 5 jobs removed
  * from a shuffled prefix of the middle-out visit order (:120-160), each put
  * back at its best position (:229-255), first-improvement insertion moves
  * within sqrt(n) places (localSearchKI :567-612), and the temperature

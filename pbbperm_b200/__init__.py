@@ -483,7 +483,7 @@ def neh_batch(instances, device=0):
 
 
 def ig_batch(instances, iterations=100, seed=0, device=0):
-    """Seeded iterated greedy from NEH on the device (one warp per instance):
+    """Seeded iterated greedy from NEH on the device (eight warps per instance):
     list of (cost, permutation); instance i draws from seed + i."""
     cnt = len(instances)
     arr, keep = _instance_array(instances)

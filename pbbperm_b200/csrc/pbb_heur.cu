@@ -1,6 +1,6 @@
 // Initial upper bounds on the device: NEH (heuristic/src/fastNEH.cpp:230-243
-// for the insertion procedure), one warp per instance, for many instances in
-// one launch -- the pool computes its admissions' bounds this way, without a
+// for the insertion procedure), one warp per instance, and iterated greedy,
+// eight warps per instance, for many instances in one launch -- the pool computes its admissions' bounds this way, without a
 // host round trip, and the engine can start from it.
 //
 // Insertion of job x into a sequence of `len` jobs uses Taillard's heads and
@@ -310,7 +310,7 @@ __global__ void __launch_bounds__(32) pbb_neh_kernel(const NehTask* tasks, int c
 // one a single warp would have come to; a pass computes the whole sequence's
 // heads and tails once for all its probes.  64 instances of 50 x 20, five
 // rounds, whole call: 23.7 ms with one warp and two whole passes per probe,
-// 2.4 ms so (NEH alone 1.2); 1500 mixed instances, three rounds: 17 and 7.
+// 2.4 ms so (NEH alone 1.2).
 __global__ void __launch_bounds__(32 * PBB_IG_WARPS) pbb_ig_kernel(const NehTask* tasks, int count, IgParams prm)
 {
     extern __shared__ __align__(16) int hs[];
@@ -463,12 +463,13 @@ cudaError_t launch_neh(const NehTask* tasks_d, int count, cudaStream_t st)
 cudaError_t launch_ig(const NehTask* tasks_d, int count, const IgParams& prm, cudaStream_t st)
 {
     if (count <= 0) return cudaSuccess;
-    // eight warps an instance while the GPU holds them all at once; past that
-    // the probes made for nothing would cost other instances their turn
-    const int warps = count <= 512 ? PBB_IG_WARPS : 2;
-    const int smem = PBB_HEUR_SMEM + warps * PBB_IG_WARP_SMEM;
+    // eight warps whatever the count, although probes made for nothing then
+    // cost other instances their turn: whole calls of 5 rounds with eight / two
+    // warps, ms, 50x20 513 instances 3.1 / 4.3, 1024 5.4 / 6.6, 4096 19.0 / 19.7;
+    // 20x10 1.3 / 1.4, 2.3 / 2.5, 8.8 / 8.7
+    const int smem = PBB_HEUR_SMEM + PBB_IG_WARPS * PBB_IG_WARP_SMEM;
     cudaFuncSetAttribute(pbb_ig_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    pbb_ig_kernel<<<count, 32 * warps, smem, st>>>(tasks_d, count, prm);
+    pbb_ig_kernel<<<count, 32 * PBB_IG_WARPS, smem, st>>>(tasks_d, count, prm);
     return cudaGetLastError();
 }
 

@@ -1,5 +1,5 @@
-// Device heuristics (pbb_heur.cu): NEH and iterated greedy, one warp per
-// instance.
+// Device heuristics (pbb_heur.cu): NEH, one warp per instance, and iterated
+// greedy, eight.
 #pragma once
 #include <cuda_runtime.h>
 #include "pbb_types.h"
@@ -28,7 +28,7 @@ struct IgParams {
 // meet on a bank more than twice.
 #define PBB_HEUR_ROW 34
 #define PBB_HEUR_REACH 8          // local-search moves reach at most sqrt(64) places
-#define PBB_IG_WARPS 8            // warps of an iterated-greedy block at most
+#define PBB_IG_WARPS 8            // warps of an iterated-greedy block
 // shared memory of one heuristic block: p, heads, tails, and per-job arrays;
 // and of each local-search warp: the rows its probe computes anew
 #define PBB_HEUR_SMEM (int)(sizeof(int) * (PBB_MAX_N * 36 + (2 * PBB_MAX_N + 1) * PBB_HEUR_ROW + 6 * PBB_MAX_N))

@@ -91,7 +91,7 @@ def test_device_ig_equals_its_restatement(iterations):
 @pytest.mark.parametrize("copies", [1, 70])
 def test_device_ig_at_the_edges_of_its_block_shapes(copies):
     """Sizes at the reach of a probe, one and 32 machines' worth of lanes, and
-    enough instances (8 x 70 > 512) for the narrow blocks."""
+    one instance a shape or many."""
     shapes = [(2, 2), (3, 2), (4, 3), (9, 32), (17, 31), (32, 4), (33, 5), (64, 2)]
     insts = [synthetic_instance(60 + i, n, m) for _ in range(copies) for i, (n, m) in enumerate(shapes)]
     got = pb.ig_batch(insts, iterations=4, seed=77)
