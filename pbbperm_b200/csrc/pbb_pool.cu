@@ -335,8 +335,8 @@ int pool_create(const pbb_pool_config* in, pbb_pool* P, int most)
     if (explorer_block_bytes(E, P->npad, P->cfg.max_jobs) > P->arena_bytes)
         return pfail(PBB_E_INVAL, "explorer_bytes is smaller than one instance's footprint");
     P->arena_bytes = std::min(P->arena_bytes, explorer_block_bytes(E, P->npad, c.max_jobs) * (size_t)P->max_slots);
-    PCK(pbbh::mem_alloc((void**)&P->arena, P->arena_bytes, P->lease), "explorer memory");
-    // after what the pool cannot do without: the general build needs none
+    // the pair bounds stand before the explorers in the store, but go back if
+    // those do not fit as well: the general build needs none
     if (P->pair_builds || P->tail_pair_builds) {
         const size_t w = std::max((size_t)P->grid * P->warps, (size_t)P->tail_grid * P->tail_warps);
         P->pair_stride = c.max_jobs * P->Ppad_max;
@@ -346,6 +346,16 @@ int pool_create(const pbb_pool_config* in, pbb_pool* P, int most)
             P->pair_builds = P->tail_pair_builds = 0;
         }
     }
+    cudaError_t room = pbbh::mem_alloc((void**)&P->arena, P->arena_bytes, P->lease);
+    if (room == cudaErrorMemoryAllocation && P->pair_stack) {
+        cudaGetLastError();
+        pbbh::mem_free(P->pair_stack, P->lease);
+        PCK(cudaStreamSynchronize(P->st), "pair bounds given back");
+        P->pair_stack = nullptr;
+        P->pair_builds = P->tail_pair_builds = 0;
+        room = pbbh::mem_alloc((void**)&P->arena, P->arena_bytes, P->lease);
+    }
+    PCK(room, "explorer memory");
     P->alloc.init(P->arena_bytes);
     P->slots.assign(S, Slot());
     return PBB_OK;
