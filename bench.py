@@ -83,7 +83,7 @@ def dist_env():
 def workload_config(extra=None):
     cfg = {"workload": "pfsp-50x20-u1-99-seed2", "n_jobs": N_JOBS, "n_machines": N_MACH, "seed": SEED,
            "bounding_mode": BOUND_MODE, "branching_mode": BRANCH_MODE, "nb_ivms": NB_IVMS,
-           "initial_ub": "NEH", "l2": "explorer state (65536 x 4.3 KB) exceeds L2; no flush"}
+           "initial_ub": "NEH", "l2": "explorer state (65536 x 22.7 KB) exceeds L2; no flush"}
     if extra:
         cfg.update(extra)
     return cfg
@@ -300,38 +300,39 @@ def run_ours(args):
 
     out = None
     if rank == 0:
-        h2d = int(p.size * 4 + N_JOBS * 192 * 8 + 2 * 192 + 2 * N_MACH * 4 + 4 + 64 * 4)
+        # processing times, Johnson entries and positions, pair machines, minimum
+        # times, bound, root
+        h2d = int(p.size * 4 + N_JOBS * 192 * 9 + 2 * 192 + 2 * N_MACH * 4 + 4 + 64 * 4)
         d2h = int(160 + 64)
         e2e = {"value": round(statistics.median(e2e_vals), 1) if e2e_vals else None, "unit": "nodes/s",
                "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
                "note": "per rank: engine creation + root/unfold + one window + result, summed over ranks, "
                        "time = slowest rank"}
 
-        # roofline of the explorer kernel.  `achieved` = the algorithmic INT32
-        # work of the bounds the reference defines per evaluation -- 5m per
-        # weak child ("m*(3 add+2 max)", bounds/src/bound_fsp_weak.cpp:132) and
-        # 4 P n + P per Johnson child (add, add-lag, max, add per job and pair
-        # over the full Johnson order, then the pair's close,
-        # bound_fsp_strong.cpp:84-100) -- times the evaluations the explorer
-        # made, per second of its device time.  The engine itself does less
-        # (its scans skip fixed jobs, and sweeps serve many children at once):
-        # its own operation count is reported beside it.
+        # roofline of the explorer kernel.  `achieved` = the INT32 operations of
+        # the bounds as the explorer executes them (Engine.kernel_stats), per
+        # second of its device time.  `equivalent` is the rate at which the
+        # reference's formulation would have to run to keep up: 5m per weak child
+        # ("m*(3 add+2 max)", bounds/src/bound_fsp_weak.cpp:132) and 4 P n + P per
+        # Johnson child (add, add-lag, max, add per job and pair over the full
+        # Johnson order, then the pair's close, bound_fsp_strong.cpp:84-100).  It
+        # is no fraction of the peak: the explorer does not execute it.
         peak = pb.int32_peak(local)
         P = N_MACH * (N_MACH - 1) // 2
         algo_ops = kern["simple_bounds"] * 5.0 * N_MACH + kern["johnson_bounds"] * (4.0 * P * N_JOBS + P)
         secs = kern["device_seconds"]
-        achieved = algo_ops / secs / 1e9 if secs > 0 else 0.0
-        engine = kern["int32_ops"] / secs / 1e9 if secs > 0 else 0.0
+        equivalent = algo_ops / secs / 1e9 if secs > 0 else 0.0
+        achieved = kern["int32_ops"] / secs / 1e9 if secs > 0 else 0.0
         roofline = {"bound": "int32", "achieved": round(achieved, 1), "peak": round(peak, 1), "unit": "Gop/s",
                     "frac": round(achieved / peak, 4) if peak else None,
-                    # DRAM bytes of one explorer launch: 16.9 MB in a 50 ms window of one
+                    # DRAM bytes of one explorer launch: 1.98 GB in a 50 ms window of one
                     # ncu capture of this workload, scaled to this window by device time
                     "traffic": round(NCU_DRAM_BYTES_PER_S * args.window),
                     "traffic_unit": "bytes per launch",
                     "peak_source": "measured: pbb_diag_int32_peak (IADD+IMNMX register chains, all SMs)",
-                    "work_model": "simple LBs x 5m + Johnson LBs x (4 P n + P), P = m(m-1)/2",
-                    "engine_ops": {"achieved": round(engine, 1), "frac": round(engine / peak, 4) if peak else None,
-                                   "work_model": kern["work_model"]}}
+                    "work_model": kern["work_model"],
+                    "equivalent": {"rate": round(equivalent, 1),
+                                   "work_model": "simple LBs x 5m + Johnson LBs x (4 P n + P), P = m(m-1)/2"}}
         cpu = None
         if ws == 1 and args.cpu_sample > 0:
             r = reference_cpu_run(p, ub, args.cpu_sample)

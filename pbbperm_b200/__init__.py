@@ -361,25 +361,37 @@ class Engine:
         _check(lib().pbb_diag_set_step_limits(self._h, int(select_budget), int(max_rounds)))
 
     def kernel_stats(self):
-        """Work of the explorer kernels since start, with the INT32 op model
-        of the bounds: weak child 5m ops (add/max chain per machine); per
-        Johnson sweep and machine pair, 5 ops per free job and pass (forward,
-        backward), 9 ops per evaluated child; per directly scanned child and
-        pair, 4 ops per free job (add, add, max, add)."""
+        """Work of the explorer kernels since start, with an INT32 op count of
+        what the search's build executes.  One-machine bounds: 4m per child.
+        Kept pair bounds (bounding mode 2, no sweeps): 8m for a child's heads or
+        tails, 5 for its comparison with each pair, 12 per position of a scanned
+        pair.  Values by position (mode 1, rows of one word): per node swept and
+        pair 4 per position, 13 per free job, 3 per child.  Sweeps with shared
+        maxima: per node swept and pair 10 per free job, 9 per child, and direct
+        scans 4 per free job and pair.  Selection, branching and the lowering of
+        the kept bounds are not counted, and a child that is pruned counts all
+        its comparisons."""
         w = _Work()
         _check(lib().pbb_work_counters(self._h, ctypes.byref(w)))
         m, n, P = w.n_machines, w.n_jobs, w.machine_pairs
-        ops = (5 * m * w.simple_bounds +
-               P * (10 * w.sweep_free_jobs + 9 * w.sweep_children) +
-               P * 4 * w.direct_free_jobs)
+        ops = 4 * m * w.simple_bounds
+        model = "4m per weak child"
+        if w.johnson_sweeps == 0 and w.direct_children > 0:
+            ops += w.direct_children * (8 * m + 5 * P) + 12 * P * w.direct_free_jobs
+            model += " + 8m + 5P per Johnson child + 12 per position of a scanned pair"
+        elif w.direct_children == 0 and n <= 32:
+            ops += P * (4 * n * w.johnson_sweeps + 13 * w.sweep_free_jobs + 3 * w.sweep_children)
+            model += " + P*(4n per node + 13 per free job + 3 per child)"
+        else:
+            ops += P * (10 * w.sweep_free_jobs + 9 * w.sweep_children + 4 * w.direct_free_jobs)
+            model += " + P*(10 per swept free job + 9 per swept child + 4 per free job of a directly scanned child)"
         return dict(device_seconds=w.device_seconds, int32_ops=float(ops), decomposed=w.decomposed,
                     simple_bounds=w.simple_bounds, johnson_bounds=w.johnson_bounds,
                     johnson_sweeps=w.johnson_sweeps, sweep_free_jobs=w.sweep_free_jobs,
                     sweep_children=w.sweep_children, direct_children=w.direct_children,
                     direct_free_jobs=w.direct_free_jobs,
                     explorers=w.explorers, warps=w.warps, status=w.status,
-                    work_model="5m per weak child + P*(10 per swept free job + 9 per swept child)"
-                               " + P*4 per free job of a directly scanned child")
+                    work_model=model)
 
     def explore(self, seconds):
         done = ctypes.c_int32(0)

@@ -1641,7 +1641,7 @@ __device__ __forceinline__ void johnson_prune(const CtaTables& T, const WarpScra
                 pair_scan<NW>(T, j, um, v, c0.y, c1.x, S.rem[m1], all, rest);
                 if (lane == 0) B.nxt[j] = all;
                 over = c0.x + c1.y + rest >= best;
-                cnt.direct_free += 2 * k;
+                cnt.direct_free += T.n;
             }
         }
         cnt.direct_children++;

@@ -1043,7 +1043,7 @@ int pbb_work_counters(pbb_engine* e, pbb_work* out)
     out->sweep_free_jobs = c.jfree;
     out->sweep_children = c.jchild;
     out->direct_children = c.jdirect;
-    out->direct_free_jobs = e->H.P > 0 ? c.jdirect_free / e->H.P : 0;   // counted per machine pair
+    out->direct_free_jobs = e->H.P > 0 ? c.jdirect_free / e->H.P : 0;   // counted over the machine pairs
     out->explorers = e->cfg.nb_ivms;
     out->warps = (e->pair_warps > 0 ? e->pair_warps : e->warps) * e->ctas;
     out->status = (int32_t)c.status;

@@ -235,9 +235,9 @@ __device__ __forceinline__ void build_lists(const WarpScratch& S, const Ivm<NW>&
 
 // 32-bit per warp (fewer live registers in the explorer loop), added to the
 // group's 64-bit counters every PBB_FLUSH_NODES decomposed nodes.  direct_free
-// grows fastest: by two passes over the free jobs for every child and pair.
-static_assert((unsigned long long)PBB_FLUSH_NODES * (PBB_MAX_N - 1) * (PBB_MAX_M * (PBB_MAX_M - 1) / 2) * 2 *
-                      (PBB_MAX_N - 1) <= 0xffffffffull,
+// grows fastest: by all positions of every child and pair.
+static_assert((unsigned long long)PBB_FLUSH_NODES * (PBB_MAX_N - 1) * (PBB_MAX_M * (PBB_MAX_M - 1) / 2) * PBB_MAX_N <=
+                  0xffffffffull,
               "a warp's 32-bit counters hold the work of PBB_FLUSH_NODES nodes");
 struct WarpCounters {
     unsigned decomposed, simple, johnson, leaves;

@@ -99,7 +99,8 @@ struct GroupCtl {
     // children evaluated by them (roofline accounting)
     unsigned long long jsweeps, jfree, jchild;
     // children bounded by direct scans, and free jobs summed over the machine
-    // pairs scanned for them
+    // pairs scanned for them (kept pair bounds: children compared, positions
+    // of the pairs scanned)
     unsigned long long jdirect, jdirect_free;
 };
 
