@@ -84,7 +84,9 @@ typedef struct pbb_config {
                                    minus the other side's, 3 the weak bound's idle time (not with
                                    boundingMode 1); 4 is rejected */
     int32_t core_warps;         /* work sharing: warps per CTA that ask for work whatever the search's
-                                   width; the others join once it is wide (0 = all) */
+                                   width; the others join once it is wide (0 = 20: all, except the
+                                   last 12 of the 32 warps that searches of more than 320 jobs x
+                                   machines run with in bounding mode 2) */
     int32_t split_depth;        /* work sharing: no split at levels deeper than n - split_depth (0 = 10, and
                                    4 while most warps wait for work) */
     int32_t share_after;        /* work sharing: an explorer hands part of its interval to an idle one only

@@ -17,18 +17,23 @@
 #define PBB_VAR_GEN(var) ((var) == 4 || (var) == 6 || (var) == 9)
 #define PBB_VAR_ALL(var) ((var) == 7 || (var) == 10)
 #define PBB_VAR_SAMPLE(var) ((var) == 2 || (var) >= 8)
-// The wide builds pay where a search is long enough to be bound by throughput;
-// below, where it is bound by the time one node takes and by how fast work
-// spreads, their spilled registers and additional warps cost a little.  The
-// tree is not known beforehand, so the line is drawn by the instance: measured
-// ms with 20 and with 32 warps, 50x20 (56 M nodes) 194 and 167, 20x20 (13 M)
-// 38.9 and 31.9, 16x20 (0.6 M) 2.35 and 2.51, 20x10 (0.12 M) 0.90 and 0.98,
-// 12x10 0.21 and 0.23.
+// The wide builds gain 14 to 20 % where a search is long and its instance has
+// many machine pairs, and lose 6 to 10 % where either is missing: a short
+// search is bound by the time one node takes and by how fast work spreads, and
+// with few pairs there is little to overlap for the spilled registers.  The
+// size of the tree is not known beforehand; the instance's size is what there is
+// to go by.  Explorer ms with 20 and with 32 warps:
+//   used from here on: 20x20 (13 M nodes) 38.9 and 32.0, 18x20 (19 M) 55.6 and
+//   44.7, 33x15 (35 M) 96.8 and 79.0, 30x20 (54 M) 131 and 106, 40x20 (60 M) 190
+//   and 164, 50x20 (56 M) 194 and 167; but 18x20 (0.9 M) 3.3 and 3.6, (0.6 M) 2.4
+//   and 2.6, 25x20 (2.6 M) 7.3 and 7.9, 40x10 (0.3 M) 2.1 and 2.2;
+//   not used: 16x20 (1.9 M) 6.1 and 6.5, 30x10 (10 M) 20.8 and 22.7, 24x10
+//   (0.5 M) 1.6 and 1.8, 14x20 (0.2 M) 1.16 and 1.29, 12x10 0.21 and 0.23.
 #define PBB_WIDE_FROM 320             // jobs x machines above which they are used
 // warps of a bound kernel's CTA at most, by the 32-job words of a row: two
 // words leave shared memory for fewer, and want more registers
 #define PBB_BOUND_WARPS(nw) ((nw) == 1 ? 16 : 12)
-#define PBB_CORE_WARPS PBB_WARPS_MAX   // default of DevSearch::core_warps
+#define PBB_CORE_WARPS PBB_WARPS_MAX   // default of DevSearch::core_warps: all but 12 in a wide build
 #define PBB_SPLIT_DEPTH 10    // default of DevSearch::split_depth
 #define PBB_SHARE_AFTER 64    // default of DevSearch::share_after
 #define PBB_SPLIT_NARROW 4    // default of DevSearch::split_narrow
