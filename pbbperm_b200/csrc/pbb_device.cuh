@@ -128,7 +128,7 @@ struct CtaTables {
     const int* min_arr;
     const int* min_dep;
     const unsigned char* posj;     // [n][posj_stride] or NULL
-    int n, m, P, Ppad, mp, je_stride, posj_stride;
+    int n, m, P, Ppad, mp, je_stride, posj_stride;   // posj_stride: of PBB_SCRATCH_ALL; else je_stride
 };
 
 struct WarpScratch {
@@ -693,7 +693,7 @@ __device__ __forceinline__ typename PosMask<NW>::type free_positions(const CtaTa
     const unsigned char* col = T.posj + i;
     M pm = 0;
     PBB_UNROLL(PBB_FREEPOS_UNROLL)
-    for (int q = 0; q < k; q++) pm |= (M)1 << col[S.rowj[q] * T.Ppad];
+    for (int q = 0; q < k; q++) pm |= (M)1 << col[S.rowj[q] * T.je_stride];
     return pm;
 }
 
@@ -718,7 +718,7 @@ __device__ __forceinline__ void fmask_build(const CtaTables& T, const WarpScratc
 
 __device__ __forceinline__ void fmask_flip(const CtaTables& T, const WarpScratch& S, int u)
 {
-    const unsigned char* col = T.posj + u * T.Ppad;
+    const unsigned char* col = T.posj + u * T.je_stride;
     for (int i = lane_id(); i < T.P; i += 32) S.fmask[i] ^= 1ull << col[i];
     __syncwarp();
 }
@@ -787,7 +787,7 @@ __device__ __forceinline__ void johnson_direct_chains(const CtaTables& T, const 
 #pragma unroll
             for (int c = 0; c < C; c++) {
                 direct_start(T, S, u[c], sd[c], m0, m1, t0[c], t1[c], B0[c], B1[c]);
-                px[c] = T.posj[u[c] * T.Ppad + i];
+                px[c] = T.posj[u[c] * T.je_stride + i];
             }
             M pm = node_positions<NW>(T, S, k, i);
             const unsigned long long* col = T.je + i;

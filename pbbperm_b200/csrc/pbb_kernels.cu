@@ -52,6 +52,14 @@ __device__ __forceinline__ unsigned ld_volatile_u32(const unsigned* p)
     return *reinterpret_cast<const volatile unsigned*>(p);
 }
 
+// shared memory the launch gave the CTA
+__device__ __forceinline__ int dynamic_smem()
+{
+    unsigned bytes;
+    asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(bytes));
+    return (int)bytes;
+}
+
 __device__ __forceinline__ int ld_volatile_s32(const int* p) { return *reinterpret_cast<const volatile int*>(p); }
 
 // Load the group's instance tables into this CTA's shared memory.
@@ -96,8 +104,14 @@ __device__ __forceinline__ void load_tables(const DevInstance& I, unsigned char*
         for (int t = tid / 32; t < I.n; t += nt / 32)
             for (int i = tid & 31; i < I.P; i += 32)
                 posj[JE_JOB(I.je[t * I.Ppad + i]) * sp.posj_stride + i] = (unsigned char)t;
-    } else if (posj_here)
-        for (int i = tid; i < I.n * I.Ppad; i += nt) posj[i] = I.posj[i];
+    } else if (posj_here) {
+        if (sp.je_stride == I.Ppad) {
+            for (int i = tid; i < I.n * I.Ppad; i += nt) posj[i] = I.posj[i];
+        } else {
+            for (int j = tid / 32; j < I.n; j += nt / 32)
+                for (int i = tid & 31; i < I.P; i += 32) posj[j * sp.je_stride + i] = I.posj[j * I.Ppad + i];
+        }
+    }
     T.je = je; T.pt = pt; T.mp = mp; T.pm0 = pm0; T.pm1 = pm1; T.min_arr = marr; T.min_dep = mdep;
     T.posj = posj_here ? posj : nullptr;
     T.je_stride = sp.je_stride;
@@ -789,7 +803,7 @@ __global__ void pbb_root_kernel(const DevGroup* groups, int ngroups, const int* 
     const int g = b / per_group;
     if (g >= ngroups) return;
     const DevGroup G = groups[g];
-    const SmemPlan sp = pbb_smem_plan(G.inst.n, G.inst.m, G.inst.Ppad, 1);
+    const SmemPlan sp = pbb_smem_plan(G.inst.n, G.inst.m, G.inst.Ppad, 1, PBB_SCRATCH_PLAIN, dynamic_smem());
     CtaTables T;
     load_tables(G.inst, smem, sp, T);
     __syncthreads();
@@ -897,29 +911,27 @@ pbb_explore_kernel(const DevGroup* groups, const int* ngroups_d, int warps_per_c
     if ((int)blockIdx.x >= G.first_cta + G.ctas) return;
     // each warp keeps its explorer's free-position masks when the launch
     // gave the room for them (the host sizes the launch with them if they fit)
-    unsigned dyn_smem;
-    asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn_smem));
+    const int room = dynamic_smem();
     // (the one-machine bound alone has no use for them)
     int fm = PBB_SCRATCH_PLAIN;
     if (PBB_VAR_ALL(VAR)) {
         fm = PBB_SCRATCH_ALL;
-        if (pbb_smem_plan(G.inst.n, G.inst.m, G.inst.Ppad, warps_per_cta, fm).total > (int)dyn_smem) {
-            if (threadIdx.x == 0) atomicOr(&G.ctl->status, PBB_ST_BADINPUT);
-            return;
-        }
     } else if (PBB_VAR_PAIRS(VAR)) {
         // the host launches this build only with room for its scratch
         fm = PBB_SCRATCH_PAIRS;
-        if (!pair_stack || G.inst.n * G.inst.Ppad > pair_stride ||
-            pbb_smem_plan(G.inst.n, G.inst.m, G.inst.Ppad, warps_per_cta, fm).total > (int)dyn_smem) {
+        if (!pair_stack || G.inst.n * G.inst.Ppad > pair_stride) {
             if (threadIdx.x == 0) atomicOr(&G.ctl->status, PBB_ST_BADINPUT);
             return;
         }
     } else if (G.inst.posj && G.search.bound_mode != 0 &&
-               pbb_smem_plan(G.inst.n, G.inst.m, G.inst.Ppad, warps_per_cta, PBB_SCRATCH_MASKS).total <= (int)dyn_smem) {
+               pbb_smem_plan(G.inst.n, G.inst.m, G.inst.Ppad, warps_per_cta, PBB_SCRATCH_MASKS, room).total <= room) {
         fm = PBB_SCRATCH_MASKS;
     }
-    const SmemPlan sp = pbb_smem_plan(G.inst.n, G.inst.m, G.inst.Ppad, warps_per_cta, fm);
+    const SmemPlan sp = pbb_smem_plan(G.inst.n, G.inst.m, G.inst.Ppad, warps_per_cta, fm, room);
+    if (sp.total > room) {
+        if (threadIdx.x == 0) atomicOr(&G.ctl->status, PBB_ST_BADINPUT);
+        return;
+    }
     CtaTables T;
     load_tables(G.inst, smem, sp, T);
     CtaShare* H = reinterpret_cast<CtaShare*>(smem + sp.share_off);
@@ -1147,7 +1159,7 @@ __global__ void pbb_bound_kernel(DevInstance I, int count, const int* sched, con
                                  unsigned int* status, int warps_per_cta, int method, BoundExtra X)
 {
     extern __shared__ __align__(16) unsigned char smem[];
-    const SmemPlan sp = pbb_smem_plan(I.n, I.m, I.Ppad, warps_per_cta);
+    const SmemPlan sp = pbb_smem_plan(I.n, I.m, I.Ppad, warps_per_cta, PBB_SCRATCH_PLAIN, dynamic_smem());
     CtaTables T;
     load_tables(I, smem, sp, T);
     __syncthreads();

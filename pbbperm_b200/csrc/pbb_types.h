@@ -222,32 +222,50 @@ __host__ __device__ inline int pbb_warp_bytes(int n, int m, int Ppad, int fmask)
 // PBB_SCRATCH_PAIRS keeps no position table, but the prefix sums of the
 // processing times, and an odd row stride of the Johnson entries, so that a
 // warp can read one pair's column as well as 32 pairs' rows.
-__host__ __device__ inline SmemPlan pbb_smem_plan(int n, int m, int Ppad, int warps, int fmask = 0)
+// CTAs of `warps` warps at 96 registers a thread that an SM holds (228 KiB of
+// shared memory, 1 KiB of it reserved for each)
+__host__ __device__ inline int pbb_sm_ctas(int total, int warps)
 {
-    const bool pairs = fmask == PBB_SCRATCH_PAIRS;
-    const int times = n * pbb_machine_pad(m) * 4;
+    const int regs = warps < 21 ? 21 / warps : 1, smem = 233472 / (total + 1024);
+    return smem < regs ? smem : regs;
+}
+
+// Rows of the Johnson table hold Ppad entries, so that lanes at different
+// positions of their pairs' orders meet no bank twice; without what is past the
+// last pair (whatever the Johnson mode, there are no more than machine pairs)
+// they take less memory, and bounding mode 1 at 50x20 runs 7 % slower.  Tight rows
+// are for tables that need it: on the host (room < 0), where the padded rows of
+// the processing times and the work-sharing block would cost the SM a CTA; in a
+// kernel, whose launch has `room` bytes, where the padded rows do not fit them.
+__host__ __device__ inline SmemPlan pbb_smem_plan(int n, int m, int Ppad, int warps, int fmask = 0, int room = -1)
+{
+    const bool pairs = fmask == PBB_SCRATCH_PAIRS, general = !pairs && fmask != PBB_SCRATCH_ALL;
+    const int times = n * pbb_machine_pad(m) * 4, share = pbb_align((int)sizeof(CtaShare) + 8 * warps, 16);
+    const int last = m * (m - 1) / 2, tight = last < Ppad ? last : Ppad;
     SmemPlan s;
-    int off = 0;
-    // without the padding past the last pair (whatever the Johnson mode, there
-    // are no more pairs than machine pairs): it pays for the padded rows of the
-    // processing times, so that no instance needs more than with tight rows
-    const int tight = m * (m - 1) / 2;
-    s.je_stride = pairs ? Ppad + 1 : (tight < Ppad ? tight : Ppad);
-    s.je_off = off;   off += pbb_align(n * s.je_stride * 8, 16);
-    s.p_off = off;    off += times;
-    s.pre_off = off;  off += pairs ? times : 0;
-    s.pm_off = off;   off += pbb_align(Ppad * 2, 16);
-    s.marr_off = off; off += pbb_align(m * 4, 16);
-    s.mdep_off = off; off += pbb_align(m * 4, 16);
-    // an odd number of words between the rows of the position table lets the
-    // lanes read one pair's positions of 32 jobs without bank conflicts
-    s.posj_stride = fmask == PBB_SCRATCH_ALL ? Ppad + 4 : Ppad;
-    s.posj_off = off; off += pairs ? 0 : pbb_align(n * s.posj_stride, 16);
-    s.share_off = off; off += pbb_align((int)sizeof(CtaShare) + 8 * warps, 16);
-    s.warp_off = off;
-    s.fmask = fmask;
-    s.warp_bytes = pbb_warp_bytes(n, m, Ppad, fmask);
-    off += s.warp_bytes * warps;
-    s.total = off;
+    s.je_stride = pairs ? Ppad + 1 : Ppad;
+    for (int pass = 0; pass < 2; pass++) {
+        int off = 0;
+        s.je_off = off;   off += pbb_align(n * s.je_stride * 8, 16);
+        s.p_off = off;    off += times;
+        s.pre_off = off;  off += pairs ? times : 0;
+        s.pm_off = off;   off += pbb_align(Ppad * 2, 16);
+        s.marr_off = off; off += pbb_align(m * 4, 16);
+        s.mdep_off = off; off += pbb_align(m * 4, 16);
+        // an odd number of words between the rows of the position table lets the
+        // lanes read one pair's positions of 32 jobs without bank conflicts; the
+        // general builds read one job's row, and use one stride for both tables
+        s.posj_stride = fmask == PBB_SCRATCH_ALL ? Ppad + 4 : s.je_stride;
+        s.posj_off = off; off += pairs ? 0 : pbb_align(n * s.posj_stride, 16);
+        s.share_off = off; off += share;
+        s.warp_off = off;
+        s.fmask = fmask;
+        s.warp_bytes = pbb_warp_bytes(n, m, Ppad, fmask);
+        off += s.warp_bytes * warps;
+        s.total = off;
+        const int grown = times - pbb_align(4 * m * n, 16) + share;
+        if (!general || (room < 0 ? pbb_sm_ctas(off, warps) >= pbb_sm_ctas(off - grown, warps) : off <= room)) break;
+        s.je_stride = tight;
+    }
     return s;
 }
