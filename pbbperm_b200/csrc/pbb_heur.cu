@@ -1,7 +1,8 @@
 // Initial upper bounds on the device: NEH (heuristic/src/fastNEH.cpp:230-243
 // for the insertion procedure), one warp per instance, and iterated greedy,
-// eight warps per instance, for many instances in one launch -- the pool computes its admissions' bounds this way, without a
-// host round trip, and the engine can start from it.
+// eight warps per instance, for many instances in one launch -- the pool
+// computes its admissions' bounds this way, without a host round trip, and the
+// engine can start from it.
 //
 // Insertion of job x into a sequence of `len` jobs uses Taillard's heads and
 // tails (fastNEH.cpp:100-178 computeHeads / computeTails / insertJob /

@@ -770,7 +770,8 @@ static int explore_window(pbb_engine* e, double seconds, int32_t* done, int eage
         }
         const bool own = variant >= 3;
         const int warps = std::min(own ? e->pair_warps : e->warps, PBB_EXPLORE_WARPS(variant));
-        CK(pbbl::launch_explore(e->nw, e->group_d, e->ngroups_d, e->ctas, warps, own ? e->pair_smem : e->smem, budget, e->max_rounds, e->select_budget, e->st,
+        CK(pbbl::launch_explore(e->nw, e->group_d, e->ngroups_d, e->ctas, warps, own ? e->pair_smem : e->smem, budget,
+                                e->max_rounds, e->select_budget, e->st,
                                 variant, eager, e->pair_stack, e->pair_stride));
         CK(cudaEventRecord(e->ev1, e->st));
         rc = wait_event(e->ev1, e->wait_limit_s < 0 ? win + 60.0 : e->wait_limit_s);

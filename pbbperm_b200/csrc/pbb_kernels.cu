@@ -1076,9 +1076,8 @@ pbb_explore_kernel(const DevGroup* groups, const int* ngroups_d, int warps_per_c
         if (best < known && lane_id() == 0) atomicMin(&H->best, best);
         if (r == 1) {
             since++;
-            bound_current<NW, (VAR == 1 || VAR == 2), PBB_VAR_SAMPLE(VAR),
-                          (PBB_VAR_ALL(VAR) ? 3 : PBB_VAR_PAIRS(VAR) ? 1 + PBB_VAR_GEN(VAR) : 0)>(G, T, S, B, id, R, mode, best,
-                                                                                            C);
+            constexpr int how = PBB_VAR_ALL(VAR) ? 3 : PBB_VAR_PAIRS(VAR) ? 1 + PBB_VAR_GEN(VAR) : 0;
+            bound_current<NW, (VAR == 1 || VAR == 2), PBB_VAR_SAMPLE(VAR), how>(G, T, S, B, id, R, mode, best, C);
         }
         if (C.decomposed >= PBB_FLUSH_NODES) flush_counters(G, C);
         if (r == 0) {
